@@ -1303,10 +1303,18 @@ static mdz_status build_hierarchy(mdz_ctx *ctx, mg_hier<T> &H) {
         T **bufv[] = {&L.xv, &L.yv, &L.fv, &L.rv, &L.idv};
         for (T **b : bufv) if (e == cudaSuccess) e = alloc0(b, L.nv());
         lev++;
-        // halve while both cell counts are even and the coarse level keeps >= 4 cells a side
-        bool can = (L.ncx % 2 == 0) && (L.ncz % 2 == 0) && L.ncx / 2 >= 4 && L.ncz / 2 >= 4;
-        if (!can) break;
-        Nx = L.ncx / 2 + 1; Nz = L.ncz / 2 + 1; dx *= 2; dz *= 2;
+        // halve while the coarse level keeps >= 4 cells a side.  An odd cell
+        // count is halved rounding up: the last coarse cell then covers one fine
+        // cell, its far wall lies one fine cell outside the box, and the fine
+        // points that would lie beyond the wall are not unknowns, so P and the
+        // Galerkin product keep their index arithmetic and footprint.  A level
+        // with an odd count that is small enough for the dense inverse stops
+        // there instead.
+        const int cx = (L.ncx + 1) / 2, cz = (L.ncz + 1) / 2;
+        const bool even = L.ncx % 2 == 0 && L.ncz % 2 == 0;
+        const long long unknowns = (long long)(L.Nx - 2) * (L.Nz - 1) + (long long)(L.Nx - 1) * (L.Nz - 2);
+        if (cx < 4 || cz < 4 || (!even && unknowns <= MG_DENSE_MAX)) break;
+        Nx = cx + 1; Nz = cz + 1; dx *= 2; dz *= 2;
     }
     H.nlev = lev;
     mg_level<T> &C = H.L[lev - 1];
