@@ -126,6 +126,38 @@ void *mdz_stage(mdz_ctx *ctx, int slot, size_t bytes);
         if (e__ != cudaSuccess) return mdz_cuda_check((ctx), e__, "kernel launch");   \
     } while (0)
 
+// ---- programmatic dependent launch ------------------------------------------
+// A kernel launched with launch_pdl may start while the launch before it in
+// the stream (or captured graph) still runs.  It must call pdl_wait() before
+// it reads or writes anything that launch, or one before it, may touch; the wait
+// returns when that launch has finished and its writes are visible.
+// pdl_release() lets the next launch start now instead of when this grid's
+// blocks end; since every launch waits, calling it first is safe.  Both do
+// nothing in a kernel launched the ordinary way.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KA, typename... A>
+static inline cudaError_t launch_pdl(void (*k)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, KA(a)...);
+}
+#define MDZ_PDL(ctx, ...)                                                             \
+    do {                                                                              \
+        (ctx)->launches++;                                                            \
+        cudaError_t e__ = launch_pdl(__VA_ARGS__);                                    \
+        if (e__ != cudaSuccess) return mdz_cuda_check((ctx), e__, "kernel launch");   \
+    } while (0)
+
 static inline int mdz_blocks(long long n, int threads = MDZ_THREADS) {
     long long b = (n + threads - 1) / threads;
     return (int)(b < 1 ? 1 : b);

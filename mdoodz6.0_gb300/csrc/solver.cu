@@ -22,7 +22,6 @@
 #include <cstdio>
 #include <cstring>
 #include <vector>
-#include <cooperative_groups.h>
 #include "stokes.cuh"
 #include "solver.cuh"
 
@@ -32,6 +31,8 @@
 #define MG_NST 31        // stencil coefficients per velocity row (15 same-component + 16 cross)
 #define MG_CENTER 7      // plane of the diagonal entry in both layouts
 #define GCR_MAX_M 48
+#define MG_TILE_LARGE 30000   // points of a level above which the restriction takes the larger tile
+#define MG_TILE_SMALL 4000    // and below which the tile kernels take the smallest
 
 // ---------------------------------------------------------------------------
 template <typename T>
@@ -83,7 +84,7 @@ struct mg_hier {
     int nlev = 0;
     bool newton = false;          // level 0 is the probed Newton block (smoothed by its stencil)
     bool built = false;           // mg_setup has filled the levels at least once
-    double *pmean = nullptr;      // preconditioner scratch: pressure sum and count
+    double *pmean = nullptr;      // preconditioner scratch: pressure sum, count and mean
     mg_level<T> L[MG_MAX_LEVELS];
 };
 
@@ -103,7 +104,6 @@ struct mdz_solver {
     int mg_jacobian = 0;         // 1: multigrid on the Newton Jacobian's velocity block (else Picard)
     int schur = 0;               // pressure block of Newton solves: 0 eta_n / cell volume, 1 the Jacobian's
                                  // D11 / 2 (tangent viscosity) where positive
-    int bottom_cs[2] = {1, 1};   // cluster size of the V-cycle bottom kernel ([0] FP64, [1] FP32)
     // preconditioner application captured as a CUDA graph, per precision
     // ([0] FP64, [1] FP32): one graph launch per Krylov iteration
     // [precision (0 FP64, 1 FP32) * 2 + newton hierarchy + 4 * tangent Schur]
@@ -191,56 +191,6 @@ __global__ void k_mg_diag(stokes_geom G, const T *__restrict__ D11, const T *__r
     }
 }
 
-// out = x + omega * D^-1 (f - A x)  (x == nullptr: x = 0)
-template <typename T>
-__global__ void __launch_bounds__(256) k_mg_smooth(stokes_geom G, stokes_coefs<T> D, const T *__restrict__ xu,
-                                                   const T *__restrict__ xv, const T *__restrict__ fu,
-                                                   const T *__restrict__ fv, const T *__restrict__ idu,
-                                                   const T *__restrict__ idv, T omega, T *__restrict__ ou,
-                                                   T *__restrict__ ov) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int Nx = G.Nx, Nz = G.Nz;
-    const T celvol = gc<T>(G, GC_CELVOL);
-    stokes_cvec<T> x{xu, xv, nullptr};
-    if (i < Nx && j <= Nz) {
-        int c = i + j * Nx;
-        T r = 0;
-        if (G.BCu[c] == -1) {
-            T ax = xu ? xrow<T, false>(G, D, x, i, j) * celvol : T(0);
-            r = (xu ? xu[c] : T(0)) + omega * idu[c] * (fu[c] - ax);
-        }
-        ou[c] = r;
-    }
-    if (i <= Nx && j < Nz) {
-        int c = i + j * (Nx + 1);
-        T r = 0;
-        if (G.BCv[c] == -1) {
-            T ax = xv ? zrow<T, false>(G, D, x, i, j) * celvol : T(0);
-            r = (xv ? xv[c] : T(0)) + omega * idv[c] * (fv[c] - ax);
-        }
-        ov[c] = r;
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_mg_residual(stokes_geom G, stokes_coefs<T> D, const T *__restrict__ xu,
-                                                     const T *__restrict__ xv, const T *__restrict__ fu,
-                                                     const T *__restrict__ fv, T *__restrict__ ru,
-                                                     T *__restrict__ rv) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int Nx = G.Nx, Nz = G.Nz;
-    const T celvol = gc<T>(G, GC_CELVOL);
-    stokes_cvec<T> x{xu, xv, nullptr};
-    if (i < Nx && j <= Nz) {
-        int c = i + j * Nx;
-        ru[c] = G.BCu[c] == -1 ? fu[c] - xrow<T, false>(G, D, x, i, j) * celvol : T(0);
-    }
-    if (i <= Nx && j < Nz) {
-        int c = i + j * (Nx + 1);
-        rv[c] = G.BCv[c] == -1 ? fv[c] - zrow<T, false>(G, D, x, i, j) * celvol : T(0);
-    }
-}
-
 // Prolongation weights along the "cell-centred" direction of a staggered
 // component: fine line j (1..ncf) -> main coarse line and neighbour, with the
 // ghost neighbour mirrored onto the main line (free slip).
@@ -267,101 +217,6 @@ __device__ __forceinline__ bool v_unknown(int i, int j, int Nx, int Nz) {
     return i >= 1 && i <= Nx - 1 && j >= 1 && j <= Nz - 2;
 }
 
-// fine x += P xc at fine point (i, j) of the (Nx+1) x (Nz+1) box (both components)
-template <typename T>
-__device__ __forceinline__ void mg_prolong_pt(const stokes_geom &F, const stokes_geom &Cg, const T *__restrict__ cu,
-                                              const T *__restrict__ cv, T *__restrict__ fu, T *__restrict__ fv,
-                                              int i, int j) {
-    const int Nx = F.Nx, Nz = F.Nz, Nxc = Cg.Nx;
-    if (i < Nx && j <= Nz && u_unknown(i, j, Nx, Nz)) {   // Vx: x node-centred, z cell-centred
-        const int c = i + j * Nx;
-        int J0, J1;
-        float w0, w1;
-        cc_weights(j, Cg.ncz, J0, w0, J1, w1);
-        const int Ia = i >> 1, Ib = (i + 1) >> 1;
-        const float wa = (i & 1) ? 0.5f : 1.0f, wb = (i & 1) ? 0.5f : 0.0f;
-        const T a0 = cu[Ia + J0 * Nxc], a1 = cu[Ia + J1 * Nxc], b0 = cu[Ib + J0 * Nxc], b1 = cu[Ib + J1 * Nxc];
-        fu[c] += (T)(wa * w0) * a0 + (T)(wa * w1) * a1 + (T)(wb * w0) * b0 + (T)(wb * w1) * b1;
-    }
-    if (i <= Nx && j < Nz && v_unknown(i, j, Nx, Nz)) {   // Vz: x cell-centred, z node-centred
-        const int c = i + j * (Nx + 1);
-        int I0, I1;
-        float w0, w1;
-        cc_weights(i, Cg.ncx, I0, w0, I1, w1);
-        const int Ja = j >> 1, Jb = (j + 1) >> 1;
-        const float wa = (j & 1) ? 0.5f : 1.0f, wb = (j & 1) ? 0.5f : 0.0f;
-        const int W = Nxc + 1;
-        const T a0 = cv[I0 + Ja * W], a1 = cv[I1 + Ja * W], b0 = cv[I0 + Jb * W], b1 = cv[I1 + Jb * W];
-        fv[c] += (T)(wa * w0) * a0 + (T)(wa * w1) * a1 + (T)(wb * w0) * b0 + (T)(wb * w1) * b1;
-    }
-}
-
-template <typename T>
-__global__ void k_mg_prolong_add(stokes_geom F, stokes_geom Cg, const T *__restrict__ cu, const T *__restrict__ cv,
-                                 T *__restrict__ fu, T *__restrict__ fv) {
-    mg_prolong_pt<T>(F, Cg, cu, cv, fu, fv, blockIdx.x * blockDim.x + threadIdx.x,
-                     blockIdx.y * blockDim.y + threadIdx.y);
-}
-
-// coarse f = P^T fine r at coarse point (I, J): the 12 fine values of each
-// component are loaded together (indices clamped into the box, weights of
-// points outside the unknowns zero)
-template <typename T>
-__device__ __forceinline__ void mg_restrict_pt(const stokes_geom &F, const stokes_geom &Cg, const T *__restrict__ ru,
-                                               const T *__restrict__ rv, T *__restrict__ cu, T *__restrict__ cv,
-                                               int I, int J) {
-    const int Nxf = F.Nx, Nzf = F.Nz, Nx = Cg.Nx, Nz = Cg.Nz;
-    if (I < Nx && J <= Nz) {
-        T s = 0;
-        if (u_unknown(I, J, Nx, Nz)) {
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                const int j = 2 * J - 2 + a;
-                int J0, J1;
-                float w0, w1;
-                cc_weights(j, Cg.ncz, J0, w0, J1, w1);
-                const float wz = (J0 == J ? w0 : 0.0f) + (J1 == J && J1 != J0 ? w1 : 0.0f);
-                const int jc = min(max(j, 0), Nzf);
-#pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    const int i = 2 * I - 1 + b;
-                    const float w = (j >= 1 && j <= F.ncz && u_unknown(i, j, Nxf, Nzf)) ? nc_weight(i, I) * wz : 0.0f;
-                    s += (T)w * ru[min(max(i, 0), Nxf - 1) + jc * Nxf];
-                }
-            }
-        }
-        cu[I + J * Nx] = s;
-    }
-    if (I <= Nx && J < Nz) {
-        T s = 0;
-        if (v_unknown(I, J, Nx, Nz)) {
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                const int i = 2 * I - 2 + a;
-                int I0, I1;
-                float w0, w1;
-                cc_weights(i, Cg.ncx, I0, w0, I1, w1);
-                const float wx = (I0 == I ? w0 : 0.0f) + (I1 == I && I1 != I0 ? w1 : 0.0f);
-                const int ic = min(max(i, 0), Nxf);
-#pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    const int j = 2 * J - 1 + b;
-                    const float w = (i >= 1 && i <= F.ncx && v_unknown(i, j, Nxf, Nzf)) ? wx * nc_weight(j, J) : 0.0f;
-                    s += (T)w * rv[ic + min(max(j, 0), Nzf - 1) * (Nxf + 1)];
-                }
-            }
-        }
-        cv[I + J * (Nx + 1)] = s;
-    }
-}
-
-template <typename T>
-__global__ void k_mg_restrict(stokes_geom F, stokes_geom Cg, const T *__restrict__ ru, const T *__restrict__ rv,
-                              T *__restrict__ cu, T *__restrict__ cv) {
-    mg_restrict_pt<T>(F, Cg, ru, rv, cu, cv, blockIdx.x * blockDim.x + threadIdx.x,
-                      blockIdx.y * blockDim.y + threadIdx.y);
-}
-
 // ---------------------------------------------------------------------------
 // Galerkin coarse operators.  Re-discretised coarse levels (averaged
 // viscosities) lose the coupling across layers of 1e5 viscosity contrast and
@@ -374,163 +229,79 @@ __global__ void k_mg_restrict(stokes_geom F, stokes_geom Cg, const T *__restrict
 // (u index (k, l) of the Nx x (Nz+1) box, v index (i, j) of the (Nx+1) x Nz box).
 // The level-0 stencil is a subset of this footprint.
 
-// y = A x for a stencil level, one u-row / v-row.  All 31 coefficients and
-// neighbour values are loaded before the first multiply (neighbour indices
-// clamped into the box, out-of-box terms masked to zero) so that the loads
-// overlap instead of waiting on each other behind the bounds tests.
+// y = A x for a stencil level, one u-row / v-row of an unknown.  The
+// coefficients are loaded by a call of their own, so that a kernel can fetch
+// them before it waits for the launch that writes x (the stencils change only
+// in mg_setup).  Neighbours outside the box are read from the nearest line
+// inside it, whose values are zero (ghost or Dirichlet nodes are never
+// unknowns).  FP64 sums run in four chains: one dependent chain of 31 FP64
+// multiply-adds is longer than the loads on the small levels.
+template <typename T>
+__device__ __forceinline__ void st_coefs(const T *__restrict__ s, size_t n, size_t c, T (&cf)[MG_NST]) {
+#pragma unroll
+    for (int q = 0; q < MG_NST; q++) cf[q] = s[(size_t)q * n + c];
+}
+
+template <typename T>
+__device__ __forceinline__ T st_urow_x(int Nx, int Nz, const T (&cf)[MG_NST], const T *__restrict__ xu,
+                                       const T *__restrict__ xv, int k, int l) {
+    constexpr int NA = sizeof(T) == 8 ? 4 : 1;
+    T s[NA] = {};
+#pragma unroll
+    for (int r = 0; r < 5; r++) {   // uu: (dk, dl) = (q % 3 - 1, q / 3 - 2)
+        const T *p = xu + (k - 1 + min(max(l + r - 2, 0), Nz) * Nx);
+#pragma unroll
+        for (int d = 0; d < 3; d++) s[(3 * r + d) % NA] += cf[3 * r + d] * p[d];
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++) {   // uv: (dI, dJ) = (q % 4 - 1, q / 4 - 2)
+        const T *p = xv + (k - 1 + min(max(l + r - 2, 0), Nz - 1) * (Nx + 1));
+#pragma unroll
+        for (int d = 0; d < 4; d++) s[(15 + 4 * r + d) % NA] += cf[15 + 4 * r + d] * p[d];
+    }
+    if constexpr (NA == 4) return (s[0] + s[1]) + (s[2] + s[3]);
+    else return s[0];
+}
+
+template <typename T>
+__device__ __forceinline__ T st_vrow_x(int Nx, int Nz, const T (&cf)[MG_NST], const T *__restrict__ xu,
+                                       const T *__restrict__ xv, int i, int j) {
+    constexpr int NA = sizeof(T) == 8 ? 4 : 1;
+    T s[NA] = {};
+    (void)Nz;
+    const int im2 = max(i - 2, 0);
+#pragma unroll
+    for (int r = 0; r < 3; r++) {   // vv: (dI, dJ) = (q % 5 - 2, q / 5 - 1)
+        const T *p = xv + (j + r - 1) * (Nx + 1);
+#pragma unroll
+        for (int d = 0; d < 5; d++)
+            s[(5 * r + d) % NA] += cf[5 * r + d] * p[d == 0 ? im2 : (d == 4 ? min(i + 2, Nx) : i + d - 2)];
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++) {   // vu: (dK, dL) = (q % 4 - 2, q / 4 - 1)
+        const T *p = xu + (j + r - 1) * Nx;
+#pragma unroll
+        for (int d = 0; d < 4; d++)
+            s[(15 + 4 * r + d) % NA] += cf[15 + 4 * r + d] * p[d == 0 ? im2 : (d == 3 ? min(i + 1, Nx - 1) : i + d - 2)];
+    }
+    if constexpr (NA == 4) return (s[0] + s[1]) + (s[2] + s[3]);
+    else return s[0];
+}
+
 template <typename T>
 __device__ __forceinline__ T st_urow(int Nx, int Nz, const T *__restrict__ su, size_t nu, const T *__restrict__ xu,
                                      const T *__restrict__ xv, int k, int l) {
-    const size_t c = (size_t)k + (size_t)l * Nx;
-    T cf[MG_NST], xn[MG_NST];
-#pragma unroll
-    for (int q = 0; q < 15; q++) {   // uu: (dk, dl) = (q % 3 - 1, q / 3 - 2)
-        const int kk = k + q % 3 - 1, ll = l + q / 3 - 2;
-        const bool in = kk >= 0 && kk < Nx && ll >= 0 && ll <= Nz;
-        const int kc = min(max(kk, 0), Nx - 1), lc = min(max(ll, 0), Nz);
-        cf[q] = su[(size_t)q * nu + c];
-        xn[q] = xu[kc + lc * Nx];
-        if (!in) cf[q] = T(0);
-    }
-#pragma unroll
-    for (int q = 0; q < 16; q++) {   // uv: (dI, dJ) = (q % 4 - 1, q / 4 - 2)
-        const int i = k + q % 4 - 1, j = l + q / 4 - 2;
-        const bool in = i >= 0 && i <= Nx && j >= 0 && j < Nz;
-        const int ic = min(max(i, 0), Nx), jc = min(max(j, 0), Nz - 1);
-        cf[15 + q] = su[(size_t)(15 + q) * nu + c];
-        xn[15 + q] = xv[ic + jc * (Nx + 1)];
-        if (!in) cf[15 + q] = T(0);
-    }
-    T s = 0;
-#pragma unroll
-    for (int q = 0; q < MG_NST; q++) s += cf[q] * xn[q];
-    return s;
+    T cf[MG_NST];
+    st_coefs<T>(su, nu, (size_t)k + (size_t)l * Nx, cf);
+    return st_urow_x<T>(Nx, Nz, cf, xu, xv, k, l);
 }
 
 template <typename T>
 __device__ __forceinline__ T st_vrow(int Nx, int Nz, const T *__restrict__ sv, size_t nv, const T *__restrict__ xu,
                                      const T *__restrict__ xv, int i, int j) {
-    const size_t c = (size_t)i + (size_t)j * (Nx + 1);
-    T cf[MG_NST], xn[MG_NST];
-#pragma unroll
-    for (int q = 0; q < 15; q++) {   // vv: (dI, dJ) = (q % 5 - 2, q / 5 - 1)
-        const int ii = i + q % 5 - 2, jj = j + q / 5 - 1;
-        const bool in = ii >= 0 && ii <= Nx && jj >= 0 && jj < Nz;
-        const int ic = min(max(ii, 0), Nx), jc = min(max(jj, 0), Nz - 1);
-        cf[q] = sv[(size_t)q * nv + c];
-        xn[q] = xv[ic + jc * (Nx + 1)];
-        if (!in) cf[q] = T(0);
-    }
-#pragma unroll
-    for (int q = 0; q < 16; q++) {   // vu: (dK, dL) = (q % 4 - 2, q / 4 - 1)
-        const int k = i + q % 4 - 2, l = j + q / 4 - 1;
-        const bool in = k >= 0 && k < Nx && l >= 0 && l <= Nz;
-        const int kc = min(max(k, 0), Nx - 1), lc = min(max(l, 0), Nz);
-        cf[15 + q] = sv[(size_t)(15 + q) * nv + c];
-        xn[15 + q] = xu[kc + lc * Nx];
-        if (!in) cf[15 + q] = T(0);
-    }
-    T s = 0;
-#pragma unroll
-    for (int q = 0; q < MG_NST; q++) s += cf[q] * xn[q];
-    return s;
-}
-
-// out = x + omega D^-1 (f - A x) on a stencil level, one u-row (i, j) or
-// v-row (i, j) (x == nullptr: x = 0)
-template <typename T>
-__device__ __forceinline__ void st_smooth_u(const stokes_geom &G, const T *__restrict__ su, const T *__restrict__ sv,
-                                            const T *__restrict__ xu, const T *__restrict__ xv,
-                                            const T *__restrict__ fu, const T *__restrict__ idu, T omega,
-                                            T *__restrict__ ou, int i, int j) {
-    const int Nx = G.Nx, Nz = G.Nz;
-    const size_t nu = (size_t)Nx * (Nz + 1);
-    const int c = i + j * Nx;
-    T r = 0;
-    if (u_unknown(i, j, Nx, Nz)) {
-        if (xu) r = xu[c] + omega * idu[c] * (fu[c] - st_urow<T>(Nx, Nz, su, nu, xu, xv, i, j));
-        else r = omega * idu[c] * fu[c];
-    }
-    ou[c] = r;
-}
-
-template <typename T>
-__device__ __forceinline__ void st_smooth_v(const stokes_geom &G, const T *__restrict__ su, const T *__restrict__ sv,
-                                            const T *__restrict__ xu, const T *__restrict__ xv,
-                                            const T *__restrict__ fv, const T *__restrict__ idv, T omega,
-                                            T *__restrict__ ov, int i, int j) {
-    const int Nx = G.Nx, Nz = G.Nz;
-    const size_t nv = (size_t)(Nx + 1) * Nz;
-    const int c = i + j * (Nx + 1);
-    T r = 0;
-    if (v_unknown(i, j, Nx, Nz)) {
-        if (xv) r = xv[c] + omega * idv[c] * (fv[c] - st_vrow<T>(Nx, Nz, sv, nv, xu, xv, i, j));
-        else r = omega * idv[c] * fv[c];
-    }
-    ov[c] = r;
-}
-
-// both rows at point (i, j) of the (Nx+1) x (Nz+1) box
-template <typename T>
-__device__ __forceinline__ void st_smooth_pt(const stokes_geom &G, const T *__restrict__ su, const T *__restrict__ sv,
-                                             const T *__restrict__ xu, const T *__restrict__ xv,
-                                             const T *__restrict__ fu, const T *__restrict__ fv,
-                                             const T *__restrict__ idu, const T *__restrict__ idv, T omega,
-                                             T *__restrict__ ou, T *__restrict__ ov, int i, int j) {
-    if (i < G.Nx && j <= G.Nz) st_smooth_u<T>(G, su, sv, xu, xv, fu, idu, omega, ou, i, j);
-    if (i <= G.Nx && j < G.Nz) st_smooth_v<T>(G, su, sv, xu, xv, fv, idv, omega, ov, i, j);
-}
-
-// one thread per row (u rows first, then v rows): twice the threads of a
-// point-per-thread launch, so that the fine stencil levels fill the machine
-template <typename T>
-__global__ void __launch_bounds__(128) k_st_smooth(stokes_geom G, const T *__restrict__ su, const T *__restrict__ sv,
-                                                   const T *__restrict__ xu, const T *__restrict__ xv,
-                                                   const T *__restrict__ fu, const T *__restrict__ fv,
-                                                   const T *__restrict__ idu, const T *__restrict__ idv, T omega,
-                                                   T *__restrict__ ou, T *__restrict__ ov) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int Nx = G.Nx, nu = Nx * (G.Nz + 1), nv = (Nx + 1) * G.Nz;
-    if (t < nu) st_smooth_u<T>(G, su, sv, xu, xv, fu, idu, omega, ou, t % Nx, t / Nx);
-    else if (t < nu + nv) st_smooth_v<T>(G, su, sv, xu, xv, fv, idv, omega, ov, (t - nu) % (Nx + 1), (t - nu) / (Nx + 1));
-}
-
-template <typename T>
-__device__ __forceinline__ void st_residual_u(const stokes_geom &G, const T *__restrict__ su, const T *__restrict__ xu,
-                                              const T *__restrict__ xv, const T *__restrict__ fu, T *__restrict__ ru,
-                                              int i, int j) {
-    const int Nx = G.Nx, Nz = G.Nz, c = i + j * Nx;
-    ru[c] = u_unknown(i, j, Nx, Nz) ? fu[c] - st_urow<T>(Nx, Nz, su, (size_t)Nx * (Nz + 1), xu, xv, i, j) : T(0);
-}
-
-template <typename T>
-__device__ __forceinline__ void st_residual_v(const stokes_geom &G, const T *__restrict__ sv, const T *__restrict__ xu,
-                                              const T *__restrict__ xv, const T *__restrict__ fv, T *__restrict__ rv,
-                                              int i, int j) {
-    const int Nx = G.Nx, Nz = G.Nz, c = i + j * (Nx + 1);
-    rv[c] = v_unknown(i, j, Nx, Nz) ? fv[c] - st_vrow<T>(Nx, Nz, sv, (size_t)(Nx + 1) * Nz, xu, xv, i, j) : T(0);
-}
-
-template <typename T>
-__device__ __forceinline__ void st_residual_pt(const stokes_geom &G, const T *__restrict__ su,
-                                               const T *__restrict__ sv, const T *__restrict__ xu,
-                                               const T *__restrict__ xv, const T *__restrict__ fu,
-                                               const T *__restrict__ fv, T *__restrict__ ru, T *__restrict__ rv,
-                                               int i, int j) {
-    if (i < G.Nx && j <= G.Nz) st_residual_u<T>(G, su, xu, xv, fu, ru, i, j);
-    if (i <= G.Nx && j < G.Nz) st_residual_v<T>(G, sv, xu, xv, fv, rv, i, j);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(128) k_st_residual(stokes_geom G, const T *__restrict__ su,
-                                                     const T *__restrict__ sv, const T *__restrict__ xu,
-                                                     const T *__restrict__ xv, const T *__restrict__ fu,
-                                                     const T *__restrict__ fv, T *__restrict__ ru,
-                                                     T *__restrict__ rv) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int Nx = G.Nx, nu = Nx * (G.Nz + 1), nv = (Nx + 1) * G.Nz;
-    if (t < nu) st_residual_u<T>(G, su, xu, xv, fu, ru, t % Nx, t / Nx);
-    else if (t < nu + nv) st_residual_v<T>(G, sv, xu, xv, fv, rv, (t - nu) % (Nx + 1), (t - nu) / (Nx + 1));
+    T cf[MG_NST];
+    st_coefs<T>(sv, nv, (size_t)i + (size_t)j * (Nx + 1), cf);
+    return st_vrow_x<T>(Nx, Nz, cf, xu, xv, i, j);
 }
 
 template <typename T>
@@ -541,6 +312,8 @@ __global__ void k_st_diag(stokes_geom G, const T *__restrict__ su, const T *__re
     if (i < (long long)nu) idu[i] = G.BCu[i] == -1 ? T(1) / su[(size_t)MG_CENTER * nu + i] : T(0);
     if (i < (long long)nv) idv[i] = G.BCv[i] == -1 ? T(1) / sv[(size_t)MG_CENTER * nv + i] : T(0);
 }
+
+#include "mg_tiles.cuh"
 
 // Level-0 probing: x = indicator of the unknowns of component comp with
 // (k mod 4, l mod 4) = (cx, cz); y = A x.  The level-0 operator (Picard or
@@ -1067,13 +840,26 @@ __global__ void __launch_bounds__(512) k_coarse_dense_setup(stokes_geom G, const
     }
 }
 
-// x = A^-1 f on the small coarsest level (zero outside the unknowns)
+// x = A^-1 f on the small coarsest level (zero outside the unknowns): eight
+// lanes per row, so that the row's products are not one chain of loads
 template <typename T>
-__global__ void __launch_bounds__(256) k_coarse_dense_solve(int n, int nu, int nv, const int *__restrict__ map,
+__device__ __forceinline__ T dense_row(int n, const T *AinvT, const T *fs, int r, int lane) {
+    T s = 0;
+    if (r < n)
+        for (int j = lane; j < n; j += 8) s += AinvT[(size_t)j * n + r] * fs[j];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(512) k_coarse_dense_solve(int n, int nu, int nv, const int *__restrict__ map,
                                                             const T *__restrict__ AinvT, const T *__restrict__ fu,
                                                             const T *__restrict__ fv, T *__restrict__ xu,
                                                             T *__restrict__ xv) {
     __shared__ T fs[MG_DENSE_MAX];
+    mg_release<T>();
+    pdl_wait();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         int m = map[i];
         fs[i] = m < nu ? fu[m] : fv[m - nu];
@@ -1081,182 +867,189 @@ __global__ void __launch_bounds__(256) k_coarse_dense_solve(int n, int nu, int n
     for (int i = threadIdx.x; i < nu; i += blockDim.x) xu[i] = T(0);
     for (int i = threadIdx.x; i < nv; i += blockDim.x) xv[i] = T(0);
     __syncthreads();
-    for (int r = threadIdx.x; r < n; r += blockDim.x) {
-        T s = 0;
-        for (int j = 0; j < n; j++) s += AinvT[(size_t)j * n + r] * fs[j];
-        int m = map[r];
-        if (m < nu) xu[m] = s; else xv[m - nu] = s;
+    for (int r0 = 0; r0 < n; r0 += blockDim.x / 8) {
+        const int r = r0 + threadIdx.x / 8;
+        const T s = dense_row<T>(n, AinvT, fs, r, threadIdx.x & 7);
+        if (r < n && (threadIdx.x & 7) == 0) {
+            const int m = map[r];
+            if (m < nu) xu[m] = s; else xv[m - nu] = s;
+        }
     }
 }
 
-
 // ---------------------------------------------------------------------------
-// Bottom of the V-cycle in one thread-block cluster.  The small levels (a few
-// thousand points each) cost one launch per sweep, residual and transfer when
-// run as grid kernels, and each such launch is several microseconds of
-// latency for little work; here the whole descent from level `first` to the
-// dense coarsest level and the ascent back run in one launch of one cluster
-// (up to 16 CTAs of 1024 threads on 16 SMs; a single CTA where clusters are
-// not available), with a cluster barrier between phases.  Same arithmetic
-// as the grid kernels (the same point functions), so the result is
-// identical.  The first level's result ends in its xu / xv buffers like the
-// grid path's.
+// Bottom of the V-cycle in one CTA, everything in shared memory.  As grid
+// kernels the smallest levels cost one launch per phase, several microseconds
+// for a few hundred rows.  Here the CTA copies the levels' stencils (unknown rows
+// only), inverse diagonals and the coarsest inverse into shared memory before
+// it waits for the launch that writes its right-hand side, then runs the
+// descent, the dense solve and the ascent between CTA barriers.  The first
+// bottom level is the first whose data, with all below, fit
+// (mg_bottom_bytes): 32 x 16 cells in FP32, 16 x 8 in FP64, on a 2 : 1 box.
+// An earlier form ran every level of at most 32k points in a 16-CTA cluster
+// out of L2, with a cluster barrier per phase: 89 us (FP32, from 128 x 64
+// cells) and 203 us (FP64, where 16 SMs are too few for the rows' FP64 work);
+// levels above the shared-memory limit are faster as grid kernels of two
+// phases each (mg_tiles.cuh).
 #define MG_BOTTOM_MAX 6
-#define MG_BOTTOM_THREADS 1024
+#define MG_BOTTOM_SMEM (220 * 1024)
+// (FP64: fewer threads with twice the registers, its levels have fewer rows)
 template <typename T>
-struct mg_bottom_level {
-    stokes_geom G;
-    const T *su, *sv, *idu, *idv;
-    T *xu, *xv, *yu, *yv, *fu, *fv, *ru, *rv;
-};
-
+constexpr int mg_bottom_threads() { return sizeof(T) == 8 ? 512 : 1024; }
 template <typename T>
 struct mg_bottom_args {
     int nlev, nu1, nu2, ndense;   // nlev levels, the last one the dense coarsest
-    int lsplit;                   // first level run by CTA 0 alone (nlev: none)
     T omega;
     const int *dmap;
     const T *AinvT;
-    mg_bottom_level<T> L[MG_BOTTOM_MAX];
+    int Nx[MG_BOTTOM_MAX], Nz[MG_BOTTOM_MAX];
+    const T *su[MG_BOTTOM_MAX], *sv[MG_BOTTOM_MAX], *idu[MG_BOTTOM_MAX], *idv[MG_BOTTOM_MAX];
+    const T *fu, *fv;             // right-hand side of the first level
+    T *xu, *xv;                   // its result
 };
 
-// points a bottom launch of `cs` CTAs takes on per level
-static inline long long mg_bottom_points(int cs) { return (long long)cs * MG_BOTTOM_THREADS * (cs == 1 ? 4 : 2); }
-
-template <typename T>
-__global__ void __launch_bounds__(MG_BOTTOM_THREADS) k_mg_bottom(const __grid_constant__ mg_bottom_args<T> A) {
-    __shared__ T fs[MG_DENSE_MAX];
-    T *xu[MG_BOTTOM_MAX], *xv[MG_BOTTOM_MAX], *yu[MG_BOTTOM_MAX], *yv[MG_BOTTOM_MAX];
-    for (int l = 0; l < A.nlev; l++) { xu[l] = A.L[l].xu; xv[l] = A.L[l].xv; yu[l] = A.L[l].yu; yv[l] = A.L[l].yv; }
-    // barrier over every thread of the launch: the grid is one cluster (or one CTA);
-    // release / acquire at cluster scope orders the global-memory phases
-    auto cbar = [&]() {
-        if (gridDim.x > 1) cooperative_groups::this_cluster().sync();
-        else __syncthreads();
-    };
-    auto tbar = [&]() { __syncthreads(); };
-    auto swap_xy = [&](int l) {
-        T *t = xu[l]; xu[l] = yu[l]; yu[l] = t;
-        t = xv[l]; xv[l] = yv[l]; yv[l] = t;
-    };
-    // one smoothing sweep / residual over a level's rows, one row per thread
-    // (u rows, then v rows: twice the threads of a point per thread, so that
-    // each phase's critical path is one 31-point row)
-    auto smooth_rows = [&](const mg_bottom_level<T> &L, const T *ixu, const T *ixv, T *ou, T *ov, int t0, int nt) {
-        const int Nx = L.G.Nx, nuL = Nx * (L.G.Nz + 1), nvL = (Nx + 1) * L.G.Nz;
-        for (int r = t0; r < nuL + nvL; r += nt) {
-            if (r < nuL) st_smooth_u<T>(L.G, L.su, L.sv, ixu, ixv, L.fu, L.idu, A.omega, ou, r % Nx, r / Nx);
-            else st_smooth_v<T>(L.G, L.su, L.sv, ixu, ixv, L.fv, L.idv, A.omega, ov, (r - nuL) % (Nx + 1),
-                                (r - nuL) / (Nx + 1));
-        }
-    };
-    auto residual_rows = [&](const mg_bottom_level<T> &L, const T *ixu, const T *ixv, int t0, int nt) {
-        const int Nx = L.G.Nx, nuL = Nx * (L.G.Nz + 1), nvL = (Nx + 1) * L.G.Nz;
-        for (int r = t0; r < nuL + nvL; r += nt) {
-            if (r < nuL) st_residual_u<T>(L.G, L.su, ixu, ixv, L.fu, L.ru, r % Nx, r / Nx);
-            else st_residual_v<T>(L.G, L.sv, ixu, ixv, L.fv, L.rv, (r - nuL) % (Nx + 1), (r - nuL) / (Nx + 1));
-        }
-    };
-    // One level's descent (pre-smoothing, residual, restriction) or ascent
-    // (prolongation, post-smoothing) by a team of threads t0, t0 + nt, ...
-    // (act = false: the thread only keeps its pointer swaps in step) with the
-    // team's barrier after each phase.
-    auto down = [&](int l, bool act, int t0, int nt, auto &&sync) {
-        const mg_bottom_level<T> &L = A.L[l];
-        if (act) smooth_rows(L, nullptr, nullptr, xu[l], xv[l], t0, nt);
-        sync();
-        for (int s = 1; s < A.nu1; s++) {
-            if (act) smooth_rows(L, xu[l], xv[l], yu[l], yv[l], t0, nt);
-            sync();
-            swap_xy(l);
-        }
-        if (act) residual_rows(L, xu[l], xv[l], t0, nt);
-        sync();
-        const mg_bottom_level<T> &C = A.L[l + 1];
-        const int Wc = C.G.Nx + 1, nptc = Wc * (C.G.Nz + 1);
-        for (int p = t0; act && p < nptc; p += nt)
-            mg_restrict_pt<T>(L.G, C.G, L.ru, L.rv, C.fu, C.fv, p % Wc, p / Wc);
-        sync();
-    };
-    auto up = [&](int l, bool act, int t0, int nt, auto &&sync) {
-        const mg_bottom_level<T> &L = A.L[l];
-        const mg_bottom_level<T> &C = A.L[l + 1];
-        const int W = L.G.Nx + 1, npt = W * (L.G.Nz + 1);
-        for (int p = t0; act && p < npt; p += nt)
-            mg_prolong_pt<T>(L.G, C.G, xu[l + 1], xv[l + 1], xu[l], xv[l], p % W, p / W);
-        sync();
-        for (int s = 0; s < A.nu2; s++) {
-            if (act) smooth_rows(L, xu[l], xv[l], yu[l], yv[l], t0, nt);
-            sync();
-            swap_xy(l);
-        }
-    };
-    auto dense = [&](bool act, int t0, int nt, auto &&sync) {   // x = A^-1 f on the coarsest level
-        const int lc = A.nlev - 1, n = A.ndense;
-        const mg_bottom_level<T> &C = A.L[lc];
-        const int nu = C.G.Nx * (C.G.Nz + 1), nv = (C.G.Nx + 1) * C.G.Nz;
-        for (int i = threadIdx.x; act && i < n; i += blockDim.x) {   // every active CTA gathers f for itself
-            const int m = A.dmap[i];
-            fs[i] = m < nu ? C.fu[m] : C.fv[m - nu];
-        }
-        for (int i = t0; act && i < nu; i += nt) xu[lc][i] = T(0);
-        for (int i = t0; act && i < nv; i += nt) xv[lc][i] = T(0);
-        sync();
-        for (int r = t0; act && r < n; r += nt) {
-            T s = 0;
-            for (int j = 0; j < n; j++) s += A.AinvT[(size_t)j * n + r] * fs[j];
-            const int m = A.dmap[r];
-            if (m < nu) xu[lc][m] = s; else xv[lc][m - nu] = s;
-        }
-        sync();
-    };
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
-    // levels lsplit .. nlev-1 are small enough for CTA 0 alone: their phases end
-    // in CTA barriers instead of cluster barriers (the other CTAs wait once)
-    const int ls = A.lsplit;
-    for (int l = 0; l < ls && l < A.nlev - 1; l++) down(l, true, tid, nthr, cbar);
-    if (ls < A.nlev) {
-        const bool act = blockIdx.x == 0;
-        for (int l = ls; l < A.nlev - 1; l++) down(l, act, threadIdx.x, blockDim.x, tbar);
-        dense(act, threadIdx.x, blockDim.x, tbar);
-        for (int l = A.nlev - 2; l >= ls; l--) up(l, act, threadIdx.x, blockDim.x, tbar);
-        cbar();
-    } else {
-        dense(true, tid, nthr, cbar);
-    }
-    for (int l = (ls < A.nlev - 1 ? ls : A.nlev - 1) - 1; l >= 0; l--) up(l, true, tid, nthr, cbar);
-    if (xu[0] != A.L[0].xu) {   // odd number of swaps on the first level: copy back
-        const mg_bottom_level<T> &L = A.L[0];
-        const int nu = L.G.Nx * (L.G.Nz + 1), nv = (L.G.Nx + 1) * L.G.Nz;
-        for (int i = tid; i < nu; i += nthr) L.xu[i] = xu[0][i];
-        for (int i = tid; i < nv; i += nthr) L.xv[i] = xv[0][i];
-    }
+// elements of one level: coefficients and inverse diagonals of the unknown
+// rows, then the vectors x, y (also the residual) and f in box layout
+__host__ __device__ inline int mg_bottom_rows_u(int Nx, int Nz) { return (Nx - 2) * (Nz - 1); }
+__host__ __device__ inline int mg_bottom_rows_v(int Nx, int Nz) { return (Nx - 1) * (Nz - 2); }
+__host__ __device__ inline int mg_bottom_box(int Nx, int Nz) { return Nx * (Nz + 1) + (Nx + 1) * Nz; }
+__host__ __device__ inline long long mg_bottom_level_elems(int Nx, int Nz) {
+    return (long long)(MG_NST + 1) * (mg_bottom_rows_u(Nx, Nz) + mg_bottom_rows_v(Nx, Nz)) +
+           3LL * mg_bottom_box(Nx, Nz);
 }
 
-// Largest cluster (16, 8 or 4 CTAs of 1024 threads) the device can place for
-// the bottom kernel, else 1 (a single CTA).
 template <typename T>
-static int mg_bottom_cluster_size() {
-    if (cudaFuncSetAttribute(k_mg_bottom<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        cudaGetLastError();
-    const int sizes[3] = {16, 8, 4};
-    for (int q = 0; q < 3; q++) {
-        const int cs = sizes[q];
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(cs);
-        cfg.blockDim = dim3(MG_BOTTOM_THREADS);
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = cs;
-        at.val.clusterDim.y = 1;
-        at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k_mg_bottom<T>, &cfg) == cudaSuccess && n >= 1) return cs;
-        cudaGetLastError();
+__global__ void __launch_bounds__(mg_bottom_threads<T>()) k_mg_bottom(const __grid_constant__ mg_bottom_args<T> A) {
+    extern __shared__ __align__(16) unsigned char bottom_sm[];
+    T *const sm = reinterpret_cast<T *>(bottom_sm);
+    mg_release<T>();
+    constexpr int NT = mg_bottom_threads<T>();
+    const int tid = threadIdx.x, lc = A.nlev - 1, n = A.ndense;
+    // ---- static data, while the launch before is still running
+    int off = 0;
+    for (int l = 0; l < lc; l++) {
+        const int Nx = A.Nx[l], Nz = A.Nz[l], Ru = mg_bottom_rows_u(Nx, Nz), Rv = mg_bottom_rows_v(Nx, Nz);
+        const size_t nu = (size_t)Nx * (Nz + 1), nv = (size_t)(Nx + 1) * Nz;
+        T *cu = sm + off, *cv = cu + (MG_NST + 1) * Ru, *vec = cv + (MG_NST + 1) * Rv;
+        for (int r = tid; r < Ru + Rv; r += NT) {
+            const bool u = r < Ru;
+            const int q = u ? r : r - Ru, w = u ? Nx - 2 : Nx - 1;
+            const size_t c = u ? (size_t)(1 + q % w) + (size_t)(1 + q / w) * Nx
+                               : (size_t)(1 + q % w) + (size_t)(1 + q / w) * (Nx + 1);
+            T cf[MG_NST];
+            st_coefs<T>(u ? A.su[l] : A.sv[l], u ? nu : nv, c, cf);
+            T *d = u ? cu + q : cv + q;
+            const int R = u ? Ru : Rv;
+#pragma unroll
+            for (int e = 0; e < MG_NST; e++) d[e * R] = cf[e];
+            d[MG_NST * R] = u ? A.idu[l][c] : A.idv[l][c];
+        }
+        for (int e = tid; e < 3 * mg_bottom_box(Nx, Nz); e += NT) vec[e] = T(0);
+        off += (int)mg_bottom_level_elems(Nx, Nz);
     }
-    return 1;
+    const int cbox = mg_bottom_box(A.Nx[lc], A.Nz[lc]);
+    T *const cx = sm + off, *const cf_ = cx + cbox, *const fs = cf_ + cbox, *const Ai = fs + n;
+    for (int e = tid; e < 2 * cbox; e += NT) cx[e] = T(0);
+    for (int e = tid; e < n * n; e += NT) Ai[e] = A.AinvT[e];
+    __syncthreads();   // the vectors are cleared before the right-hand side goes into one
+    pdl_wait();
+    {
+        const int nu = A.Nx[0] * (A.Nz[0] + 1), box = mg_bottom_box(A.Nx[0], A.Nz[0]);
+        T *f = sm + (MG_NST + 1) * (mg_bottom_rows_u(A.Nx[0], A.Nz[0]) + mg_bottom_rows_v(A.Nx[0], A.Nz[0])) + 2 * box;
+        for (int e = tid; e < box; e += NT) f[e] = e < nu ? A.fu[e] : A.fv[e - nu];
+    }
+    __syncthreads();
+    unsigned par = 0;   // bit l: level l's x is in its second vector
+    // mode 0: x = omega D^-1 f; 1: y = x + omega D^-1 (f - A x); 2: y = f - A x
+    auto rows = [&](int base, int Nx, int Nz, bool odd, int mode) {
+        const int Ru = mg_bottom_rows_u(Nx, Nz), Rv = mg_bottom_rows_v(Nx, Nz), nu = Nx * (Nz + 1),
+                  box = mg_bottom_box(Nx, Nz);
+        const T *cu = sm + base, *cv = cu + (MG_NST + 1) * Ru;
+        T *vec = sm + base + (MG_NST + 1) * (Ru + Rv);
+        T *x = vec + (odd ? box : 0), *y = vec + (odd ? 0 : box);
+        const T *f = vec + 2 * box;
+        for (int r = tid; r < Ru + Rv; r += NT) {
+            const bool u = r < Ru;
+            const int q = u ? r : r - Ru, w = u ? Nx - 2 : Nx - 1, R = u ? Ru : Rv;
+            const int k = 1 + q % w, l = 1 + q / w, c = u ? k + l * Nx : nu + k + l * (Nx + 1);
+            const T *d = u ? cu + q : cv + q;
+            const T id = d[MG_NST * R];
+            if (mode == 0) { x[c] = A.omega * id * f[c]; continue; }
+            T cf[MG_NST];
+#pragma unroll
+            for (int e = 0; e < MG_NST; e++) cf[e] = d[e * R];
+            const T ax = u ? st_urow_x<T>(Nx, Nz, cf, x, x + nu, k, l) : st_vrow_x<T>(Nx, Nz, cf, x, x + nu, k, l);
+            y[c] = mode == 1 ? x[c] + A.omega * id * (f[c] - ax) : f[c] - ax;
+        }
+        __syncthreads();
+    };
+    auto vecs = [&](int base, int l) {   // start of level l's vectors
+        return l == lc ? cx : sm + base + (MG_NST + 1) * (mg_bottom_rows_u(A.Nx[l], A.Nz[l]) + mg_bottom_rows_v(A.Nx[l], A.Nz[l]));
+    };
+    int base = 0;
+    for (int l = 0; l < lc; l++) {
+        const int Nx = A.Nx[l], Nz = A.Nz[l], next = base + (int)mg_bottom_level_elems(Nx, Nz);
+        rows(base, Nx, Nz, false, 0);
+        bool odd = false;
+        for (int s = 1; s < A.nu1; s++) { rows(base, Nx, Nz, odd, 1); odd = !odd; }
+        if (odd) par |= 1u << l;
+        rows(base, Nx, Nz, odd, 2);
+        // restriction of the residual
+        const box_geom F{Nx, Nz, Nx - 1, Nz - 1}, C{A.Nx[l + 1], A.Nz[l + 1], A.Nx[l + 1] - 1, A.Nz[l + 1] - 1};
+        const int box = mg_bottom_box(Nx, Nz), nu = Nx * (Nz + 1), nuc = C.Nx * (C.Nz + 1);
+        const T *r = vecs(base, l) + (odd ? 0 : box);
+        T *f = vecs(next, l + 1) + (l + 1 == lc ? 1 : 2) * mg_bottom_box(C.Nx, C.Nz);
+        const int Ru = mg_bottom_rows_u(C.Nx, C.Nz), Rv = mg_bottom_rows_v(C.Nx, C.Nz);
+        for (int p = tid; p < Ru + Rv; p += NT) {
+            if (p < Ru) {
+                const int I = 1 + p % (C.Nx - 2), J = 1 + p / (C.Nx - 2);
+                f[I + J * C.Nx] = restricted_u<T>(F, C, r, I, J);
+            } else {
+                const int q = p - Ru, I = 1 + q % (C.Nx - 1), J = 1 + q / (C.Nx - 1);
+                f[nuc + I + J * (C.Nx + 1)] = restricted_v<T>(F, C, r + nu, I, J);
+            }
+        }
+        __syncthreads();
+        base = next;
+    }
+    {   // coarsest level: x = A^-1 f
+        for (int i = tid; i < n; i += NT) fs[i] = cf_[A.dmap[i]];
+        __syncthreads();
+        for (int r0 = 0; r0 < n; r0 += NT / 8) {
+            const int r = r0 + tid / 8;
+            const T s = dense_row<T>(n, Ai, fs, r, tid & 7);
+            if (r < n && (tid & 7) == 0) cx[A.dmap[r]] = s;
+        }
+        __syncthreads();
+    }
+    for (int l = lc - 1; l >= 0; l--) {
+        const int Nx = A.Nx[l], Nz = A.Nz[l], next = base;
+        base -= (int)mg_bottom_level_elems(Nx, Nz);
+        bool odd = par >> l & 1;
+        const box_geom F{Nx, Nz, Nx - 1, Nz - 1}, C{A.Nx[l + 1], A.Nz[l + 1], A.Nx[l + 1] - 1, A.Nz[l + 1] - 1};
+        const int box = mg_bottom_box(Nx, Nz), nu = Nx * (Nz + 1), nuc = C.Nx * (C.Nz + 1);
+        T *x = vecs(base, l) + (odd ? box : 0);
+        const T *c = vecs(next, l + 1) + (par >> (l + 1) & 1 ? mg_bottom_box(C.Nx, C.Nz) : 0);
+        const int Ru = mg_bottom_rows_u(Nx, Nz), Rv = mg_bottom_rows_v(Nx, Nz);
+        for (int p = tid; p < Ru + Rv; p += NT) {
+            if (p < Ru) {
+                const int k = 1 + p % (Nx - 2), j = 1 + p / (Nx - 2);
+                x[k + j * Nx] = prolonged_u<T>(F, C, c, x, k, j);
+            } else {
+                const int q = p - Ru, i = 1 + q % (Nx - 1), j = 1 + q / (Nx - 1);
+                x[nu + i + j * (Nx + 1)] = prolonged_v<T>(F, C, c + nuc, x + nu, i, j);
+            }
+        }
+        __syncthreads();
+        for (int s = 0; s < A.nu2; s++) { rows(base, Nx, Nz, odd, 1); odd = !odd; }
+        par = odd ? par | 1u << l : par & ~(1u << l);
+    }
+    const int nu0 = A.Nx[0] * (A.Nz[0] + 1), box0 = mg_bottom_box(A.Nx[0], A.Nz[0]);
+    const T *x = vecs(0, 0) + (par & 1 ? box0 : 0);
+    for (int e = tid; e < box0; e += NT) {
+        if (e < nu0) A.xu[e] = x[e];
+        else A.xv[e - nu0] = x[e];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1294,7 +1087,7 @@ static mdz_status build_hierarchy(mdz_ctx *ctx, mg_hier<T> &H) {
             if (e == cudaSuccess) e = alloc0(&L.D11, (size_t)L.ncx * L.ncz);
             if (e == cudaSuccess) e = alloc0(&L.D33, (size_t)Nx * Nz);
             if (e == cudaSuccess) e = alloc0(&L.pz, (size_t)L.ncx * L.ncz);
-            if (e == cudaSuccess) e = alloc0(&H.pmean, 2);
+            if (e == cudaSuccess) e = alloc0(&H.pmean, 4);
         }
         if (e == cudaSuccess) e = alloc0(&L.su, (size_t)MG_NST * L.nu());
         if (e == cudaSuccess) e = alloc0(&L.sv, (size_t)MG_NST * L.nv());
@@ -1415,8 +1208,8 @@ mdz_status mdz_solver_ensure(mdz_ctx *ctx) {
     if ((s = alloc_gcr<float>(ctx, S->g32, S->restart)) != MDZ_OK) return s;
     MDZ_CUDA(ctx, cudaMallocHost((void **)&S->sc, 64 * sizeof(double)));
     memset(S->sc, 0, 64 * sizeof(double));
-    S->bottom_cs[0] = mg_bottom_cluster_size<double>();
-    S->bottom_cs[1] = mg_bottom_cluster_size<float>();
+    MDZ_CUDA(ctx, cudaFuncSetAttribute(k_mg_bottom<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_BOTTOM_SMEM));
+    MDZ_CUDA(ctx, cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_BOTTOM_SMEM));
     MDZ_CUDA(ctx, cudaFuncSetAttribute(k_coarse_dense_setup<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        MG_DENSE_SMEM));
     MDZ_CUDA(ctx, cudaFuncSetAttribute(k_coarse_dense_setup<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1604,37 +1397,51 @@ static mdz_status mg_setup(mdz_ctx *ctx, mg_hier<T> &H, const double *eta_n, con
 
 static inline dim3 box_grid(int Nx, int Nz) { return dim3((Nx + 1 + 31) / 32, (Nz + 1 + 7) / 8); }
 
+// Shared memory of the bottom kernel run from level l down.
+template <typename T>
+static size_t mg_bottom_bytes(const mg_hier<T> &H, int l) {
+    long long n = 0;
+    for (int q = l; q < H.nlev - 1; q++) n += mg_bottom_level_elems(H.L[q].Nx, H.L[q].Nz);
+    const mg_level<T> &C = H.L[H.nlev - 1];
+    n += 2LL * mg_bottom_box(C.Nx, C.Nz) + (long long)C.ndense * (C.ndense + 1);
+    return (size_t)n * sizeof(T);
+}
+
+// Whether vcycle() runs level l and all below it in the one-launch bottom
+// kernel: as soon as their data fit in one CTA's shared memory.
+template <typename T>
+static bool vcycle_bottom(const mg_hier<T> &H, int l) {
+    const bool viscous = l == 0 && !H.newton;   // level 0 of a Picard hierarchy: stencil from eta directly
+    return !viscous && l < H.nlev - 1 && H.L[H.nlev - 1].ndense && H.nlev - l <= MG_BOTTOM_MAX &&
+           mg_bottom_bytes<T>(H, l) <= MG_BOTTOM_SMEM;
+}
+
 // Whether vcycle() smooths level l with its own sweeps (not the dense
 // coarsest solve, the coarse CG, nor the one-launch bottom kernel).
 template <typename T>
-static bool vcycle_smoothed(const mdz_ctx *ctx, const mg_hier<T> &H, int l) {
-    const mg_level<T> &L = H.L[l];
-    if (l == H.nlev - 1) return false;
-    const bool viscous = l == 0 && !H.newton;
-    const mg_level<T> &Cd = H.L[H.nlev - 1];
-    const int cs = ctx->solver->bottom_cs[sizeof(T) == 8 ? 0 : 1];
-    return !(!viscous && Cd.ndense && H.nlev - l <= MG_BOTTOM_MAX &&
-             (long long)(L.Nx + 1) * (L.Nz + 1) <= mg_bottom_points(cs));
+static bool vcycle_smoothed(const mg_hier<T> &H, int l) {
+    return l < H.nlev - 1 && !vcycle_bottom<T>(H, l);
 }
 
 // One V-cycle: H.L[l].x <- approx A^-1 H.L[l].f.  Level 0 smooths with the
 // re-discretised stencil (viscosities read directly), coarser levels with the
 // Galerkin stencils.  x0_done: the first sweep from x = 0 (x = omega D^-1 f)
-// was already written into L.xu / L.xv with the right-hand side
-// (k_precond_rhs); out_u / out_v: where the last post-smoothing sweep writes
-// (the caller's vector), else the level's own buffers.  Both only for a level
-// that vcycle_smoothed() accepts.
+// was already written into L.xu / L.xv with the right-hand side (by
+// k_precond, or by the finer level's restriction); out_u / out_v: where
+// the last post-smoothing sweep writes (the caller's vector), else the level's
+// own buffers.  Both only for a level that vcycle_smoothed() accepts.  zp: the
+// pressure to shift by its mean in the last launch (viscous level 0, nu2 = 1).
 template <typename T>
 static mdz_status vcycle(mdz_ctx *ctx, mg_hier<T> &H, int l, int nu1, int nu2, T omega, cudaStream_t st,
-                         bool x0_done = false, T *out_u = nullptr, T *out_v = nullptr) {
+                         bool x0_done = false, T *out_u = nullptr, T *out_v = nullptr, T *zp = nullptr) {
     mg_level<T> &L = H.L[l];
     stokes_geom G = L.geom();
     stokes_coefs<T> D = L.coefs();
-    dim3 bl(32, 8), gr = box_grid(L.Nx, L.Nz);
+    const dim3 bl(32, 8), gr = box_grid(L.Nx, L.Nz);
+    // (const views: launch_pdl converts its arguments to the kernel's types)
     if (l == H.nlev - 1 && L.ndense) {
-        k_coarse_dense_solve<T><<<1, 256, 0, st>>>(L.ndense, (int)L.nu(), (int)L.nv(), L.dmap, L.AinvT, L.fu, L.fv,
-                                                   L.xu, L.xv);
-        MDZ_LAUNCHED(ctx);
+        MDZ_PDL(ctx, k_coarse_dense_solve<T>, 1, 512, 0, st, L.ndense, (int)L.nu(), (int)L.nv(), L.dmap, L.AinvT,
+                L.fu, L.fv, L.xu, L.xv);
         return MDZ_OK;
     }
     if (l == H.nlev - 1) {
@@ -1645,73 +1452,70 @@ static mdz_status vcycle(mdz_ctx *ctx, mg_hier<T> &H, int l, int nu1, int nu2, T
         return MDZ_OK;
     }
     const bool viscous = l == 0 && !H.newton;   // level 0 of a Picard hierarchy: stencil from eta directly
-    const mg_level<T> &Cd = H.L[H.nlev - 1];
-    const int cs = ctx->solver->bottom_cs[sizeof(T) == 8 ? 0 : 1];
-    if (!viscous && Cd.ndense && H.nlev - l <= MG_BOTTOM_MAX &&
-        (long long)(L.Nx + 1) * (L.Nz + 1) <= mg_bottom_points(cs)) {   // this level and all below in one launch
+    if (vcycle_bottom<T>(H, l)) {   // this level and all below in one launch
+        const mg_level<T> &Cd = H.L[H.nlev - 1];
         mg_bottom_args<T> A;
         A.nlev = H.nlev - l; A.nu1 = nu1; A.nu2 = nu2; A.ndense = Cd.ndense; A.omega = omega;
-        A.lsplit = A.nlev;
-        for (int q = 0; q < A.nlev; q++)   // levels of at most one point per thread of one CTA
-            if ((long long)(H.L[l + q].Nx + 1) * (H.L[l + q].Nz + 1) <= MG_BOTTOM_THREADS) { A.lsplit = q; break; }
         A.dmap = Cd.dmap; A.AinvT = Cd.AinvT;
         for (int q = 0; q < A.nlev; q++) {
             const mg_level<T> &B = H.L[l + q];
-            A.L[q] = mg_bottom_level<T>{B.geom(), B.su, B.sv, B.idu, B.idv, B.xu, B.xv, B.yu, B.yv,
-                                        B.fu, B.fv, B.ru, B.rv};
+            A.Nx[q] = B.Nx; A.Nz[q] = B.Nz;
+            A.su[q] = B.su; A.sv[q] = B.sv; A.idu[q] = B.idu; A.idv[q] = B.idv;
         }
-        if (cs > 1) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(cs);
-            cfg.blockDim = dim3(MG_BOTTOM_THREADS);
-            cfg.stream = st;
-            cudaLaunchAttribute at;
-            at.id = cudaLaunchAttributeClusterDimension;
-            at.val.clusterDim.x = cs;
-            at.val.clusterDim.y = 1;
-            at.val.clusterDim.z = 1;
-            cfg.attrs = &at;
-            cfg.numAttrs = 1;
-            MDZ_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_mg_bottom<T>, A));
-        } else {
-            k_mg_bottom<T><<<1, MG_BOTTOM_THREADS, 0, st>>>(A);
-        }
-        MDZ_LAUNCHED(ctx);
+        A.fu = L.fu; A.fv = L.fv; A.xu = L.xu; A.xv = L.xv;
+        MDZ_PDL(ctx, k_mg_bottom<T>, 1, mg_bottom_threads<T>(), mg_bottom_bytes<T>(H, l), st, A);
         return MDZ_OK;
     }
-    const int rows_grid = mdz_blocks(L.nu() + L.nv(), 128);
-    auto smooth = [&](const T *xu, const T *xv, T *ou, T *ov) {
-        if (viscous) k_mg_smooth<T><<<gr, bl, 0, st>>>(G, D, xu, xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
-        else k_st_smooth<T><<<rows_grid, 128, 0, st>>>(G, L.su, L.sv, xu, xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
+    const int rows_grid = mdz_blocks(L.nu() + L.nv(), ST_THREADS);
+    auto smooth = [&](const T *xu, const T *xv, T *ou, T *ov) -> mdz_status {
+        if (viscous) MDZ_PDL(ctx, k_mg_smooth<T>, gr, bl, 0, st, G, D, xu, xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
+        else MDZ_PDL(ctx, k_st_smooth<T>, rows_grid, ST_THREADS, 0, st, G, L.su, L.sv, xu, xv, L.fu, L.fv, L.idu, L.idv,
+                     omega, ou, ov);
+        return MDZ_OK;
     };
+    mdz_status s;
     // pre-smoothing from x = 0
-    if (!x0_done) {
-        smooth(nullptr, nullptr, L.xu, L.xv);
-        MDZ_LAUNCHED(ctx);
-    }
-    for (int s = 1; s < nu1; s++) {
-        smooth(L.xu, L.xv, L.yu, L.yv);
-        MDZ_LAUNCHED(ctx);
+    if (!x0_done && (s = smooth(nullptr, nullptr, L.xu, L.xv)) != MDZ_OK) return s;
+    for (int q = 1; q < nu1; q++) {
+        if ((s = smooth(L.xu, L.xv, L.yu, L.yv)) != MDZ_OK) return s;
         std::swap(L.xu, L.yu); std::swap(L.xv, L.yv);
     }
-    if (viscous) k_mg_residual<T><<<gr, bl, 0, st>>>(G, D, L.xu, L.xv, L.fu, L.fv, L.ru, L.rv);
-    else k_st_residual<T><<<rows_grid, 128, 0, st>>>(G, L.su, L.sv, L.xu, L.xv, L.fu, L.fv, L.ru, L.rv);
-    MDZ_LAUNCHED(ctx);
+    // residual, restriction and the coarse level's first sweep in one launch
     mg_level<T> &C = H.L[l + 1];
-    k_mg_restrict<T><<<box_grid(C.Nx, C.Nz), bl, 0, st>>>(G, C.geom(), L.ru, L.rv, C.fu, C.fv);
-    MDZ_LAUNCHED(ctx);
-    mdz_status s = vcycle<T>(ctx, H, l + 1, nu1, nu2, omega, st);
-    if (s != MDZ_OK) return s;
-    k_mg_prolong_add<T><<<gr, bl, 0, st>>>(G, C.geom(), C.xu, C.xv, L.xu, L.xv);
-    MDZ_LAUNCHED(ctx);
-    for (int q = 0; q < nu2; q++) {
-        if (q == nu2 - 1 && out_u) {   // the last sweep straight into the caller's vector
-            smooth(L.xu, L.xv, out_u, out_v);
-            MDZ_LAUNCHED(ctx);
-            break;
-        }
-        smooth(L.xu, L.xv, L.yu, L.yv);
-        MDZ_LAUNCHED(ctx);
+    const stokes_geom GC = C.geom();
+    const bool c0 = vcycle_smoothed<T>(H, l + 1);
+    T *cxu = c0 ? C.xu : nullptr, *cxv = c0 ? C.xv : nullptr;
+    const int cw = C.Nx + 1, ch = C.Nz + 1;
+    const long long cpts = (long long)cw * ch;
+#define MG_RR(kernel, TX, TY, NT, ...)                                                                                \
+    MDZ_PDL(ctx, kernel<T, TX, TY, NT>, dim3((cw + TX - 1) / TX, (ch + TY - 1) / TY), NT, 0, st, G, __VA_ARGS__, L.xu, \
+            L.xv, L.fu, L.fv, GC, C.fu, C.fv, C.idu, C.idv, omega, cxu, cxv)
+    if (viscous) MG_RR(k_mg_resid_restrict, 16, 8, 384, D);
+    else if (cpts > MG_TILE_LARGE) MG_RR(k_st_resid_restrict, 16, 8, 416, L.su, L.sv);
+    else if (cpts > MG_TILE_SMALL) MG_RR(k_st_resid_restrict, 8, 4, 352, L.su, L.sv);
+    else MG_RR(k_st_resid_restrict, 4, 2, 128, L.su, L.sv);
+#undef MG_RR
+    if ((s = vcycle<T>(ctx, H, l + 1, nu1, nu2, omega, st, c0)) != MDZ_OK) return s;
+    if (nu2 == 0) {
+        MDZ_PDL(ctx, k_mg_prolong_add<T>, gr, bl, 0, st, G, GC, C.xu, C.xv, L.xu, L.xv);
+        return MDZ_OK;
+    }
+    // prolongation and the first post-smoothing sweep in one launch; the last
+    // sweep goes straight into the caller's vector
+    T *ou = nu2 == 1 && out_u ? out_u : L.yu, *ov = nu2 == 1 && out_u ? out_v : L.yv;
+    if (viscous)
+        MDZ_PDL(ctx, k_mg_prolong_smooth<T, 32, 8>, gr, 256, 0, st, G, D, GC, C.xu, C.xv, L.xu, L.xv, L.fu, L.fv, L.idu,
+                L.idv, omega, ou, ov, zp, H.pmean);
+    else if ((long long)(L.Nx + 1) * (L.Nz + 1) > MG_TILE_SMALL)
+        MDZ_PDL(ctx, k_st_prolong_smooth<T, 16, 8>, dim3((L.Nx + 16) / 16, (L.Nz + 8) / 8), 256, 0, st, G, GC, L.su, L.sv,
+                C.xu, C.xv, L.xu, L.xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
+    else
+        MDZ_PDL(ctx, k_st_prolong_smooth<T, 8, 4>, dim3((L.Nx + 8) / 8, (L.Nz + 4) / 4), 64, 0, st, G, GC, L.su, L.sv,
+                C.xu, C.xv, L.xu, L.xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
+    if (ou == L.yu) { std::swap(L.xu, L.yu); std::swap(L.xv, L.yv); }
+    for (int q = 1; q < nu2; q++) {
+        if (q == nu2 - 1 && out_u) return smooth(L.xu, L.xv, out_u, out_v);
+        if ((s = smooth(L.xu, L.xv, L.yu, L.yv)) != MDZ_OK) return s;
         std::swap(L.xu, L.yu); std::swap(L.xv, L.yv);
     }
     return MDZ_OK;
@@ -1743,126 +1547,126 @@ __global__ void k_psub(int np, const signed char *__restrict__ tp, const double 
 
 // ---------------------------------------------------------------------------
 // Block preconditioner: zp = (eta_n / celvol) rp ; zu = V-cycle(ru - B zp).
-// (eta_n / celvol from the level-0 copy D11 = 2 eta_n in precision T), and
-// the sum and count of zp over the pressure equations (as k_psum) for the
-// zero-mean projection applied by k_copy_out
+// One launch writes zp (eta_n / celvol from the level-0 copy D11 = 2 eta_n in
+// precision T, or from the Jacobian's tangent D11 where that is positive),
+// f = r_vel - B zp on the fine level (B: celvol-scaled pressure gradient; the
+// rows form the two zp they need again), with xu non-null the V-cycle's first
+// sweep from x = 0, x = omega D^-1 f, and the sum, count and mean of zp over the
+// pressure equations for the zero-mean projection in the last launch.
 template <typename T>
-__global__ void __launch_bounds__(256) k_precond_p(stokes_geom G, const T *__restrict__ D11, const T *__restrict__ Dt,
-                                                   const T *__restrict__ rp, T *__restrict__ zp, double *part,
-                                                   unsigned int *counter, double *psum) {
-    const int np = G.ncx * G.ncz;
-    const T c = T(0.5) * gc<T>(G, GC_IXZ);
+__global__ void __launch_bounds__(256) k_precond(stokes_geom G, const T *__restrict__ D11, const T *__restrict__ Dt,
+                                                 const T *__restrict__ ru, const T *__restrict__ rv,
+                                                 const T *__restrict__ rp, T *__restrict__ zp, T *__restrict__ fu,
+                                                 T *__restrict__ fv, const T *__restrict__ idu,
+                                                 const T *__restrict__ idv, T omega, T *__restrict__ xu,
+                                                 T *__restrict__ xv, double *part, unsigned int *counter,
+                                                 double *psum) {
+    mg_release<T>();
+    const int Nx = G.Nx, Nz = G.Nz, ncx = G.ncx, ncz = G.ncz;
+    const int ntx = (Nx + 32) / 32, ntiles = ntx * ((Nz + 8) / 8);
+    const T half_ivol = T(0.5) * gc<T>(G, GC_IXZ);
+    auto z = [&](int c) {
+        T d = D11[c];
+        if (Dt) {
+            const T t = Dt[c];
+            if (t > T(0)) d = t;
+        }
+        return half_ivol * d * rp[c];
+    };
     T acc = 0;
     int cnt = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-        T v = 0;
-        if (G.BCp[i] == -1) {
-            T d = D11[i];
-            if (Dt) {   // the Jacobian's tangent D11 where it is positive
-                const T t = Dt[i];
-                if (t > T(0)) d = t;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int i = (tile % ntx) * 32 + (threadIdx.x & 31), j = (tile / ntx) * 8 + (threadIdx.x >> 5);
+        const int c2 = i - 1 + (j - 1) * ncx;
+        if (i < Nx && j <= Nz) {
+            const int c = i + j * Nx;
+            T r = 0, x0 = 0;
+            if (u_unknown(i, j, Nx, Nz)) {
+                r = ru[c] - gc<T>(G, GC_DZ) * (z(c2 + 1) - z(c2));
+                if (xu) x0 = omega * idu[c] * r;
             }
-            v = c * d * rp[i];
+            fu[c] = r;
+            if (xu) xu[c] = x0;
+        }
+        if (i <= Nx && j < Nz) {
+            const int c = i + j * (Nx + 1);
+            T r = 0, x0 = 0;
+            if (v_unknown(i, j, Nx, Nz)) {
+                r = rv[c] - gc<T>(G, GC_DX) * (z(c2 + ncx) - z(c2));
+                if (xv) x0 = omega * idv[c] * r;
+            }
+            fv[c] = r;
+            if (xv) xv[c] = x0;
+        }
+        if (i < ncx && j < ncz) {
+            const T v = z(i + j * ncx);
+            zp[i + j * ncx] = v;
             acc += v;
             cnt++;
         }
-        zp[i] = v;
     }
-    const T v[2] = {acc, (T)cnt};
-    mdz_grid_sum<2, T>(v, part, counter, psum);
-}
-
-// f = r_vel - B zp  on the fine MG level (B: celvol-scaled pressure gradient);
-// with xu non-null also the V-cycle's first sweep from x = 0, x = omega D^-1 f
-// (the smoother's own arithmetic for a zero x), in the same pass
-template <typename T>
-__global__ void k_precond_rhs(stokes_geom G, const T *__restrict__ ru, const T *__restrict__ rv,
-                              const T *__restrict__ zp, T *__restrict__ fu, T *__restrict__ fv,
-                              const T *__restrict__ idu, const T *__restrict__ idv, T omega, T *__restrict__ xu,
-                              T *__restrict__ xv) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int Nx = G.Nx, Nz = G.Nz, ncx = G.ncx;
-    if (i < Nx && j <= Nz) {
-        int c = i + j * Nx;
-        T r = 0, x0 = 0;
-        if (G.BCu[c] == -1) {
-            int c2 = i - 1 + (j - 1) * ncx;
-            r = ru[c] - gc<T>(G, GC_DZ) * (zp[c2 + 1] - zp[c2]);
-            if (xu) x0 = T(0) + omega * idu[c] * (r - T(0));
-        }
-        fu[c] = r;
-        if (xu) xu[c] = x0;
-    }
-    if (i <= Nx && j < Nz) {
-        int c = i + j * (Nx + 1);
-        T r = 0, x0 = 0;
-        if (G.BCv[c] == -1) {
-            int c2 = i - 1 + (j - 1) * ncx;
-            r = rv[c] - gc<T>(G, GC_DX) * (zp[c2 + ncx] - zp[c2]);
-            if (xv) x0 = T(0) + omega * idv[c] * (r - T(0));
-        }
-        fv[c] = r;
-        if (xv) xv[c] = x0;
+    const T v[2] = {acc, (T)cnt};   // (counts per thread are small integers: exact in T)
+    if (mdz_grid_sum<2, T>(v, part, counter, psum)) {
+        __syncthreads();
+        if (threadIdx.x == 0) psum[2] = psum[1] > 0 ? (double)((T)psum[0] / (T)psum[1]) : 0.0;
     }
 }
 
 // z pressure <- zero mean over the pressure equations (the mean cancels in
 // the gradient of the right-hand side, so it is removed only here)
 template <typename T>
-__global__ void k_pmean_out(int np, const signed char *__restrict__ tp, const double *__restrict__ psum,
-                            T *__restrict__ zp) {
+__global__ void k_pmean_out(int np, const double *__restrict__ psum, T *__restrict__ zp) {
+    mg_release<T>();
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < np && tp[i] == -1 && psum[1] > 0) zp[i] -= (T)psum[0] / (T)psum[1];
+    if (i < np) zp[i] -= (T)psum[2];
 }
 
-// z velocity <- the V-cycle's result; z pressure <- zero mean over the
-// pressure equations (the mean cancels in the gradient of the right-hand side,
-// so it is removed only here)
+// z velocity <- the V-cycle's result; z pressure <- zero mean, as k_pmean_out
 template <typename T>
 __global__ void k_copy_out(size_t nu, size_t nv, int np, const T *__restrict__ xu, const T *__restrict__ xv,
-                           const signed char *__restrict__ tp, const double *__restrict__ psum, T *__restrict__ zu,
-                           T *__restrict__ zv, T *__restrict__ zp) {
+                           const double *__restrict__ psum, T *__restrict__ zu, T *__restrict__ zv,
+                           T *__restrict__ zp) {
+    mg_release<T>();
+    pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < nu) zu[i] = xu[i];
     if (i < nv) zv[i] = xv[i];
-    if (i < (size_t)np && tp[i] == -1 && psum[1] > 0) zp[i] -= (T)psum[0] / (T)psum[1];
+    if (i < (size_t)np) zp[i] -= (T)psum[2];
 }
 
+// (captured: the first launch must be an ordinary one, so that the graph as a
+// whole follows the stream's earlier work)
 template <typename T>
-static mdz_status precondition(mdz_ctx *ctx, mg_hier<T> &H, const double *eta_n, const T *Dt, const T *r, T *z,
-                               size_t nu, size_t nv, cudaStream_t st) {
+static mdz_status precondition(mdz_ctx *ctx, mg_hier<T> &H, const T *Dt, const T *r, T *z, size_t nu, size_t nv,
+                               cudaStream_t st) {
     mg_level<T> &F = H.L[0];
     stokes_geom G = F.geom();
     const int np = F.ncx * F.ncz;
-    // zero-mean pressure block: constants are the operator's null space; left
-    // in, they grow in the iterates and cost the FP32 gradients their accuracy
-    {
-        int blocks = mdz_blocks(np, 256);
-        if (blocks > 152 * 4) blocks = 152 * 4;
-        k_precond_p<T><<<blocks, 256, 0, st>>>(G, F.D11, Dt, r + nu + nv, z + nu + nv, ctx->red_part + MDZ_RP_PRECP,
-                                               ctx->red_cnt + MDZ_RC_PRECP, H.pmean);
-        MDZ_LAUNCHED(ctx);
-    }
     mdz_solver *S = ctx->solver;
     // a level-0 V-cycle of its own sweeps takes its first sweep from the
     // right-hand side kernel and writes its last sweep into z
-    const bool fused = vcycle_smoothed<T>(ctx, H, 0) && S->nu2 > 0;
-    k_precond_rhs<T><<<box_grid(F.Nx, F.Nz), dim3(32, 8), 0, st>>>(G, r, r + nu, z + nu + nv, F.fu, F.fv, F.idu,
-                                                                  F.idv, (T)S->omega, fused ? F.xu : nullptr,
-                                                                  fused ? F.xv : nullptr);
+    const bool fused = vcycle_smoothed<T>(H, 0) && S->nu2 > 0;
+    const bool mean_fused = fused && !H.newton && S->nu2 == 1;
+    T *const zp = z + nu + nv;
+    // zero-mean pressure block: constants are the operator's null space; left
+    // in, they grow in the iterates and cost the FP32 gradients their accuracy
+    int blocks = ((F.Nx + 32) / 32) * ((F.Nz + 8) / 8);
+    if (blocks > 152 * 8) blocks = 152 * 8;
+    k_precond<T><<<blocks, 256, 0, st>>>(G, F.D11, Dt, r, r + nu, r + nu + nv, zp, F.fu, F.fv, F.idu, F.idv,
+                                         (T)S->omega, fused ? F.xu : nullptr, fused ? F.xv : nullptr,
+                                         ctx->red_part + MDZ_RP_PRECP, ctx->red_cnt + MDZ_RC_PRECP, H.pmean);
     MDZ_LAUNCHED(ctx);
     mdz_status s = vcycle<T>(ctx, H, 0, S->nu1, S->nu2, (T)S->omega, st, fused, fused ? z : nullptr,
-                             fused ? z + nu : nullptr);
-    if (s != MDZ_OK) return s;
+                             fused ? z + nu : nullptr, mean_fused ? zp : nullptr);
+    if (s != MDZ_OK || mean_fused) return s;
     if (fused) {
-        k_pmean_out<T><<<mdz_blocks(np), MDZ_THREADS, 0, st>>>(np, G.BCp, H.pmean, z + nu + nv);
+        MDZ_PDL(ctx, k_pmean_out<T>, mdz_blocks(np), MDZ_THREADS, 0, st, np, H.pmean, zp);
     } else {
         size_t n = nu > nv ? nu : nv;
         if ((size_t)np > n) n = np;
-        k_copy_out<T><<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(nu, nv, np, F.xu, F.xv, G.BCp, H.pmean, z, z + nu,
-                                                             z + nu + nv);
+        MDZ_PDL(ctx, k_copy_out<T>, mdz_blocks(n), MDZ_THREADS, 0, st, nu, nv, np, F.xu, F.xv, H.pmean, z, z + nu, zp);
     }
-    MDZ_LAUNCHED(ctx);
     return MDZ_OK;
 }
 
@@ -2189,7 +1993,7 @@ static mdz_status precond_graph(mdz_ctx *ctx, gcr_space<T> &S, mg_hier<T> &H, co
     if (SV->pre[slot]) { cudaGraphExecDestroy(SV->pre[slot]); SV->pre[slot] = nullptr; }
     const long long l0 = ctx->launches;
     MDZ_CUDA(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    mdz_status s = precondition<T>(ctx, H, eta_n, Dt, S.pin, S.z, S.nu, S.nv, st);
+    mdz_status s = precondition<T>(ctx, H, Dt, S.pin, S.z, S.nu, S.nv, st);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &g);
     if (s != MDZ_OK) { if (g) cudaGraphDestroy(g); return s; }
