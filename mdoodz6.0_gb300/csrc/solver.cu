@@ -27,7 +27,7 @@
 
 #define MG_MAX_LEVELS 16
 #define MG_DENSE_MAX 256
-#define MG_DENSE_SMEM (96 * 1024)   // [A | I] of the coarsest level in shared memory up to this size (n <= 78)
+#define MG_DENSE_SMEM (200 * 1024)  // the coarsest level is inverted in shared memory up to this size (FP64: n <= 160)
 #define MG_NST 31        // stencil coefficients per velocity row (15 same-component + 16 cross)
 #define MG_CENTER 7      // plane of the diagonal entry in both layouts
 #define GCR_MAX_M 48
@@ -54,7 +54,7 @@ struct mg_level {
     // coarsest level with at most MG_DENSE_MAX unknowns: explicit inverse
     int ndense = 0;
     int *dmap = nullptr;                        // dense index -> u index, or nu + v index
-    double *Awork = nullptr;                    // 2 ndense^2 FP64: [A | I] for Gauss-Jordan
+    T *Awork = nullptr;                         // ndense^2: the elimination, where it does not fit in shared memory
     T *AinvT = nullptr;                         // inverse, column-major
     size_t nu() const { return (size_t)Nx * (Nz + 1); }
     size_t nv() const { return (size_t)(Nx + 1) * Nz; }
@@ -84,6 +84,8 @@ struct mg_hier {
     int nlev = 0;
     bool newton = false;          // level 0 is the probed Newton block (smoothed by its stencil)
     bool built = false;           // mg_setup has filled the levels at least once
+    bool viscous = false;         // the last mg_setup left level 0 to its viscosities (no stencils stored)
+    stokes_geom setup_geom{};     // level 0 of that set-up
     double *pmean = nullptr;      // preconditioner scratch: pressure sum, count and mean
     mg_level<T> L[MG_MAX_LEVELS];
 };
@@ -408,91 +410,79 @@ __global__ void k_probe_collect(stokes_geom G, int comp, int cx, int cz, const T
 //   v-row (i, j), cN = inN D22[N], cS = inS D22[S], dE = inE D33[E], dW = inW D33[W]:
 //     v(i, j+-1): -2/3 cN|cS / dz^2   v(i+-1, j): -dE|dW / dx^2   v(i, j): the sum of their negatives
 //     u(i, j+1): cN/3 - dE   u(i-1, j+1): dW - cN/3   u(i, j): dE - cS/3   u(i-1, j): cS/3 - dW   (/ dx dz)
+// (The free-slip box of u_unknown / v_unknown, checked before a hierarchy is
+// built: every centroid and vertex is active, in* = 0 only for the shear
+// stress beside a free-slip wall.)
+template <typename T>
+__device__ __forceinline__ void picard_coefs_u(const stokes_geom &G, const T *__restrict__ D11,
+                                               const T *__restrict__ D33, int k, int l, T (&a)[MG_NST]) {
+    const int Nx = G.Nx, Nz = G.Nz, c1 = k + l * Nx, c2 = k - 1 + (l - 1) * G.ncx;
+    const T celvol = gc<T>(G, GC_CELVOL), ixx = gc<T>(G, GC_IXX), izz = gc<T>(G, GC_IZZ), ixz = gc<T>(G, GC_IXZ);
+#pragma unroll
+    for (int q = 0; q < MG_NST; q++) a[q] = T(0);
+    const T aE = D11[c2 + 1], aW = D11[c2];
+    const T bN = l < Nz - 1 ? D33[c1] : T(0), bS = l > 1 ? D33[c1 - Nx] : T(0);
+    const T uE = -T(2.0 * T(1.0 / 3.0)) * aE * ixx, uW = -T(2.0 * T(1.0 / 3.0)) * aW * ixx;
+    const T uN = -bN * izz, uS = -bS * izz;
+    auto isu = [&](int kk, int ll, T v) { return u_unknown(kk, ll, Nx, Nz) ? v * celvol : T(0); };
+    auto isv = [&](int ii, int jj, T v) { return v_unknown(ii, jj, Nx, Nz) ? v * celvol : T(0); };
+    a[(0 + 1) + 3 * (0 + 2)] = -(uE + uW + uN + uS) * celvol;
+    a[(1 + 1) + 3 * (0 + 2)] = isu(k + 1, l, uE);
+    a[(-1 + 1) + 3 * (0 + 2)] = isu(k - 1, l, uW);
+    a[(0 + 1) + 3 * (1 + 2)] = isu(k, l + 1, uN);
+    a[(0 + 1) + 3 * (-1 + 2)] = isu(k, l - 1, uS);
+    a[15 + (1 + 1) + 4 * (0 + 2)] = isv(k + 1, l, (aE * T(1.0 / 3.0) - bN) * ixz);
+    a[15 + (1 + 1) + 4 * (-1 + 2)] = isv(k + 1, l - 1, (bS - aE * T(1.0 / 3.0)) * ixz);
+    a[15 + (0 + 1) + 4 * (0 + 2)] = isv(k, l, (bN - aW * T(1.0 / 3.0)) * ixz);
+    a[15 + (0 + 1) + 4 * (-1 + 2)] = isv(k, l - 1, (aW * T(1.0 / 3.0) - bS) * ixz);
+}
+
+template <typename T>
+__device__ __forceinline__ void picard_coefs_v(const stokes_geom &G, const T *__restrict__ D11,
+                                               const T *__restrict__ D33, int k, int l, T (&a)[MG_NST]) {
+    const int Nx = G.Nx, Nz = G.Nz, c1 = k + l * Nx, c2 = k - 1 + (l - 1) * G.ncx;
+    const T celvol = gc<T>(G, GC_CELVOL), ixx = gc<T>(G, GC_IXX), izz = gc<T>(G, GC_IZZ), ixz = gc<T>(G, GC_IXZ);
+#pragma unroll
+    for (int q = 0; q < MG_NST; q++) a[q] = T(0);
+    const T cN = D11[c2 + G.ncx], cS = D11[c2];
+    const T dE = k < Nx - 1 ? D33[c1] : T(0), dW = k > 1 ? D33[c1 - 1] : T(0);
+    const T vN = -T(2.0 * T(1.0 / 3.0)) * cN * izz, vS = -T(2.0 * T(1.0 / 3.0)) * cS * izz;
+    const T vE = -dE * ixx, vW = -dW * ixx;
+    auto isu = [&](int kk, int ll, T v) { return u_unknown(kk, ll, Nx, Nz) ? v * celvol : T(0); };
+    auto isv = [&](int ii, int jj, T v) { return v_unknown(ii, jj, Nx, Nz) ? v * celvol : T(0); };
+    a[(0 + 2) + 5 * (0 + 1)] = -(vN + vS + vE + vW) * celvol;
+    a[(0 + 2) + 5 * (1 + 1)] = isv(k, l + 1, vN);
+    a[(0 + 2) + 5 * (-1 + 1)] = isv(k, l - 1, vS);
+    a[(1 + 2) + 5 * (0 + 1)] = isv(k + 1, l, vE);
+    a[(-1 + 2) + 5 * (0 + 1)] = isv(k - 1, l, vW);
+    a[15 + (0 + 2) + 4 * (1 + 1)] = isu(k, l + 1, (cN * T(1.0 / 3.0) - dE) * ixz);
+    a[15 + (-1 + 2) + 4 * (1 + 1)] = isu(k - 1, l + 1, (dW - cN * T(1.0 / 3.0)) * ixz);
+    a[15 + (0 + 2) + 4 * (0 + 1)] = isu(k, l, (dE - cS * T(1.0 / 3.0)) * ixz);
+    a[15 + (-1 + 2) + 4 * (0 + 1)] = isu(k - 1, l, (cS * T(1.0 / 3.0) - dW) * ixz);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_picard_stencil(stokes_geom G, const T *__restrict__ D11,
                                                         const T *__restrict__ D33, T *__restrict__ su,
                                                         T *__restrict__ sv) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int Nx = G.Nx, Nz = G.Nz, nx = Nx, ncx = G.ncx, nxvz = Nx + 1;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int Nx = G.Nx, Nz = G.Nz;
     const size_t nu = (size_t)Nx * (Nz + 1), nv = (size_t)(Nx + 1) * Nz;
-    const T celvol = gc<T>(G, GC_CELVOL), ixx = gc<T>(G, GC_IXX), izz = gc<T>(G, GC_IZZ),
-            ixz = gc<T>(G, GC_IXZ);
-    if (i < Nx && j <= Nz) {   // u-row (k, l) = (i, j)
-        const int k = i, l = j, c1 = k + l * nx;
-        T a[MG_NST];
+    T a[MG_NST];
+    if (i < Nx && j <= Nz) {
+        const bool unk = u_unknown(i, j, Nx, Nz);
+        if (unk) picard_coefs_u<T>(G, D11, D33, i, j, a);
 #pragma unroll
-        for (int q = 0; q < MG_NST; q++) a[q] = T(0);
-        if (G.BCu[c1] == -1) {
-            const int c2 = k - 1 + (l - 1) * ncx, iPrW = c2, iPrE = c2 + 1, ixyN = c1, ixyS = c1 - nx;
-            const T inW = G.BCp[iPrW] == -1 ? T(1) : T(0), inE = G.BCp[iPrE] == -1 ? T(1) : T(0);
-            const T inS = (G.BCg[ixyS] != 30 && G.BCu[c1 - nx] != 13) ? T(1) : T(0);
-            const T inN = (G.BCg[ixyN] != 30 && G.BCu[c1 + nx] != 13) ? T(1) : T(0);
-            const T aE = inE * D11[iPrE], aW = inW * D11[iPrW];
-            const T bN = inN * D33[ixyN], bS = inS * D33[ixyS];
-            const T uE = -T(2.0 * T(1.0 / 3.0)) * aE * ixx, uW = -T(2.0 * T(1.0 / 3.0)) * aW * ixx;
-            const T uN = -bN * izz, uS = -bS * izz;
-            auto isu = [&](int kk, int ll) { return G.BCu[kk + ll * nx] == -1 ? T(1) : T(0); };
-            auto isv = [&](int ii, int jj) { return G.BCv[ii + jj * nxvz] == -1 ? T(1) : T(0); };
-            a[(0 + 1) + 3 * (0 + 2)] = -(uE + uW + uN + uS);
-            a[(1 + 1) + 3 * (0 + 2)] = uE * isu(k + 1, l);
-            a[(-1 + 1) + 3 * (0 + 2)] = uW * isu(k - 1, l);
-            a[(0 + 1) + 3 * (1 + 2)] = uN * isu(k, l + 1);
-            a[(0 + 1) + 3 * (-1 + 2)] = uS * isu(k, l - 1);
-            a[15 + (1 + 1) + 4 * (0 + 2)] = (aE * T(1.0 / 3.0) - bN) * ixz * isv(k + 1, l);
-            a[15 + (1 + 1) + 4 * (-1 + 2)] = (bS - aE * T(1.0 / 3.0)) * ixz * isv(k + 1, l - 1);
-            a[15 + (0 + 1) + 4 * (0 + 2)] = (bN - aW * T(1.0 / 3.0)) * ixz * isv(k, l);
-            a[15 + (0 + 1) + 4 * (-1 + 2)] = (aW * T(1.0 / 3.0) - bS) * ixz * isv(k, l - 1);
-        }
-#pragma unroll
-        for (int q = 0; q < MG_NST; q++) su[(size_t)q * nu + c1] = a[q] * celvol;
+        for (int q = 0; q < MG_NST; q++) su[(size_t)q * nu + i + j * Nx] = unk ? a[q] : T(0);
     }
-    if (i <= Nx && j < Nz) {   // v-row (k, l) = (i, j)
-        const int k = i, l = j, c3 = k + l * nxvz;
-        T a[MG_NST];
+    if (i <= Nx && j < Nz) {
+        const bool unk = v_unknown(i, j, Nx, Nz);
+        if (unk) picard_coefs_v<T>(G, D11, D33, i, j, a);
 #pragma unroll
-        for (int q = 0; q < MG_NST; q++) a[q] = T(0);
-        if (G.BCv[c3] == -1) {
-            const int c1 = k + l * nx, c2 = k - 1 + (l - 1) * ncx;
-            const int iPrS = c2, iPrN = c2 + ncx, ixyW = c1 - 1, ixyE = c1;
-            T inS = 0, inN = 0;
-            const bool s30 = G.BCv[c3 - nxvz] == 30, n30 = G.BCv[c3 + nxvz] == 30;
-            if (!s30 && !n30) { inS = 1; inN = 1; }
-            if (s30 && !n30) inN = 1;
-            if (!s30 && n30) inS = 1;
-            if (G.BCp[iPrS] == -1) inS = 1;
-            if (G.BCp[iPrN] == -1) inN = 1;
-            const T inW = (G.BCg[ixyW] != 30 && G.BCv[c3 - 1] != 13) ? T(1) : T(0);
-            const T inE = (G.BCg[ixyE] != 30 && G.BCv[c3 + 1] != 13) ? T(1) : T(0);
-            const T cN = inN * D11[iPrN], cS = inS * D11[iPrS];
-            const T dE = inE * D33[ixyE], dW = inW * D33[ixyW];
-            const T vN = -T(2.0 * T(1.0 / 3.0)) * cN * izz, vS = -T(2.0 * T(1.0 / 3.0)) * cS * izz;
-            const T vE = -dE * ixx, vW = -dW * ixx;
-            auto isu = [&](int kk, int ll) { return G.BCu[kk + ll * nx] == -1 ? T(1) : T(0); };
-            auto isv = [&](int ii, int jj) { return G.BCv[ii + jj * nxvz] == -1 ? T(1) : T(0); };
-            a[(0 + 2) + 5 * (0 + 1)] = -(vN + vS + vE + vW);
-            a[(0 + 2) + 5 * (1 + 1)] = vN * isv(k, l + 1);
-            a[(0 + 2) + 5 * (-1 + 1)] = vS * isv(k, l - 1);
-            a[(1 + 2) + 5 * (0 + 1)] = vE * isv(k + 1, l);
-            a[(-1 + 2) + 5 * (0 + 1)] = vW * isv(k - 1, l);
-            a[15 + (0 + 2) + 4 * (1 + 1)] = (cN * T(1.0 / 3.0) - dE) * ixz * isu(k, l + 1);
-            a[15 + (-1 + 2) + 4 * (1 + 1)] = (dW - cN * T(1.0 / 3.0)) * ixz * isu(k - 1, l + 1);
-            a[15 + (0 + 2) + 4 * (0 + 1)] = (dE - cS * T(1.0 / 3.0)) * ixz * isu(k, l);
-            a[15 + (-1 + 2) + 4 * (0 + 1)] = (cS * T(1.0 / 3.0) - dW) * ixz * isu(k - 1, l);
-        }
-#pragma unroll
-        for (int q = 0; q < MG_NST; q++) sv[(size_t)q * nv + c3] = a[q] * celvol;
+        for (int q = 0; q < MG_NST; q++) sv[(size_t)q * nv + i + j * (Nx + 1)] = unk ? a[q] : T(0);
     }
 }
 
-// Coarse stencils = R A P, four threads per coarse row (one fine line of the
-// restriction each, summed in shared memory at the end), accumulated in the
-// level's precision (FP64 throughput is a small fraction of FP32 on this
-// part) in shared memory (plane-major, one column per thread).  Every level of the
-// hierarchy follows the tag rule (u_unknown / v_unknown), so the kernel
-// reads no tags.  Each fine row's 31 coefficients are loaded in
-// one batch before use: loaded one at a time behind the zero test they
-// serialise on memory latency.  An entry landing outside the footprint
-// (impossible with this P) sets *bad.
 // parents of fine u node (i, j) / v node (i, j) as coarse (I, J) pairs
 __device__ __forceinline__ void u_parents_ij(int i, int j, int nczc, int *I, int *J, float *w) {
     int J0, J1;
@@ -517,132 +507,116 @@ __device__ __forceinline__ void v_parents_ij(int i, int j, int ncxc, int *I, int
     I[3] = I1; J[3] = Jb; w[3] = wb * w1;
 }
 
-#define GAL_THREADS 128
-#define GAL_SPLIT 4   // threads per coarse row: each takes one of the 4 fine lines of the restriction
-template <typename T>
+// Coarse stencils = R A P.  A block forms 32 coarse rows of one component:
+// each of its 12 warps takes one of the 12 fine rows a coarse row restricts
+// from (3 node-centred x 4 cell-centred lines), for the 32 coarse rows of its
+// lanes, so the parity of the fine indices, and with it the pattern of the
+// parents, is the same across a warp; every lane accumulates its 31 entries in
+// a column of shared memory of its own and the 12 columns are added up at the
+// end, in warp order, together with the row's inverse diagonal.  Accumulation in
+// the level's precision (FP64 throughput is a small fraction of FP32 on this
+// part).  From a viscous fine level (VISC) the 9 Picard coefficients of a row are
+// formed from the viscosities instead of reading 31 stored ones.  An entry
+// landing outside the footprint (impossible with this P) sets *bad.
+// An earlier form (four threads per coarse row, three fine rows each one
+// after the other, u and v rows in the same thread) took 80-90 us on every
+// level however small, and 236 us on the first level of 1025 x 513 in FP32.
+#define GAL_WARPS 12
+#define GAL_THREADS (32 * GAL_WARPS)
+template <typename T, bool VISC>
 __global__ void __launch_bounds__(GAL_THREADS) k_galerkin(stokes_geom F, const T *__restrict__ suF,
-                                                          const T *__restrict__ svF, stokes_geom Cg,
-                                                          T *__restrict__ suC, T *__restrict__ svC, int *bad) {
-    __shared__ T acc_sh[MG_NST * GAL_THREADS];
-    T *acc = acc_sh + threadIdx.x;
-#define ACC(q) acc[(q) * GAL_THREADS]
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int t = (int)(gt / GAL_SPLIT), sub = (int)(gt % GAL_SPLIT);   // coarse row, fine line of it
-    const int col0 = threadIdx.x - sub;                                  // the row's first column here
+                                                          const T *__restrict__ svF, const T *__restrict__ D11,
+                                                          const T *__restrict__ D33, stokes_geom Cg, int ublocks,
+                                                          T *__restrict__ suC, T *__restrict__ svC,
+                                                          T *__restrict__ idu, T *__restrict__ idv, int *bad) {
+    extern __shared__ __align__(16) unsigned char gal_sm[];
+    T *const acc_sh = reinterpret_cast<T *>(gal_sm);
+    T *const acc = acc_sh + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool ublock = (int)blockIdx.x < ublocks;
     const int Nxf = F.Nx, Nzf = F.Nz, Nxc = Cg.Nx, Nzc = Cg.Nz;
-    const size_t nuf = (size_t)Nxf * (Nzf + 1), nvf = (size_t)(Nxf + 1) * Nzf;
-    const int nuc = Nxc * (Nzc + 1), nvc = (Nxc + 1) * Nzc;
+    const int t0 = 32 * (ublock ? (int)blockIdx.x : (int)blockIdx.x - ublocks), t = t0 + lane;
+    const int n = ublock ? Nxc * (Nzc + 1) : (Nxc + 1) * Nzc, w = ublock ? Nxc : Nxc + 1;
+    const int K = t % w, L = t / w;   // coarse u node (K, L) or v node (K, L)
+    const bool row = t < n && (ublock ? u_unknown(K, L, Nxc, Nzc) : v_unknown(K, L, Nxc, Nzc));
+#pragma unroll
+    for (int q = 0; q < MG_NST; q++) acc[q * GAL_THREADS] = T(0);
+    const int cc = warp / 3, nc = warp % 3;   // cell-centred line 2 X - 2 + cc, node-centred 2 X - 1 + nc
+    const float wn = nc == 1 ? 1.0f : 0.5f;
     int PI[4], PJ[4];
     float pw[4];
     T a[MG_NST];
-    if (t < nuc) {   // coarse u-row (K, L)
-        const int K = t % Nxc, L = t / Nxc;
-        for (int q = 0; q < MG_NST; q++) ACC(q) = T(0);
-        if (u_unknown(K, L, Nxc, Nzc)) {
-            for (int lf = 2 * L - 2 + sub; lf <= 2 * L - 2 + sub; lf++) {
-                if (lf < 1 || lf > F.ncz) continue;
-                int J0, J1;
-                float w0, w1;
-                cc_weights(lf, Cg.ncz, J0, w0, J1, w1);
-                const float wz = (J0 == L ? w0 : 0.0f) + (J1 == L && J1 != J0 ? w1 : 0.0f);
-                if (wz == 0.0f) continue;
-                for (int k = 2 * K - 1; k <= 2 * K + 1; k++) {
-                    if (!u_unknown(k, lf, Nxf, Nzf)) continue;
-                    const size_t f = (size_t)k + (size_t)lf * Nxf;
-                    const T R = (T)(nc_weight(k, K) * wz);
+    pdl_wait();
+    auto add = [&](int slot, int di, int dj, int lo_i, int hi_i, int lo_j, int hi_j, int sd, T v) {
+        if (di < lo_i || di > hi_i || dj < lo_j || dj > hi_j) { *bad = 1; return; }
+        acc[(slot + (di - lo_i) + sd * (dj - lo_j)) * GAL_THREADS] += v;
+    };
+    if (row && ublock) {
+        const int k = 2 * K - 1 + nc, l = 2 * L - 2 + cc;
+        if (l >= 1 && l <= F.ncz && u_unknown(k, l, Nxf, Nzf)) {
+            const T R = weight<T>(wn * cc_restrict_weight(L, cc, Cg.ncz));
+            if (VISC) picard_coefs_u<T>(F, D11, D33, k, l, a);
+            else st_coefs<T>(suF, (size_t)Nxf * (Nzf + 1), (size_t)k + (size_t)l * Nxf, a);
 #pragma unroll
-                    for (int q = 0; q < MG_NST; q++) a[q] = __ldg(suF + (size_t)q * nuf + f);
+            for (int q = 0; q < 15; q++) {   // uu entries of the fine row
+                if (a[q] == T(0)) continue;
+                u_parents_ij(k + q % 3 - 1, l + q / 3 - 2, Cg.ncz, PI, PJ, pw);
+                const T ra = R * a[q];
 #pragma unroll
-                    for (int q = 0; q < 15; q++) {   // uu entries of the fine row
-                        if (a[q] == T(0)) continue;
-                        u_parents_ij(k + q % 3 - 1, lf + q / 3 - 2, Cg.ncz, PI, PJ, pw);
-                        const T ra = R * a[q];
+                for (int s = 0; s < 4; s++)
+                    if (pw[s] != 0.0f && u_unknown(PI[s], PJ[s], Nxc, Nzc))
+                        add(0, PI[s] - K, PJ[s] - L, -1, 1, -2, 2, 3, ra * weight<T>(pw[s]));
+            }
 #pragma unroll
-                        for (int s = 0; s < 4; s++) {
-                            if (pw[s] == 0.0f || !u_unknown(PI[s], PJ[s], Nxc, Nzc)) continue;
-                            const int dK = PI[s] - K, dL = PJ[s] - L;
-                            if (dK < -1 || dK > 1 || dL < -2 || dL > 2) { *bad = 1; continue; }
-                            ACC((dK + 1) + 3 * (dL + 2)) += ra * (T)pw[s];
-                        }
-                    }
+            for (int q = 0; q < 16; q++) {   // uv entries
+                if (a[15 + q] == T(0)) continue;
+                v_parents_ij(k + q % 4 - 1, l + q / 4 - 2, Cg.ncx, PI, PJ, pw);
+                const T ra = R * a[15 + q];
 #pragma unroll
-                    for (int q = 0; q < 16; q++) {   // uv entries of the fine row
-                        if (a[15 + q] == T(0)) continue;
-                        v_parents_ij(k + q % 4 - 1, lf + q / 4 - 2, Cg.ncx, PI, PJ, pw);
-                        const T ra = R * a[15 + q];
+                for (int s = 0; s < 4; s++)
+                    if (pw[s] != 0.0f && v_unknown(PI[s], PJ[s], Nxc, Nzc))
+                        add(15, PI[s] - K, PJ[s] - L, -1, 2, -2, 1, 4, ra * weight<T>(pw[s]));
+            }
+        }
+    } else if (row) {
+        const int i = 2 * K - 2 + cc, j = 2 * L - 1 + nc;
+        if (i >= 1 && i <= F.ncx && v_unknown(i, j, Nxf, Nzf)) {
+            const T R = weight<T>(wn * cc_restrict_weight(K, cc, Cg.ncx));
+            if (VISC) picard_coefs_v<T>(F, D11, D33, i, j, a);
+            else st_coefs<T>(svF, (size_t)(Nxf + 1) * Nzf, (size_t)i + (size_t)j * (Nxf + 1), a);
 #pragma unroll
-                        for (int s = 0; s < 4; s++) {
-                            if (pw[s] == 0.0f || !v_unknown(PI[s], PJ[s], Nxc, Nzc)) continue;
-                            const int dI = PI[s] - K, dJ = PJ[s] - L;
-                            if (dI < -1 || dI > 2 || dJ < -2 || dJ > 1) { *bad = 1; continue; }
-                            ACC(15 + (dI + 1) + 4 * (dJ + 2)) += ra * (T)pw[s];
-                        }
-                    }
-                }
+            for (int q = 0; q < 15; q++) {   // vv entries
+                if (a[q] == T(0)) continue;
+                v_parents_ij(i + q % 5 - 2, j + q / 5 - 1, Cg.ncx, PI, PJ, pw);
+                const T ra = R * a[q];
+#pragma unroll
+                for (int s = 0; s < 4; s++)
+                    if (pw[s] != 0.0f && v_unknown(PI[s], PJ[s], Nxc, Nzc))
+                        add(0, PI[s] - K, PJ[s] - L, -2, 2, -1, 1, 5, ra * weight<T>(pw[s]));
+            }
+#pragma unroll
+            for (int q = 0; q < 16; q++) {   // vu entries
+                if (a[15 + q] == T(0)) continue;
+                u_parents_ij(i + q % 4 - 2, j + q / 4 - 1, Cg.ncz, PI, PJ, pw);
+                const T ra = R * a[15 + q];
+#pragma unroll
+                for (int s = 0; s < 4; s++)
+                    if (pw[s] != 0.0f && u_unknown(PI[s], PJ[s], Nxc, Nzc))
+                        add(15, PI[s] - K, PJ[s] - L, -2, 1, -1, 2, 4, ra * weight<T>(pw[s]));
             }
         }
     }
     __syncthreads();
-    if (t < nuc)
-        for (int q = sub; q < MG_NST; q += GAL_SPLIT) {
-            const T *c = acc_sh + q * GAL_THREADS + col0;
-            suC[(size_t)q * nuc + t] = (c[0] + c[1]) + (c[2] + c[3]);
-        }
-    __syncthreads();
-    if (t < nvc) {   // coarse v-row (I, J)
-        const int I = t % (Nxc + 1), J = t / (Nxc + 1);
-        for (int q = 0; q < MG_NST; q++) ACC(q) = T(0);
-        if (v_unknown(I, J, Nxc, Nzc)) {
-            for (int i = 2 * I - 2 + sub; i <= 2 * I - 2 + sub; i++) {
-                if (i < 1 || i > F.ncx) continue;
-                int I0, I1;
-                float w0, w1;
-                cc_weights(i, Cg.ncx, I0, w0, I1, w1);
-                const float wx = (I0 == I ? w0 : 0.0f) + (I1 == I && I1 != I0 ? w1 : 0.0f);
-                if (wx == 0.0f) continue;
-                for (int j = 2 * J - 1; j <= 2 * J + 1; j++) {
-                    if (!v_unknown(i, j, Nxf, Nzf)) continue;
-                    const size_t f = (size_t)i + (size_t)j * (Nxf + 1);
-                    const T R = (T)(wx * nc_weight(j, J));
+    T *out = ublock ? suC : svC, *id = ublock ? idu : idv;
+    for (int q = warp; q < MG_NST; q += GAL_WARPS) {
+        if (t >= n) continue;
+        const T *c = acc_sh + q * GAL_THREADS + lane;
+        T s = 0;
 #pragma unroll
-                    for (int q = 0; q < MG_NST; q++) a[q] = __ldg(svF + (size_t)q * nvf + f);
-#pragma unroll
-                    for (int q = 0; q < 15; q++) {   // vv entries
-                        if (a[q] == T(0)) continue;
-                        v_parents_ij(i + q % 5 - 2, j + q / 5 - 1, Cg.ncx, PI, PJ, pw);
-                        const T ra = R * a[q];
-#pragma unroll
-                        for (int s = 0; s < 4; s++) {
-                            if (pw[s] == 0.0f || !v_unknown(PI[s], PJ[s], Nxc, Nzc)) continue;
-                            const int dI = PI[s] - I, dJ = PJ[s] - J;
-                            if (dI < -2 || dI > 2 || dJ < -1 || dJ > 1) { *bad = 1; continue; }
-                            ACC((dI + 2) + 5 * (dJ + 1)) += ra * (T)pw[s];
-                        }
-                    }
-#pragma unroll
-                    for (int q = 0; q < 16; q++) {   // vu entries
-                        if (a[15 + q] == T(0)) continue;
-                        u_parents_ij(i + q % 4 - 2, j + q / 4 - 1, Cg.ncz, PI, PJ, pw);
-                        const T ra = R * a[15 + q];
-#pragma unroll
-                        for (int s = 0; s < 4; s++) {
-                            if (pw[s] == 0.0f || !u_unknown(PI[s], PJ[s], Nxc, Nzc)) continue;
-                            const int dK = PI[s] - I, dL = PJ[s] - J;
-                            if (dK < -2 || dK > 1 || dL < -1 || dL > 2) { *bad = 1; continue; }
-                            ACC(15 + (dK + 2) + 4 * (dL + 1)) += ra * (T)pw[s];
-                        }
-                    }
-                }
-            }
-        }
+        for (int e = 0; e < GAL_WARPS; e++) s += c[32 * e];
+        out[(size_t)q * n + t] = s;
+        if (q == MG_CENTER) id[t] = row ? T(1) / s : T(0);
     }
-    __syncthreads();
-    if (t < nvc)
-        for (int q = sub; q < MG_NST; q += GAL_SPLIT) {
-            const T *c = acc_sh + q * GAL_THREADS + col0;
-            svC[(size_t)q * nvc + t] = (c[0] + c[1]) + (c[2] + c[3]);
-        }
-#undef ACC
 }
 
 template <typename T>
@@ -731,27 +705,28 @@ __device__ __forceinline__ int dense_v(int Nx, int Nz, int i, int j) {
     return (i >= 1 && i <= Nx - 1 && j >= 1 && j <= Nz - 2) ? (Nx - 2) * (Nz - 1) + (i - 1) + (j - 1) * (Nx - 1) : -1;
 }
 
+// In the hierarchy's precision: the FP32 hierarchy's inverse is stored in FP32
+// and only corrects a V-cycle.  In place (the pivot column's slot takes the
+// inverse's), in shared memory where it fits (the launch passes the dynamic
+// size), else in the global work array; per step one warp finds the pivot and
+// its reciprocal, then the pivot row and column are copied, then every element
+// is updated: three barriers.  (Eliminating [A | I] with seven barriers and a
+// division per thread and step took 300 us in FP64 and 155 us in FP32 for the
+// 52 unknowns of 8 x 4 cells.)
 template <typename T>
 __global__ void __launch_bounds__(512) k_coarse_dense_setup(stokes_geom G, const T *__restrict__ su,
                                                             const T *__restrict__ sv, int n,
-                                                            const int *__restrict__ map, double *Ag,
+                                                            const int *__restrict__ map, T *Ag,
                                                             T *__restrict__ AinvT, int *status) {
-    // [A | I] in shared memory when it fits (the launch passes the dynamic
-    // size), else in the global work array: each of the n elimination steps
-    // reads and writes all of it between barriers
-    // in the hierarchy's precision: the FP32 hierarchy's inverse is stored in
-    // FP32 and only corrects a V-cycle; FP64 elimination runs at a small
-    // fraction of the FP32 rate on this part (one CTA: ~300 us per set-up)
-    extern __shared__ double dsm[];
-    T *A = (size_t)2 * n * n * sizeof(T) <= MG_DENSE_SMEM ? reinterpret_cast<T *>(dsm) : reinterpret_cast<T *>(Ag);
-    __shared__ T col[MG_DENSE_MAX];
-    __shared__ int bad;
-    const int Nx = G.Nx, Nz = G.Nz;
+    extern __shared__ __align__(16) unsigned char dsm[];
+    T *A = (size_t)n * n * sizeof(T) <= MG_DENSE_SMEM ? reinterpret_cast<T *>(dsm) : Ag;
+    __shared__ T prow[MG_DENSE_MAX], col[MG_DENSE_MAX], s_inv;
+    __shared__ int perm[MG_DENSE_MAX], s_pr;
+    const int Nx = G.Nx, Nz = G.Nz, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
     const size_t nu = (size_t)Nx * (Nz + 1), nv = (size_t)(Nx + 1) * Nz;
-    if (threadIdx.x == 0) bad = 0;
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) A[e] = T(0);
+    for (int e = tid; e < n * n; e += blockDim.x) A[e] = T(0);
     __syncthreads();
-    for (int r = threadIdx.x; r < n; r += blockDim.x) {
+    for (int r = tid; r < n; r += blockDim.x) {
         const int m = map[r];
         if (m < (int)nu) {
             const int k = m % Nx, l = m / Nx;
@@ -776,67 +751,61 @@ __global__ void __launch_bounds__(512) k_coarse_dense_setup(stokes_geom G, const
         }
     }
     __syncthreads();
-    // Gauss-Jordan on [A | I] with partial pivoting (the Newton block is
-    // neither symmetric nor definite); B ends as A^-1
-    T *B = A + (size_t)n * n;
-    __shared__ T red_v[32];
-    __shared__ int red_i[32];
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) B[e] = (e / n == e % n) ? T(1) : T(0);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    // Gauss-Jordan with partial pivoting (the Newton block is neither
+    // symmetric nor definite)
     for (int k = 0; k < n; k++) {
-        T bv = T(-1);
-        int bi = k;
-        for (int i = k + threadIdx.x; i < n; i += blockDim.x) {
-            const T v = fabs(A[(size_t)i * n + k]);
-            if (v > bv) { bv = v; bi = i; }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            const T ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-        }
-        if (lane == 0) { red_v[wid] = bv; red_i[wid] = bi; }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < nw; w++)
-                if (red_v[w] > red_v[0] || (red_v[w] == red_v[0] && red_i[w] < red_i[0])) {
-                    red_v[0] = red_v[w];
-                    red_i[0] = red_i[w];
-                }
-        }
-        __syncthreads();
-        const T pmax = red_v[0];
-        const int pr = red_i[0];
-        if (!(pmax > T(0)) || !isfinite(pmax)) { if (threadIdx.x == 0) bad = 1; break; }   // uniform
-        if (pr != k)
-            for (int j = threadIdx.x; j < n; j += blockDim.x) {
-                T t = A[(size_t)k * n + j]; A[(size_t)k * n + j] = A[(size_t)pr * n + j]; A[(size_t)pr * n + j] = t;
-                t = B[(size_t)k * n + j]; B[(size_t)k * n + j] = B[(size_t)pr * n + j]; B[(size_t)pr * n + j] = t;
+        if (wid == 0) {
+            T bv = T(-1);
+            int bi = k;
+            for (int i = k + lane; i < n; i += 32) {
+                const T v = fabs(A[(size_t)i * n + k]);
+                if (v > bv) { bv = v; bi = i; }
             }
-        __syncthreads();
-        const T inv = T(1) / A[(size_t)k * n + k];
-        __syncthreads();
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            A[(size_t)k * n + j] *= inv;
-            B[(size_t)k * n + j] *= inv;
+            for (int o = 16; o > 0; o >>= 1) {
+                const T ov = __shfl_xor_sync(0xffffffffu, bv, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+            }
+            if (lane == 0) {
+                const bool ok = bv > T(0) && isfinite(bv);
+                s_pr = ok ? bi : -1;
+                s_inv = ok ? T(1) / A[(size_t)bi * n + k] : T(0);
+            }
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) col[i] = A[(size_t)i * n + k];
+        const int pr = s_pr;
+        const T inv = s_inv;
+        if (pr < 0) {   // uniform
+            if (tid == 0) *status = 1;
+            return;
+        }
+        for (int j = tid; j < n; j += blockDim.x) {
+            const T ap = A[(size_t)pr * n + j], ak = A[(size_t)k * n + j];
+            prow[j] = j == k ? inv : ap * inv;
+            col[j] = j == pr ? A[(size_t)k * n + k] : A[(size_t)j * n + k];
+            if (j == 0) perm[k] = pr;
+            if (pr != k && j != k) A[(size_t)pr * n + j] = ak;   // (column k is rewritten below)
+        }
         __syncthreads();
-        for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-            const int i = e / n, j = e % n;
-            if (i == k) continue;
-            A[(size_t)i * n + j] -= col[i] * A[(size_t)k * n + j];
-            B[(size_t)i * n + j] -= col[i] * B[(size_t)k * n + j];
+        for (int i = wid; i < n; i += nw) {
+            const T c = col[i];
+            for (int j = lane; j < n; j += 32) {
+                T *a = A + (size_t)i * n + j;
+                *a = i == k ? prow[j] : (j == k ? T(0) : *a) - c * prow[j];
+            }
         }
         __syncthreads();
     }
+    // the row interchanges become column interchanges of the inverse, last first
+    int *src = reinterpret_cast<int *>(col);
+    for (int j = tid; j < n; j += blockDim.x) src[j] = j;
     __syncthreads();
-    if (bad) { if (threadIdx.x == 0) *status = 1; return; }
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        int i = e / n, j = e % n;
-        AinvT[(size_t)j * n + i] = (T)B[(size_t)i * n + j];
+    if (tid == 0)
+        for (int k = n - 1; k >= 0; k--) { const int t = src[k]; src[k] = src[perm[k]]; src[perm[k]] = t; }
+    __syncthreads();
+    for (int e = tid; e < n * n; e += blockDim.x) {
+        const int i = e / n, j = e % n;
+        AinvT[(size_t)j * n + i] = A[(size_t)i * n + src[j]];
     }
 }
 
@@ -1100,17 +1069,15 @@ static mdz_status build_hierarchy(mdz_ctx *ctx, mg_hier<T> &H) {
         // count is halved rounding up: the last coarse cell then covers one fine
         // cell, its far wall lies one fine cell outside the box, and the fine
         // points that would lie beyond the wall are not unknowns, so P and the
-        // Galerkin product keep their index arithmetic and footprint.  A level
-        // with an odd count that is small enough for the dense inverse stops
-        // there instead.  (k_mg_coarse_cg, the one-CTA conjugate gradients of a
-        // level too large for the inverse, took 2.2 ms of every FP64 V-cycle
-        // on the 25 x 25 cells a 401^2 box used to end in, against 0.2 ms for
-        // the levels that replace it: 101^2 defect solve 225 -> 16.2 ms, 401^2
-        // shear-band step 310 -> 104 ms.)
+        // Galerkin product keep their index arithmetic and footprint.
+        // (k_mg_coarse_cg, the one-CTA conjugate gradients of a coarsest level
+        // too large for the dense inverse, took 2.2 ms of every FP64 V-cycle on
+        // the 25 x 25 cells a 401^2 box used to end in, against 0.2 ms for the
+        // levels that replace it: 101^2 defect solve 225 -> 16.2 ms, 401^2
+        // shear-band step 310 -> 104 ms.  It is left for boxes some four times
+        // longer than high and more.)
         const int cx = (L.ncx + 1) / 2, cz = (L.ncz + 1) / 2;
-        const bool even = L.ncx % 2 == 0 && L.ncz % 2 == 0;
-        const long long unknowns = (long long)(L.Nx - 2) * (L.Nz - 1) + (long long)(L.Nx - 1) * (L.Nz - 2);
-        if (cx < 4 || cz < 4 || (!even && unknowns <= MG_DENSE_MAX)) break;
+        if (cx < 4 || cz < 4) break;
         Nx = cx + 1; Nz = cz + 1; dx *= 2; dz *= 2;
     }
     H.nlev = lev;
@@ -1126,7 +1093,7 @@ static mdz_status build_hierarchy(mdz_ctx *ctx, mg_hier<T> &H) {
         size_t n2 = (size_t)C.ndense * C.ndense;
         if (e == cudaSuccess) e = alloc0(&C.dmap, map.size());
         if (e == cudaSuccess) e = cudaMemcpy(C.dmap, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = alloc0(&C.Awork, 2 * n2);
+        if (e == cudaSuccess) e = alloc0(&C.Awork, n2);
         if (e == cudaSuccess) e = alloc0(&C.AinvT, n2);
     } else {
         for (int q = 0; q < 4; q++) {
@@ -1208,6 +1175,12 @@ mdz_status mdz_solver_ensure(mdz_ctx *ctx) {
     if ((s = alloc_gcr<float>(ctx, S->g32, S->restart)) != MDZ_OK) return s;
     MDZ_CUDA(ctx, cudaMallocHost((void **)&S->sc, 64 * sizeof(double)));
     memset(S->sc, 0, 64 * sizeof(double));
+#define MG_SMEM_ATTR(k, bytes) MDZ_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))
+    MG_SMEM_ATTR((k_galerkin<double, true>), sizeof(double) * MG_NST * GAL_THREADS);
+    MG_SMEM_ATTR((k_galerkin<double, false>), sizeof(double) * MG_NST * GAL_THREADS);
+    MG_SMEM_ATTR((k_galerkin<float, true>), sizeof(float) * MG_NST * GAL_THREADS);
+    MG_SMEM_ATTR((k_galerkin<float, false>), sizeof(float) * MG_NST * GAL_THREADS);
+#undef MG_SMEM_ATTR
     MDZ_CUDA(ctx, cudaFuncSetAttribute(k_mg_bottom<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_BOTTOM_SMEM));
     MDZ_CUDA(ctx, cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_BOTTOM_SMEM));
     MDZ_CUDA(ctx, cudaFuncSetAttribute(k_coarse_dense_setup<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1220,12 +1193,17 @@ mdz_status mdz_solver_ensure(mdz_ctx *ctx) {
 }
 
 template <typename T>
-static mdz_status copy_stencils(mdz_ctx *ctx, const mg_hier<T> &H, int level, int *Nx, int *Nz, double *su,
+static mdz_status copy_stencils(mdz_ctx *ctx, mg_hier<T> &H, int level, int *Nx, int *Nz, double *su,
                                 double *sv) {
     if (level < 0 || level >= H.nlev) return mdz_fail(ctx, MDZ_ERR_ARG, "mg_stencils: level %d of %d", level, H.nlev);
     const mg_level<T> &L = H.L[level];
     *Nx = L.Nx;
     *Nz = L.Nz;
+    if (level == 0 && H.viscous && (su || sv)) {   // the viscous level keeps no stencils of its own
+        k_picard_stencil<T><<<dim3((L.Nx + 32) / 32, (L.Nz + 8) / 8), dim3(32, 8), 0, ctx->stream>>>(
+            H.setup_geom, L.D11, L.D33, L.su, L.sv);
+        MDZ_LAUNCHED(ctx);
+    }
     MDZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const T *src[2] = {L.su, L.sv};
     double *dst[2] = {su, sv};
@@ -1334,6 +1312,8 @@ static mdz_status mg_setup(mdz_ctx *ctx, mg_hier<T> &H, const double *eta_n, con
     int nc = F.ncx * F.ncz, nv = F.Nx * F.Nz;
     H.newton = newton;
     H.built = true;
+    H.viscous = !newton;
+    H.setup_geom = F.geom();
     cudaEvent_t ev;
     mdz_prof_begin(ctx, MDZ_PROF_MG_SETUP, st, &ev);
     k_fill_D11_D33<T><<<mdz_blocks(nv > nc ? nv : nc), MDZ_THREADS, 0, st>>>(nc, nv, eta_n, eta_s, F.D11, F.D33);
@@ -1341,9 +1321,11 @@ static mdz_status mg_setup(mdz_ctx *ctx, mg_hier<T> &H, const double *eta_n, con
     // level-0 stencils: the Picard block written out from eta, or the Newton
     // Jacobian's velocity block probed with 2 x 16 colour classes
     const dim3 bl(32, 8), gr0((F.Nx + 1 + 31) / 32, (F.Nz + 1 + 7) / 8);
-    if (!newton) {
-        k_picard_stencil<T><<<gr0, bl, 0, st>>>(F.geom(), F.D11, F.D33, F.su, F.sv);
-        MDZ_LAUNCHED(ctx);
+    if (!newton) {   // (stored only where something reads them: mdz_mg_stencils writes them out on request)
+        if (H.nlev == 1) {
+            k_picard_stencil<T><<<gr0, bl, 0, st>>>(F.geom(), F.D11, F.D33, F.su, F.sv);
+            MDZ_LAUNCHED(ctx);
+        }
     } else {
     MDZ_CUDA(ctx, cudaMemsetAsync(F.su, 0, sizeof(T) * MG_NST * F.nu(), st));
     MDZ_CUDA(ctx, cudaMemsetAsync(F.sv, 0, sizeof(T) * MG_NST * F.nv(), st));
@@ -1369,25 +1351,28 @@ static mdz_status mg_setup(mdz_ctx *ctx, mg_hier<T> &H, const double *eta_n, con
     MDZ_CUDA(ctx, cudaMemsetAsync(status, 0, 2 * sizeof(int), st));
     for (int l = 1; l < H.nlev; l++) {
         mg_level<T> &P = H.L[l - 1], &L = H.L[l];
-        size_t n = L.nu() > L.nv() ? L.nu() : L.nv();
-        k_galerkin<T><<<mdz_blocks((long long)n * GAL_SPLIT, GAL_THREADS), GAL_THREADS, 0, st>>>(P.geom(), P.su, P.sv, L.geom(), L.su, L.sv, status + 1);
-        MDZ_LAUNCHED(ctx);
-        k_st_diag<T><<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(L.geom(), L.su, L.sv, L.idu, L.idv);
-        MDZ_LAUNCHED(ctx);
+        const int ub = (int)((L.nu() + 31) / 32), vb = (int)((L.nv() + 31) / 32);
+        const size_t smem = sizeof(T) * MG_NST * GAL_THREADS;
+        if (l == 1 && !newton)
+            MDZ_PDL(ctx, k_galerkin<T, true>, ub + vb, GAL_THREADS, smem, st, P.geom(), nullptr, nullptr, P.D11, P.D33,
+                    L.geom(), ub, L.su, L.sv, L.idu, L.idv, status + 1);
+        else
+            MDZ_PDL(ctx, k_galerkin<T, false>, ub + vb, GAL_THREADS, smem, st, P.geom(), P.su, P.sv, nullptr, nullptr,
+                    L.geom(), ub, L.su, L.sv, L.idu, L.idv, status + 1);
     }
     mg_level<T> &C = H.L[H.nlev - 1];
     if (C.ndense) {
-        const size_t smem = (size_t)2 * C.ndense * C.ndense * sizeof(T);
+        const size_t smem = (size_t)C.ndense * C.ndense * sizeof(T);
         k_coarse_dense_setup<T><<<1, 512, smem <= MG_DENSE_SMEM ? smem : 0, st>>>(C.geom(), C.su, C.sv, C.ndense,
                                                                               C.dmap, C.Awork, C.AinvT, status);
         MDZ_LAUNCHED(ctx);
     }
-    {   // algorithmic bytes: viscosities in, D11 / D33 out; level-0 stencils
-        // written once; each Galerkin level reads the finer stencils once and
+    {   // algorithmic bytes: viscosities in, D11 / D33 out; each Galerkin level
+        // reads the finer stencils (the first one the viscosities) once and
         // writes its own plus the inverse diagonal
-        double b = 8.0 * (nc + nv) + sizeof(T) * (nc + nv) + sizeof(T) * MG_NST * (double)(F.nu() + F.nv());
+        double b = 8.0 * (nc + nv) + 2.0 * sizeof(T) * (nc + nv);
         for (int l = 1; l < H.nlev; l++)
-            b += sizeof(T) * (MG_NST * (double)(H.L[l - 1].nu() + H.L[l - 1].nv()) +
+            b += sizeof(T) * ((l > 1 || newton ? MG_NST : 0.0) * (double)(H.L[l - 1].nu() + H.L[l - 1].nv()) +
                               (MG_NST + 1.0) * (double)(H.L[l].nu() + H.L[l].nv()));
         mdz_prof_end(ctx, MDZ_PROF_MG_SETUP, b, st, ev);
     }
