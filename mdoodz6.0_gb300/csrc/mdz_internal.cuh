@@ -92,6 +92,7 @@ struct mdz_ctx {
     double *red_part = nullptr;
     unsigned int *red_cnt = nullptr;
     bool bcs_checked = false, bcs_ok = false, bcs_neumann = false;
+    bool bcs_box = false;        // tags are the free-slip Dirichlet box (box_tags in stokes.cu)
     // optional per-launch event timing of the main kernel classes (bench roofline)
     bool profiling = false;
     struct prof_rec { int cls; cudaEvent_t a, b; double bytes; };

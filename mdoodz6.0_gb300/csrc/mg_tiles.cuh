@@ -314,48 +314,127 @@ __global__ void __launch_bounds__(2 * TW * TH) k_st_prolong_smooth(
 
 // ---- level 0 of a Picard hierarchy (viscosities read directly) ---------------
 // Picard momentum rows of the free-slip box that every hierarchy starts from
-// (checked before it is built), without reading tags: xrow / zrow with all
-// centroids active and the shear stress dropped on the free-slip walls.
-template <typename T, typename RS>
-__device__ __forceinline__ T picard_urow(const stokes_geom &G, const stokes_coefs<T> &D, int k, int l, const RS &rs) {
+// (checked before it is built; no tags are read).  A block first forms the
+// stresses its rows difference, once per centroid and vertex, into shared
+// memory, with the cell volume and the grid spacings folded into their
+// constants:
+//   sx = D11 (2/3 du/dx - 1/3 dw/dz) dz      sz = D11 (2/3 dw/dz - 1/3 du/dx) dx
+//   g  = D33 (du/dz + dw/dx) dx              (0 on the walls: free slip)
+//   A u = (sx_W - sx_E) + (g_S - g_N)        A w = (sz_S - sz_N) + (dz / dx) (g_W - g_E)
+// In FP64 these kernels are bound by the FP64 pipe (80 % active): evaluated
+// row by row (picard_urow / picard_vrow) a point cost 60 FP64 instructions, from
+// the tile about 27; 401^2 sweep 24 -> 15 us, residual + restriction 34 -> 19,
+// prolongation + sweep 29 -> 20.  FP32 has the instructions to spare and no use
+// for the extra barrier (one V-cycle at 1025 x 513: 109 us row by row, 118 from
+// the tile), so it evaluates row by row.
+template <typename T>
+constexpr bool mg_stress_tile() { return sizeof(T) == 8; }
+
+// rates of an accessor X.u(k, l), X.v(k, l)
+template <typename T, typename VEL>
+struct rates_of {
+    VEL X;
+    T idx, idz;
+    __device__ __forceinline__ pair2<T> exx(int kc, int lc) const {
+        const T dudx = (X.u(kc + 1, lc + 1) - X.u(kc, lc + 1)) * idx, dvdz = (X.v(kc + 1, lc + 1) - X.v(kc + 1, lc)) * idz;
+        const T div = dudx + dvdz;
+        return pair2<T>{dudx - div * T(1.0 / 3.0), dvdz - div * T(1.0 / 3.0)};
+    }
+    __device__ __forceinline__ T gxz(int kv, int lv) const {
+        return (X.u(kv, lv + 1) - X.u(kv, lv)) * idz + (X.v(kv + 1, lv) - X.v(kv, lv)) * idx;
+    }
+};
+template <typename T, typename VEL>
+__device__ __forceinline__ T picard_urow(const stokes_geom &G, const stokes_coefs<T> &D, int k, int l, const VEL &X) {
+    const rates_of<T, VEL> rs{X, gc<T>(G, GC_IDX), gc<T>(G, GC_IDZ)};
     const int nx = G.Nx, c1 = k + l * nx, c2 = k - 1 + (l - 1) * G.ncx;
     const T TxxE = D.D11[c2 + 1] * rs.exx(k, l - 1).x, TxxW = D.D11[c2] * rs.exx(k - 1, l - 1).x;
     const T TxzN = l < G.Nz - 1 ? D.D33[c1] * rs.gxz(k, l) : T(0), TxzS = l > 1 ? D.D33[c1 - nx] * rs.gxz(k, l - 1) : T(0);
-    return -(TxxE - TxxW) * gc<T>(G, GC_IDX) - (TxzN - TxzS) * gc<T>(G, GC_IDZ);
+    return (-(TxxE - TxxW) * rs.idx - (TxzN - TxzS) * rs.idz) * gc<T>(G, GC_CELVOL);
 }
-template <typename T, typename RS>
-__device__ __forceinline__ T picard_vrow(const stokes_geom &G, const stokes_coefs<T> &D, int k, int l, const RS &rs) {
+template <typename T, typename VEL>
+__device__ __forceinline__ T picard_vrow(const stokes_geom &G, const stokes_coefs<T> &D, int k, int l, const VEL &X) {
+    const rates_of<T, VEL> rs{X, gc<T>(G, GC_IDX), gc<T>(G, GC_IDZ)};
     const int c1 = k + l * G.Nx, c2 = k - 1 + (l - 1) * G.ncx;
     const T TzzN = D.D22[c2 + G.ncx] * rs.exx(k - 1, l).y, TzzS = D.D22[c2] * rs.exx(k - 1, l - 1).y;
     const T TxzE = k < G.Nx - 1 ? D.D33[c1] * rs.gxz(k, l) : T(0), TxzW = k > 1 ? D.D33[c1 - 1] * rs.gxz(k - 1, l) : T(0);
-    return -(TzzN - TzzS) * gc<T>(G, GC_IDZ) - (TxzE - TxzW) * gc<T>(G, GC_IDX);
+    return (-(TzzN - TzzS) * rs.idz - (TxzE - TxzW) * rs.idx) * gc<T>(G, GC_CELVOL);
 }
 
-// out = x + omega * D^-1 (f - A x)  (x == nullptr: x = 0)
+template <typename T, int W, int H>
+struct visc_tile {
+    T sx[H][W], sz[H][W], g[H][W];   // centroids and vertices from (x0, z0)
+    // X: X.u(k, l), X.v(k, l) at nodes inside the box
+    template <typename VEL>
+    __device__ __forceinline__ void fill(const stokes_geom &G, const stokes_coefs<T> &D, const VEL &X, int x0, int z0,
+                                         int tid, int nt) {
+        const T dx = gc<T>(G, GC_DX), dz = gc<T>(G, GC_DZ), idx = gc<T>(G, GC_IDX), idz = gc<T>(G, GC_IDZ);
+        const T third = T(1.0 / 3.0), xx = T(2) * third * (dz * idx), xz = third, zz = T(2) * third * (dx * idz),
+                gx = dx * idz;
+        for (int t = tid; t < W * H; t += nt) {
+            const int a = t % W, b = t / W, k = x0 + a, l = z0 + b;
+            T vx = 0, vz = 0, vg = 0;
+            if (k >= 0 && k < G.ncx && l >= 0 && l < G.ncz) {
+                const T du = X.u(k + 1, l + 1) - X.u(k, l + 1), dv = X.v(k + 1, l + 1) - X.v(k + 1, l);
+                const T d = D.D11[k + l * G.ncx];
+                vx = d * (xx * du - xz * dv);
+                vz = d * (zz * dv - xz * du);
+            }
+            if (k >= 1 && k <= G.Nx - 2 && l >= 1 && l <= G.Nz - 2)
+                vg = D.D33[k + l * G.Nx] * (gx * (X.u(k, l + 1) - X.u(k, l)) + (X.v(k + 1, l) - X.v(k, l)));
+            sx[b][a] = vx;
+            sz[b][a] = vz;
+            g[b][a] = vg;
+        }
+    }
+    // rows at point (k, l) = tile position (a, b): centroid (k - 1, l - 1) is (a - 1, b - 1)
+    __device__ __forceinline__ T urow(int a, int b) const {
+        return (sx[b - 1][a - 1] - sx[b - 1][a]) + (g[b - 1][a] - g[b][a]);
+    }
+    __device__ __forceinline__ T vrow(int a, int b, T ratio) const {
+        return (sz[b - 1][a - 1] - sz[b][a - 1]) + ratio * (g[b][a - 1] - g[b][a]);
+    }
+};
+
+template <typename T>
+struct vel_global {
+    const T *xu, *xv;
+    int Nx;
+    __device__ __forceinline__ T u(int k, int l) const { return xu[k + l * Nx]; }
+    __device__ __forceinline__ T v(int i, int j) const { return xv[i + j * (Nx + 1)]; }
+};
+
+// out = x + omega * D^-1 (f - A x)  (x == nullptr: x = 0), 32 x 8 points per block
 template <typename T>
 __global__ void __launch_bounds__(256) k_mg_smooth(stokes_geom G, stokes_coefs<T> D, const T *__restrict__ xu,
                                                    const T *__restrict__ xv, const T *__restrict__ fu,
                                                    const T *__restrict__ fv, const T *__restrict__ idu,
                                                    const T *__restrict__ idv, T omega, T *__restrict__ ou,
                                                    T *__restrict__ ov) {
+    constexpr bool TILE = mg_stress_tile<T>();
+    __shared__ visc_tile<T, TILE ? 33 : 1, TILE ? 9 : 1> S;
     mg_release<T>();
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int Nx = G.Nx, Nz = G.Nz;
-    const T celvol = gc<T>(G, GC_CELVOL);
-    const rates_direct<T> rs{xu, xv, Nx, Nx + 1, gc<T>(G, GC_IDX), gc<T>(G, GC_IDZ)};
+    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 8, a = threadIdx.x & 31, b = threadIdx.x >> 5;
+    const int i = i0 + a, j = j0 + b, Nx = G.Nx, Nz = G.Nz;
+    const vel_global<T> X{xu, xv, Nx};
+    if (TILE && xu) {
+        S.fill(G, D, X, i0 - 1, j0 - 1, threadIdx.x, 256);
+        __syncthreads();
+    }
+    const T ratio = gc<T>(G, GC_DZ) * gc<T>(G, GC_IDX);
+    auto au = [&]() { if constexpr (TILE) return S.urow(a + 1, b + 1); else return picard_urow<T>(G, D, i, j, X); };
+    auto av = [&]() { if constexpr (TILE) return S.vrow(a + 1, b + 1, ratio); else return picard_vrow<T>(G, D, i, j, X); };
     if (i < Nx && j <= Nz) {
         const int c = i + j * Nx;
         T r = 0;
-        if (u_unknown(i, j, Nx, Nz))
-            r = xu ? xu[c] + omega * idu[c] * (fu[c] - picard_urow<T>(G, D, i, j, rs) * celvol) : omega * idu[c] * fu[c];
+        if (u_unknown(i, j, Nx, Nz)) r = xu ? xu[c] + omega * idu[c] * (fu[c] - au()) : omega * idu[c] * fu[c];
         ou[c] = r;
     }
     if (i <= Nx && j < Nz) {
         const int c = i + j * (Nx + 1);
         T r = 0;
-        if (v_unknown(i, j, Nx, Nz))
-            r = xv ? xv[c] + omega * idv[c] * (fv[c] - picard_vrow<T>(G, D, i, j, rs) * celvol) : omega * idv[c] * fv[c];
+        if (v_unknown(i, j, Nx, Nz)) r = xv ? xv[c] + omega * idv[c] * (fv[c] - av()) : omega * idv[c] * fv[c];
         ov[c] = r;
     }
 }
@@ -369,20 +448,32 @@ __global__ void __launch_bounds__(NT) k_mg_resid_restrict(stokes_geom F, stokes_
                                                           T omega, T *__restrict__ cxu, T *__restrict__ cxv) {
     constexpr int UW = 2 * TX + 1, UH = 2 * TY + 2, VW = 2 * TX + 2, VH = 2 * TY + 1;
     __shared__ T ru[UH][UW], rv[VH][VW];
+    constexpr bool TILE = mg_stress_tile<T>();
+    __shared__ visc_tile<T, TILE ? 2 * TX + 3 : 1, TILE ? 2 * TY + 3 : 1> S;   // from (2 I0 - 3, 2 J0 - 3)
     const int Nx = F.Nx, Nz = F.Nz, I0 = blockIdx.x * TX, J0 = blockIdx.y * TY;
-    const T celvol = gc<T>(F, GC_CELVOL);
-    const rates_direct<T> rs{xu, xv, Nx, Nx + 1, gc<T>(F, GC_IDX), gc<T>(F, GC_IDZ)};
     mg_release<T>();
     pdl_wait();
+    const vel_global<T> X{xu, xv, Nx};
+    if constexpr (TILE) {
+        S.fill(F, D, X, 2 * I0 - 3, 2 * J0 - 3, threadIdx.x, NT);
+        __syncthreads();
+    }
+    const T ratio = gc<T>(F, GC_DZ) * gc<T>(F, GC_IDX);
     for (int t = threadIdx.x; t < UW * UH + VW * VH; t += NT) {
         T r = 0;
         if (t < UW * UH) {
             const int a = t % UW, b = t / UW, k = 2 * I0 - 1 + a, l = 2 * J0 - 2 + b;
-            if (u_unknown(k, l, Nx, Nz)) r = fu[k + l * Nx] - picard_urow<T>(F, D, k, l, rs) * celvol;
+            if (u_unknown(k, l, Nx, Nz)) {
+                if constexpr (TILE) r = fu[k + l * Nx] - S.urow(a + 2, b + 1);
+                else r = fu[k + l * Nx] - picard_urow<T>(F, D, k, l, X);
+            }
             ru[b][a] = r;
         } else {
             const int q = t - UW * UH, a = q % VW, b = q / VW, i = 2 * I0 - 2 + a, j = 2 * J0 - 1 + b;
-            if (v_unknown(i, j, Nx, Nz)) r = fv[i + j * (Nx + 1)] - picard_vrow<T>(F, D, i, j, rs) * celvol;
+            if (v_unknown(i, j, Nx, Nz)) {
+                if constexpr (TILE) r = fv[i + j * (Nx + 1)] - S.vrow(a + 1, b + 2, ratio);
+                else r = fv[i + j * (Nx + 1)] - picard_vrow<T>(F, D, i, j, X);
+            }
             rv[b][a] = r;
         }
     }
@@ -390,22 +481,13 @@ __global__ void __launch_bounds__(NT) k_mg_resid_restrict(stokes_geom F, stokes_
     restrict_tile<T, TX, TY>(Cg, ru, rv, I0, J0, cu, cv, cidu, cidv, omega, cxu, cxv);
 }
 
-// strain rates from a tile of velocities that starts at node (i0, j0) of both components
+// velocities of a tile in shared memory that starts at node (i0, j0) of both components
 template <typename T, int W>
-struct rates_xtile {
+struct vel_tile {
     const T (*pu)[W], (*pv)[W];
     int i0, j0;
-    T idx, idz;
     __device__ __forceinline__ T u(int k, int l) const { return pu[l - j0][k - i0]; }
     __device__ __forceinline__ T v(int k, int l) const { return pv[l - j0][k - i0]; }
-    __device__ __forceinline__ pair2<T> exx(int kc, int lc) const {
-        const T dudx = (u(kc + 1, lc + 1) - u(kc, lc + 1)) * idx, dvdz = (v(kc + 1, lc + 1) - v(kc + 1, lc)) * idz;
-        const T div = dudx + dvdz;
-        return pair2<T>{dudx - div * T(1.0 / 3.0), dvdz - div * T(1.0 / 3.0)};
-    }
-    __device__ __forceinline__ T gxz(int kv, int lv) const {
-        return (u(kv, lv + 1) - u(kv, lv)) * idz + (v(kv + 1, lv) - v(kv, lv)) * idx;
-    }
 };
 
 template <typename T, int TW, int TH>
@@ -415,7 +497,9 @@ __global__ void __launch_bounds__(TW *TH) k_mg_prolong_smooth(
     const T *__restrict__ idu, const T *__restrict__ idv, T omega, T *__restrict__ ou, T *__restrict__ ov,
     T *__restrict__ zp, const double *__restrict__ pmean) {
     constexpr int W = TW + 2, H = TH + 2;
+    constexpr bool TILE = mg_stress_tile<T>();
     __shared__ T pu[H][W], pv[H][W];
+    __shared__ visc_tile<T, TILE ? TW + 1 : 1, TILE ? TH + 1 : 1> S;
     mg_release<T>();
     pdl_wait();
     const int Nx = F.Nx, Nz = F.Nz, i0 = blockIdx.x * TW, j0 = blockIdx.y * TH;
@@ -425,25 +509,25 @@ __global__ void __launch_bounds__(TW *TH) k_mg_prolong_smooth(
         pv[b][a] = prolonged_v<T>(F, Cg, cv, xv, i0 - 1 + a, j0 - 1 + b);
     }
     __syncthreads();
-    const int li = threadIdx.x % TW, lj = threadIdx.x / TW, i = i0 + li, j = j0 + lj;
-    const T celvol = gc<T>(F, GC_CELVOL);
-    const rates_xtile<T, W> rs{pu, pv, i0 - 1, j0 - 1, gc<T>(F, GC_IDX), gc<T>(F, GC_IDZ)};
+    const vel_tile<T, W> X{pu, pv, i0 - 1, j0 - 1};
+    if constexpr (TILE) {
+        S.fill(F, D, X, i0 - 1, j0 - 1, threadIdx.x, TW * TH);
+        __syncthreads();
+    }
+    const int a = threadIdx.x % TW, b = threadIdx.x / TW, i = i0 + a, j = j0 + b;
+    const T ratio = gc<T>(F, GC_DZ) * gc<T>(F, GC_IDX);
+    auto au = [&]() { if constexpr (TILE) return S.urow(a + 1, b + 1); else return picard_urow<T>(F, D, i, j, X); };
+    auto av = [&]() { if constexpr (TILE) return S.vrow(a + 1, b + 1, ratio); else return picard_vrow<T>(F, D, i, j, X); };
     if (i < Nx && j <= Nz) {
         const int c = i + j * Nx;
         T r = 0;
-        if (u_unknown(i, j, Nx, Nz)) {
-            const T ax = picard_urow<T>(F, D, i, j, rs) * celvol;
-            r = pu[lj + 1][li + 1] + omega * idu[c] * (fu[c] - ax);
-        }
+        if (u_unknown(i, j, Nx, Nz)) r = pu[b + 1][a + 1] + omega * idu[c] * (fu[c] - au());
         ou[c] = r;
     }
     if (i <= Nx && j < Nz) {
         const int c = i + j * (Nx + 1);
         T r = 0;
-        if (v_unknown(i, j, Nx, Nz)) {
-            const T ax = picard_vrow<T>(F, D, i, j, rs) * celvol;
-            r = pv[lj + 1][li + 1] + omega * idv[c] * (fv[c] - ax);
-        }
+        if (v_unknown(i, j, Nx, Nz)) r = pv[b + 1][a + 1] + omega * idv[c] * (fv[c] - av());
         ov[c] = r;
     }
     if (zp && i < F.ncx && j < F.ncz) zp[i + j * F.ncx] -= (T)pmean[2];   // as k_pmean_out

@@ -140,25 +140,6 @@ __global__ void k_level_tags(int Nx, int Nz, signed char *BCu, signed char *BCv,
     if (i < ng) BCg[i] = -1;
 }
 
-static bool fine_tags_follow_rule(const mdz_grid_desc &d) {
-    int Nx = d.Nx, Nz = d.Nz;
-    for (int l = 0; l <= Nz; l++)
-        for (int k = 0; k < Nx; k++) {
-            signed char t = -1;
-            if (k == 0 || k == Nx - 1) t = 0;
-            if (l == 0 || l == Nz) t = 13;
-            if (d.BCu_type[k + l * Nx] != t) return false;
-        }
-    for (int l = 0; l < Nz; l++)
-        for (int k = 0; k <= Nx; k++) {
-            signed char t = -1;
-            if (l == 0 || l == Nz - 1) t = 0;
-            if (k == 0 || k == Nx) t = 13;
-            if (d.BCv_type[k + l * (Nx + 1)] != t) return false;
-        }
-    return true;
-}
-
 // ---------------------------------------------------------------------------
 // Multigrid kernels (velocity block, Picard, homogeneous boundaries).
 template <typename T>
@@ -1165,7 +1146,7 @@ mdz_status mdz_solver_ensure(mdz_ctx *ctx) {
     if (ctx->solver && ctx->solver->ready) return MDZ_OK;
     mdz_status s = mdz_check_stokes_bcs(ctx);
     if (s != MDZ_OK) return s;
-    if (!fine_tags_follow_rule(ctx->host_desc))
+    if (!ctx->bcs_box)
         return mdz_fail(ctx, MDZ_ERR_UNSUPPORTED, "solver: boundary tags must be the free-slip box pattern");
     if (!ctx->solver) ctx->solver = new mdz_solver();
     mdz_solver *S = ctx->solver;
@@ -1393,12 +1374,16 @@ static size_t mg_bottom_bytes(const mg_hier<T> &H, int l) {
 }
 
 // Whether vcycle() runs level l and all below it in the one-launch bottom
-// kernel: as soon as their data fit in one CTA's shared memory.
+// kernel: as soon as their data fit in one CTA's shared memory and, in FP64,
+// the level has at most 256 rows (more are too much for one SM's FP64 units:
+// 312 rows took 37 us, as grid kernels some 22).
 template <typename T>
 static bool vcycle_bottom(const mg_hier<T> &H, int l) {
+    const mg_level<T> &L = H.L[l];
     const bool viscous = l == 0 && !H.newton;   // level 0 of a Picard hierarchy: stencil from eta directly
     return !viscous && l < H.nlev - 1 && H.L[H.nlev - 1].ndense && H.nlev - l <= MG_BOTTOM_MAX &&
-           mg_bottom_bytes<T>(H, l) <= MG_BOTTOM_SMEM;
+           mg_bottom_bytes<T>(H, l) <= MG_BOTTOM_SMEM &&
+           (sizeof(T) == 4 || mg_bottom_rows_u(L.Nx, L.Nz) + mg_bottom_rows_v(L.Nx, L.Nz) <= 256);
 }
 
 // Whether vcycle() smooths level l with its own sweeps (not the dense
@@ -1453,7 +1438,7 @@ static mdz_status vcycle(mdz_ctx *ctx, mg_hier<T> &H, int l, int nu1, int nu2, T
     }
     const int rows_grid = mdz_blocks(L.nu() + L.nv(), ST_THREADS);
     auto smooth = [&](const T *xu, const T *xv, T *ou, T *ov) -> mdz_status {
-        if (viscous) MDZ_PDL(ctx, k_mg_smooth<T>, gr, bl, 0, st, G, D, xu, xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
+        if (viscous) MDZ_PDL(ctx, k_mg_smooth<T>, gr, 256, 0, st, G, D, xu, xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
         else MDZ_PDL(ctx, k_st_smooth<T>, rows_grid, ST_THREADS, 0, st, G, L.su, L.sv, xu, xv, L.fu, L.fv, L.idu, L.idv,
                      omega, ou, ov);
         return MDZ_OK;
@@ -1534,8 +1519,7 @@ __global__ void k_psub(int np, const signed char *__restrict__ tp, const double 
 // Block preconditioner: zp = (eta_n / celvol) rp ; zu = V-cycle(ru - B zp).
 // One launch writes zp (eta_n / celvol from the level-0 copy D11 = 2 eta_n in
 // precision T, or from the Jacobian's tangent D11 where that is positive),
-// f = r_vel - B zp on the fine level (B: celvol-scaled pressure gradient; the
-// rows form the two zp they need again), with xu non-null the V-cycle's first
+// f = r_vel - B zp on the fine level (B: celvol-scaled pressure gradient), with xu non-null the V-cycle's first
 // sweep from x = 0, x = omega D^-1 f, and the sum, count and mean of zp over the
 // pressure equations for the zero-mean projection in the last launch.
 template <typename T>
@@ -1547,27 +1531,34 @@ __global__ void __launch_bounds__(256) k_precond(stokes_geom G, const T *__restr
                                                  T *__restrict__ xv, double *part, unsigned int *counter,
                                                  double *psum) {
     mg_release<T>();
-    const int Nx = G.Nx, Nz = G.Nz, ncx = G.ncx, ncz = G.ncz;
+    __shared__ T s_z[9][33];   // zp of the centroids (i0 - 1 .. i0 + 31, j0 - 1 .. j0 + 7)
+    const int Nx = G.Nx, Nz = G.Nz, ncx = G.ncx, ncz = G.ncz, a = threadIdx.x & 31, h = threadIdx.x >> 5;
     const int ntx = (Nx + 32) / 32, ntiles = ntx * ((Nz + 8) / 8);
     const T half_ivol = T(0.5) * gc<T>(G, GC_IXZ);
-    auto z = [&](int c) {
-        T d = D11[c];
-        if (Dt) {
-            const T t = Dt[c];
-            if (t > T(0)) d = t;
-        }
-        return half_ivol * d * rp[c];
-    };
     T acc = 0;
     int cnt = 0;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int i = (tile % ntx) * 32 + (threadIdx.x & 31), j = (tile / ntx) * 8 + (threadIdx.x >> 5);
-        const int c2 = i - 1 + (j - 1) * ncx;
+        const int i0 = (tile % ntx) * 32, j0 = (tile / ntx) * 8, i = i0 + a, j = j0 + h;
+        for (int t = threadIdx.x; t < 33 * 9; t += 256) {
+            const int k = i0 - 1 + t % 33, l = j0 - 1 + t / 33;
+            T v = 0;
+            if (k >= 0 && k < ncx && l >= 0 && l < ncz) {
+                const int c = k + l * ncx;
+                T d = D11[c];
+                if (Dt) {   // the Jacobian's tangent D11 where it is positive
+                    const T dt = Dt[c];
+                    if (dt > T(0)) d = dt;
+                }
+                v = half_ivol * d * rp[c];
+            }
+            s_z[t / 33][t % 33] = v;
+        }
+        __syncthreads();
         if (i < Nx && j <= Nz) {
             const int c = i + j * Nx;
             T r = 0, x0 = 0;
             if (u_unknown(i, j, Nx, Nz)) {
-                r = ru[c] - gc<T>(G, GC_DZ) * (z(c2 + 1) - z(c2));
+                r = ru[c] - gc<T>(G, GC_DZ) * (s_z[h][a + 1] - s_z[h][a]);
                 if (xu) x0 = omega * idu[c] * r;
             }
             fu[c] = r;
@@ -1577,18 +1568,19 @@ __global__ void __launch_bounds__(256) k_precond(stokes_geom G, const T *__restr
             const int c = i + j * (Nx + 1);
             T r = 0, x0 = 0;
             if (v_unknown(i, j, Nx, Nz)) {
-                r = rv[c] - gc<T>(G, GC_DX) * (z(c2 + ncx) - z(c2));
+                r = rv[c] - gc<T>(G, GC_DX) * (s_z[h + 1][a] - s_z[h][a]);
                 if (xv) x0 = omega * idv[c] * r;
             }
             fv[c] = r;
             if (xv) xv[c] = x0;
         }
         if (i < ncx && j < ncz) {
-            const T v = z(i + j * ncx);
+            const T v = s_z[h + 1][a + 1];
             zp[i + j * ncx] = v;
             acc += v;
             cnt++;
         }
+        __syncthreads();
     }
     const T v[2] = {acc, (T)cnt};   // (counts per thread are small integers: exact in T)
     if (mdz_grid_sum<2, T>(v, part, counter, psum)) {
@@ -2087,7 +2079,7 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
         mdz_prof_end(ctx, MDZ_PROF_MG_SMOOTH, SV->pre_bytes[pslot], st, ev);
         mdz_prof_begin(ctx, MDZ_PROF_STOKES_APPLY, st, &ev);
         stokes_apply_launch<P>(G, K, stokes_cvec<P>{SP.z, SP.z + nu, SP.z + nu + nv},
-                               stokes_vec<P>{SP.w, SP.w + nu, SP.w + nu + nv}, nullptr, newton, st);
+                               stokes_vec<P>{SP.w, SP.w + nu, SP.w + nu + nv}, nullptr, newton, true, st);
         MDZ_LAUNCHED(ctx);
         {   // algorithmic bytes: input and output vectors, the D-tensor read once, tags
             size_t nc = S.np, ng = (size_t)G.Nx * G.Nz;
@@ -2194,7 +2186,7 @@ mdz_status mdz_dev_solve(mdz_ctx *ctx, const mdz_fields &f, bool newton, int pre
         double r0 = -1.0, prev = 1e300;
         auto defect = [&]() -> mdz_status {   // r64 = F - K64 dx
             stokes_apply_launch<double>(G, K64, stokes_cvec<double>{dx, dx + nu, dx + nu + nv},
-                                        stokes_vec<double>{S64.t, S64.t + nu, S64.t + nu + nv}, nullptr, newton, st);
+                                        stokes_vec<double>{S64.t, S64.t + nu, S64.t + nu + nv}, nullptr, newton, true, st);
             MDZ_LAUNCHED(ctx);
             MDZ_CUDA(ctx, cudaMemcpyAsync(S64.r, F, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
             k_axpby<double><<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, -1.0, S64.t, 1.0, S64.r);

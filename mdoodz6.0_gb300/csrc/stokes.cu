@@ -70,29 +70,161 @@ __global__ void __launch_bounds__(256) k_stokes_apply(stokes_geom G, stokes_coef
     }
 }
 
+// The same on the free-slip Dirichlet box (box: no Neumann rows, every centroid
+// active), where the row flags of xrow / zrow differ from all-ones only beside
+// the walls.  The block forms, once per node of its 32 x 8 tile and halo, the
+// strain rates (as k_stokes_apply), then the tangent stresses from them
+// (normal stresses per centroid with the four-vertex mean of the shear rate,
+// shear stress per vertex with the four-centroid means of rates and pressure,
+// zero on the walls), and a row is two stress differences and the pressure
+// gradient; the cell volume is folded into the spacings.  A row next to a
+// free-slip wall drops the wall vertex on its own line from the mean of its
+// two centroids (weight 1/3 on the other three, as the reference's
+// coefficients have it): those rows correct their stresses by D13 (D23) times
+// the difference of the means.
+// The FP64 Newton apply is bound by the FP64 pipe: row by row it took 200 FP64
+// instructions a point, here about 60: 401^2 77 -> 31 us, 1025 x 513 203 -> 82 us;
+// FP32 1025 x 513 25 -> 16 us.
+constexpr int SB_W = 33, SB_H = 9;   // stresses: centroids and vertices from (i0 - 1, j0 - 1)
+template <typename T, bool NEWTON, bool RES>
+__global__ void __launch_bounds__(256) k_stokes_apply_box(stokes_geom G, stokes_coefs<T> D, stokes_cvec<T> x,
+                                                          stokes_vec<T> y, stokes_cvec<T> b) {
+    __shared__ T s_ex[RT_H][RT_W], s_ez[RT_H][RT_W], s_g[RT_H][RT_W], s_p[NEWTON ? RT_H : 1][RT_W];
+    __shared__ T s_xx[SB_H][SB_W], s_zz[SB_H][SB_W], s_xz[SB_H][SB_W];
+    const int Nx = G.Nx, Nz = G.Nz, ncx = G.ncx, ncz = G.ncz, nxvz = Nx + 1;
+    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 8, tid = threadIdx.x;
+    const T idx = gc<T>(G, GC_IDX), idz = gc<T>(G, GC_IDZ), dx = gc<T>(G, GC_DX), dz = gc<T>(G, GC_DZ);
+    const T third = T(1.0 / 3.0);
+    // rates at centroids from (i0 - 2, j0 - 2) and vertices from (i0 - 1, j0 - 1)
+    for (int t = tid; t < RT_W * RT_H; t += 256) {
+        const int a = t % RT_W, h = t / RT_W;
+        const int kc = i0 - 2 + a, lc = j0 - 2 + h, kv = kc + 1, lv = lc + 1;
+        T ex = 0, ez = 0, g = 0, pc = 0;
+        if (kc >= 0 && kc < ncx && lc >= 0 && lc < ncz) {
+            const int cu = kc + (lc + 1) * Nx, cv = kc + 1 + lc * nxvz;
+            const T dudx = (x.u[cu + 1] - x.u[cu]) * idx, dvdz = (x.v[cv + nxvz] - x.v[cv]) * idz;
+            const T div = (dudx + dvdz) * third;
+            ex = dudx - div;
+            ez = dvdz - div;
+            if (NEWTON) pc = x.p[kc + lc * ncx];
+        }
+        if (kv >= 0 && kv < Nx && lv >= 0 && lv < Nz) {
+            const int cu = kv + lv * Nx, cv = kv + lv * nxvz;
+            g = (x.u[cu + Nx] - x.u[cu]) * idz + (x.v[cv + 1] - x.v[cv]) * idx;
+        }
+        s_ex[h][a] = ex;
+        s_ez[h][a] = ez;
+        s_g[h][a] = g;
+        if (NEWTON) s_p[h][a] = pc;
+    }
+    __syncthreads();
+    for (int t = tid; t < SB_W * SB_H; t += 256) {
+        const int a = t % SB_W, h = t / SB_W, k = i0 - 1 + a, l = j0 - 1 + h;
+        T xx = 0, zz = 0, xz = 0;
+        if (k >= 0 && k < ncx && l >= 0 && l < ncz) {   // centroid (k, l): vertices (k .. k+1, l .. l+1)
+            const int c = k + l * ncx;
+            const T ex = s_ex[h + 1][a + 1], ez = s_ez[h + 1][a + 1];
+            if (NEWTON) {
+                const T gm = T(0.25) * ((s_g[h][a] + s_g[h][a + 1]) + (s_g[h + 1][a] + s_g[h + 1][a + 1]));
+                const T p = s_p[h + 1][a + 1];
+                xx = D.D11[c] * ex + D.D12[c] * ez + D.D13[c] * gm + D.D14[c] * p;
+                zz = D.D21[c] * ex + D.D22[c] * ez + D.D23[c] * gm + D.D24[c] * p;
+            } else {
+                xx = D.D11[c] * ex;
+                zz = D.D22[c] * ez;
+            }
+        }
+        if (k >= 1 && k <= Nx - 2 && l >= 1 && l <= Nz - 2) {   // inner vertex (k, l): centroids (k-1 .. k, l-1 .. l)
+            const int c = k + l * Nx;
+            xz = D.D33[c] * s_g[h][a];
+            if (NEWTON) {
+                const T ex = (s_ex[h][a] + s_ex[h][a + 1]) + (s_ex[h + 1][a] + s_ex[h + 1][a + 1]);
+                const T ez = (s_ez[h][a] + s_ez[h][a + 1]) + (s_ez[h + 1][a] + s_ez[h + 1][a + 1]);
+                const T p = (s_p[h][a] + s_p[h][a + 1]) + (s_p[h + 1][a] + s_p[h + 1][a + 1]);
+                xz += T(0.25) * (D.D31[c] * ex + D.D32[c] * ez + D.D34[c] * p);
+            }
+        }
+        s_xx[h][a] = xx;
+        s_zz[h][a] = zz;
+        s_xz[h][a] = xz;
+    }
+    __syncthreads();
+    const int a = (tid & 31) + 1, h = (tid >> 5) + 1, i = i0 + a - 1, j = j0 + h - 1;   // (a, h): tile position of (i, j)
+    auto gm4 = [&](int q, int e) {   // mean shear rate of the centroid at tile position (q, e), as above
+        return T(0.25) * ((s_g[e][q] + s_g[e][q + 1]) + (s_g[e + 1][q] + s_g[e + 1][q + 1]));
+    };
+    if (i < Nx && j <= Nz) {            // Vx node (i, j)
+        const int c = i + j * Nx;
+        T r = 0;
+        if (i >= 1 && i <= Nx - 2 && j >= 1 && j <= Nz - 1) {
+            const int e = i + (j - 1) * ncx, w = e - 1;
+            T E = s_xx[h - 1][a], W = s_xx[h - 1][a - 1];
+            if (NEWTON && (j == 1 || j == Nz - 1)) {
+                // the wall vertex (i, j - 1) or (i, j) is left out of both means
+                const T in = j == 1 ? s_g[h][a] : s_g[h - 1][a];
+                E += D.D13[e] * (third * (in + s_g[h][a + 1] + s_g[h - 1][a + 1]) - gm4(a, h - 1));
+                W += D.D13[w] * (third * (in + s_g[h][a - 1] + s_g[h - 1][a - 1]) - gm4(a - 1, h - 1));
+            }
+            r = dz * ((W - E) + (x.p[e] - x.p[w])) + dx * (s_xz[h - 1][a] - s_xz[h][a]);
+            if (RES) r -= b.u[c] * gc<T>(G, GC_CELVOL);
+        }
+        y.u[c] = r;
+    }
+    if (i <= Nx && j < Nz) {            // Vz node (i, j)
+        const int c = i + j * nxvz;
+        T r = 0;
+        if (i >= 1 && i <= Nx - 1 && j >= 1 && j <= Nz - 2) {
+            const int s = i - 1 + (j - 1) * ncx, n = s + ncx;
+            T N = s_zz[h][a - 1], S = s_zz[h - 1][a - 1];
+            if (NEWTON && (i == 1 || i == Nx - 1)) {
+                // the wall vertex (i - 1, j) or (i, j) is left out of both means
+                const T in = i == 1 ? s_g[h][a] : s_g[h][a - 1];
+                S += D.D23[s] * (third * (in + s_g[h - 1][a - 1] + s_g[h - 1][a]) - gm4(a - 1, h - 1));
+                N += D.D23[n] * (third * (in + s_g[h + 1][a - 1] + s_g[h + 1][a]) - gm4(a - 1, h));
+            }
+            r = dx * ((S - N) + (x.p[n] - x.p[s])) + dz * (s_xz[h][a - 1] - s_xz[h][a]);
+            if (RES) r -= b.v[c] * gc<T>(G, GC_CELVOL);
+        }
+        y.v[c] = r;
+    }
+    if (i < ncx && j < ncz) {           // centroid (i, j)
+        const int c = i + j * ncx, cu = i + (j + 1) * Nx, cv = i + 1 + j * nxvz;
+        T r = dz * (x.u[cu + 1] - x.u[cu]) + dx * (x.v[cv + nxvz] - x.v[cv]);
+        if (RES) r -= b.p[c] * gc<T>(G, GC_CELVOL);
+        y.p[c] = r;
+    }
+}
+
 stokes_geom mdz_stokes_geom(const mdz_ctx *ctx) {
     const mdz_dgrid &g = ctx->g;
     return make_geom(g.Nx, g.Nz, g.dx, g.dz, g.BCu, g.BCv, g.BCp, g.BCg);
 }
 
+// box: the context's tags are the free-slip Dirichlet box (mdz_ctx::bcs_box)
 template <typename T>
 void stokes_apply_launch(const stokes_geom &G, const stokes_coefs<T> &D, stokes_cvec<T> x, stokes_vec<T> y,
-                         const stokes_cvec<T> *b, bool newton, cudaStream_t st) {
-    dim3 bl(32, 8), gr((G.Nx + 1 + 31) / 32, (G.Nz + 1 + 7) / 8);
-    T celvol = gc<T>(G, GC_CELVOL);
-    stokes_cvec<T> bb = b ? *b : stokes_cvec<T>{nullptr, nullptr, nullptr};
+                         const stokes_cvec<T> *b, bool newton, bool box, cudaStream_t st) {
+    const dim3 gr((G.Nx + 1 + 31) / 32, (G.Nz + 1 + 7) / 8);
+    const T celvol = gc<T>(G, GC_CELVOL);
+    const stokes_cvec<T> bb = b ? *b : stokes_cvec<T>{nullptr, nullptr, nullptr};
+#define APPLY(NEWTON, RES)                                                                     \
+    do {                                                                                       \
+        if (box) k_stokes_apply_box<T, NEWTON, RES><<<gr, 256, 0, st>>>(G, D, x, y, bb);       \
+        else k_stokes_apply<T, NEWTON, RES><<<gr, dim3(32, 8), 0, st>>>(G, D, x, y, bb, celvol); \
+    } while (0)
     if (b) {
-        if (newton) k_stokes_apply<T, true, true><<<gr, bl, 0, st>>>(G, D, x, y, bb, celvol);
-        else k_stokes_apply<T, false, true><<<gr, bl, 0, st>>>(G, D, x, y, bb, celvol);
+        if (newton) APPLY(true, true);
+        else APPLY(false, true);
     } else {
-        if (newton) k_stokes_apply<T, true, false><<<gr, bl, 0, st>>>(G, D, x, y, bb, celvol);
-        else k_stokes_apply<T, false, false><<<gr, bl, 0, st>>>(G, D, x, y, bb, celvol);
+        if (newton) APPLY(true, false);
+        else APPLY(false, false);
     }
+#undef APPLY
 }
 template void stokes_apply_launch<double>(const stokes_geom &, const stokes_coefs<double> &, stokes_cvec<double>,
-                                          stokes_vec<double>, const stokes_cvec<double> *, bool, cudaStream_t);
+                                          stokes_vec<double>, const stokes_cvec<double> *, bool, bool, cudaStream_t);
 template void stokes_apply_launch<float>(const stokes_geom &, const stokes_coefs<float> &, stokes_cvec<float>,
-                                         stokes_vec<float>, const stokes_cvec<float> *, bool, cudaStream_t);
+                                         stokes_vec<float>, const stokes_cvec<float> *, bool, bool, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Sums of squares per equation block and counts of equations: out[0..2] = sum F^2
@@ -163,9 +295,32 @@ static bool supported_bcs(const mdz_ctx *ctx, bool *neumann) {
     return true;
 }
 
+// Tags of the free-slip pure-shear box (the rule of k_level_tags in solver.cu):
+// Vx Dirichlet on the W/E lines, free-slip ghosts on the S/N rows; Vz Dirichlet
+// on the S/N lines, ghosts on W/E; everything else inner.
+static bool box_tags(const mdz_grid_desc &d) {
+    int Nx = d.Nx, Nz = d.Nz;
+    for (int l = 0; l <= Nz; l++)
+        for (int k = 0; k < Nx; k++) {
+            signed char t = -1;
+            if (k == 0 || k == Nx - 1) t = 0;
+            if (l == 0 || l == Nz) t = 13;
+            if (d.BCu_type[k + l * Nx] != t) return false;
+        }
+    for (int l = 0; l < Nz; l++)
+        for (int k = 0; k <= Nx; k++) {
+            signed char t = -1;
+            if (l == 0 || l == Nz - 1) t = 0;
+            if (k == 0 || k == Nx) t = 13;
+            if (d.BCv_type[k + l * (Nx + 1)] != t) return false;
+        }
+    return true;
+}
+
 mdz_status mdz_check_stokes_bcs(mdz_ctx *ctx) {
     if (!ctx->bcs_checked) {
         ctx->bcs_ok = supported_bcs(ctx, &ctx->bcs_neumann);
+        ctx->bcs_box = ctx->bcs_ok && !ctx->bcs_neumann && box_tags(ctx->host_desc);
         ctx->bcs_checked = true;
     }
     if (!ctx->bcs_ok)
@@ -373,7 +528,7 @@ mdz_status mdz_dev_residual(mdz_ctx *ctx, const mdz_fields &f, double *d_norms6,
     stokes_geom G = mdz_stokes_geom(ctx);
     stokes_cvec<double> x{f.u, f.v, f.p_corr}, b{f.roger_x, f.roger_z, f.rhs_p};
     stokes_vec<double> y{f.ru, f.rv, f.rp};
-    stokes_apply_launch<double>(G, mdz_coefs64(f), x, y, &b, false, st);
+    stokes_apply_launch<double>(G, mdz_coefs64(f), x, y, &b, false, ctx->bcs_checked && ctx->bcs_box, st);
     MDZ_LAUNCHED(ctx);
     mdz_status s = neumann_launch(ctx, true, false, f, x, f.ru, f.rv, st);
     if (s != MDZ_OK) return s;
@@ -421,7 +576,7 @@ extern "C" mdz_status mdz_StokesOperatorApply(mdz_ctx *ctx, mdz_fields *f, int j
     MDZ_CUDA(ctx, cudaMemcpyAsync(dxv, xv, nv * 8, cudaMemcpyHostToDevice, st));
     MDZ_CUDA(ctx, cudaMemcpyAsync(dxp, xp, np * 8, cudaMemcpyHostToDevice, st));
     stokes_apply_launch<double>(mdz_stokes_geom(ctx), mdz_coefs64(ctx->d), stokes_cvec<double>{dxu, dxv, dxp},
-                                stokes_vec<double>{dyu, dyv, dyp}, nullptr, jacobian != 0, st);
+                                stokes_vec<double>{dyu, dyv, dyp}, nullptr, jacobian != 0, ctx->bcs_box, st);
     MDZ_LAUNCHED(ctx);
     if ((s = neumann_launch(ctx, false, jacobian != 0, ctx->d, stokes_cvec<double>{dxu, dxv, dxp}, dyu, dyv, st)) !=
         MDZ_OK)

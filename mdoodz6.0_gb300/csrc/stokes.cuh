@@ -9,7 +9,7 @@ mdz_status mdz_check_stokes_bcs(mdz_ctx *ctx);
 
 template <typename T>
 void stokes_apply_launch(const stokes_geom &G, const stokes_coefs<T> &D, stokes_cvec<T> x, stokes_vec<T> y,
-                         const stokes_cvec<T> *b, bool newton, cudaStream_t st);
+                         const stokes_cvec<T> *b, bool newton, bool box, cudaStream_t st);
 template <typename T>
 mdz_status stokes_norms_launch(mdz_ctx *ctx, stokes_cvec<T> f, double *d_out6, cudaStream_t st);
 
