@@ -21,6 +21,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <atomic>
 #include <vector>
 #include "stokes.cuh"
 #include "solver.cuh"
@@ -31,6 +32,7 @@
 #define MG_NST 31        // stencil coefficients per velocity row (15 same-component + 16 cross)
 #define MG_CENTER 7      // plane of the diagonal entry in both layouts
 #define GCR_MAX_M 48
+#define GCR_NOTE 32       // slots of mdz_solver::sc the device writes: running squared norm, ticket
 #define MG_TILE_LARGE 30000   // points of a level above which the restriction takes the larger tile
 #define MG_TILE_SMALL 4000    // and below which the tile kernels take the smallest
 
@@ -68,6 +70,8 @@ struct mg_level {
 template <typename T>
 struct gcr_space {
     size_t nu = 0, nv = 0, np = 0, n = 0;
+    size_t ld = 0;                      // n rounded up to whole 128-byte lines: the vectors' stride and allocated
+                                        // length, zero beyond n, so that the vector kernels load 16 bytes a thread
     int m = 0;
     T *Z = nullptr, *W = nullptr;       // m basis vectors each (u, v, p contiguous)
     T *x = nullptr, *r = nullptr, *z = nullptr, *w = nullptr, *t = nullptr;
@@ -97,6 +101,7 @@ struct mdz_solver {
     gcr_space<double> g64;
     gcr_space<float> g32;
     double *sc = nullptr;        // host-pinned scalars
+    double ticket = 0.0;         // of the newest GCR iteration (gcr_wait_note)
     bool ready = false;
     int nu1 = 2, nu2 = 1;        // fewer sweeps, a few more Krylov iterations: faster overall at 1025x513
     double omega = 0.7;
@@ -1106,11 +1111,12 @@ static mdz_status alloc_gcr(mdz_ctx *ctx, gcr_space<T> &S, int m) {
     const mdz_dgrid &g = ctx->g;
     S.nu = (size_t)g.Nx * (g.Nz + 1); S.nv = (size_t)(g.Nx + 1) * g.Nz; S.np = (size_t)g.ncx * g.ncz;
     S.n = S.nu + S.nv + S.np;
+    S.ld = (S.n + 31) / 32 * 32;
     S.m = m;
-    cudaError_t e = alloc0(&S.Z, S.n * m);
-    if (e == cudaSuccess) e = alloc0(&S.W, S.n * m);
+    cudaError_t e = alloc0(&S.Z, S.ld * m);
+    if (e == cudaSuccess) e = alloc0(&S.W, S.ld * m);
     T **v[] = {&S.x, &S.r, &S.z, &S.w, &S.t, &S.pin};
-    for (T **b : v) if (e == cudaSuccess) e = alloc0(b, S.n);
+    for (T **b : v) if (e == cudaSuccess) e = alloc0(b, S.ld);
     if (e == cudaSuccess) e = cudaMalloc((void **)&S.dA0, sizeof(T *) * (GCR_MAX_M + 4));
     if (e == cudaSuccess) e = cudaMalloc((void **)&S.dA1, sizeof(T *) * (GCR_MAX_M + 4));
     if (e == cudaSuccess) e = cudaMalloc((void **)&S.dA2, sizeof(T *) * (GCR_MAX_M + 4));
@@ -1120,7 +1126,7 @@ static mdz_status alloc_gcr(mdz_ctx *ctx, gcr_space<T> &S, int m) {
     // pointer tables: rows 0..m-1 = W_i, row m = w, row m+1 = r
     std::vector<const T *> a0(m + 2), a1(m + 2), a2(m + 2);
     for (int i = 0; i < m + 2; i++) {
-        const T *base = i < m ? S.W + S.n * i : (i == m ? S.w : S.r);
+        const T *base = i < m ? S.W + S.ld * i : (i == m ? S.w : S.r);
         a0[i] = base; a1[i] = base + S.nu; a2[i] = base + S.nu + S.nv;
     }
     cudaMemcpy(S.dA0, a0.data(), sizeof(T *) * (m + 2), cudaMemcpyHostToDevice);
@@ -1661,7 +1667,11 @@ static mdz_status precondition(mdz_ctx *ctx, mg_hier<T> &H, const T *Dt, const T
 // whose coefficients the finish applies; sc[0] = 1/||w||, sc[1] = alpha,
 // sc[2] = ||w||^2, sc[3] = running ||r||^2 (so the host reads it only every
 // few iterations).
-__device__ void gcr_scalars(int k, const double *d, double *sc, double *tri, bool second) {
+// The running norm also goes to the host's memory with the iteration's ticket:
+// the host decides on the next iteration while the finish is still running,
+// instead of copying sc[3] back after it.
+__device__ void gcr_scalars(int k, const double *d, double *sc, double *tri, bool second, volatile double *note,
+                            double ticket) {
     // column k of U: the pass's Gram-Schmidt coefficients (added to the first
     // pass's after a second pass) and the new direction's norm
     double *U = tri + (size_t)k * GCR_MAX_M;
@@ -1679,6 +1689,9 @@ __device__ void gcr_scalars(int k, const double *d, double *sc, double *tri, boo
     sc[2] = nrm2;
     sc[3] -= alpha * alpha;   // ||r_k||^2 = ||r_k-1||^2 - alpha_k^2
     sc[8 + k] = alpha;
+    note[0] = sc[3];
+    __threadfence_system();
+    note[1] = ticket;
 }
 
 // gamma = U^-1 alpha (back substitution, one thread): x = x0 + Z gamma with
@@ -1700,6 +1713,7 @@ __global__ void k_gcr_gamma(int k, const double *__restrict__ sc, double *__rest
 template <typename P>
 __global__ void k_gcr_orth_if(size_t n, int k, const P *__restrict__ W, const double *__restrict__ beta,
                               const double *__restrict__ sc, P *__restrict__ w) {
+    pdl_wait();
     if (sc[5] == 0.0) return;
     __shared__ P bsh[GCR_MAX_M];
     for (int q = threadIdx.x; q < k; q += blockDim.x) bsh[q] = (P)beta[q];
@@ -1723,11 +1737,23 @@ __global__ void k_set_scalar(double *dst, const double *src) {
 // iteration this reads the basis W twice (the sums and here) and nothing of
 // Z: about 2k + 7 vectors against 3k + 11 for the form that orthogonalised
 // z and updated r every iteration.
+template <typename T>
+struct alignas(16) vec16 {
+    static constexpr int N = 16 / sizeof(T);
+    T v[N];
+};
+
+// (16 bytes of each vector per thread; n is the padded length.  Memory bound:
+// 1025 x 513 in FP32, 12 vectors on average, 12.1 us, 23.6 with 4-byte loads)
 template <typename P>
-__global__ void k_gcr_finish(size_t n, int k, P *__restrict__ W, P *__restrict__ Z, const double *__restrict__ dots1,
-                             const double *__restrict__ dots2, const double *__restrict__ sc,
-                             const P *__restrict__ z, const P *__restrict__ w, P *__restrict__ pin,
-                             double *__restrict__ next1, double *__restrict__ next2) {
+__global__ void __launch_bounds__(256) k_gcr_finish(size_t n, int k, P *__restrict__ W, P *__restrict__ Z,
+                                                    const double *__restrict__ dots1,
+                                                    const double *__restrict__ dots2, const double *__restrict__ sc,
+                                                    const P *__restrict__ z, const P *__restrict__ w,
+                                                    P *__restrict__ pin, double *__restrict__ next1,
+                                                    double *__restrict__ next2) {
+    typedef vec16<P> V;
+    pdl_wait();
     // the next iteration accumulates into the other parity's buffers, which
     // no kernel of this iteration reads: clear them here instead of by memsets
     if (blockIdx.x == 0 && next1)
@@ -1736,14 +1762,22 @@ __global__ void k_gcr_finish(size_t n, int k, P *__restrict__ W, P *__restrict__
     const double *__restrict__ beta = sc[5] != 0.0 ? dots2 : dots1;
     for (int q = threadIdx.x; q < k; q += blockDim.x) bsh[q] = (P)beta[q];
     __syncthreads();
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V::N;
     if (i >= n) return;
-    P ws = w[i];
-    for (int q = 0; q < k; q++) ws -= bsh[q] * W[q * n + i];
-    ws *= (P)sc[0];
-    W[(size_t)k * n + i] = ws;
-    pin[i] = ws;
-    Z[(size_t)k * n + i] = z[i];
+    V ws = *reinterpret_cast<const V *>(w + i);
+    const V zi = *reinterpret_cast<const V *>(z + i);
+#pragma unroll 4
+    for (int q = 0; q < k; q++) {
+        const V wq = *reinterpret_cast<const V *>(W + q * n + i);
+#pragma unroll
+        for (int e = 0; e < V::N; e++) ws.v[e] -= bsh[q] * wq.v[e];
+    }
+    const P s = (P)sc[0];
+#pragma unroll
+    for (int e = 0; e < V::N; e++) ws.v[e] *= s;
+    *reinterpret_cast<V *>(W + (size_t)k * n + i) = ws;
+    *reinterpret_cast<V *>(pin + i) = ws;
+    *reinterpret_cast<V *>(Z + (size_t)k * n + i) = zi;
 }
 
 // r = r - sum alpha_q W_q over the basis (end of a basis); the P copy of the
@@ -1822,30 +1856,42 @@ static mdz_status remove_pressure_mean(mdz_ctx *ctx, double *p, cudaStream_t st)
     return MDZ_OK;
 }
 
-// out[q] = (a_q, b) for the nq vectors of the pointer table (each of length
-// n, contiguous u|v|p like b).  FP32 vectors: one thread keeps Q = 8 running
-// sums, so b is read once per 8 vectors and the loads of 8 independent chains
-// overlap, and products, sums and the warp reductions stay FP32 with only the
-// warp sums entering FP64 (FP64 instructions issue at a small fraction of
-// the FP32 rate on this part, so even a per-thread FP64 reduction tree
-// dominated the kernel).  FP64 vectors: Q = 1, one vector per block row (the
-// per-element FP64 multiply-add is the bound there).  Block row y handles
-// vectors y Q .. y Q + Q - 1; its blocks write their partials to
+// out[q] = (a_q, b) for the nq vectors of the pointer table (each of padded
+// length n, contiguous u|v|p like b).  One thread keeps Q running sums and loads
+// 16 bytes of each vector and of b at a time, so b is read once per Q vectors
+// and the loads of all of them are in flight together.  FP32 vectors (Q = 8):
+// products, sums and the warp reductions stay FP32 with only the warp sums
+// entering FP64 (FP64 instructions issue at a small fraction of the FP32 rate
+// on this part, so even a per-thread FP64 reduction tree dominated the
+// kernel).  FP64 vectors (Q = 4) are bound by their FP64 multiply-adds.  Block
+// row y handles vectors y Q .. y Q + Q - 1; its blocks write their partials to
 // part[q * gridDim.x + blockIdx.x] and the last block of the row to finish
 // adds them up in block order (reduce.cuh): deterministic.  cnt: one arrival
 // counter per block row.  A non-null flag holding 0 makes the launch a no-op.
+// 1025 x 513 in FP32, up to 8 / 16 / 24 vectors: 13.8 / 21.2 / 29.6 us, with
+// 4-byte loads 18.9 / 32.7 / 51.7.
+template <typename T>
+constexpr int dots_q() { return sizeof(T) == 4 ? 8 : 4; }
 template <typename T, int MDOT_Q>
 __device__ __forceinline__ void dots_block(int nq, size_t n, const T *const *ap, const T *__restrict__ b,
                                            double *part, double (&bs)[MDOT_Q], double *sh) {
+    typedef vec16<T> V;
     T p[MDOT_Q];
 #pragma unroll
     for (int j = 0; j < MDOT_Q; j++) p[j] = T(0);
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const T bi = b[i];
+    const size_t stride = (size_t)gridDim.x * blockDim.x * V::N;
+    for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V::N; i < n; i += stride) {
+        const V bi = *reinterpret_cast<const V *>(b + i);
+        V a[MDOT_Q];
 #pragma unroll
         for (int j = 0; j < MDOT_Q; j++)
-            if (ap[j]) p[j] += ap[j][i] * bi;
+            if (ap[j]) a[j] = *reinterpret_cast<const V *>(ap[j] + i);
+#pragma unroll
+        for (int j = 0; j < MDOT_Q; j++)
+            if (ap[j]) {
+#pragma unroll
+                for (int e = 0; e < V::N; e++) p[j] += a[j].v[e] * bi.v[e];
+            }
     }
     mdz_block_sum<MDOT_Q, T>(p, bs, sh);
     const int q0 = blockIdx.y * MDOT_Q;
@@ -1885,7 +1931,8 @@ template <typename T, int MDOT_Q>
 __global__ void __launch_bounds__(256) k_gcr_dots(int k, size_t n, const T *const *__restrict__ a,
                                                   const T *__restrict__ w, const T *__restrict__ r, double *part,
                                                   double *out, const double *flag, int mode, double *sc,
-                                                  double *tri, unsigned int *cnt) {
+                                                  double *tri, unsigned int *cnt, double *note, double ticket) {
+    pdl_wait();
     if (flag && *flag == 0.0) return;
     __shared__ double sh[32 * MDOT_Q];
     const int nq = k + 2, q0 = blockIdx.y * MDOT_Q;
@@ -1917,21 +1964,27 @@ __global__ void __launch_bounds__(256) k_gcr_dots(int k, size_t n, const T *cons
         }
         sc[5] = 0.0;
     }
-    gcr_scalars(k, d, sc, tri, mode == 2);
+    gcr_scalars(k, d, sc, tri, mode == 2, note, ticket);
+}
+
+// grid of a dots launch over nq vectors: block rows of Q vectors, about four
+// blocks per SM in all, each thread at least one 16-byte load per vector
+template <typename T>
+static dim3 dots_grid(size_t n, int nq) {
+    constexpr int Q = dots_q<T>();
+    const int rows = (nq + Q - 1) / Q;
+    int bx = mdz_blocks((long long)n, 256 * vec16<T>::N);
+    const int cap = (152 * 4 + rows - 1) / rows;
+    if (bx > cap) bx = cap;
+    return dim3(bx, rows);
 }
 
 template <typename T>
 static mdz_status gcr_dots_launch(mdz_ctx *ctx, gcr_space<T> &S, int k, const T *w, const T *r, double *out,
-                                  const double *flag, int mode, double *sc, cudaStream_t st) {
-    constexpr int Q = sizeof(T) == 4 ? 8 : 1;
-    const int tiles = (k + 2 + Q - 1) / Q;
-    int bx = mdz_blocks((long long)S.n, 256 * (sizeof(T) == 4 ? 8 : 4));
-    const int cap = (sizeof(T) == 4 ? 152 * 8 : 152 * 4 + tiles - 1) / tiles;
-    if (bx > cap) bx = cap;
-    if (bx < 8) bx = 8;
-    k_gcr_dots<T, Q><<<dim3(bx, tiles), 256, 0, st>>>(k, S.n, S.dA0, w, r, ctx->red_part + MDZ_RP_DOTS, out, flag,
-                                                       mode, sc, S.tri, ctx->red_cnt + MDZ_RC_GCR);
-    MDZ_LAUNCHED(ctx);
+                                  const double *flag, int mode, double *sc, double ticket, cudaStream_t st) {
+    MDZ_PDL(ctx, k_gcr_dots<T, dots_q<T>()>, dots_grid<T>(S.ld, k + 2), 256, 0, st, k, S.ld, S.dA0, w, r,
+            ctx->red_part + MDZ_RP_DOTS, out, flag, mode, sc, S.tri, ctx->red_cnt + MDZ_RC_GCR,
+            ctx->solver->sc + GCR_NOTE, ticket);
     return MDZ_OK;
 }
 
@@ -1939,17 +1992,25 @@ template <typename T>
 static mdz_status dots_launch(mdz_ctx *ctx, gcr_space<T> &S, int q0, int nq, const T *b, double *out,
                               cudaStream_t st, const double *flag = nullptr) {
     if (nq <= 0) return MDZ_OK;
-    // FP32: 8 vectors per block row, ~8 elements per thread; FP64: one vector
-    // per block row, about 600 blocks in all
-    constexpr int Q = sizeof(T) == 4 ? 8 : 1;
-    const int tiles = (nq + Q - 1) / Q;
-    int bx = mdz_blocks((long long)S.n, 256 * (sizeof(T) == 4 ? 8 : 4));
-    const int cap = (sizeof(T) == 4 ? 152 * 8 : 152 * 4 + tiles - 1) / tiles;
-    if (bx > cap) bx = cap;
-    if (bx < 8) bx = 8;
-    k_dots<T, Q><<<dim3(bx, tiles), 256, 0, st>>>(nq, S.n, S.dA0 + q0, b, ctx->red_part + MDZ_RP_DOTS,
-                                                   ctx->red_cnt + MDZ_RC_DOTS, out, flag);
+    k_dots<T, dots_q<T>()><<<dots_grid<T>(S.ld, nq), 256, 0, st>>>(nq, S.ld, S.dA0 + q0, b, ctx->red_part + MDZ_RP_DOTS,
+                                                                   ctx->red_cnt + MDZ_RC_DOTS, out, flag);
     MDZ_LAUNCHED(ctx);
+    return MDZ_OK;
+}
+
+// The running norm of the iteration with this ticket, as gcr_scalars wrote it
+// to host memory (GCR_NOTE), usually before the iteration's last launch ends.
+static mdz_status gcr_wait_note(mdz_ctx *ctx, double ticket, cudaStream_t st, double *rn2) {
+    volatile double *note = ctx->solver->sc + GCR_NOTE;
+    for (long long spin = 1; note[1] != ticket; spin++) {
+        if (spin % 4096) continue;
+        const cudaError_t e = cudaStreamQuery(st);   // a failed launch never writes its ticket
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess) return mdz_cuda_check(ctx, e, "GCR iteration");
+        if (note[1] != ticket) return mdz_fail(ctx, MDZ_ERR_STATE, "GCR: an iteration ended without its norm");
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    *rn2 = note[0];
     return MDZ_OK;
 }
 
@@ -2016,8 +2077,10 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
     constexpr bool mixed = sizeof(T) != sizeof(P);
     mdz_solver *SV = ctx->solver;
     stokes_geom G = mdz_stokes_geom(ctx);
-    const size_t n = S.n, nu = S.nu, nv = S.nv;
+    // vector kernels run over the padded length (zeros beyond the n unknowns)
+    const size_t n = S.ld, nu = S.nu, nv = S.nv;
     int nb = mdz_blocks(n);
+    const int nb16 = mdz_blocks((long long)n, 256 * vec16<P>::N);
     MDZ_CUDA(ctx, cudaMemsetAsync(S.x, 0, sizeof(T) * n, st));
     // ||r0||
     // S.dots layout (doubles, B = GCR_MAX_M + 8): first-pass sums of even / odd
@@ -2026,10 +2089,7 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
     const int B = GCR_MAX_M + 8;
     double *sc = S.dots + (GCR_MAX_M + 4), *dots = S.dots + 3 * B;
     double *dots1p[2] = {S.dots, S.dots + 4 * B}, *dots2p[2] = {S.dots + 2 * B, S.dots + 5 * B};
-    for (int q = 0; q < 2; q++) {
-        MDZ_CUDA(ctx, cudaMemsetAsync(dots1p[q], 0, sizeof(double) * (GCR_MAX_M + 3), st));
-        MDZ_CUDA(ctx, cudaMemsetAsync(dots2p[q], 0, sizeof(double) * (GCR_MAX_M + 3), st));
-    }
+    MDZ_CUDA(ctx, cudaMemsetAsync(S.dots, 0, sizeof(double) * 8 * B, st));
     mdz_status s;
     cudaGraphExec_t pre = nullptr;
     long long pre_launches = 0;
@@ -2084,7 +2144,7 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
         {   // algorithmic bytes: input and output vectors, the D-tensor read once, tags
             size_t nc = S.np, ng = (size_t)G.Nx * G.Nz;
             double coef = newton ? (8.0 * nc + 4.0 * ng) : (2.0 * nc + ng);
-            double bytes = sizeof(P) * (2.0 * n + coef) + (double)(nu + nv + nc + ng);
+            double bytes = sizeof(P) * (2.0 * S.n + coef) + (double)(nu + nv + nc + ng);
             mdz_prof_end(ctx, MDZ_PROF_STOKES_APPLY, bytes, st, ev);
         }
         mdz_prof_begin(ctx, MDZ_PROF_KRYLOV, st, &ev);
@@ -2095,28 +2155,25 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
         // whether a second pass runs.
         const int ng = nb < 152 * 8 ? nb : 152 * 8;
         double *d1 = dots1p[it & 1], *d2 = dots2p[it & 1];
-        if ((s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, d1, nullptr, 1, sc, st)) != MDZ_OK) return s;
+        SV->ticket += 1.0;
+        if ((s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, d1, nullptr, 1, sc, SV->ticket, st)) != MDZ_OK) return s;
         if (k > 0) {   // second pass (each launch returns at once unless sc[5] = 1)
-            k_gcr_orth_if<P><<<ng, MDZ_THREADS, 0, st>>>(n, k, SP.W, d1, sc, SP.w);
-            MDZ_LAUNCHED(ctx);
-            if ((s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, d2, sc + 5, 2, sc, st)) != MDZ_OK) return s;
+            MDZ_PDL(ctx, k_gcr_orth_if<P>, ng, MDZ_THREADS, 0, st, n, k, SP.W, d1, sc, SP.w);
+            if ((s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, d2, sc + 5, 2, sc, SV->ticket, st)) != MDZ_OK) return s;
         }
-        k_gcr_finish<P><<<nb, MDZ_THREADS, 0, st>>>(n, k, SP.W, SP.Z, d1, d2, sc, SP.z, SP.w, SP.pin,
-                                                     dots1p[(it + 1) & 1], dots2p[(it + 1) & 1]);
-        MDZ_LAUNCHED(ctx);
+        MDZ_PDL(ctx, k_gcr_finish<P>, nb16, 256, 0, st, n, k, SP.W, SP.Z, d1, d2, sc, SP.z, SP.w, SP.pin,
+                dots1p[(it + 1) & 1], dots2p[(it + 1) & 1]);
         {   // algorithmic bytes (one Gram-Schmidt pass): the sums read W_q,
             // w and r0 (k + 2 P vectors); the finish reads W_q, w, z and
             // writes W_k, Z_k and the next input (k + 5)
             double pv = 2.0 * k + 7.0;
-            mdz_prof_end(ctx, MDZ_PROF_KRYLOV, (double)n * sizeof(P) * pv, st, ev);
+            mdz_prof_end(ctx, MDZ_PROF_KRYLOV, (double)S.n * sizeof(P) * pv, st, ev);
         }
         k++;
         // the running norm lives on the device; the host looks every `check`
         // iterations, at each restart and at the iteration limit
         if ((it + 1) % check != 0 && k != S.m && it + 1 < maxit) continue;
-        MDZ_CUDA(ctx, cudaMemcpyAsync(SV->sc, sc, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
-        MDZ_CUDA(ctx, cudaStreamSynchronize(st));
-        rn2 = SV->sc[3];
+        if ((s = gcr_wait_note(ctx, SV->ticket, st, &rn2)) != MDZ_OK) return s;
         if (!std::isfinite(rn2)) return mdz_fail(ctx, MDZ_ERR_NAN, "GCR: NaN in the Krylov iteration");
         if (rn2 <= rtol * rtol * rn02 || (k == S.m)) {
             // fold the basis in and take the true norm of r at convergence
