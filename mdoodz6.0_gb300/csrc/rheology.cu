@@ -130,28 +130,106 @@ __device__ __forceinline__ float mpow(float x, float y) { return powf(x, y); }
 template <typename Real>
 __device__ __forceinline__ Real dmin(Real a, Real b) { return a <= b ? a : b; }
 
-// Materials as the local solves read them: the public parameters plus
-// lnK_pwl = ln(pref F A^(-1/n) f^(-r/n)), the part of the logarithm of the
-// dislocation prefactor B_pwl (Viscosity, SOURCE/RheologyDensity.c:153-154)
-// that depends on neither the node nor the iteration.  Taken once per
-// launch on the host; NaN where the product is not positive and finite, and the
-// solve then multiplies the reference's factors out as they stand.
-struct mdz_mat_k : mdz_materials {
-    double lnK_pwl[MDZ_MAX_PHASES];
+// ---- constants of the local solves, taken once per launch on the host -----------
+// The local solves are bound by the FP64 pipe (77 % active): a transcendental
+// function is 20-100 FP64 instructions, a division ten, and every comparison
+// or conversion of an FP64 value is one too.  So whatever depends on the
+// phase and the model switches alone is formed here: reciprocals, prefactors,
+// powers of the reference grain size, and flags in place of comparisons.
+enum {
+    VP_CST = 1, VP_PWL = 2, VP_LIN = 4, VP_EXP = 8, VP_GBS = 16, VP_TENS = 32,   // mechanisms (cstv, pwlv, ...)
+    VP_LOGF = 64,      // FP64 dislocation creep in log form (lnK_pwl below)
+    VP_LIN1 = 128,     // n_lin = 1: linear diffusion creep
+    VP_VP1 = 256,      // n_vp = 1: linear viscoplastic regularisation
+    VP_PWL_D = 512, VP_PWL_PHI = 1024, VP_LIN_D = 2048, VP_LIN_PHI = 4096,   // grain size / melt exponents not 0
+    VP_GBS_D = 8192, VP_GBS_PHI = 16384
+};
+template <typename Real>
+struct visc_phase {
+    int flags;
+    // dislocation creep: B = K0 exp((Q + P V) in / RT) d^md exp(-a phi), K0 = pref F A^-in f^(-r in), lnK its
+    // logarithm; in = 1 / n, md = m in, a = a in (the others alike)
+    Real n_pwl, in_pwl, Q_pwl, V_pwl, K0_pwl, lnK_pwl, md_pwl, a_pwl;
+    Real n_lin, in_lin, Q_lin, V_lin, K0_lin, m_lin, a_lin, dm_lin, dmn_lin;   // gs_ref^-m, gs_ref^(m in)
+    Real n_gbs, in_gbs, Q_gbs, V_gbs, K0_gbs, md_gbs, a_gbs;
+    Real Gexp, Qexp, Sexp, Eexp, nexp;
+    Real eta0, ieta0, gs_ref, igs_ref, Slim, eta_vp, in_vp;
+};
+template <typename Real>
+struct visc_prm {
+    int iselastic, step, clamp_tangent;
+    Real R, dt, idt, Emin, Tmin, Tpeierls, eta_big, P_tens, mineta, maxeta;
+};
+template <typename Real>
+struct visc_mat {
+    int n_phases;
+    visc_prm<Real> prm;
+    visc_phase<Real> ph[MDZ_MAX_PHASES];
 };
 
-static mdz_mat_k mat_k(const mdz_materials &m) {
-    mdz_mat_k k;
-    static_cast<mdz_materials &>(k) = m;
-    for (int p = 0; p < MDZ_MAX_PHASES; p++) {
-        double v = NAN;
+// lnK_pwl = ln(pref F A^(-1/n) f^(-r/n)): the part of the logarithm of the
+// dislocation prefactor B_pwl (Viscosity, SOURCE/RheologyDensity.c:153-154)
+// that depends on neither the node nor the iteration; without VP_LOGF, where
+// the product is not positive and finite, the solve multiplies the reference's
+// factors out as they stand.
+template <typename Real>
+static visc_mat<Real> make_visc_mat(const mdz_materials &m, const mdz_rheo_params &prm) {
+    visc_mat<Real> k{};
+    k.n_phases = m.n_phases;
+    visc_prm<Real> &q = k.prm;
+    q.iselastic = prm.iselastic; q.step = prm.step; q.clamp_tangent = prm.clamp_tangent;
+    q.R = (Real)m.R; q.dt = (Real)prm.dt; q.idt = (Real)(1.0 / prm.dt);
+    q.Emin = (Real)(1e-30 / prm.scale_E); q.Tmin = (Real)(ZEROC / prm.scale_T);
+    q.Tpeierls = (Real)((1200.0 + ZEROC) / prm.scale_T); q.eta_big = (Real)(1.0e100 / prm.scale_eta);
+    q.P_tens = (Real)(-25e6 / prm.scale_S); q.mineta = (Real)prm.mineta; q.maxeta = (Real)prm.maxeta;
+    auto prefactor = [](double pf, double A, double n, double f, double r) {
+        double v = pf * std::pow(A, -1.0 / n);
+        if (r != 0) v *= std::pow(f, -r / n);
+        return v;
+    };
+    for (int p = 0; p < m.n_phases; p++) {
+        visc_phase<Real> &v = k.ph[p];
         const double n = m.npwl[p], pf = m.pref_pwl[p] * m.Fpwl[p], A = m.Apwl[p], f = m.fpwl[p], r = m.rpwl[p];
-        if (p < m.n_phases && m.pwlv[p] != 0 && n != 0 && pf > 0 && A > 0 && (r == 0 || f > 0)) {
-            v = std::log(pf) - std::log(A) / n;
-            if (r != 0) v -= r / n * std::log(f);
-            if (!std::isfinite(v)) v = NAN;
+        int fl = (m.cstv[p] ? VP_CST : 0) | (m.pwlv[p] ? VP_PWL : 0) | (m.linv[p] ? VP_LIN : 0) | (m.expv[p] ? VP_EXP : 0) |
+                 (m.gbsv[p] ? VP_GBS : 0) | (m.is_tensile[p] ? VP_TENS : 0);
+        if (m.pwlv[p]) {
+            if (m.mpwl[p] != 0) fl |= VP_PWL_D;
+            if (m.apwl[p] != 0) fl |= VP_PWL_PHI;
+            v.n_pwl = (Real)n; v.in_pwl = (Real)(1.0 / n); v.Q_pwl = (Real)m.Qpwl[p]; v.V_pwl = (Real)m.Vpwl[p];
+            v.K0_pwl = (Real)prefactor(pf, A, n, f, r);
+            v.md_pwl = (Real)(m.mpwl[p] / n); v.a_pwl = (Real)(m.apwl[p] / n);
+            if (sizeof(Real) == 8 && pf > 0 && A > 0 && (r == 0 || f > 0)) {
+                double l = std::log(pf) - std::log(A) / n;
+                if (r != 0) l -= r / n * std::log(f);
+                if (std::isfinite(l)) { v.lnK_pwl = (Real)l; fl |= VP_LOGF; }
+            }
         }
-        k.lnK_pwl[p] = v;
+        if (m.linv[p]) {
+            const double nl = m.nlin[p];
+            if (nl == 1.0) fl |= VP_LIN1;
+            if (m.mlin[p] != 0) fl |= VP_LIN_D;
+            if (m.alin[p] != 0) fl |= VP_LIN_PHI;
+            v.n_lin = (Real)nl; v.in_lin = (Real)(1.0 / nl); v.Q_lin = (Real)m.Qlin[p]; v.V_lin = (Real)m.Vlin[p];
+            v.K0_lin = (Real)prefactor(m.Flin[p], m.Alin[p], nl, m.flin[p], m.rlin[p]);
+            v.m_lin = (Real)m.mlin[p]; v.a_lin = (Real)(m.alin[p] / nl);
+            v.dm_lin = (Real)(m.mlin[p] == 0 ? 1.0 : std::pow(m.gs_ref[p], -m.mlin[p]));
+            v.dmn_lin = (Real)(m.mlin[p] == 0 ? 1.0 : std::pow(m.gs_ref[p], m.mlin[p] / nl));
+        }
+        if (m.gbsv[p]) {
+            const double ng = m.ngbs[p];
+            if (m.mgbs[p] != 0) fl |= VP_GBS_D;
+            if (m.agbs[p] != 0) fl |= VP_GBS_PHI;
+            v.n_gbs = (Real)ng; v.in_gbs = (Real)(1.0 / ng); v.Q_gbs = (Real)m.Qgbs[p]; v.V_gbs = (Real)m.Vgbs[p];
+            v.K0_gbs = (Real)prefactor(m.Fgbs[p], m.Agbs[p], ng, m.fgbs[p], m.rgbs[p]);
+            v.md_gbs = (Real)(m.mgbs[p] / ng); v.a_gbs = (Real)(m.agbs[p] / ng);
+        }
+        v.Gexp = (Real)m.Gexp[p]; v.Qexp = (Real)m.Qexp[p]; v.Sexp = (Real)m.Sexp[p]; v.Eexp = (Real)m.Eexp[p];
+        v.nexp = (Real)m.nexp[p];
+        v.eta0 = (Real)m.eta0[p]; v.ieta0 = (Real)(1.0 / m.eta0[p]);
+        v.gs_ref = (Real)m.gs_ref[p]; v.igs_ref = (Real)(1.0 / m.gs_ref[p]);
+        v.Slim = (Real)m.Slim[p]; v.eta_vp = (Real)m.eta_vp[p]; v.in_vp = (Real)(1.0 / m.n_vp[p]);
+        if (m.n_vp[p] == 1.0) fl |= VP_VP1;
+        v.flags = fl;
     }
     return k;
 }
@@ -164,144 +242,113 @@ __device__ __forceinline__ double ln1p_series(double x) {
     return x * (1.0 + x * (-0.5 + x * (1.0 / 3.0 + x * (-0.25 + x * (0.2 + x * (-1.0 / 6.0 + x * (1.0 / 7.0)))))));
 }
 
-// pow with the exponents the creep laws make trivial (0, 1, 2, -1, -2:
-// grain-size and melt exponents switched off, linear diffusion creep and its
-// tangent, squares) taken exactly; each costs a full FP64 log/exp pair
-// otherwise, and FP64 throughput is what bounds the local solves on this part.
-template <typename Real, typename Y>
-__device__ __forceinline__ Real fpow(Real x, Y y0) {
-    const Real y = Real(y0);
-    if (y == Real(0)) return Real(1);
-    if (y == Real(1)) return x;
-    if (y == Real(2)) return x * x;
-    if (y == Real(-1)) return Real(1) / x;
-    if (y == Real(-2)) return Real(1) / (x * x);
-    return mpow(x, y);
-}
-
-// exp with the zero argument of switched-off melt weakening taken exactly
+// One (node, phase) solve.  The reference's Gxx.. (rates with the anisotropic
+// elastic correction) equal Exx.. in this isotropic subset, and its f_ani =
+// Gii / Eii is 1.  ie: 1 / (mu dt) where the model is elastic.
 template <typename Real>
-__device__ __forceinline__ Real fexp(Real x) { return x == Real(0) ? Real(1) : mexp(x); }
-
-template <typename Real>
-__device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Real X0, Real Exx,
-                           Real Ezz, Real Exz, Real Gxx, Real Gzz, Real Gxz, Real Txx0, Real Tzz0,
-                           Real Txz0, const mdz_mat_k &m, const mdz_rheo_params &prm, Real dil, Real fric,
-                           Real C, Real P0, Real beta, visc_res &o, const float *guess) {
-    const Real R = Real(m.R), dt = Real(prm.dt), tol = sizeof(Real) == 8 ? Real(1.0e-11) : Real(1.0e-4);
-    const int nitmax = 20;
-    int elastic = prm.iselastic, it;
-    const bool constant = Real(m.cstv[p]) != 0, dislocation = Real(m.pwlv[p]) != 0, diffusion = Real(m.linv[p]) != 0;
+__device__ void visc_local_t(const visc_phase<Real> &m, const visc_prm<Real> &prm, Real G, Real ie, Real T, Real P,
+                             Real d, Real phi, Real X0, Real Exx, Real Ezz, Real Exz, Real Txx0, Real Tzz0, Real Txz0,
+                             Real dil, Real fric, Real C, Real P0, Real beta, visc_res &o, const float *guess) {
+    const Real dt = prm.dt, tol = sizeof(Real) == 8 ? Real(1.0e-11) : Real(1.0e-4);
+    const int nitmax = 20, fl = m.flags;
+    int it;
+    const bool elastic = prm.iselastic != 0 && prm.step != 0;
+    const bool constant = fl & VP_CST, dislocation = fl & VP_PWL, diffusion = fl & VP_LIN, lin1 = fl & VP_LIN1,
+               vp1 = fl & VP_VP1, logform = sizeof(Real) == 8 && (fl & VP_LOGF);
     // Peierls creep only below 1200 C (tested before the 0 C clamp, :137),
     // grain-boundary sliding, tension cut-off; the learned start models none
     // of them, so their solves take the reference's start
-    const bool peierls = m.expv[p] != 0 && T < Real((1200.0 + ZEROC) / prm.scale_T);
-    const bool gbs = m.gbsv[p] != 0, tensile = m.is_tensile[p] != 0;
+    const bool peierls = (fl & VP_EXP) && T < prm.Tpeierls, gbs = fl & VP_GBS, tensile = fl & VP_TENS;
     if (peierls || gbs || tensile) guess = nullptr;
-    Real K = Real(1.0) / beta, res = Real(0.0);
+    Real res = Real(0.0);
     const Real Tii0 = msqrt(Txx0 * Txx0 + Txz0 * Txz0);
-    const Real n_pwl = Real(m.npwl[p]), Va_pwl = Real(m.Vpwl[p]), n_lin = Real(m.nlin[p]), m_lin = Real(m.mlin[p]);
-    Real B_lin = 0, C_pwl = 0, C_lin = 0, dCpwldP = 0, dClindP = 0;
-    Real eta_pwl = Real(0.0), eta_lin = Real(0.0), eta_cst = Real(0.0), eta_vep = Real(0.0), eta_vp = Real(0.0);
-    const Real eta_vp0 = Real(m.eta_vp[p]), n_vp = Real(m.n_vp[p]);
+    const Real n_pwl = m.n_pwl, n_lin = m.n_lin;
+    Real C_pwl = 0, C_lin = 0;
+    Real eta_pwl = Real(0.0), eta_lin = Real(0.0), eta_vep = Real(0.0), eta_vp = Real(0.0);
+    const Real eta_vp0 = m.eta_vp;
     Real Eii_pwl = 0, Eii_lin = 0, Eii_cst = 0, Eii_exp = 0, Eii_gbs = 0;
     o.Eii_pl = Real(0.0); o.OverS = Real(0.0); o.ve_fail = 0; o.vp_fail = 0; o.vp_its = 0;
 
-    Real Eyy = -(Exx + Ezz), Gyy = -(Gxx + Gzz);
-    Real Eii = msqrt(Real(1.0) / Real(2.0) * (Exx * Exx + Ezz * Ezz + Eyy * Eyy) + Exz * Exz);
-    Real Gii = msqrt(Real(1.0) / Real(2.0) * (Gxx * Gxx + Gzz * Gzz + Gyy * Gyy) + Gxz * Gxz);
-    if (Eii * Real(prm.scale_E) < Real(1e-30)) Eii = Real(1e-30) / Real(prm.scale_E);
-    if (Gii * Real(prm.scale_E) < Real(1e-30)) Gii = Real(1e-30) / Real(prm.scale_E);
-    const Real f_ani = Gii / Eii;
-    // reciprocals taken once per solve: an FP64 division is a long instruction
-    // sequence on this part, and the reference's formulas divide some fifty
-    // times per local solve
-    const Real iEii = Real(1.0) / Eii, iGii = Real(1.0) / Gii;
+    const Real Eyy = -(Exx + Ezz);
+    Real Eii = msqrt(Real(0.5) * (Exx * Exx + Ezz * Ezz + Eyy * Eyy) + Exz * Exz);
+    if (Eii < prm.Emin) Eii = prm.Emin;
+    const Real iEii = Real(1.0) / Eii;
     o.Pcorr = P;
-    if (prm.step == 0) elastic = 0;
-    o.d1 = Real(m.gs_ref[p]);
-    if (elastic == 0) { G = Real(1e1); K = Real(1e1); dil = Real(0.0); }
-    if (T < Real(ZEROC) / Real(prm.scale_T)) T = Real(ZEROC) / Real(prm.scale_T);
-    const Real iRT = Real(1.0) / (R * T);
+    o.d1 = m.gs_ref;
+    // without elasticity the reference sets G = K = 10 and no dilation
+    if (!elastic) { G = Real(1e1); dil = Real(0.0); }
+    const Real eta_el = G * dt;
+    const Real i2eta_el = Real(0.5) * (elastic && prm.iselastic == 1 ? ie : Real(1.0) / eta_el);
+    if (T < prm.Tmin) T = prm.Tmin;
+    const Real iRT = Real(1.0) / (prm.R * T);
     // FP64 dislocation creep in log form: ln B_pwl from the per-phase constant,
-    // then C_pwl = (2 f_ani B_pwl)^-n and eta_pwl = B_pwl Eii^(1/n - 1) as two
+    // then C_pwl = (2 B_pwl)^-n and eta_pwl = B_pwl Eii^(1/n - 1) as two
     // exponentials after one logarithm (the product form takes three pow and an
-    // exp), and in the learned polish Eii_pwl = exp(ln C_pwl + n ln Tii) with
-    // ln Tii = lnTE + ln eta_ve known.  FP32 keeps the product form: rounding of
+    // exp), and in the iterations Eii_pwl = exp(ln C_pwl + n ln Tii) with
+    // ln Tii = lnTE + ln eta_ve.  FP32 keeps the product form: rounding of
     // the logarithms' sums there is at the size of its convergence test.
-    const bool logform = sizeof(Real) == 8 && dislocation && isfinite(m.lnK_pwl[p]);
     Real lnC_pwl = Real(0.0), lnTE = Real(0.0), ln_eta_pwl = Real(0.0);
     if (dislocation) {
-        const Real in = Real(1.0) / n_pwl;
+        const Real in = m.in_pwl;
         if (logform) {
-            Real lnB = Real(m.lnK_pwl[p]) + (Real(m.Qpwl[p]) + P * Va_pwl) * iRT * in;
-            if (Real(m.mpwl[p]) != Real(0.0)) lnB += Real(m.mpwl[p]) * in * mlog(d);
-            if (Real(m.apwl[p]) != Real(0.0)) lnB -= Real(m.apwl[p]) * phi * in;
-            // ln(2 f_ani): f_ani = Gii / Eii is 1 up to rounding for isotropic rates,
-            // where ln 2 + x - x^2/2 + x^3/3 (x = f_ani - 1, |x| < 2^-20) is exact
-            // to rounding and spares an FP64 logarithm
-            const Real xf = f_ani - Real(1.0);
-            const Real LE = mlog(Eii),
-                       LF = mfabs(xf) < Real(9.5367431640625e-07)
-                                ? Real(0.69314718055994530942) + xf * (Real(1.0) + xf * (Real(-0.5) + xf * Real(1.0 / 3.0)))
-                                : mlog(Real(2.0) * f_ani);   // ln 2; 2^-20
-            lnTE = LF + LE;   // ln(2 f_ani Eii) = ln Tii - ln eta_ve
-            lnC_pwl = -n_pwl * (LF + lnB);
+            Real lnB = m.lnK_pwl + (m.Q_pwl + P * m.V_pwl) * iRT * in;
+            if (fl & VP_PWL_D) lnB += m.md_pwl * mlog(d);
+            if (fl & VP_PWL_PHI) lnB -= m.a_pwl * phi;
+            const Real ln2 = Real(0.69314718055994530942), LE = mlog(Eii);
+            lnTE = ln2 + LE;   // ln(2 Eii) = ln Tii - ln eta_ve
+            lnC_pwl = -n_pwl * (ln2 + lnB);
             C_pwl = mexp(lnC_pwl);
             ln_eta_pwl = lnB + (in - Real(1.0)) * LE;
             eta_pwl = mexp(ln_eta_pwl);
         } else {
-            Real B_pwl = Real(m.pref_pwl[p]) * Real(m.Fpwl[p]) * fpow(Real(m.Apwl[p]), -in) * mexp((Real(m.Qpwl[p]) + P * Va_pwl) * iRT * in) *
-                           fpow(d, Real(m.mpwl[p]) * in) * fpow(Real(m.fpwl[p]), -Real(m.rpwl[p]) * in) * fexp(-Real(m.apwl[p]) * phi * in);
-            C_pwl = fpow(Real(2.0) * f_ani * B_pwl, -n_pwl);
-            eta_pwl = B_pwl * fpow(Eii, in - Real(1.0));
+            Real B_pwl = m.K0_pwl * mexp((m.Q_pwl + P * m.V_pwl) * iRT * in);
+            if (fl & VP_PWL_D) B_pwl *= mpow(d, m.md_pwl);
+            if (fl & VP_PWL_PHI) B_pwl *= mexp(-m.a_pwl * phi);
+            C_pwl = mpow(Real(2.0) * B_pwl, -n_pwl);
+            eta_pwl = B_pwl * mpow(Eii, in - Real(1.0));
         }
-        dCpwldP = -C_pwl * Va_pwl * iRT;
     }
+    Real B_lin = 0;
     if (diffusion) {
-        const Real in = Real(1.0) / n_lin;
-        B_lin = Real(m.Flin[p]) * fpow(Real(m.Alin[p]), -in) * mexp((Real(m.Qlin[p]) + P * Real(m.Vlin[p])) * iRT * in) *
-                fpow(Real(m.flin[p]), -Real(m.rlin[p]) * in) * fexp(-Real(m.alin[p]) * phi * in);
-        C_lin = fpow(Real(2.0) * f_ani * B_lin, -n_lin);
-        dClindP = -C_lin * Real(m.Vlin[p]) * iRT;
-        eta_lin = B_lin * fpow(Eii, in - Real(1.0)) * fpow(d, m_lin * in);
+        B_lin = m.K0_lin * mexp((m.Q_lin + P * m.V_lin) * iRT * m.in_lin);
+        if (fl & VP_LIN_PHI) B_lin *= mexp(-m.a_lin * phi);
+        C_lin = lin1 ? Real(0.5) / B_lin : mpow(Real(2.0) * B_lin, -n_lin);
+        eta_lin = lin1 ? B_lin : B_lin * mpow(Eii, m.in_lin - Real(1.0));
+        if (fl & VP_LIN_D) eta_lin *= mpow(d, m.m_lin * m.in_lin);
     }
     // grain-boundary sliding: a creep law of the dislocation form (:176-180)
-    const Real n_gbs = Real(m.ngbs[p]);
     Real C_gbs = Real(0.0), eta_gbs = Real(0.0);
     if (gbs) {
-        const Real in = Real(1.0) / n_gbs;
-        const Real B_gbs = Real(m.Fgbs[p]) * fpow(Real(m.Agbs[p]), -in) *
-                           mexp((Real(m.Qgbs[p]) + P * Real(m.Vgbs[p])) * iRT * in) * fpow(d, Real(m.mgbs[p]) * in) *
-                           fpow(Real(m.fgbs[p]), -Real(m.rgbs[p]) * in) * fexp(-Real(m.agbs[p]) * phi * in);
-        C_gbs = fpow(Real(2.0) * f_ani * B_gbs, -n_gbs);
-        eta_gbs = B_gbs * fpow(Eii, in - Real(1.0));
+        Real B_gbs = m.K0_gbs * mexp((m.Q_gbs + P * m.V_gbs) * iRT * m.in_gbs);
+        if (fl & VP_GBS_D) B_gbs *= mpow(d, m.md_gbs);
+        if (fl & VP_GBS_PHI) B_gbs *= mexp(-m.a_gbs * phi);
+        C_gbs = mpow(Real(2.0) * B_gbs, -m.n_gbs);
+        eta_gbs = B_gbs * mpow(Eii, m.in_gbs - Real(1.0));
     }
     // Peierls creep, exponential law as a power law of exponent ST + n
     // (:181-199): ST = Q / RT 2 gamma (1 - gamma)
-    const Real n_exp = Real(m.nexp[p]);
+    const Real n_exp = m.nexp;
     Real ST = Real(0.0), B_exp = Real(0.0), C_exp = Real(0.0), eta_exp = Real(0.0);
     if (peierls) {
-        const Real gam = Real(m.Gexp[p]), Ea = Real(m.Qexp[p]);
+        const Real gam = m.Gexp, Ea = m.Qexp;
         ST = Ea * iRT * Real(2.0) * gam * (Real(1.0) - gam);
         const Real sn = ST + n_exp, isn = Real(1.0) / sn;
         const Real Arr = mexp(-Ea * iRT * (Real(1.0) - gam) * (Real(1.0) - gam));
         const Real F_exp = mpow(mpow(Real(2.0), Real(1.0) - ST - n_exp) / mpow(msqrt(Real(3.0)), sn + Real(1.0)), isn);
-        B_exp = F_exp * (mpow(gam * Real(m.Sexp[p]), ST * isn) / mpow(Real(m.Eexp[p]) * Arr, isn));
-        C_exp = mpow(Real(2.0) * f_ani * B_exp, -sn);
+        B_exp = F_exp * (mpow(gam * m.Sexp, ST * isn) / mpow(m.Eexp * Arr, isn));
+        C_exp = mpow(Real(2.0) * B_exp, -sn);
         eta_exp = B_exp * mpow(Eii, isn - Real(1.0));
     }
     Real cos_fric, sin_fric;
     msincos(fric, &sin_fric, &cos_fric);
     Real sin_dil = dil == Real(0.0) ? Real(0.0) : msin(dil);
     Real Tyield = C * cos_fric + P * sin_fric;
-    if (Real(m.Slim[p]) < Tyield) { sin_fric = Real(0.0); cos_fric = Real(1.0); sin_dil = Real(0.0); C = Real(m.Slim[p]); Tyield = Real(m.Slim[p]); }
+    if (m.Slim < Tyield) { sin_fric = Real(0.0); cos_fric = Real(1.0); sin_dil = Real(0.0); C = m.Slim; Tyield = m.Slim; }
     // tension cut-off (:204-213): below the tension pressure -25 MPa the yield
     // line turns to pass through (P_tens, 0)
     bool tens = false;
     if (tensile) {
-        const Real P_tens = Real(-25e6) / Real(prm.scale_S);
-        const Real sin_fric_tens = -C * cos_fric / P_tens;
+        const Real sin_fric_tens = -C * cos_fric / prm.P_tens;
         if (C * cos_fric + P * sin_fric_tens < Tyield) {
             sin_fric = sin_fric_tens;
             Tyield = C * cos_fric + P * sin_fric_tens;
@@ -309,10 +356,8 @@ __device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Re
         }
     }
     o.X1 = X0;
-    const Real eta_el = G * dt;
-    if (constant) eta_cst = Real(m.eta0[p]);
-    Real eta_up = Real(1.0e100) / Real(prm.scale_eta);
-    if (constant) eta_up = dmin(eta_up, eta_cst);
+    Real eta_up = prm.eta_big;
+    if (constant) eta_up = dmin(eta_up, m.eta0);
     if (dislocation) eta_up = dmin(eta_up, eta_pwl);
     if (elastic) eta_up = dmin(eta_up, eta_el);
     if (peierls) eta_up = dmin(eta_up, eta_exp);
@@ -320,12 +365,14 @@ __device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Re
     if (gbs) eta_up = dmin(eta_up, eta_gbs);
     // local Newton on the visco-elastic viscosity
     Real eta_ve = eta_up, Tii;
-    const Real dm_lin = fpow(o.d1, -m_lin);
+    const Real dm_lin = m.dm_lin;
     bool ve_done = false;
     o.eta_up = eta_up;
     o.learned = guess != nullptr;
     o.fallback = 0;
-    const Real i2eta_el = Real(0.5) / eta_el, ifcst = constant ? Real(0.5) / (f_ani * eta_cst) : Real(0.0);
+    const Real ifcst = constant ? Real(0.5) * m.ieta0 : Real(0.0), iel = elastic ? i2eta_el : Real(0.0);
+    // logarithm of the start, known where dislocation creep sets it
+    const bool start_pwl = logform && eta_up == eta_pwl;
     if (guess) {
         // Learned start s = mlog(eta_ve), polished by Halley steps on
         // g(s) = mlog(sum of the strain rates) - mlog(Eii): every mechanism's
@@ -335,14 +382,14 @@ __device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Re
         // means the reference's own test below holds.  The network predicts
         // ln(eta_ve / eta_up), eta_up being the reference's start (the
         // smallest viscosity of the active mechanisms).
-        Real s = (logform && eta_up == eta_pwl ? ln_eta_pwl : mlog(eta_up)) + (Real)guess[0];
+        Real s = (start_pwl ? ln_eta_pwl : mlog(eta_up)) + (Real)guess[0];
         for (it = 0; it <= MDZ_POLISH_STEPS; it++) {
             eta_ve = mexp(s);
-            Tii = Real(2.0) * f_ani * eta_ve * Eii;
-            const Real Eel = elastic ? Tii * i2eta_el : Real(0.0);
-            if (constant) Eii_cst = Tii * ifcst;
-            if (dislocation) Eii_pwl = logform ? mexp(lnC_pwl + n_pwl * (lnTE + s)) : C_pwl * fpow(Tii, n_pwl);
-            if (diffusion) Eii_lin = C_lin * fpow(Tii, n_lin) * dm_lin;
+            Tii = Real(2.0) * eta_ve * Eii;
+            const Real Eel = Tii * iel;
+            Eii_cst = Tii * ifcst;
+            if (dislocation) Eii_pwl = logform ? mexp(lnC_pwl + n_pwl * (lnTE + s)) : C_pwl * mpow(Tii, n_pwl);
+            if (diffusion) Eii_lin = C_lin * (lin1 ? Tii : mpow(Tii, n_lin)) * dm_lin;
             const Real S0 = Eel + Eii_pwl + Eii_lin + Eii_cst;
             res = mfabs((Eii - S0) * iEii);
             // a start is accepted only after one update: a warm start can
@@ -352,8 +399,9 @@ __device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Re
             if (it > 0 && res < tol / 100) { ve_done = true; break; }
             if (it == MDZ_POLISH_STEPS) break;
             if (!(S0 > Real(0.0))) break;
-            const Real S1 = Eel + n_pwl * Eii_pwl + n_lin * Eii_lin + Eii_cst;
-            const Real S2 = Eel + n_pwl * n_pwl * Eii_pwl + n_lin * n_lin * Eii_lin + Eii_cst;
+            const Real E1 = n_pwl * Eii_pwl, E2 = lin1 ? Eii_lin : n_lin * Eii_lin;
+            const Real S1 = Eel + E1 + E2 + Eii_cst;
+            const Real S2 = Eel + n_pwl * E1 + (lin1 ? E2 : n_lin * E2) + Eii_cst;
             const Real iS0 = Real(1.0) / S0;
             const Real q = S0 * iEii;
             const Real g = (sizeof(Real) == 8 && mfabs(q - Real(1.0)) < Real(0.03125)) ? Real(ln1p_series(double(q - Real(1.0)))) : mlog(q);
@@ -368,94 +416,116 @@ __device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Re
             Eii_pwl = 0; Eii_lin = 0; Eii_cst = 0;
         }
     }
-    const Real dfel = elastic ? -Eii / eta_el : Real(0.0), dfcst = constant ? -Eii / eta_cst : Real(0.0);
+    // the reference's Newton iteration, eta_ve -= r / f', with f' multiplied by eta_ve
+    const Real dfl = -Real(2.0) * Eii * (iel + ifcst);
     for (it = 0; !ve_done && it < nitmax; it++) {
-        Tii = Real(2.0) * f_ani * eta_ve * Eii;
-        if (constant) Eii_cst = Tii * ifcst;
-        if (dislocation) Eii_pwl = C_pwl * fpow(Tii, n_pwl);
-        if (gbs) Eii_gbs = C_gbs * fpow(Tii, n_gbs);
+        Tii = Real(2.0) * eta_ve * Eii;
+        Eii_cst = Tii * ifcst;
+        if (dislocation) {
+            if (logform) Eii_pwl = mexp(lnC_pwl + n_pwl * (lnTE + (it == 0 && start_pwl ? ln_eta_pwl : mlog(eta_ve))));
+            else Eii_pwl = C_pwl * mpow(Tii, n_pwl);
+        }
+        if (gbs) Eii_gbs = C_gbs * mpow(Tii, m.n_gbs);
         if (peierls) Eii_exp = C_exp * mpow(Tii, ST + n_exp);
-        if (diffusion) Eii_lin = C_lin * fpow(Tii, n_lin) * dm_lin;
-        Real r = Eii - elastic * Tii * i2eta_el - (Eii_pwl + Eii_exp + Eii_lin + Eii_gbs + Eii_cst);
+        if (diffusion) Eii_lin = C_lin * (lin1 ? Tii : mpow(Tii, n_lin)) * dm_lin;
+        const Real r = Eii - Tii * iel - (Eii_pwl + Eii_exp + Eii_lin + Eii_gbs + Eii_cst);
         res = mfabs(r * iEii);
         if (res < tol / 100) break;
-        const Real ieta = Real(1.0) / eta_ve;
-        Real dfdeta = dfel + dfcst;
         // (grain-boundary sliding has no term here in the reference)
-        if (peierls) dfdeta += -Eii_exp * (ST + n_exp) * ieta;
-        if (diffusion) dfdeta += -Eii_lin * n_lin * ieta;
-        if (dislocation) dfdeta += -Eii_pwl * n_pwl * ieta;
-        eta_ve -= r / dfdeta;
+        Real S1 = (lin1 ? Eii_lin : Eii_lin * n_lin) + Eii_pwl * n_pwl;
+        if (peierls) S1 += Eii_exp * (ST + n_exp);
+        eta_ve -= r * eta_ve / (dfl * eta_ve - S1);
     }
     if (!ve_done) {   // iterations of a failed polish count too
         o.ve_its = it + (guess ? MDZ_POLISH_STEPS : 0);
         if (it == nitmax - 1 && res > tol) o.ve_fail = 1;
     }
     o.eta_ve = eta_ve;
-    // Eii_pwl = C_pwl Tii^n_pwl was evaluated at the final eta_ve when the
-    // iteration stopped on its convergence test (not when it ran out): then
-    // Tii^n_pwl is Eii_pwl / C_pwl, and the powers of Tii below follow from it
-    // without another FP64 pow each
-    const bool pwl_fresh = dislocation && (ve_done || res < tol / 100) && C_pwl > Real(0.0) && Eii_pwl > Real(0.0);
-    Tii = Real(2.0) * eta_ve * f_ani * Eii;
-    const Real Tn = !dislocation ? Real(0.0) : (pwl_fresh ? Eii_pwl / C_pwl : fpow(Tii, n_pwl));   // Tii^n_pwl
-    const Real iTii = Real(1.0) / Tii, TG = Tii * iGii;   // Tii / (f_ani Eii) = Tii / Gii
-    Real Txx = Gxx * TG, Tzz = Gzz * TG, Txz = Gxz * TG;
+    // the rates were evaluated at the final eta_ve when the iteration stopped
+    // on its convergence test (not when it ran out): viscosities and powers of
+    // Tii below then follow from them, eta_k = Tii / (2 Eii_k) and
+    // C_pwl Tii^n = Eii_pwl, without another FP64 pow each
+    const bool fresh = ve_done || res < tol / 100;
+    Tii = Real(2.0) * eta_ve * Eii;
+    if (dislocation && !fresh) Eii_pwl = C_pwl * mpow(Tii, n_pwl);
+    const Real iTii = Real(1.0) / Tii, two_eta = Real(2.0) * eta_ve;   // Tii / Eii
+    Real Txx = Exx * two_eta, Tzz = Ezz * two_eta, Txz = Exz * two_eta;
     Real Exx_lin = 0, Ezz_lin = 0, Exz_lin = 0, Exx_cst = 0, Ezz_cst = 0, Exz_cst = 0;
     Real Exx_exp = 0, Ezz_exp = 0, Exz_exp = 0;
+    Real inv_eta_diss = Real(0.0);
     if (peierls) {
         eta_exp = B_exp * mpow(Eii_exp, Real(1.0) / (ST + n_exp) - Real(1.0));
         const Real h = Real(0.5) / eta_exp;
+        inv_eta_diss += Real(2.0) * h;
         Exx_exp = Txx * h; Ezz_exp = Tzz * h; Exz_exp = Txz * h;
     }
-    if (dislocation) eta_pwl = Tii / (Real(2.0) * C_pwl * Tn);   // (2 C)^-1 Tii^(1-n)
+    Real h_pwl = Eii_pwl * iTii;   // 1 / (2 eta_pwl) = C_pwl Tii^(n-1)
+    if (dislocation) inv_eta_diss += Real(2.0) * h_pwl;
     if (diffusion) {
-        const Real in = Real(1.0) / n_lin;
-        eta_lin = B_lin * fpow(Eii_lin, in - Real(1.0)) * fpow(o.d1, m_lin * in);
-        const Real h = Real(0.5) / eta_lin;
+        const Real h = fresh ? Eii_lin * iTii
+                             : Real(0.5) / (B_lin * (lin1 ? Real(1.0) : mpow(Eii_lin, m.in_lin - Real(1.0))) * m.dmn_lin);
+        inv_eta_diss += Real(2.0) * h;
         Exx_lin = Txx * h; Ezz_lin = Tzz * h; Exz_lin = Txz * h;
     }
     if (constant) {
-        const Real h = Real(0.5) / eta_cst;
+        const Real h = Real(0.5) * m.ieta0;
+        inv_eta_diss += m.ieta0;
         Exx_cst = Txx * h; Ezz_cst = Tzz * h; Exz_cst = Txz * h;
     }
     // visco-elastic tangent
     Real deta = Real(0.0);
-    if (dislocation) deta += -C_pwl * (Tn * iTii * iTii * iTii) * (n_pwl - Real(1.0));   // Tii^(n-3)
+    if (dislocation) deta += -(Eii_pwl * iTii * iTii * iTii) * (n_pwl - Real(1.0));   // C Tii^(n-3)
     if (peierls) deta += -C_exp * mpow(Tii, n_exp + ST - Real(3.0)) * (n_exp + ST - Real(1.0));
-    if (diffusion) deta += -C_lin * fpow(Tii, n_lin - Real(3.0)) * (n_lin - Real(1.0)) * dm_lin;
-    const Real e2 = fpow(eta_ve, Real(2.0));
-    Real dTxx = deta * (Real(2.0) * Txx + Tzz) * e2, dTzz = deta * (Real(2.0) * Tzz + Txx) * e2, dTxz = Real(2.0) * deta * Txz * e2;
-    Real den = Real(1.0) - Real(2.0) * (dTxx * Exx + dTzz * Ezz + dTxz * Exz);
-    const Real e2den = Real(2.0) * eta_ve / den;
-    Real dve_dExx = dTxx * e2den, dve_dEzz = dTzz * e2den;
-    Real dve_dExz = dTxz * e2den;
-    Real dummy = Real(0.0), Jii = Tii * Tii;
-    if (dislocation) dummy += -Real(2.0) * (Tn * iTii) * dCpwldP;   // Jii^((n-1)/2) = Tii^(n-1)
-    if (diffusion) dummy += -Real(2.0) * fpow(Jii, (Real(1.0) / Real(2.0)) * n_lin - Real(1.0) / Real(2.0)) * fpow(d, -m_lin) * dClindP;
-    Real dve_dP = fpow(eta_ve, 2) * dummy;
+    if (diffusion && !lin1) deta += -C_lin * mpow(Tii, n_lin - Real(3.0)) * (n_lin - Real(1.0)) * dm_lin;
+    const Real e2 = eta_ve * eta_ve, de2 = deta * e2;
+    const Real dTxx = de2 * (Real(2.0) * Txx + Tzz), dTzz = de2 * (Real(2.0) * Tzz + Txx), dTxz = Real(2.0) * de2 * Txz;
+    const Real den = Real(1.0) - Real(2.0) * (dTxx * Exx + dTzz * Ezz + dTxz * Exz);
+    const Real e2den = two_eta / den;
+    const Real dve_dExx = dTxx * e2den, dve_dEzz = dTzz * e2den, dve_dExz = dTxz * e2den;
+    Real dummy = Real(0.0);
+    if (dislocation) dummy += Real(2.0) * h_pwl * m.V_pwl * iRT;   // -2 Tii^(n-1) dC/dP, dC/dP = -C V / RT
+    if (diffusion && m.V_lin != Real(0.0)) {
+        Real t = Real(2.0) * C_lin * m.V_lin * iRT;
+        if (!lin1) t *= mpow(Tii, n_lin - Real(1.0));
+        if (fl & VP_LIN_D) t *= mpow(d, -m.m_lin);
+        dummy += t;
+    }
+    const Real dve_dP = e2 * dummy;
     // plastic return mapping on gdot
     Real gdot = Real(0.0), dQdtxx = 0, dQdtzz = 0, dQdtxz = 0, dQdP = 0, divp = Real(0.0), Pc = P;
     Real dlamdExx = 0, dlamdEzz = 0, dlamdExz = 0, dlamdP = 0;
     Real dvep_dExx = 0, dvep_dEzz = 0, dvep_dExz = 0, dvep_dP = 0;
     Real F_trial = Tii - Tyield;
+    const bool is_pl = F_trial > Real(1e-17);
+    Real Kdt = Real(0.0);
+    if (is_pl || tens) Kdt = elastic ? dt / beta : Real(1e1) * dt;
     // tensile domain: the dilation angle that returns the stress to the
     // tension corner (:456-465, SimpleYields.m of the reference)
     if (tens) {
-        eta_vp = eta_vp0 * fpow(Eii, Real(1.0) / n_vp - Real(1.0));
+        eta_vp = vp1 ? eta_vp0 : eta_vp0 * mpow(Eii, m.in_vp - Real(1.0));
         const Real Pc_chk = -(C * cos_fric) / (-Tii / P + sin_fric);
         sin_dil = (P * eta_ve + P * eta_vp - Pc_chk * eta_ve - Pc_chk * eta_vp) /
-                  (K * dt * (C * cos_fric + Pc_chk * sin_fric - Tii));
+                  (Kdt * (C * cos_fric + Pc_chk * sin_fric - Tii));
     }
-    const bool is_pl = F_trial > Real(1e-17);
     Real dsdExx = Real(0.0), dsdEzz = Real(0.0), dsdExz = Real(0.0), dsdP = Real(0.0);   // d sin_dil / d .
     if (is_pl) {
-        const Real in_vp = Real(1.0) / n_vp;
-        eta_vp = eta_vp0 * fpow(Eii, in_vp - 1);
-        gdot = F_trial / (eta_ve + eta_vp + K * dt * sin_fric * sin_dil);
-        dQdtxx = Txx * Real(0.5) * iTii; dQdtzz = Tzz * Real(0.5) * iTii; dQdtxz = Txz * iTii;
-        const Real F_trial0 = F_trial, iF0 = Real(1.0) / F_trial0;
+        const Real in_vp = m.in_vp, Kss = Kdt * sin_fric * sin_dil, Ccf = C * cos_fric;
+        eta_vp = vp1 ? eta_vp0 : eta_vp0 * mpow(Eii, in_vp - Real(1.0));
+        gdot = F_trial / (eta_ve + eta_vp + Kss);
+        const Real hT = Real(0.5) * iTii;
+        dQdtxx = Txx * hT; dQdtzz = Tzz * hT; dQdtxz = Txz * iTii;
+        const Real tol0 = tol * F_trial;   // |F| / F_trial0 < tol
+        dQdP = -sin_dil;
         bool vp_done = false;
+        auto eval = [&]() {   // F at gdot (Pc, eta_vp, Tyield)
+            divp = gdot * sin_dil;
+            Pc = P + Kdt * divp;
+            if (!vp1) eta_vp = eta_vp0 * mpow(mfabs(gdot), in_vp - Real(1.0));
+            Tyield = Ccf + Pc * sin_fric + gdot * eta_vp;
+            F_trial = Tii - eta_ve * gdot - Tyield;
+            res = mfabs(F_trial);
+            return res < tol || res < tol0;
+        };
         if (guess) {
             // learned start: gdot = fraction * 2 Eii, at most MDZ_POLISH_STEPS
             // Newton updates, the reference's own convergence test
@@ -464,17 +534,10 @@ __device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Re
             const Real gdot_plain = gdot;
             gdot = frac * Real(2.0) * Eii;
             for (it = 0; it <= MDZ_POLISH_STEPS; it++) {
-                dQdP = -sin_dil;
-                divp = -gdot * dQdP;
-                Pc = P + K * dt * divp;
-                eta_vp = eta_vp0 * fpow(mfabs(gdot), in_vp - Real(1.0));
-                Tyield = C * cos_fric + Pc * sin_fric + gdot * eta_vp;
-                F_trial = Tii - eta_ve * gdot - Tyield;
-                res = mfabs(F_trial);
-                if (it > 0 && (res < tol || res * iF0 < tol)) { vp_done = true; break; }
+                const bool ok = eval();
+                if (it > 0 && ok) { vp_done = true; break; }
                 if (it == MDZ_POLISH_STEPS) break;
-                Real dFdgdot = -eta_ve - eta_vp * in_vp - K * dt * sin_fric * sin_dil;
-                gdot -= F_trial / dFdgdot;
+                gdot += F_trial / (eta_ve + eta_vp * in_vp + Kss);
             }
             o.vp_its = it;
             if (!vp_done) {
@@ -483,77 +546,62 @@ __device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Re
             }
         }
         for (it = 0; !vp_done && it < nitmax; it++) {
-            dQdP = -sin_dil;
-            divp = -gdot * dQdP;
-            Pc = P + K * dt * divp;
-            eta_vp = eta_vp0 * fpow(mfabs(gdot), in_vp - Real(1.0));
-            Tyield = C * cos_fric + Pc * sin_fric + gdot * eta_vp;
-            F_trial = Tii - eta_ve * gdot - Tyield;
-            res = mfabs(F_trial);
-            if (res < tol || res * iF0 < tol) break;
-            Real dFdgdot = -eta_ve - eta_vp * in_vp - K * dt * sin_fric * sin_dil;
-            gdot -= F_trial / dFdgdot;
+            if (eval()) break;
+            gdot += F_trial / (eta_ve + eta_vp * in_vp + Kss);
         }
         if (!vp_done) {
             o.vp_its = it + (guess ? MDZ_POLISH_STEPS : 0);
-            if (it == nitmax - 1 && (res > tol || res * iF0 > tol)) o.vp_fail = 1;
+            if (it == nitmax - 1 && (res > tol || res > tol0)) o.vp_fail = 1;
         }
-        Txx = Real(2.0) * eta_ve * (Exx - gdot * dQdtxx);
-        Tzz = Real(2.0) * eta_ve * (Ezz - gdot * dQdtzz);
-        Real Tyy = -(Txx + Tzz);
-        Txz = Real(2.0) * eta_ve * (Exz - gdot * dQdtxz / Real(2.0));
-        Tii = msqrt(Real(0.5) * (fpow(Txx, Real(2.0)) + fpow(Tzz, Real(2.0)) + fpow(Tyy, Real(2.0))) + fpow(Txz, Real(2.0)));
+        Txx = two_eta * (Exx - gdot * dQdtxx);
+        Tzz = two_eta * (Ezz - gdot * dQdtzz);
+        const Real Tyy = -(Txx + Tzz);
+        Txz = two_eta * (Exz - gdot * dQdtxz * Real(0.5));
+        Tii = msqrt(Real(0.5) * (Txx * Txx + Tzz * Tzz + Tyy * Tyy) + Txz * Txz);
         eta_vep = Tii * Real(0.5) * iEii;
-        o.Eii_pl = gdot / Real(2.0);
-        Tii = Real(2.0) * eta_vep * Eii;
+        o.Eii_pl = gdot * Real(0.5);
         o.OverS = eta_vp * gdot;
         o.Pcorr = Pc;
         // visco-elasto-plastic tangent
         if (tens) {   // derivatives of the tensile dilation angle (:578-587)
             const Real dEii_dExx = (Real(2.0) * Exx + Ezz) * Real(0.5) * iEii, dEii_dEzz = (Real(2.0) * Ezz + Exx) * Real(0.5) * iEii;
             const Real dEii_dExz = Exz * iEii;
-            const Real Ccf = C * cos_fric, A = Real(2.0) * Eii * eta_ve - P * sin_fric, A2 = A * A;
-            const Real iden = Real(1.0) / (K * dt * A * (C * P * cos_fric * sin_fric + (Ccf - Real(2.0) * Eii * eta_ve) * A));
+            const Real A = Real(2.0) * Eii * eta_ve - P * sin_fric, A2 = A * A;
+            const Real iden = Real(1.0) / (Kdt * A * (C * P * cos_fric * sin_fric + (Ccf - Real(2.0) * Eii * eta_ve) * A));
             const Real Q = C * P * cos_fric * sin_fric + A2;
             auto dsd = [&](Real dve, Real dE) {
                 const Real dT = Eii * dve + dE * eta_ve;
-                return (Real(2.0) * K * dt * sin_dil * dT * Q +
+                return (Real(2.0) * Kdt * sin_dil * dT * Q +
                         P * (-Ccf * dve * A + Real(2.0) * Ccf * (eta_ve + eta_vp) * dT + dve * A2)) * iden;
             };
             dsdExx = dsd(dve_dExx, dEii_dExx);
             dsdEzz = dsd(dve_dEzz, dEii_dEzz);
             dsdExz = dsd(dve_dExz, dEii_dExz);
             dsdP = (Real(2.0) * C * Eii * cos_fric * (eta_ve + eta_vp) * (P * dve_dP - eta_ve) - C * P * cos_fric * dve_dP * A +
-                    Real(2.0) * Eii * K * dt * sin_dil * (C * cos_fric * sin_fric * (P * dve_dP - eta_ve) + dve_dP * A2) +
+                    Real(2.0) * Eii * Kdt * sin_dil * (C * cos_fric * sin_fric * (P * dve_dP - eta_ve) + dve_dP * A2) +
                     A2 * (P * dve_dP + eta_ve + eta_vp)) * iden;
         }
-        const Real ev = eta_ve * iEii;
-        Real dFdExx = (Real(2.0) * Exx + Ezz) * ev + Real(2.0) * Eii * dve_dExx;
-        Real dFdEzz = (Real(2.0) * Ezz + Exx) * ev + Real(2.0) * Eii * dve_dEzz;
-        Real dFdExz = Real(2.0) * Exz * ev + Real(2.0) * Eii * dve_dExz;
-        Real dFdP = -sin_fric + Real(2.0) * Eii * dve_dP;
-        Real gg = Real(1.0) / (eta_ve + eta_vp * in_vp + K * dt * sin_fric * sin_dil);
-        dlamdExx = gg * (dFdExx - gdot * (dve_dExx + K * dt * sin_fric * dsdExx));
-        dlamdEzz = gg * (dFdEzz - gdot * (dve_dEzz + K * dt * sin_fric * dsdEzz));
-        dlamdExz = gg * (dFdExz - gdot * (dve_dExz + K * dt * sin_fric * dsdExz));
-        dlamdP = gg * (dFdP - gdot * (dve_dP + K * dt * sin_fric * dsdP));
-        Real q = in_vp - Real(1.0);
-        const Real evg = eta_vp / gdot;
-        Real dvp_dExx = evg * dlamdExx * q, dvp_dEzz = evg * dlamdEzz * q;
-        Real dvp_dExz = evg * dlamdExz * q, dvp_dP = evg * dlamdP * q;
-        Real a = eta_vp + K * dt * sin_fric * sin_dil;
-        const Real TyE3 = Tyield * Real(0.5) * iEii * iEii * iEii, h2 = Real(0.5) * iEii;   // Tyield / (2 Eii^3), 1 / (2 Eii)
-        dvep_dExx = -Real(0.5) * (Real(2.0) * Exx + Ezz) * TyE3 + (a * dlamdExx + gdot * dvp_dExx + gdot * K * dt * sin_fric * dsdExx) * h2;
-        dvep_dEzz = -Real(0.5) * (Real(2.0) * Ezz + Exx) * TyE3 + (a * dlamdEzz + gdot * dvp_dEzz + gdot * K * dt * sin_fric * dsdEzz) * h2;
-        dvep_dExz = -Exz * TyE3 + (a * dlamdExz + gdot * dvp_dExz + gdot * K * dt * sin_fric * dsdExz) * h2;
-        dvep_dP = (sin_fric + a * dlamdP + gdot * dvp_dP + gdot * K * dt * sin_fric * dsdP) * h2;
+        const Real ev = eta_ve * iEii, E2 = Real(2.0) * Eii, Ksf = Kdt * sin_fric;
+        const Real xx2 = Real(2.0) * Exx + Ezz, zz2 = Real(2.0) * Ezz + Exx;
+        const Real gg = Real(1.0) / (eta_ve + eta_vp * in_vp + Kss);
+        dlamdExx = gg * (xx2 * ev + E2 * dve_dExx - gdot * (dve_dExx + Ksf * dsdExx));
+        dlamdEzz = gg * (zz2 * ev + E2 * dve_dEzz - gdot * (dve_dEzz + Ksf * dsdEzz));
+        dlamdExz = gg * (Real(2.0) * Exz * ev + E2 * dve_dExz - gdot * (dve_dExz + Ksf * dsdExz));
+        dlamdP = gg * (-sin_fric + E2 * dve_dP - gdot * (dve_dP + Ksf * dsdP));
+        Real dvp_dExx = 0, dvp_dEzz = 0, dvp_dExz = 0, dvp_dP = 0;   // (linear regularisation: constant eta_vp)
+        if (!vp1) {
+            const Real evq = eta_vp / gdot * (in_vp - Real(1.0));
+            dvp_dExx = evq * dlamdExx; dvp_dEzz = evq * dlamdEzz;
+            dvp_dExz = evq * dlamdExz; dvp_dP = evq * dlamdP;
+        }
+        const Real a = eta_vp + Kss;
+        const Real h2 = Real(0.5) * iEii, TyE3 = Tyield * h2 * iEii * iEii;   // 1 / (2 Eii), Tyield / (2 Eii^3)
+        dvep_dExx = -Real(0.5) * xx2 * TyE3 + (a * dlamdExx + gdot * (dvp_dExx + Ksf * dsdExx)) * h2;
+        dvep_dEzz = -Real(0.5) * zz2 * TyE3 + (a * dlamdEzz + gdot * (dvp_dEzz + Ksf * dsdEzz)) * h2;
+        dvep_dExz = -Exz * TyE3 + (a * dlamdExz + gdot * (dvp_dExz + Ksf * dsdExz)) * h2;
+        dvep_dP = (sin_fric + a * dlamdP + gdot * (dvp_dP + Ksf * dsdP)) * h2;
     }
     o.gdot = gdot;
-    Real inv_eta_diss = Real(0.0);
-    if (peierls) inv_eta_diss += Real(1.0) / eta_exp;
-    if (dislocation) inv_eta_diss += Real(1.0) / eta_pwl;
-    if (diffusion) inv_eta_diss += Real(1.0) / eta_lin;
-    if (constant) inv_eta_diss += Real(1.0) / eta_cst;
     if (!is_pl) {
         o.detadexx = dve_dExx; o.detadezz = dve_dEzz; o.detadexz = dve_dExz; o.detadp = dve_dP;
         o.etaVE = eta_ve;
@@ -564,39 +612,36 @@ __device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Re
         o.ddivpdexx = -dQdP * dlamdExx + gdot * dsdExx;
         o.ddivpdezz = -dQdP * dlamdEzz + gdot * dsdEzz;
         o.ddivpdexz = -dQdP * dlamdExz + gdot * dsdExz;
-        o.ddivpdp = -dQdP * dlamdP + gdot * dsdP + Real(0.0);
+        o.ddivpdp = -dQdP * dlamdP + gdot * dsdP;
         inv_eta_diss += Real(1.0) / eta_vep;
+        // the dislocation parts of the reported rates are taken at the returned stress
+        if (dislocation)
+            h_pwl = !(C_pwl > Real(0.0)) ? Real(0.0)
+                  : logform ? mexp(lnC_pwl + (n_pwl - Real(1.0)) * mlog(Tii)) : C_pwl * mpow(Tii, n_pwl - Real(1.0));
     }
-    // eta_pwl is re-evaluated unconditionally in the reference (C_pwl = 0 when
-    // dislocation creep is off, which makes the dislocation parts vanish); Tii
-    // is still the visco-elastic one unless the plastic branch changed it
-    // 1 / (2 eta_pwl) = C_pwl Tii^(n-1): no division of the reference's
-    // fpow(2 C_pwl, -1) fpow(Tii, 1 - n) is needed where Tii^n is known
-    const Real h_pwl = !(C_pwl > Real(0.0)) ? Real(0.0) : (dislocation && !is_pl ? C_pwl * Tn * iTii : C_pwl * fpow(Tii, n_pwl - Real(1.0)));
-    eta_pwl = Real(0.5) / h_pwl;
-    o.Exx_el = (Real)elastic * (Txx - Txx0) * i2eta_el;
-    o.Ezz_el = (Real)elastic * (Tzz - Tzz0) * i2eta_el;
-    o.Exz_el = (Real)elastic * (Txz - Txz0) * i2eta_el;
+    o.Exx_el = elastic ? (Txx - Txx0) * i2eta_el : Real(0.0);
+    o.Ezz_el = elastic ? (Tzz - Tzz0) * i2eta_el : Real(0.0);
+    o.Exz_el = elastic ? (Txz - Txz0) * i2eta_el : Real(0.0);
     o.Exx_diss = gdot * dQdtxx + Exx_lin + Txx * h_pwl + Exx_exp + Exx_cst;
     o.Ezz_diss = gdot * dQdtzz + Ezz_lin + Tzz * h_pwl + Ezz_exp + Ezz_cst;
-    o.Exz_diss = gdot * dQdtxz / Real(2.0) + Exz_lin + Txz * h_pwl + Exz_exp + Exz_cst;
-    o.Eii_el = (Real)elastic * mfabs(Tii - Tii0) * i2eta_el;
+    o.Exz_diss = gdot * dQdtxz * Real(0.5) + Exz_lin + Txz * h_pwl + Exz_exp + Exz_cst;
+    o.Eii_el = elastic ? mfabs(Tii - Tii0) * i2eta_el : Real(0.0);
     o.Eii_pwl = Tii * h_pwl;
     o.Eii_lin = Eii_lin;
     o.Eii_cst = Eii_cst;
     o.Eii_exp = Eii_exp;
     o.Eii_gbs = Eii_gbs;
     o.div_pl = divp;
-    o.div_el = -(Pc - P0) / (K * dt);
+    o.div_el = -(Pc - P0) * (elastic ? beta * prm.idt : Real(0.1) * prm.idt);
     Real eta = Real(1.0) / inv_eta_diss;
-    o.VEcoeff = elastic == 0 ? Real(0.0) : Real(2.0) * eta_ve * i2eta_el;
+    o.VEcoeff = elastic ? two_eta * i2eta_el : Real(0.0);
     if (prm.step == 0) o.etaVE = eta;
     o.txx = Txx; o.tzz = Tzz; o.txz = Txz;
-    if (eta > Real(prm.maxeta)) eta = Real(prm.maxeta);
-    if (eta < Real(prm.mineta)) eta = Real(prm.mineta);
-    const bool clamped = o.etaVE > Real(prm.maxeta) || o.etaVE < Real(prm.mineta);
-    if (o.etaVE > Real(prm.maxeta)) o.etaVE = Real(prm.maxeta);
-    if (o.etaVE < Real(prm.mineta)) o.etaVE = Real(prm.mineta);
+    if (eta > prm.maxeta) eta = prm.maxeta;
+    if (eta < prm.mineta) eta = prm.mineta;
+    const bool clamped = o.etaVE > prm.maxeta || o.etaVE < prm.mineta;
+    if (o.etaVE > prm.maxeta) o.etaVE = prm.maxeta;
+    if (o.etaVE < prm.mineta) o.etaVE = prm.mineta;
     if (clamped && prm.clamp_tangent) {   // the limiter is flat: its tangent is zero
         o.detadexx = Real(0.0); o.detadezz = Real(0.0); o.detadexz = Real(0.0); o.detadp = Real(0.0);
     }
@@ -607,57 +652,50 @@ __device__ void visc_local_t(int p, Real G, Real T, Real P, Real d, Real phi, Re
     o.lab_y = (float)(gdot * Real(0.5) * iEii);
 }
 
-
-// The reference's local solve in FP64 (all call sites but the inexact FP32
-// evaluations of k_viscosity_* use this one).
-__device__ __forceinline__ void visc_local(int p, double G, double T, double P, double d, double phi, double X0,
-                                           double Exx, double Ezz, double Exz, double Gxx, double Gzz, double Gxz,
-                                           double Txx0, double Tzz0, double Txz0, const mdz_mat_k &m,
-                                           const mdz_rheo_params &prm, double dil, double fric, double C, double P0,
-                                           double beta, visc_res &o, const float *guess = nullptr) {
-    visc_local_t<double>(p, G, T, P, d, phi, X0, Exx, Ezz, Exz, Gxx, Gzz, Gxz, Txx0, Tzz0, Txz0, m, prm, dil, fric,
-                         C, P0, beta, o, guess);
-}
+// Materials of a launch: FP64, and FP32 for the inexact evaluations.
+template <bool FP32>
+struct visc_mats {
+    visc_mat<double> d;
+    visc_mat<float> f;
+};
+template <>
+struct visc_mats<false> {
+    visc_mat<double> d;
+};
 
 // One (node, phase) local solve: in FP32 when asked (an inexact evaluation
 // for a non-linear iteration far from convergence; FP64 transcendental
 // functions issue at a small fraction of the FP32 rate on this part), with
 // the FP64 solve taking over wherever the FP32 one failed or overflowed;
 // otherwise the FP64 solve, from the learned start when one is given.
-__device__ __forceinline__ void visc_node_phase(bool fp32, int p, double G, double T, double P, double d, double phi,
-                                                double X0, const double *E, double Txx0, double Tzz0, double Txz0,
-                                                const mdz_mat_k &m, const mdz_rheo_params &prm, double dil,
-                                                double fric, double C, double P0, double beta, visc_res &o,
-                                                const float *guess) {
-    if (fp32) {
-        visc_local_t<float>(p, (float)G, (float)T, (float)P, (float)d, (float)phi, (float)X0, (float)E[0],
-                            (float)E[1], (float)E[2], (float)E[3], (float)E[4], (float)E[5], (float)Txx0,
-                            (float)Tzz0, (float)Txz0, m, prm, (float)dil, (float)fric, (float)C, (float)P0,
-                            (float)beta, o, nullptr);
+template <bool FP32>
+__device__ __forceinline__ void visc_node_phase(const visc_mats<FP32> &m, int p, double G, double ie, double T, double P,
+                                                double d, double phi, double X0, const double *E, double Txx0,
+                                                double Tzz0, double Txz0, double dil, double fric, double C, double P0,
+                                                double beta, visc_res &o, const float *guess) {
+    if constexpr (FP32) {
+        visc_local_t<float>(m.f.ph[p], m.f.prm, (float)G, (float)ie, (float)T, (float)P, (float)d, (float)phi, (float)X0,
+                            (float)E[0], (float)E[1], (float)E[2], (float)Txx0, (float)Tzz0, (float)Txz0, (float)dil,
+                            (float)fric, (float)C, (float)P0, (float)beta, o, nullptr);
         const bool ok = !o.ve_fail && !o.vp_fail && isfinite(o.eta) && isfinite(o.etaVE) && isfinite(o.txx) &&
                         isfinite(o.tzz) && isfinite(o.txz) && isfinite(o.detadexx) && isfinite(o.detadezz) &&
                         isfinite(o.detadexz) && isfinite(o.detadp) && isfinite(o.Pcorr);
         if (ok) return;
     }
-    visc_local(p, G, T, P, d, phi, X0, E[0], E[1], E[2], E[3], E[4], E[5], Txx0, Tzz0, Txz0, m, prm, dil, fric, C,
-               P0, beta, o, guess);
+    visc_local_t<double>(m.d.ph[p], m.d.prm, G, ie, T, P, d, phi, X0, E[0], E[1], E[2], Txx0, Tzz0, Txz0, dil, fric, C,
+                         P0, beta, o, guess);
 }
 
 // Effective rates entering the local solve (isotropic form of the elastic
 // stress correction, NonNewtonianViscosityGrid :1060-1094): E[0..2] Exx, Ezz,
 // Exz and E[3..5] Gxx, Gzz, Gxz, with the reference's inverse of Da evaluated
-// for ani = 0 (iDa11 = iDa22 = 1/2, iDa33 = 1, off-diagonals 0).
+// for ani = 0 (iDa11 = iDa22 = 1/2, iDa33 = 1, off-diagonals 0), where the two
+// agree; ie = 1 / (mu dt) of an elastic model, 1 otherwise.
 __device__ __forceinline__ void eff_rates(double exx, double ezz, double exz, double sxx0, double szz0, double sxz0,
-                                          double etae, double *E) {
-    const double i11 = 0.5, i22 = 0.5, i33 = 1.0, z = 0.0, ie = 1.0 / etae;   // one division, not four
-    double Exx = exx + (i11 * sxx0 + z * szz0 + z * sxz0) * ie;
-    double Ezz = ezz + (z * sxx0 + i22 * szz0 + z * sxz0) * ie;
-    double Exz = exz + (z * sxx0 + z * szz0 + i33 * sxz0) * 0.5 * ie;
-    double gxz = 2.0 * exz + (z * sxx0 + z * szz0 + i33 * sxz0) * ie;
-    E[0] = Exx; E[1] = Ezz; E[2] = Exz;
-    E[3] = Exx * 1.0 + Ezz * z + gxz * z;
-    E[4] = Ezz * 1.0 + Exx * z - gxz * z;
-    E[5] = Exx * z - Exx * z + gxz * 0.5;
+                                          double ie, double *E) {
+    const double h = 0.5 * ie, Exz = exz + sxz0 * h;
+    E[0] = exx + sxx0 * h; E[1] = ezz + szz0 * h; E[2] = Exz;
+    E[3] = E[0]; E[4] = E[1]; E[5] = Exz;
 }
 
 __device__ __forceinline__ void put(double *p, int i, double v) {
@@ -683,13 +721,15 @@ __device__ __forceinline__ void count_local(int *counters, int fails, int fallba
 }
 
 // One thread per centroid: loop over phases with a fraction above 1e-13.
-__global__ void __launch_bounds__(128) k_viscosity_centroids(mdz_dgrid g, mdz_mat_k m, mdz_rheo_params prm,
+template <bool FP32>
+__global__ void __launch_bounds__(128) k_viscosity_centroids(mdz_dgrid g, const __grid_constant__ visc_mats<FP32> m,
+                                                             mdz_rheo_params prm,
                                                              mdz_fields f, int *__restrict__ counters,
-                                                             const float2 *guess, float2 *labels, int fp32) {
+                                                             const float2 *guess, float2 *labels) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     int nc = g.ncx * g.ncz;
     if (c >= nc) return;
-    const int avg = prm.eta_avg, nph = m.n_phases;
+    const int avg = prm.eta_avg, nph = m.d.n_phases;
     double eta = 0, eta_phys = 0, VE = 0, sxx = 0, szz = 0, sxz = 0, eel = 0, epl = 0, epwl = 0, elin = 0, ecst = 0,
            eexp = 0, egbs = 0,
            dn = 0, xel = 0, xdi = 0, zel = 0, zdi = 0, dexx = 0, dezz = 0, dgxz = 0, dp = 0, vxx = 0, vzz = 0,
@@ -697,11 +737,11 @@ __global__ void __launch_bounds__(128) k_viscosity_centroids(mdz_dgrid g, mdz_ma
     int fails = 0, fallbacks = 0, learned = 0, iters = 0;
     signed char t = g.BCp[c];
     if (t != 30 && t != 31) {
-        const double etae = prm.iselastic == 1 ? prm.dt * f.mu_n[c] : 1.0;
+        const double ie = prm.iselastic == 1 ? 1.0 / (prm.dt * f.mu_n[c]) : 1.0;
         const double exx = f.exxd[c], ezz = f.ezzd[c], exz = f.exz_n[c];
         const double sxx0 = f.sxxd0[c], szz0 = f.szzd0[c], sxz0 = f.sxz0_n[c];
         double E[6];
-        eff_rates(exx, ezz, exz, sxx0, szz0, sxz0, etae, E);
+        eff_rates(exx, ezz, exz, sxx0, szz0, sxz0, ie, E);
         const double mu = f.mu_n[c], T = f.T[c], P = f.p[c], d0 = f.d0_n[c], phi0 = f.phi0_n[c];
         const double X0 = f.X0_n ? f.X0_n[c] : 0.0, P0 = f.p0_n ? f.p0_n[c] : 0.0;
         const double dil = f.dil_n[c], fric = f.fric_n[c], Coh = f.C_n[c], bet = f.bet_n[c];
@@ -714,8 +754,8 @@ __global__ void __launch_bounds__(128) k_viscosity_centroids(mdz_dgrid g, mdz_ma
                 const float2 q = guess[(size_t)p * nc + c];
                 gs[0] = q.x; gs[1] = q.y;
             }
-            visc_node_phase(fp32 != 0, p, mu, T, P, d0, phi0, X0, E, sxx0, szz0, sxz0, m, prm, dil, fric, Coh, P0, bet, o,
-                            guess ? gs : nullptr);
+            visc_node_phase<FP32>(m, p, mu, ie, T, P, d0, phi0, X0, E, sxx0, szz0, sxz0, dil, fric, Coh, P0, bet, o,
+                                  guess ? gs : nullptr);
             // labels may be the guess buffer itself: this thread read its entry above
             if (labels) labels[(size_t)p * nc + c] = make_float2(o.lab_x, o.lab_y);
             fails += o.ve_fail + o.vp_fail;
@@ -728,7 +768,7 @@ __global__ void __launch_bounds__(128) k_viscosity_centroids(mdz_dgrid g, mdz_ma
             }
             if (avg == 0 || avg == 2) { sxx += w * o.txx; szz += w * o.tzz; sxz += w * o.txz; }
             VE += w * o.VEcoeff; eel += w * o.Eii_el; epl += w * o.Eii_pl; epwl += w * o.Eii_pwl;
-            elin += w * o.Eii_lin; ecst += w * o.Eii_cst; dn += w * 1.0 / o.d1;
+            elin += w * o.Eii_lin; ecst += w * o.Eii_cst; dn += w * m.d.ph[p].igs_ref;
             eexp += w * o.Eii_exp; egbs += w * o.Eii_gbs;
             xel += w * o.Exx_el; xdi += w * o.Exx_diss; zel += w * o.Ezz_el; zdi += w * o.Ezz_diss;
             Wt += w * (o.txx * exx + o.tzz * ezz + (o.txx + o.tzz) * (exx + ezz) + 2.0 * o.txz * exz);
@@ -775,21 +815,23 @@ __global__ void __launch_bounds__(128) k_viscosity_centroids(mdz_dgrid g, mdz_ma
     count_local(counters, fails, fallbacks, learned, iters);
 }
 
-__global__ void __launch_bounds__(128) k_viscosity_vertices(mdz_dgrid g, mdz_mat_k m, mdz_rheo_params prm,
+template <bool FP32>
+__global__ void __launch_bounds__(128) k_viscosity_vertices(mdz_dgrid g, const __grid_constant__ visc_mats<FP32> m,
+                                                             mdz_rheo_params prm,
                                                             mdz_fields f, int *__restrict__ counters,
-                                                            const float2 *guess, float2 *labels, int fp32) {
+                                                            const float2 *guess, float2 *labels) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     int nv = g.Nx * g.Nz;
     if (c >= nv) return;
-    const int avg = prm.eta_avg, nph = m.n_phases;
+    const int avg = prm.eta_avg, nph = m.d.n_phases;
     double VE = 0, sxz = 0, eta_phys = 0, eta = 0, zel = 0, zdi = 0, dexx = 0, dezz = 0, dgxz = 0, dp = 0, X = 0,
            OS = 0;
     int fails = 0, fallbacks = 0, learned = 0, iters = 0;
     if (g.BCg[c] != 30) {
-        const double etae = prm.iselastic == 1 ? prm.dt * f.mu_s[c] : 1.0;
+        const double ie = prm.iselastic == 1 ? 1.0 / (prm.dt * f.mu_s[c]) : 1.0;
         const double sxx0 = f.sxxd0_s[c], szz0 = f.szzd0_s[c], sxz0 = f.sxz0[c];
         double E[6];
-        eff_rates(f.exxd_s[c], f.ezzd_s[c], f.exz[c], sxx0, szz0, sxz0, etae, E);
+        eff_rates(f.exxd_s[c], f.ezzd_s[c], f.exz[c], sxx0, szz0, sxz0, ie, E);
         const double mu = f.mu_s[c], T = f.T_s[c], P = f.P_s[c], d0 = f.d0_s[c], phi0 = f.phi0_s[c];
         const double X0 = f.X0_s ? f.X0_s[c] : 0.0, P0 = f.p0_s ? f.p0_s[c] : 0.0;
         const double dil = f.dil_s[c], fric = f.fric_s[c], Coh = f.C_s[c], bet = f.bet_s[c];
@@ -802,8 +844,8 @@ __global__ void __launch_bounds__(128) k_viscosity_vertices(mdz_dgrid g, mdz_mat
                 const float2 q = guess[(size_t)p * nv + c];
                 gs[0] = q.x; gs[1] = q.y;
             }
-            visc_node_phase(fp32 != 0, p, mu, T, P, d0, phi0, X0, E, sxx0, szz0, sxz0, m, prm, dil, fric, Coh, P0, bet, o,
-                            guess ? gs : nullptr);
+            visc_node_phase<FP32>(m, p, mu, ie, T, P, d0, phi0, X0, E, sxx0, szz0, sxz0, dil, fric, Coh, P0, bet, o,
+                                  guess ? gs : nullptr);
             // labels may be the guess buffer itself: this thread read its entry above
             if (labels) labels[(size_t)p * nv + c] = make_float2(o.lab_x, o.lab_y);
             fails += o.ve_fail + o.vp_fail;
@@ -858,8 +900,8 @@ __global__ void k_operators(mdz_dgrid g, mdz_rheo_params prm, mdz_fields f, int 
             double eta = f.eta_n[k];
             d11 = 2.0 * eta; d22 = 2.0 * eta;
             if (jacobian) {
-                double etae = prm.iselastic == 1 ? prm.dt * f.mu_n[k] : 1.0, E[6];
-                eff_rates(f.exxd[k], f.ezzd[k], f.exz_n[k], f.sxxd0[k], f.szzd0[k], f.sxz0_n[k], etae, E);
+                double ie = prm.iselastic == 1 ? 1.0 / (prm.dt * f.mu_n[k]) : 1.0, E[6];
+                eff_rates(f.exxd[k], f.ezzd[k], f.exz_n[k], f.sxxd0[k], f.szzd0[k], f.sxz0_n[k], ie, E);
                 // K = 0 (incompressible): the K*dt*ddivp terms vanish
                 d11 += 2.0 * f.detadexx_n[k] * E[3];
                 d12 = 2.0 * f.detadezz_n[k] * E[3];
@@ -881,8 +923,8 @@ __global__ void k_operators(mdz_dgrid g, mdz_rheo_params prm, mdz_fields f, int 
             double eta = f.eta_s[k];
             d33 = eta;
             if (jacobian) {
-                double etae = prm.iselastic == 1 ? prm.dt * f.mu_s[k] : 1.0, E[6];
-                eff_rates(f.exxd_s[k], f.ezzd_s[k], f.exz[k], f.sxxd0_s[k], f.szzd0_s[k], f.sxz0[k], etae, E);
+                double ie = prm.iselastic == 1 ? 1.0 / (prm.dt * f.mu_s[k]) : 1.0, E[6];
+                eff_rates(f.exxd_s[k], f.ezzd_s[k], f.exz[k], f.sxxd0_s[k], f.szzd0_s[k], f.sxz0[k], ie, E);
                 d31 = 2.0 * f.detadexx_s[k] * E[5];
                 d32 = 2.0 * f.detadezz_s[k] * E[5];
                 d33 += 2.0 * f.detadgxz_s[k] * E[5];
@@ -1021,13 +1063,13 @@ __global__ void __launch_bounds__(256) k_mlp_guess(mdz_dgrid g, int nph, mdz_rhe
         if (act) {
             double E[6];
             if (CENT) {
-                const double etae = prm.iselastic == 1 ? prm.dt * f.mu_n[c] : 1.0;
-                eff_rates(f.exxd[c], f.ezzd[c], f.exz_n[c], f.sxxd0[c], f.szzd0[c], f.sxz0_n[c], etae, E);
+                const double ie = prm.iselastic == 1 ? 1.0 / (prm.dt * f.mu_n[c]) : 1.0;
+                eff_rates(f.exxd[c], f.ezzd[c], f.exz_n[c], f.sxxd0[c], f.szzd0[c], f.sxz0_n[c], ie, E);
                 T = f.T[c];
                 P = f.p[c];
             } else {
-                const double etae = prm.iselastic == 1 ? prm.dt * f.mu_s[c] : 1.0;
-                eff_rates(f.exxd_s[c], f.ezzd_s[c], f.exz[c], f.sxxd0_s[c], f.szzd0_s[c], f.sxz0[c], etae, E);
+                const double ie = prm.iselastic == 1 ? 1.0 / (prm.dt * f.mu_s[c]) : 1.0;
+                eff_rates(f.exxd_s[c], f.ezzd_s[c], f.exz[c], f.sxxd0_s[c], f.szzd0_s[c], f.sxz0[c], ie, E);
                 T = f.T_s[c];
                 P = f.P_s[c];
             }
@@ -1082,7 +1124,8 @@ __device__ __forceinline__ double mlp_u01(unsigned long long seed, long long i, 
     return (double)(z >> 11) * (1.0 / 9007199254740992.0);
 }
 
-__global__ void __launch_bounds__(128) k_mlp_samples(long long n, unsigned long long seed, mdz_mat_k m,
+__global__ void __launch_bounds__(128) k_mlp_samples(long long n, unsigned long long seed, mdz_materials m,
+                                                     const __grid_constant__ visc_mats<false> mk,
                                                      mdz_rheo_params prm, double lo0, double hi0, double lo1,
                                                      double hi1, double lo2, double hi2, double lo3, double hi3,
                                                      mdz_mlp_norm nm, uint4 *__restrict__ X, float2 *__restrict__ Y) {
@@ -1098,8 +1141,11 @@ __global__ void __launch_bounds__(128) k_mlp_samples(long long n, unsigned long 
     q.dt = dt;
     if (T < ZEROC / q.scale_T) T = ZEROC / q.scale_T;
     visc_res o;
-    visc_local(ph, m.mu[ph], T, P, m.gs_ref[ph], 0.0, 0.0, Eii, -Eii, 0.0, Eii, -Eii, 0.0, 0.0, 0.0, 0.0, m, q,
-               m.psi[ph], m.phi[ph], m.C[ph], P, m.bet[ph], o);
+    visc_prm<double> vq = mk.d.prm;   // the tuple's own time step
+    vq.dt = dt;
+    vq.idt = 1.0 / dt;
+    visc_local_t<double>(mk.d.ph[ph], vq, m.mu[ph], 1.0 / (dt * m.mu[ph]), T, P, m.gs_ref[ph], 0.0, 0.0, Eii, -Eii, 0.0,
+                         0.0, 0.0, 0.0, m.psi[ph], m.phi[ph], m.C[ph], P, m.bet[ph], o, nullptr);
     float2 lab = mlp_labels(o.eta_ve, o.eta_up, o.gdot, Eii);
     lab.x = fminf(fmaxf(lab.x, -8.f), 1.f);
     lab.y = fminf(fmaxf(lab.y, 0.f), 1.f);
@@ -1112,7 +1158,7 @@ __global__ void __launch_bounds__(128) k_mlp_samples(long long n, unsigned long 
 mdz_status mdz_dev_mlp_samples(mdz_ctx *ctx, const mdz_materials *m, const mdz_rheo_params *prm, long long n,
                                unsigned long long seed, const double lo[4], const double hi[4],
                                const mdz_mlp_norm &norm, uint4 *X, float2 *Y, cudaStream_t st) {
-    k_mlp_samples<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, seed, mat_k(*m), *prm, lo[0], hi[0], lo[1], hi[1], lo[2],
+    k_mlp_samples<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, seed, *m, visc_mats<false>{make_visc_mat<double>(*m, *prm)}, *prm, lo[0], hi[0], lo[1], hi[1], lo[2],
                                                                 hi[2], lo[3], hi[3], norm, X, Y);
     MDZ_LAUNCHED(ctx);
     return MDZ_OK;
@@ -1142,10 +1188,17 @@ mdz_status mdz_dev_viscosity(mdz_ctx *ctx, const mdz_materials *m, const mdz_rhe
     }
     cudaEvent_t ev;
     mdz_prof_begin(ctx, MDZ_PROF_VISCOSITY, st, &ev);
-    const mdz_mat_k mk = mat_k(*m);
-    k_viscosity_centroids<<<mdz_blocks(nc, 128), 128, 0, st>>>(g, mk, *prm, f, d_counters, guess_n, lab_n, fp32 ? 1 : 0);
-    MDZ_LAUNCHED(ctx);
-    k_viscosity_vertices<<<mdz_blocks(nv, 128), 128, 0, st>>>(g, mk, *prm, f, d_counters, guess_s, lab_s, fp32 ? 1 : 0);
+    if (fp32) {
+        const visc_mats<true> mk{make_visc_mat<double>(*m, *prm), make_visc_mat<float>(*m, *prm)};
+        k_viscosity_centroids<true><<<mdz_blocks(nc, 128), 128, 0, st>>>(g, mk, *prm, f, d_counters, guess_n, lab_n);
+        MDZ_LAUNCHED(ctx);
+        k_viscosity_vertices<true><<<mdz_blocks(nv, 128), 128, 0, st>>>(g, mk, *prm, f, d_counters, guess_s, lab_s);
+    } else {
+        const visc_mats<false> mk{make_visc_mat<double>(*m, *prm)};
+        k_viscosity_centroids<false><<<mdz_blocks(nc, 128), 128, 0, st>>>(g, mk, *prm, f, d_counters, guess_n, lab_n);
+        MDZ_LAUNCHED(ctx);
+        k_viscosity_vertices<false><<<mdz_blocks(nv, 128), 128, 0, st>>>(g, mk, *prm, f, d_counters, guess_s, lab_s);
+    }
     MDZ_LAUNCHED(ctx);
     // algorithmic bytes: per centroid 17 + n_phases FP64 inputs and 35 outputs,
     // per vertex 17 + n_phases inputs and 12 outputs, plus the tags
