@@ -61,7 +61,7 @@ void mdz_reseed_free(mdz_ctx *ctx) {
 // Quarter-grid geometry, every constant formed as the reference forms it.
 struct quarter_geom {
     int nxl, nzl, Ncx, Ncz, Nx;
-    double dx, dz, xge, zge, qx0, qz0;   // extended vertex origin; quarter-index origin xc_e0 - dx/4
+    double dx, dz, idx2, idz2, xge, zge, qx0, qz0;   // extended vertex origin; quarter-index origin xc_e0 - dx/4
     double xg0, zg0, xc0, zc0, xmin, xmax, zmin, zmax;
 };
 
@@ -71,6 +71,7 @@ static quarter_geom make_quarter_geom(const mdz_ctx *ctx) {
     q.Ncx = d.Nx - 1; q.Ncz = d.Nz - 1; q.Nx = d.Nx;
     q.nxl = 2 * (q.Ncx + 2); q.nzl = 2 * (q.Ncz + 2);
     q.dx = d.dx; q.dz = d.dz;
+    q.idx2 = 2.0 / d.dx; q.idz2 = 2.0 / d.dz;
     q.xg0 = d.xg[0]; q.zg0 = d.zg[0]; q.xc0 = d.xc[0]; q.zc0 = d.zc[0];
     q.xge = q.xg0 - q.dx;
     q.zge = q.zg0 - q.dz;
@@ -84,16 +85,23 @@ static quarter_geom make_quarter_geom(const mdz_ctx *ctx) {
 // ceil(v + 0.5) - 1 of the reference's nearest-node formula, as an int
 __device__ __forceinline__ int nearest_of(double v) { return (int)(ceil(__dadd_rn(v, 0.5)) - 1.0); }
 
+// Quarter-cell index of a marker at distance d from the first quarter line, by
+// the mantissa where the roundings cannot matter (2^-19 of a quarter cell from a
+// line), by the reference's quotient, product and sum elsewhere.
+__device__ __forceinline__ int quarter_index(double d, double h, double ih2, int n) {
+    int i;
+    if (!line_index(d, ih2, 0.5, i)) i = nearest_of(__dmul_rn(__ddiv_rn(d, h), 2.0));
+    return i < 0 ? 0 : (i > n - 1 ? n - 1 : i);
+}
+
 __global__ void k_quarter_count(int n, const double *__restrict__ x, const double *__restrict__ z,
                                 const int *__restrict__ phase, quarter_geom q, int *__restrict__ qcell,
                                 int *__restrict__ qcount) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     if (phase[k] < 0) { qcell[k] = -1; return; }
-    int ic = nearest_of(__dmul_rn(__ddiv_rn(x[k] - q.qx0, q.dx), 2.0));
-    int jc = nearest_of(__dmul_rn(__ddiv_rn(z[k] - q.qz0, q.dz), 2.0));
-    ic = ic < 0 ? 0 : (ic > q.nxl - 1 ? q.nxl - 1 : ic);
-    jc = jc < 0 ? 0 : (jc > q.nzl - 1 ? q.nzl - 1 : jc);
+    const int ic = quarter_index(x[k] - q.qx0, q.dx, q.idx2, q.nxl);
+    const int jc = quarter_index(z[k] - q.qz0, q.dz, q.idz2, q.nzl);
     const int c = ic + jc * q.nxl;
     qcell[k] = c;
     atomicAdd(&qcount[c], 1);

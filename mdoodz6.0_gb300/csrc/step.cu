@@ -183,7 +183,7 @@ __global__ void k_marker_update(int n, mdz_dgrid g, const double *__restrict__ m
     // what & 4: pressure increment (UpdateParticlePressure, before the advection)
     // centroids, ghosted frame (Interp_Grid2P_centroids2, non-periodic)
     if (what & 5) {
-        int jp = (int)ceil_quot(x - g.xvz[0], dx, idx, 0.0) - 1, ip = (int)ceil_quot(z - g.zvx[0], dz, idz, 0.0) - 1;
+        int jp = quot_index(x - g.xvz[0], dx, idx, 0.0), ip = quot_index(z - g.zvx[0], dz, idz, 0.0);
         int jw = jp - 1, je = jp, is = ip - 1, in_ = ip;
         if (jp <= 0) { jw = 0; je = 0; }
         if (jp >= ncx) { jw = ncx - 1; je = ncx - 1; }
@@ -206,7 +206,7 @@ __global__ void k_marker_update(int n, mdz_dgrid g, const double *__restrict__ m
     }
     // vertices (Interp_Grid2P)
     if (what & 1) {
-        int jp = (int)ceil_quot(x - g.xg[0], dx, idx, 0.0) - 1, ip = (int)ceil_quot(z - g.zg[0], dz, idz, 0.0) - 1;
+        int jp = quot_index(x - g.xg[0], dx, idx, 0.0), ip = quot_index(z - g.zg[0], dz, idz, 0.0);
         jp = jp < 0 ? 0 : (jp > Nx - 2 ? Nx - 2 : jp);
         ip = ip < 0 ? 0 : (ip > Nz - 2 ? Nz - 2 : ip);
         double dxm = fabs(x - g.xg[jp]), dzm = fabs(z - g.zg[ip]);
@@ -222,7 +222,7 @@ __global__ void k_marker_update(int n, mdz_dgrid g, const double *__restrict__ m
     }
     // strain increments on centroid lines (AccumulatedStrainII :235-350)
     if (what & 2) {
-        int jp = (int)ceil_quot(x - g.xc[0], dx, idx, 0.0) - 1, ip = (int)ceil_quot(z - g.zc[0], dz, idz, 0.0) - 1;
+        int jp = quot_index(x - g.xc[0], dx, idx, 0.0), ip = quot_index(z - g.zc[0], dz, idz, 0.0);
         jp = jp < 0 ? 0 : (jp > ncx - 2 ? ncx - 2 : jp);
         ip = ip < 0 ? 0 : (ip > ncz - 2 ? ncz - 2 : ip);
         double dxm = x - g.xc[jp], dzm = z - g.zc[ip];
@@ -230,6 +230,15 @@ __global__ void k_marker_update(int n, mdz_dgrid g, const double *__restrict__ m
         const signed char *t = g.BCp;
         double e = 0, ep = 0, s = 0, w;
         const double wx = dxm * idx, wz = dzm * idz;
+        const bool solid = !is_air(t[SW]) && !is_air(t[SE]) && !is_air(t[NW]) && !is_air(t[NE]);
+        if (solid) {   // the four weights sum to 1: no quotients
+            const double s0 = dstrain[SW] + wx * (dstrain[SE] - dstrain[SW]), s1 = dstrain[NW] + wx * (dstrain[NE] - dstrain[NW]);
+            const double p0 = dstrain_pl[SW] + wx * (dstrain_pl[SE] - dstrain_pl[SW]);
+            const double p1 = dstrain_pl[NW] + wx * (dstrain_pl[NE] - dstrain_pl[NW]);
+            strain[k] += s0 + wz * (s1 - s0);
+            strain_pl[k] += p0 + wz * (p1 - p0);
+            return;
+        }
         if (!is_air(t[SW])) { w = (1.0 - wx) * (1.0 - wz); e += w * dstrain[SW]; ep += w * dstrain_pl[SW]; s += w; }
         if (!is_air(t[SE])) { w = wx * (1.0 - wz); e += w * dstrain[SE]; ep += w * dstrain_pl[SE]; s += w; }
         if (!is_air(t[NW])) { w = (1.0 - wx) * wz; e += w * dstrain[NW]; ep += w * dstrain_pl[NW]; s += w; }
