@@ -117,11 +117,12 @@ extern "C" mdz_status mdz_create(mdz_ctx **out, const mdz_grid_desc *d, int n_ph
     for (int a = 0; a < MDZ_M_NATTR; a++) UP(ctx->m.attr[a], (const double *)nullptr, cap);
     int ncells = (Nx - 1) * (Nz - 1);
     ctx->bins.ncells = ncells;
+    ctx->bins.quads = ncells < (1 << 29) - 1024 ? 4 : 1;   // bins are counted in 32 bits
+    const size_t nbins = (size_t)ctx->bins.quads * ncells;
     UP(ctx->bins.cell, (const int *)nullptr, cap); UP(ctx->bins.sorted, (const int *)nullptr, cap);
-    UP(ctx->bins.qvert, (const int *)nullptr, cap);
-    UP(ctx->bins.count, (const int *)nullptr, ncells + 1); UP(ctx->bins.start, (const int *)nullptr, ncells + 1);
-    UP(ctx->bins.cursor, (const int *)nullptr, ncells + 1);
-    UP(ctx->bins.scan_partials, (const int *)nullptr, (ncells + 1) / 1024 + 2);
+    UP(ctx->bins.arrival, (const int *)nullptr, cap);
+    UP(ctx->bins.count, (const int *)nullptr, nbins + 1); UP(ctx->bins.start, (const int *)nullptr, nbins + 1);
+    UP(ctx->bins.scan_partials, (const int *)nullptr, (nbins + 1) / 1024 + 2);
     UP(ctx->red_part, (const double *)nullptr, MDZ_RED_PART);
     UP(ctx->red_cnt, (const unsigned int *)nullptr, MDZ_RED_COUNTERS);
 #undef UP
@@ -147,7 +148,7 @@ extern "C" void mdz_destroy(mdz_ctx *ctx) {
     mdz_dgrid &g = ctx->g;
     void *ptrs[] = {g.xg, g.zg, g.xc, g.zc, g.xvz, g.zvx, g.BCu, g.BCv, g.BCp, g.BCg, g.BCu_val, g.BCv_val,
                     ctx->m.x, ctx->m.z, ctx->m.vx, ctx->m.vz, ctx->m.phase, ctx->bins.cell, ctx->bins.sorted,
-                    ctx->bins.qvert, ctx->bins.count, ctx->bins.start, ctx->bins.cursor, ctx->bins.scan_partials,
+                    ctx->bins.arrival, ctx->bins.count, ctx->bins.start, ctx->bins.scan_partials,
                     ctx->red_part, ctx->red_cnt, ctx->ale_sums};
     for (void *p : ptrs)
         if (p) cudaFree(p);

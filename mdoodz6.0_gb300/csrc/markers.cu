@@ -26,21 +26,55 @@ __device__ __forceinline__ int lower_line(double x, double X0, double h, double 
     return quot_index(x - X0, h, ih, 0.0);
 }
 
+// Two sets of lines with one spacing, and the distance of their first lines in
+// 2^-20 of it (line_indices).
+struct line_pair {
+    const double *X, *Xh;
+    double h, ih;
+    long long off;
+    int n;   // lines of the first set
+};
+
+static line_pair make_line_pair(const double *X, const double *Xh, double first, double first_h, double h, int n) {
+    const double ih = 1.0 / h;
+    return line_pair{X, Xh, h, ih, (long long)std::llround((first - first_h) * ih * 1048576.0), n};
+}
+
 // ---------------------------------------------------------------------------
 // Binning: cell of each active marker = nearest centroid (the same formula and
-// clamps as P2Mastah on centroids), per-cell counts.
+// clamps as P2Mastah on centroids), and inside the cell the quadrant of its
+// nearest vertex (the cell's corner (q & 1, q >> 1)): bin `quads` cell + q.  A
+// cell is then the nearest-centroid list of its centroid and a quadrant a
+// quarter of the nearest-vertex list of its corner, both contiguous.  quads is
+// 1, without quadrants, where four times the cells leave 32 bits.
+// cell[k]: the bin, arrival[k]: how many of the bin came before (in any order:
+// the segments are sorted below), which saves the scatter its atomics.
+// Bound by the FP64 pipe: four indices one by one took 135 us for 8.4 M markers,
+// in pairs 85.
+__device__ __forceinline__ void cell_and_side(const line_pair &L, double x, int &c, int &side) {
+    int v;
+    if (!line_indices(x - L.X[0], L.ih, 0.5, L.off, c, v)) {
+        c = nearest_line(x, L.X[0], L.h, L.ih, L.n);
+        v = nearest_line(x, L.Xh[0], L.h, L.ih, L.n + 1);
+    }
+    c = c < 0 ? 0 : (c > L.n - 1 ? L.n - 1 : c);
+    v = v < 0 ? 0 : (v > L.n ? L.n : v);
+    side = v > c;   // the vertex lines lie half a cell to either side of the centroid's
+}
+
 __global__ void k_bin_count(int n, const double *__restrict__ x, const double *__restrict__ z,
-                            const int *__restrict__ phase, const double *__restrict__ xc,
-                            const double *__restrict__ zc, double dx, double dz, double idx, double idz, int ncx,
-                            int ncz, int *__restrict__ cell, int *__restrict__ count) {
+                            const int *__restrict__ phase, line_pair LX, line_pair LZ, int quads,
+                            int *__restrict__ cell, int *__restrict__ arrival, int *__restrict__ count) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     if (phase[k] == -1) { cell[k] = -1; return; }
-    int ic = nearest_line(x[k], xc[0], dx, idx, ncx);
-    int jc = nearest_line(z[k], zc[0], dz, idz, ncz);
-    int c = ic + jc * ncx;
+    int ic, jc, qx, qz;
+    cell_and_side(LX, x[k], ic, qx);
+    cell_and_side(LZ, z[k], jc, qz);
+    int c = ic + jc * LX.n;
+    if (quads == 4) c = 4 * c + qx + 2 * qz;
     cell[k] = c;
-    atomicAdd(&count[c], 1);
+    arrival[k] = atomicAdd(&count[c], 1);
 }
 
 // Block-wise inclusive scan (1024 elements per block) of int counts; writes
@@ -103,17 +137,15 @@ __global__ void k_scan_add(int n, int *__restrict__ out, const int *__restrict__
     if (i < n) out[i + 1] += partial[blockIdx.x];
 }
 
-__global__ void k_bin_scatter(int n, const int *__restrict__ cell, const int *__restrict__ start,
-                              int *__restrict__ cursor, int *__restrict__ sorted) {
+__global__ void k_bin_scatter(int n, const int *__restrict__ cell, const int *__restrict__ arrival,
+                              const int *__restrict__ start, int *__restrict__ sorted) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     int c = cell[k];
-    if (c < 0) return;
-    int pos = start[c] + atomicAdd(&cursor[c], 1);
-    sorted[pos] = k;
+    if (c >= 0) sorted[start[c] + arrival[k]] = k;
 }
 
-// Make the order inside each cell ascending in marker index, so that every
+// Make the order inside each bin ascending in marker index, so that every
 // projection sums in a fixed order (bit-reproducible run to run).
 __global__ void k_bin_sort_segments(int ncells, const int *__restrict__ start, int *__restrict__ sorted) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -126,61 +158,40 @@ __global__ void k_bin_sort_segments(int ncells, const int *__restrict__ start, i
     }
 }
 
-// Nearest vertex of the marker at each sorted position (the projection onto
-// vertices tests every marker of its four candidate cells against the node:
-// with the index stored once per binning the three markers in four that
-// belong to another vertex cost an integer compare instead of two FP64 index
-// computations, FP64 being a small fraction of the FP32 rate on this part).
-// Same formula, lines and clamps as the projection's own nearest_line.
-__global__ void k_bin_vertices(int n, const int *__restrict__ nbinned, const int *__restrict__ sorted,
-                               const double *__restrict__ x, const double *__restrict__ z,
-                               const double *__restrict__ xg, const double *__restrict__ zg, double dx, double dz,
-                               double idx, double idz, int Nx, int Nz, int *__restrict__ qvert) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n || q >= *nbinned) return;
-    const int k = sorted[q];
-    const int ip = nearest_line(x[k], xg[0], dx, idx, Nx), jp = nearest_line(z[k], zg[0], dz, idz, Nz);
-    qvert[q] = ip | (jp << 16);
-}
-
 mdz_status mdz_ensure_bins(mdz_ctx *ctx, cudaStream_t st) {
     mdz_bins &B = ctx->bins;
     if (B.valid) return MDZ_OK;
     const mdz_dgrid &g = ctx->g;
-    int n = ctx->m.n, nc = B.ncells;
-    MDZ_CUDA(ctx, cudaMemsetAsync(B.count, 0, sizeof(int) * (nc + 1), st));
-    MDZ_CUDA(ctx, cudaMemsetAsync(B.cursor, 0, sizeof(int) * (nc + 1), st));
+    const int n = ctx->m.n, nb = B.quads * B.ncells;
+    MDZ_CUDA(ctx, cudaMemsetAsync(B.count, 0, sizeof(int) * ((size_t)nb + 1), st));
     if (n > 0) {
-        k_bin_count<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, ctx->m.x, ctx->m.z, ctx->m.phase, g.xc, g.zc, g.dx, g.dz,
-                                                           g.idx, g.idz, g.ncx, g.ncz, B.cell, B.count);
+        const mdz_grid_desc &hd = ctx->host_desc;
+        k_bin_count<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, ctx->m.x, ctx->m.z, ctx->m.phase,
+                                                           make_line_pair(g.xc, g.xg, hd.xc[0], hd.xg[0], g.dx, g.ncx),
+                                                           make_line_pair(g.zc, g.zg, hd.zc[0], hd.zg[0], g.dz, g.ncz),
+                                                           B.quads, B.cell, B.arrival, B.count);
         MDZ_LAUNCHED(ctx);
     }
-    int nb = (nc + 1023) / 1024;
-    k_scan_blocks<<<nb, 1024, 0, st>>>(nc, B.count, B.start, B.scan_partials);
+    const int blocks = (int)(((size_t)nb + 1023) / 1024);
+    k_scan_blocks<<<blocks, 1024, 0, st>>>(nb, B.count, B.start, B.scan_partials);
     MDZ_LAUNCHED(ctx);
-    k_scan_partials<<<1, 1024, 0, st>>>(nb, B.scan_partials);
+    k_scan_partials<<<1, 1024, 0, st>>>(blocks, B.scan_partials);
     MDZ_LAUNCHED(ctx);
-    k_scan_add<<<nb, 1024, 0, st>>>(nc, B.start, B.scan_partials);
-    MDZ_LAUNCHED(ctx);
-    if (n > 0) {
-        k_bin_scatter<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, B.cell, B.start, B.cursor, B.sorted);
-        MDZ_LAUNCHED(ctx);
-    }
-    k_bin_sort_segments<<<mdz_blocks(nc), MDZ_THREADS, 0, st>>>(nc, B.start, B.sorted);
+    k_scan_add<<<blocks, 1024, 0, st>>>(nb, B.start, B.scan_partials);
     MDZ_LAUNCHED(ctx);
     if (n > 0) {
-        k_bin_vertices<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, B.start + nc, B.sorted, ctx->m.x, ctx->m.z, g.xg,
-                                                              g.zg, g.dx, g.dz, g.idx, g.idz, g.Nx, g.Nz, B.qvert);
+        k_bin_scatter<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, B.cell, B.arrival, B.start, B.sorted);
         MDZ_LAUNCHED(ctx);
     }
+    k_bin_sort_segments<<<mdz_blocks(nb), MDZ_THREADS, 0, st>>>(nb, B.start, B.sorted);
+    MDZ_LAUNCHED(ctx);
     B.valid = true;
     return MDZ_OK;
 }
 
 // ---------------------------------------------------------------------------
-// Batched projection.  One thread per node gathers, from the markers of the
-// cells that can hold its contributors, exactly the tent weights P2Mastah
-// scatters: each marker finds its nearest node (ip, jp) with the reference's
+// Batched projection.  Every node gathers, from the markers of the cells that
+// can hold its contributors, exactly the tent weights P2Mastah scatters: each marker finds its nearest node (ip, jp) with the reference's
 // formula and clamps, then contributes to (ip, jp) and, for the 9-cell
 // stencil, to the 8 neighbours, with distances measured from X[ip] +/- dx.
 struct p2g_fields {
@@ -202,12 +213,44 @@ __device__ __forceinline__ void cell_range(int i, int h, int kind, int n_nodes, 
     hi = hi > n_cells - 1 ? n_cells - 1 : hi;
 }
 
+// Node value B / W by the reciprocal of W that the node's fields share: one step
+// on the remainder makes the quotient the rounded one but for rare last bits
+// (Markstein, IBM J. Res. Dev. 34, 1990), in 3 FP64 instructions.
+__device__ __forceinline__ double over_weight(double B, double W, double rW) {
+    const double q = B * rW;
+    const unsigned e = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;   // biased exponent: 0 for a zero, 2^-900 .. 2^900
+    if ((e < 123u || e > 1923u) && (__double_as_longlong(B) << 1) != 0) return B / W;
+    return __fma_rn(__fma_rn(-q, W, B), rW, q);
+}
+
+template <int NF, int NPH>
+__device__ __forceinline__ void p2g_finish(int node, int nn, signed char tag, double Wm, const double *BmWm,
+                                           const double *Wph, const p2g_fields &F, int nph_rt,
+                                           double *__restrict__ phase_perc) {
+    const bool air = tag == 30 || tag == 31;
+    const bool skip = fabs(Wm) < 1e-30 || air;
+    if (F.empty && phase_perc && !air && fabs(Wm) < 1e-30) atomicAdd(F.empty, 1);
+    const double rW = 1.0 / Wm;
+#pragma unroll
+    for (int f = 0; f < NF; f++) {
+        if (skip) continue;
+        double v = over_weight(BmWm[f], Wm, rW);
+        if (F.avg[f] == 1) v = 1.0 / v;
+        if (F.avg[f] == 2) v = exp(v);
+        F.out[f][node] = v;
+    }
+    if (phase_perc) {
+#pragma unroll
+        for (int p = 0; p < NPH; p++)
+            if (p < nph_rt) phase_perc[(size_t)p * nn + node] = skip ? Wph[p] : over_weight(Wph[p], Wm, rW);
+    }
+}
+
 template <int NF, int NPH>
 __global__ void __launch_bounds__(128) k_p2g_gather(
     int nnx, int nnz, const double *__restrict__ X, const double *__restrict__ Z, const signed char *__restrict__ tag,
     int kindx, int kindz, int h, double dx, double dz, double idx, double idz, double idxi, double idzi, int ncx,
-    int ncz, const int *__restrict__ start, const int *__restrict__ sorted, const int *__restrict__ qvert,
-    const double *__restrict__ mx, const double *__restrict__ mz, const int *__restrict__ mphase, p2g_fields F,
+    int ncz, int quads, const int *__restrict__ start, const int *__restrict__ sorted, const double *__restrict__ mx, const double *__restrict__ mz, const int *__restrict__ mphase, p2g_fields F,
     int nph_rt, double *__restrict__ phase_perc) {
     int node = blockIdx.x * blockDim.x + threadIdx.x;
     if (node >= nnx * nnz) return;
@@ -246,74 +289,224 @@ __global__ void __launch_bounds__(128) k_p2g_gather(
             BmWm[f] += v * w;
         }
     };
-    // Markers in the order the reference's loop meets them: cell rows
-    // upwards, cells left to right, markers by index inside a cell.
-    const bool cellnode = kindx == 0 && kindz == 0;   // centroids: the bin cell is the nearest centroid
+    // Markers by cell rows upwards, cells left to right, bins in order inside a cell.
     for (int r = rlo; r <= rhi; r++) {
-        if (cellnode) {
-            for (int c = clo; c <= chi; c++) {
-                const int di = i - c, dj = j - r;
-                if (di < -h || di > h || dj < -h || dj > h) continue;
-                const int cell = c + r * ncx;
-                for (int q = start[cell], e = start[cell + 1]; q < e; q++) add(sorted[q], c, r, di, dj);
-            }
-            continue;
-        }
-        int b = start[clo + r * ncx], e = start[chi + r * ncx + 1];
-        for (int q = b; q < e; q++) {
-            int ip, jp;
-            if (qvert) {   // vertices: the stored nearest vertex
-                const int pk = qvert[q];
-                ip = pk & 0xffff;
-                jp = pk >> 16;
-            } else {
-                const int k = sorted[q];
-                ip = nearest_line(mx[k], X0, dx, idx, nnx);
-                jp = nearest_line(mz[k], Z0, dz, idz, nnz);
-            }
+        const size_t b = start[(size_t)quads * (clo + r * ncx)], e = start[(size_t)quads * (chi + r * ncx + 1)];
+        for (size_t q = b; q < e; q++) {
+            const int k = sorted[q];
+            const int ip = nearest_line(mx[k], X0, dx, idx, nnx), jp = nearest_line(mz[k], Z0, dz, idz, nnz);
             int di = i - ip, dj = j - jp;
             if (di < -h || di > h || dj < -h || dj > h) continue;
-            add(sorted[q], ip, jp, di, dj);
+            add(k, ip, jp, di, dj);
         }
     }
-    const bool air = tag[node] == 30 || tag[node] == 31;
-    bool skip = fabs(Wm) < 1e-30 || air;
-    if (F.empty && phase_perc && !air && fabs(Wm) < 1e-30) atomicAdd(F.empty, 1);
+    p2g_finish<NF, NPH>(node, nnx * nnz, tag[node], Wm, BmWm, Wph, F, nph_rt, phase_perc);
+}
+
+// Projection on centroids or vertices, whose nearest-node lists are contiguous
+// runs of the bins (one per centroid, one per quadrant around a vertex).  A CTA
+// has 4 rows of 32 nodes; the markers of the nodes and, for the nine-cell
+// stencil (H = 1), of the ring of nodes around them go through shared memory
+// four per owner node at a time: read by four neighbouring lanes per owner (a
+// full 32-byte sector where the markers lie in bin order), transformed once
+// (reciprocal, logarithm), and summed by one lane per node.
+//
+// With a thread per node reading its markers from global memory a load
+// touched 32 sectors for 32 values and, with more nodes in flight than L1 has
+// sectors for, most markers came from L2 several times; vertices tested every
+// marker of their candidate cells (four for one that counts, 16 for nine), and
+// the nine-cell stencil took reciprocals and logarithms nine times per marker.
+// Four markers per owner at a time: with two or eight the six-field centroid
+// projection takes 2.4 and 1.4 times as long (half sectors; two CTAs per SM).
+// Now bound by the FP64 pipe (72 % active; 20 instructions a marker): 8.4 M
+// markers onto 1024 x 512 centroids, six fields and four phases, 1249 -> 350 us;
+// 1.1 M onto 302 x 151 vertices, nine cells, three harmonic means, 945 -> 311 us.
+constexpr int P2G_W = 32, P2G_R = 4, P2G_LEN = 4, P2G_PAD = 5;   // padded owner: no bank conflicts in the sums
+
+template <int NF, int H>
+constexpr size_t p2g_tile_bytes() {
+    return (size_t)(P2G_W + 2 * H) * (P2G_R + 2 * H) * (P2G_PAD * ((2 + NF) * 8 + 4) + 8 * 4);
+}
+
+template <int NF, int NPH, int H>
+__global__ void __launch_bounds__(P2G_W *P2G_R) k_p2g_tile(
+    int nnx, int nnz, int vert, const double *__restrict__ X, const double *__restrict__ Z,
+    const signed char *__restrict__ tag, double dx, double dz, double idxi, double idzi, int ncx, int ncz,
+    const int *__restrict__ start, const int *__restrict__ sorted, const double *__restrict__ mx,
+    const double *__restrict__ mz, const int *__restrict__ mphase, p2g_fields F, int nph_rt,
+    double *__restrict__ phase_perc) {
+    constexpr int OW = P2G_W + 2 * H, OR = P2G_R + 2 * H, NO = OW * OR;
+    constexpr int NONE = -2147483647 - 1;   // no marker in this place
+    extern __shared__ double sm[];
+    double *sx = sm, *sz = sx + NO * P2G_PAD, *sv = sz + NO * P2G_PAD;
+    int *sp = (int *)(sv + NF * NO * P2G_PAD), *run = sp + NO * P2G_PAD, *end = run + 4 * NO;
+    const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    const int tiles = (nnx + P2G_W - 1) / P2G_W;
+    const int i0 = (blockIdx.x % tiles) * P2G_W, j0 = (blockIdx.x / tiles) * P2G_R;
+    // H = 0: the owners of a row are its own nodes, and a warp needs no other
+    const int o_lo = H ? threadIdx.x : row * OW + lane, o_hi = H ? NO : row * OW + OW;
+    const int o_step = H ? P2G_W * P2G_R : 32;
+    auto meet = [&]() {
+        if (H) __syncthreads();
+        else __syncwarp();
+    };
+    // runs of the owners: marker m of owner o is sorted[run[r][o] + m], r the run with m < end[r][o]
+    int longest = 0;
+    for (int o = o_lo; o < o_hi; o += o_step) {
+        const int i = i0 + o % OW - H, j = j0 + o / OW - H;
+        const bool in = i >= 0 && i < nnx && j >= 0 && j < nnz;
+        int len = 0;
 #pragma unroll
-    for (int f = 0; f < NF; f++) {
-        if (skip) continue;
-        double v = BmWm[f] / Wm;
-        if (F.avg[f] == 1) v = 1.0 / v;
-        if (F.avg[f] == 2) v = exp(v);
-        F.out[f][node] = v;
+        for (int r = 0; r < 4; r++) {
+            int b = 0, e = 0;
+            if (in && vert) {
+                const int ci = i - 1 + (r & 1), cj = j - 1 + (r >> 1);
+                if (ci >= 0 && ci < ncx && cj >= 0 && cj < ncz) {
+                    const size_t q = 4 * (size_t)(ci + cj * ncx) + 3 - r;
+                    b = start[q];
+                    e = start[q + 1];
+                }
+            } else if (in && r == 0) {
+                const size_t q = 4 * (size_t)(i + j * ncx);
+                b = start[q];
+                e = start[q + 4];
+            }
+            run[r * NO + o] = b - len;
+            len += e - b;
+            end[r * NO + o] = len;
+        }
+        longest = len > longest ? len : longest;
     }
-    if (phase_perc) {
-        int nn = nnx * nnz;
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (H) {
+        __shared__ int s_longest[P2G_R];
+        if (lane == 0) s_longest[row] = longest;
+        __syncthreads();
+        for (int w = 0; w < P2G_R; w++) longest = s_longest[w] > longest ? s_longest[w] : longest;
+    }
+    const int i = i0 + lane, j = j0 + row;
+    const bool valid = i < nnx && j < nnz;
+    // coordinates of the node, and of its owners' lines seen from there: X[ip] +- dx
+    double Xn[2 * H + 1], Zn[2 * H + 1];
 #pragma unroll
-        for (int p = 0; p < NPH; p++)
-            if (p < nph_rt) phase_perc[(size_t)p * nn + node] = skip ? Wph[p] : Wph[p] / Wm;
+    for (int d = -H; d <= H; d++) {
+        const int ip = i - d, jp = j - d;   // owner at distance d
+        Xn[d + H] = ip >= 0 && ip < nnx ? (d > 0 ? X[ip] + dx : d < 0 ? X[ip] - dx : X[ip]) : 0.0;
+        Zn[d + H] = jp >= 0 && jp < nnz ? (d > 0 ? Z[jp] + dz : d < 0 ? Z[jp] - dz : Z[jp]) : 0.0;
+    }
+    double Wm = 0.0, BmWm[NF > 0 ? NF : 1], Wph[NPH > 0 ? NPH : 1];
+#pragma unroll
+    for (int f = 0; f < NF; f++) BmWm[f] = 0.0;
+#pragma unroll
+    for (int p = 0; p < NPH; p++) Wph[p] = 0.0;
+    for (int t = 0; t < longest; t += P2G_LEN) {
+        meet();
+        // four places per lane at a time, so that their loads are in flight together
+        const int s_hi = o_hi * P2G_LEN;
+        for (int s0 = H ? (int)threadIdx.x : row * OW * P2G_LEN + lane; s0 < s_hi; s0 += 4 * o_step) {
+            int k[4], p[4], at[4];
+            double a[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int s = s0 + u * o_step, o = s / P2G_LEN, m = t + s % P2G_LEN;
+                at[u] = s < s_hi ? o * P2G_PAD + s % P2G_LEN : -1;
+                k[u] = -1;
+                p[u] = NONE;
+                if (s < s_hi && m < end[3 * NO + o]) {
+                    int r = 0;
+                    if (vert) r = (m >= end[o]) + (m >= end[NO + o]) + (m >= end[2 * NO + o]);
+                    k[u] = sorted[run[r * NO + o] + m];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (k[u] >= 0) p[u] = mphase[k[u]];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (at[u] >= 0) sp[at[u]] = p[u];
+#pragma unroll
+            for (int f = -2; f < NF; f++) {
+                const double *src = f == -2 ? mx : f == -1 ? mz : F.val[f < 0 ? 0 : f];
+                const bool per_phase = f >= 0 && F.per_phase[f < 0 ? 0 : f];
+                const int avg = f >= 0 ? F.avg[f < 0 ? 0 : f] : 0;
+#pragma unroll
+                for (int u = 0; u < 4; u++) a[u] = k[u] >= 0 ? src[per_phase ? p[u] : k[u]] : 1.0;
+                if (avg == 1) {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) a[u] = 1.0 / a[u];
+                } else if (avg == 2) {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) a[u] = log(a[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (k[u] >= 0) sm[(f + 2) * NO * P2G_PAD + at[u]] = a[u];
+            }
+        }
+        meet();
+        if (!valid) continue;
+#pragma unroll
+        for (int dj = H; dj >= -H; dj--) {   // owner rows upwards, owners left to right
+#pragma unroll
+            for (int di = H; di >= -H; di--) {
+                const int o = (row + H - dj) * OW + lane + H - di;
+#pragma unroll
+                for (int m = 0; m < P2G_LEN; m++) {
+                    const int at = o * P2G_PAD + m, p = sp[at];
+                    if (p == NONE) break;
+                    const double dxm = fabs(Xn[di + H] - sx[at]), dzm = fabs(Zn[dj + H] - sz[at]);
+                    const double w = (1.0 - dxm * idxi) * (1.0 - dzm * idzi);
+                    Wm += w;
+#pragma unroll
+                    for (int pp = 0; pp < NPH; pp++)
+                        if (p == pp) Wph[pp] += w;
+#pragma unroll
+                    for (int f = 0; f < NF; f++) BmWm[f] += sv[f * NO * P2G_PAD + at] * w;
+                }
+            }
+        }
+    }
+    if (valid) {
+        const int node = i + j * nnx;
+        p2g_finish<NF, NPH>(node, nnx * nnz, tag[node], Wm, BmWm, Wph, F, nph_rt, phase_perc);
     }
 }
 
-template <int NF>
-static void launch_p2g_nf(int nph, dim3 gr, dim3 bl, cudaStream_t st, int nnx, int nnz, const double *X,
-                          const double *Z, const signed char *tag, int kx, int kz, int h, double dx, double dz,
-                          double dxi, double dzi, int ncx, int ncz, const mdz_ctx *ctx, const p2g_fields &F,
-                          double *pp) {
+template <int NF, int NPH, int H>
+static cudaError_t launch_p2g_tile(int vert, cudaStream_t st, const mdz_nodeset &ns, double dxi, double dzi,
+                                   const mdz_ctx *ctx, const p2g_fields &F, int nph, double *pp) {
+    const mdz_dgrid &g = ctx->g;
+    const long long tiles = (long long)((ns.nx + P2G_W - 1) / P2G_W) * ((ns.nz + P2G_R - 1) / P2G_R);
+    const size_t bytes = p2g_tile_bytes<NF, H>();
+    cudaError_t e = cudaFuncSetAttribute(k_p2g_tile<NF, NPH, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    k_p2g_tile<NF, NPH, H><<<(unsigned)tiles, P2G_W * P2G_R, bytes, st>>>(
+        ns.nx, ns.nz, vert, ns.X, ns.Z, ns.tag, g.dx, g.dz, 1.0 / dxi, 1.0 / dzi, g.ncx, g.ncz, ctx->bins.start,
+        ctx->bins.sorted, ctx->m.x, ctx->m.z, ctx->m.phase, F, nph, pp);
+    return cudaSuccess;
+}
+
+template <int NF, int NPH>
+static cudaError_t launch_p2g(int kx, int kz, int h, cudaStream_t st, const mdz_nodeset &ns, double dxi, double dzi,
+                              const mdz_ctx *ctx, const p2g_fields &F, int nph, double *pp) {
+    const mdz_dgrid &g = ctx->g;
     const mdz_bins &B = ctx->bins;
-    const int *qv = kx == 1 && kz == 1 ? B.qvert : nullptr;   // vertex lines in both directions
-    if (pp == nullptr || nph <= 0)
-        k_p2g_gather<NF, 0><<<gr, bl, 0, st>>>(nnx, nnz, X, Z, tag, kx, kz, h, dx, dz, 1.0 / dx, 1.0 / dz, 1.0 / dxi,
-                                               1.0 / dzi, ncx, ncz, B.start,
-                                               B.sorted, qv, ctx->m.x, ctx->m.z, ctx->m.phase, F, 0, nullptr);
-    else if (nph <= 4)
-        k_p2g_gather<NF, 4><<<gr, bl, 0, st>>>(nnx, nnz, X, Z, tag, kx, kz, h, dx, dz, 1.0 / dx, 1.0 / dz, 1.0 / dxi,
-                                               1.0 / dzi, ncx, ncz, B.start,
-                                               B.sorted, qv, ctx->m.x, ctx->m.z, ctx->m.phase, F, nph, pp);
-    else
-        k_p2g_gather<NF, MDZ_MAX_PHASES><<<gr, bl, 0, st>>>(nnx, nnz, X, Z, tag, kx, kz, h, dx, dz, 1.0 / dx, 1.0 / dz,
-                                                            1.0 / dxi, 1.0 / dzi, ncx, ncz, B.start, B.sorted, qv, ctx->m.x,
-                                                            ctx->m.z, ctx->m.phase, F, nph, pp);
+    // centroids and vertices with quadrant bins; velocity nodes have one line of either kind
+    if (B.quads == 4 && kx == kz)
+        return h ? launch_p2g_tile<NF, NPH, 1>(kx, st, ns, dxi, dzi, ctx, F, nph, pp)
+                 : launch_p2g_tile<NF, NPH, 0>(kx, st, ns, dxi, dzi, ctx, F, nph, pp);
+    k_p2g_gather<NF, NPH><<<mdz_blocks(ns.nx * ns.nz, 128), 128, 0, st>>>(
+        ns.nx, ns.nz, ns.X, ns.Z, ns.tag, kx, kz, h, g.dx, g.dz, 1.0 / g.dx, 1.0 / g.dz, 1.0 / dxi, 1.0 / dzi, g.ncx,
+        g.ncz, B.quads, B.start, B.sorted, ctx->m.x, ctx->m.z, ctx->m.phase, F, nph, pp);
+    return cudaSuccess;
+}
+
+template <int NF>
+static cudaError_t launch_p2g_nf(int nph, int kx, int kz, int h, cudaStream_t st, const mdz_nodeset &ns, double dxi,
+                                 double dzi, const mdz_ctx *ctx, const p2g_fields &F, double *pp) {
+    if (pp == nullptr || nph <= 0) return launch_p2g<NF, 0>(kx, kz, h, st, ns, dxi, dzi, ctx, F, 0, nullptr);
+    if (nph <= 4) return launch_p2g<NF, 4>(kx, kz, h, st, ns, dxi, dzi, ctx, F, nph, pp);
+    return launch_p2g<NF, MDZ_MAX_PHASES>(kx, kz, h, st, ns, dxi, dzi, ctx, F, nph, pp);
 }
 
 // Core projection on the resident markers (device pointers everywhere).
@@ -333,14 +526,13 @@ static mdz_status p2g_core(mdz_ctx *ctx, const p2g_fields &F, int nf, double *d_
     double dxi = itp_stencil == 9 ? 3.0 * g.dx / 2.0 : g.dx / 2.0;
     double dzi = itp_stencil == 9 ? 3.0 * g.dz / 2.0 : g.dz / 2.0;
     int nn = ns.nx * ns.nz;
-    dim3 bl(128), gr(mdz_blocks(nn, 128));
     int nph = d_phase_perc ? ctx->n_phases : 0;
     p2g_fields Fc = F;
     Fc.empty = d_phase_perc ? ctx->p2g_empty : nullptr;
     cudaEvent_t ev;
     mdz_prof_begin(ctx, MDZ_PROF_P2G, st, &ev);
     switch (nf) {
-#define CASE(N) case N: launch_p2g_nf<N>(nph, gr, bl, st, ns.nx, ns.nz, ns.X, ns.Z, ns.tag, kx, kz, h, g.dx, g.dz, dxi, dzi, g.ncx, g.ncz, ctx, Fc, d_phase_perc); break;
+#define CASE(N) case N: MDZ_CUDA(ctx, launch_p2g_nf<N>(nph, kx, kz, h, st, ns, dxi, dzi, ctx, Fc, d_phase_perc)); break;
         CASE(0) CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8)
 #undef CASE
     }
@@ -430,7 +622,7 @@ extern "C" mdz_status mdz_P2Mastah(mdz_ctx *ctx, const double *mat_prop, double 
 // Counts per cell / vertex and per (node, phase): integer, exact.
 template <int NPH>
 __global__ void k_count_nodes(int nnx, int nnz, int kindx, int kindz, const double *__restrict__ X,
-                              const double *__restrict__ Z, double dx, double dz, int ncx, int ncz,
+                              const double *__restrict__ Z, double dx, double dz, int ncx, int ncz, int quads,
                               const int *__restrict__ start, const int *__restrict__ sorted,
                               const double *__restrict__ mx, const double *__restrict__ mz,
                               const int *__restrict__ mphase, int nph, int *__restrict__ count,
@@ -445,7 +637,7 @@ __global__ void k_count_nodes(int nnx, int nnz, int kindx, int kindz, const doub
 #pragma unroll
     for (int p = 0; p < NPH; p++) pc[p] = 0;
     for (int r = rlo; r <= rhi; r++) {
-        int b = start[clo + r * ncx], e = start[chi + r * ncx + 1];
+        int b = start[(size_t)quads * (clo + r * ncx)], e = start[(size_t)quads * (chi + r * ncx + 1)];
         for (int q = b; q < e; q++) {
             int k = sorted[q];
             if (nearest_line(mx[k], X[0], dx, 1.0 / dx, nnx) != i || nearest_line(mz[k], Z[0], dz, 1.0 / dz, nnz) != j)
@@ -486,13 +678,13 @@ extern "C" mdz_status mdz_count_markers(mdz_ctx *ctx, int *nb_part_cell, int *nb
         if (!dc || !dp) return mdz_fail(ctx, MDZ_ERR_CUDA, "count: staging allocation failed");
         if (ctx->n_phases <= 4)
             k_count_nodes<4><<<mdz_blocks(nn), MDZ_THREADS, 0, st>>>(ns.nx, ns.nz, kind, kind, ns.X, ns.Z, g.dx, g.dz,
-                                                                    g.ncx, g.ncz, ctx->bins.start, ctx->bins.sorted,
-                                                                    ctx->m.x, ctx->m.z, ctx->m.phase, ctx->n_phases,
+                                                                    g.ncx, g.ncz, ctx->bins.quads, ctx->bins.start,
+                                                                    ctx->bins.sorted, ctx->m.x, ctx->m.z, ctx->m.phase, ctx->n_phases,
                                                                     dc, dp);
         else
             k_count_nodes<MDZ_MAX_PHASES><<<mdz_blocks(nn), MDZ_THREADS, 0, st>>>(
-                ns.nx, ns.nz, kind, kind, ns.X, ns.Z, g.dx, g.dz, g.ncx, g.ncz, ctx->bins.start, ctx->bins.sorted,
-                ctx->m.x, ctx->m.z, ctx->m.phase, ctx->n_phases, dc, dp);
+                ns.nx, ns.nz, kind, kind, ns.X, ns.Z, g.dx, g.dz, g.ncx, g.ncz, ctx->bins.quads, ctx->bins.start,
+                ctx->bins.sorted, ctx->m.x, ctx->m.z, ctx->m.phase, ctx->n_phases, dc, dp);
         MDZ_LAUNCHED(ctx);
         if (hc) MDZ_CUDA(ctx, cudaMemcpyAsync(hc, dc, sizeof(int) * nn, cudaMemcpyDeviceToHost, st));
         if (hp) MDZ_CUDA(ctx, cudaMemcpyAsync(hp, dp, sizeof(int) * (size_t)nn * ctx->n_phases, cudaMemcpyDeviceToHost, st));
@@ -604,24 +796,9 @@ extern "C" mdz_status mdz_Interp_Grid2P(mdz_ctx *ctx, const double *node_field, 
 // [0, N-2], tag-30 substitutions as in the reference.
 //
 // Both components need the position on the vertex lines and on the ghosted
-// lines half a cell below: one fma gives both indices, the second by an
-// integer sum (`off`: the distance of the two first lines in 2^-20 of a cell).
-struct line_pair {
-    const double *X, *Xh;   // vertex lines, ghosted lines
-    double h, ih;
-    long long off;
-    int n;                  // vertex lines
-};
-
+// lines half a cell below: one fma gives both indices.
 __device__ __forceinline__ void line_pair_indices(const line_pair &L, double x, int &i, int &ih) {
-    const double d = x - L.X[0], t = __fma_rn(d, L.ih, 6442450944.0);
-    const unsigned long long a = (unsigned long long)__double_as_longlong(t), b = a + (unsigned long long)L.off;
-    // three units: half of one for the rounding of `off`
-    if ((unsigned)(a >> 52) == 0x41Fu && ((unsigned)a & 0xfffffu) - 3u <= 0xffffau &&
-        ((unsigned)b & 0xfffffu) - 3u <= 0xffffau && (unsigned)(b >> 52) == 0x41Fu) {
-        i = (int)((unsigned)(a >> 20) ^ 0x80000000u);
-        ih = (int)((unsigned)(b >> 20) ^ 0x80000000u);
-    } else {
+    if (!line_indices(x - L.X[0], L.ih, 0.0, L.off, i, ih)) {
         i = lower_line(x, L.X[0], L.h, L.ih);
         ih = lower_line(x, L.Xh[0], L.h, L.ih);
     }
@@ -733,13 +910,9 @@ mdz_status mdz_dev_rk4(mdz_ctx *ctx, const double *du, const double *dv, double 
         };
         const box_keys box{key(g.xmin, true), key(g.xmax, false), key(g.zmin, true), key(g.zmax, false)};
         const mdz_grid_desc &hd = ctx->host_desc;
-        auto lines = [](const double *X, const double *Xh, double first, double first_h, double h, int nl) {
-            const double ih = 1.0 / h;
-            return line_pair{X, Xh, h, ih, (long long)std::llround((first - first_h) * ih * 1048576.0), nl};
-        };
         k_rk4<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, ctx->m.x, ctx->m.z, ctx->m.phase, ctx->m.vx, ctx->m.vz, du, dv,
-                                                     lines(g.xg, g.xvz, hd.xg[0], hd.xvz[0], g.dx, g.Nx),
-                                                     lines(g.zg, g.zvx, hd.zg[0], hd.zvx[0], g.dz, g.Nz), g.BCu, g.BCv,
+                                                     make_line_pair(g.xg, g.xvz, hd.xg[0], hd.xvz[0], g.dx, g.Nx),
+                                                     make_line_pair(g.zg, g.zvx, hd.zg[0], hd.zvx[0], g.dz, g.Nz), g.BCu, g.BCv,
                                                      dt, 0.5 * dt, box);
         MDZ_LAUNCHED(ctx);
     }

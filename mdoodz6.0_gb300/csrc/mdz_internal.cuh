@@ -58,6 +58,16 @@ __device__ __forceinline__ bool line_index(double d, double ih, double add, int 
     i = (int)(((hi << 12) | (lo >> 20)) ^ 0x80000000u);
     return (hi >> 20) == 0x41Fu && (lo & 0xfffffu) - 2u <= 0xffffcu;
 }
+// The same on two sets of lines, the second's first line `off` units of 2^-20 of
+// a cell below the first's (rounded, hence a third unit of margin).
+__device__ __forceinline__ bool line_indices(double d, double ih, double add, long long off, int &i, int &j) {
+    const unsigned long long a = (unsigned long long)__double_as_longlong(__fma_rn(d, ih, add + 6442450944.0));
+    const unsigned long long b = a + (unsigned long long)off;
+    i = (int)((unsigned)(a >> 20) ^ 0x80000000u);
+    j = (int)((unsigned)(b >> 20) ^ 0x80000000u);
+    return (unsigned)(a >> 52) == 0x41Fu && (unsigned)(b >> 52) == 0x41Fu &&
+           ((unsigned)a & 0xfffffu) - 3u <= 0xffffau && ((unsigned)b & 0xfffffu) - 3u <= 0xffffau;
+}
 __device__ __forceinline__ int quot_index(double d, double h, double ih, double add) {
     int i;
     if (!line_index(d, ih, add, i)) i = (int)ceil_quot(d, h, ih, add) - 1;
@@ -73,16 +83,17 @@ struct mdz_markers {
     double *attr[MDZ_M_NATTR] = {nullptr};
 };
 
-// Cell binning of the resident markers: markers sorted by cell (stable).
+// Binning of the resident markers (k_bin_count): by cell and, within the cell,
+// by the quadrant of the nearest vertex; ascending marker index inside a bin.
 struct mdz_bins {
     bool valid = false;
     int ncells = 0;
-    int *cell = nullptr;        // per marker: cell index or -1 (inactive)
-    int *count = nullptr;       // per cell
-    int *start = nullptr;       // per cell + 1: exclusive scan of count
-    int *cursor = nullptr;      // scratch for the scatter
-    int *sorted = nullptr;      // marker indices grouped by cell, ascending inside a cell
-    int *qvert = nullptr;       // per sorted position: the marker's nearest vertex, ip | jp << 16
+    int quads = 4;              // bins per cell: 4, or 1 on grids of more than 2^29 cells
+    int *cell = nullptr;        // per marker: bin, or -1 (inactive)
+    int *arrival = nullptr;     // per marker: place in the bin before the sort
+    int *count = nullptr;       // per bin
+    int *start = nullptr;       // per bin + 1: exclusive scan of count
+    int *sorted = nullptr;      // marker indices grouped by bin
     int *scan_partials = nullptr;
 };
 
@@ -193,14 +204,14 @@ struct mdz_nodeset {
 };
 mdz_nodeset mdz_get_nodeset(const mdz_ctx *ctx, int centroid);
 
-// Binning (markers.cu): the cell bins, and the scan / scatter / per-bin
+// Binning (markers.cu): the marker bins, and the scan / scatter / per-bin
 // sort kernels the quarter-cell bins of the reseeding reuse.
 mdz_status mdz_ensure_bins(mdz_ctx *ctx, cudaStream_t st);
 __global__ void k_scan_blocks(int n, const int *__restrict__ in, int *__restrict__ out, int *__restrict__ partial);
 __global__ void k_scan_partials(int nb, int *partial);
 __global__ void k_scan_add(int n, int *__restrict__ out, const int *__restrict__ partial);
-__global__ void k_bin_scatter(int n, const int *__restrict__ cell, const int *__restrict__ start,
-                              int *__restrict__ cursor, int *__restrict__ sorted);
+__global__ void k_bin_scatter(int n, const int *__restrict__ cell, const int *__restrict__ arrival,
+                              const int *__restrict__ start, int *__restrict__ sorted);
 __global__ void k_bin_sort_segments(int ncells, const int *__restrict__ start, int *__restrict__ sorted);
 
 // Marker reseeding (reseed.cu): the reseeding of CountPartCell on the resident

@@ -41,7 +41,7 @@ struct mdz_reseed_ws {
     long long cap = 0;
     int nq = 0, ni = 0;
     int *qcell = nullptr, *qsorted = nullptr;            // per marker
-    int *qcount = nullptr, *qstart = nullptr, *qcursor = nullptr, *qpart = nullptr;   // per quarter cell
+    int *qcount = nullptr, *qstart = nullptr, *qpart = nullptr;   // per quarter cell
     int *flag = nullptr, *rank = nullptr, *src = nullptr, *ipart = nullptr;           // per inner quarter cell
     int *inact = nullptr, *islot = nullptr, *reuse = nullptr, *mpart = nullptr;       // per marker
     int *status = nullptr;                               // [0] no-neighbour flag
@@ -50,7 +50,7 @@ struct mdz_reseed_ws {
 void mdz_reseed_free(mdz_ctx *ctx) {
     mdz_reseed_ws *W = ctx->reseed;
     if (!W) return;
-    int *p[] = {W->qcell, W->qsorted, W->qcount, W->qstart, W->qcursor, W->qpart, W->flag, W->rank,
+    int *p[] = {W->qcell, W->qsorted, W->qcount, W->qstart, W->qpart, W->flag, W->rank,
                 W->src, W->ipart, W->inact, W->islot, W->reuse, W->mpart, W->status};
     for (int *q : p)
         if (q) cudaFree(q);
@@ -96,7 +96,7 @@ __device__ __forceinline__ int quarter_index(double d, double h, double ih2, int
 
 __global__ void k_quarter_count(int n, const double *__restrict__ x, const double *__restrict__ z,
                                 const int *__restrict__ phase, quarter_geom q, int *__restrict__ qcell,
-                                int *__restrict__ qcount) {
+                                int *__restrict__ arrival, int *__restrict__ qcount) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     if (phase[k] < 0) { qcell[k] = -1; return; }
@@ -104,7 +104,7 @@ __global__ void k_quarter_count(int n, const double *__restrict__ x, const doubl
     const int jc = quarter_index(z[k] - q.qz0, q.dz, q.idz2, q.nzl);
     const int c = ic + jc * q.nxl;
     qcell[k] = c;
-    atomicAdd(&qcount[c], 1);
+    arrival[k] = atomicAdd(&qcount[c], 1);
 }
 
 // Window of AddPartCell2's neighbour list, in the reference's visiting order.
@@ -309,7 +309,6 @@ static mdz_status reseed_ws(mdz_ctx *ctx, const quarter_geom &q, mdz_reseed_ws *
     MDZ_CUDA(ctx, A(W->qsorted, cap));
     MDZ_CUDA(ctx, A(W->qcount, nq + 1));
     MDZ_CUDA(ctx, A(W->qstart, nq + 1));
-    MDZ_CUDA(ctx, A(W->qcursor, nq + 1));
     MDZ_CUDA(ctx, A(W->qpart, (nq + 1023) / 1024 + 1));
     MDZ_CUDA(ctx, A(W->flag, ni));
     MDZ_CUDA(ctx, A(W->rank, ni + 1));
@@ -342,17 +341,17 @@ mdz_status mdz_dev_reseed(mdz_ctx *ctx, int min_part_cell, int direct, const dou
     if (s != MDZ_OK) return s;
     const int n = ctx->m.n, nq = W->nq, ni = W->ni;
     // quarter-cell bins, ascending marker index inside each
+    int *const arrival = W->inact;   // free until the inactive slots are listed
     MDZ_CUDA(ctx, cudaMemsetAsync(W->qcount, 0, sizeof(int) * (nq + 1), st));
-    MDZ_CUDA(ctx, cudaMemsetAsync(W->qcursor, 0, sizeof(int) * (nq + 1), st));
     MDZ_CUDA(ctx, cudaMemsetAsync(W->status, 0, sizeof(int) * 4, st));
     if (n > 0) {
         k_quarter_count<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, ctx->m.x, ctx->m.z, ctx->m.phase, q, W->qcell,
-                                                               W->qcount);
+                                                               arrival, W->qcount);
         MDZ_LAUNCHED(ctx);
     }
     if ((s = scan_ints(ctx, nq, W->qcount, W->qstart, W->qpart, st)) != MDZ_OK) return s;
     if (n > 0) {
-        k_bin_scatter<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, W->qcell, W->qstart, W->qcursor, W->qsorted);
+        k_bin_scatter<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, W->qcell, arrival, W->qstart, W->qsorted);
         MDZ_LAUNCHED(ctx);
     }
     k_bin_sort_segments<<<mdz_blocks(nq), MDZ_THREADS, 0, st>>>(nq, W->qstart, W->qsorted);

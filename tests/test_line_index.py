@@ -47,7 +47,7 @@ def test_line_index_matches_division(n, x0, x1):
 
 @pytest.mark.parametrize("n,x0,x1", [(3, 0.0, 1.0), (33, -7.3, 11.9), (513, 1e6, 1e6 + 0.5), (1025, -1.0, 1.0)])
 def test_ghosted_index_by_integer_sum(n, x0, x1):
-    """line_pair_indices (csrc/markers.cu): the index on the lines half a cell
+    """line_indices (csrc/mdz_internal.cuh): the index on the lines half a cell
     below from the same mantissa plus the rounded distance of the first lines."""
     h = (x1 - x0) / (n - 1)
     x, L = positions(n, x0, x1, h)
