@@ -231,9 +231,9 @@ __global__ void __launch_bounds__(128) k_mlp_train(const unsigned char *__restri
             const int row = g + ((r & 2) ? 8 : 0), col = 2 * t + (r & 1);
             const float v = acc[q][r];
             if (tau < 32) {
-                P[MLP_P_W2 + (16 * (tau >> 3) + row) * 64 + 8 * (tau & 7) + col] = v;
+                P[mlp_part_w2(16 * (tau >> 3) + row, 8 * (tau & 7) + col)] = v;
             } else if (tau < 36) {
-                P[MLP_P_W1 + (16 * (tau - 32) + row) * 8 + col] = v;
+                P[mlp_part_w1(16 * (tau - 32) + row, col)] = v;
             } else if (row < 2) {
                 P[MLP_P_W3 + row * 64 + 8 * (tau - 36) + col] = v;
             }
@@ -250,27 +250,42 @@ __global__ void __launch_bounds__(128) k_mlp_train(const unsigned char *__restri
 // Sum of the CTA partials in a fixed order (8 interleaved slices of the CTAs,
 // then the slices in order); optionally one Adam step on the FP32 master
 // weights, which also rewrites the packed BF16 image.  Block: 32 parameters x
-// 8 slices.
+// 8 slices.  Starts while the gradient pass ends (pdl_wait), as the next pass
+// does while this kernel runs.
 __global__ void __launch_bounds__(256) k_mlp_reduce(int nblk, const float *__restrict__ partials,
                                                     float *__restrict__ grad, float *__restrict__ params,
                                                     float *__restrict__ m, float *__restrict__ v,
                                                     unsigned char *packed, float lr, float b1, float b2, float eps,
-                                                    float bc1, float bc2, int adam, const int *__restrict__ tc_err) {
+                                                    float bc1, float bc2, int adam, const int *__restrict__ tc_err,
+                                                    float *__restrict__ loss_out) {
     __shared__ float part[8][33];
-    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
-    if (*tc_err) return;   // a timed-out tensor-core pass leaves the weights alone
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, q = blockIdx.x * 32 + lane;
+    pdl_wait();
+    pdl_release();
+    const int failed = *tc_err;   // a timed-out tensor-core pass leaves the weights alone
     float s = 0.f;
-    if (p <= MLP_NPARAM) {
-#pragma unroll 4
-        for (int b = slice; b < nblk; b += 8) s += partials[(size_t)b * (MLP_NPARAM + 1) + p];
+    if (q <= MLP_NPARAM) {
+        // 20 loads in flight: the sum of 304 partials is two trips through L2
+        const float *P = partials + q;
+        constexpr int U = 20;
+        for (int b0 = slice; b0 < nblk; b0 += 8 * U) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = b0 + 8 * u < nblk ? P[(size_t)(b0 + 8 * u) * (MLP_NPARAM + 1)] : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (b0 + 8 * u < nblk) s += v[u];
+        }
     }
     part[slice][lane] = s;
     __syncthreads();
-    if (slice != 0 || p > MLP_NPARAM) return;
+    if (failed || slice != 0 || q > MLP_NPARAM) return;
     s = part[0][lane];
 #pragma unroll
-    for (int q = 1; q < 8; q++) s += part[q][lane];
+    for (int i = 1; i < 8; i++) s += part[i][lane];
+    const int p = mlp_part_param(q);
     grad[p] = s;
+    if (loss_out && p == MLP_NPARAM) *loss_out = s;
     if (!adam || p == MLP_NPARAM) return;
     const float mm = b1 * m[p] + (1.f - b1) * s, vv = b2 * v[p] + (1.f - b2) * s * s;
     m[p] = mm;
@@ -330,7 +345,7 @@ static mdz_status mlp_ensure(mdz_ctx *ctx) {
     if (e == cudaSuccess) e = cudaMemset(M->packed, 0, MLP_PACK_BYTES);
     // partial gradient rows: one per CTA, two CTAs per SM for the tcgen05 pass
     if (e == cudaSuccess) e = cudaMalloc((void **)&M->partials, sizeof(float) * (MLP_NPARAM + 1) * 2 * M->max_blocks);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&M->grad, sizeof(float) * (MLP_NPARAM + 1));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&M->grad, sizeof(float) * (MLP_NPARAM + 1 + MLP_LOSSES));
     if (e == cudaSuccess) e = cudaMalloc((void **)&M->tc_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(M->tc_err, 0, sizeof(int));
     if (e == cudaSuccess)
@@ -478,7 +493,7 @@ static mdz_status mlp_tc_status(mdz_ctx *ctx);
 
 // one pass over `rows` rows starting at row0: partial gradients + reduction (+ Adam)
 static mdz_status mlp_step(mdz_ctx *ctx, const uint4 *X, const float2 *Y, long long row0, int rows, int adam,
-                           float lr) {
+                           float lr, float *loss_out = nullptr) {
     mdz_mlp *M = ctx->mlp;
     cudaStream_t st = ctx->stream;
     const int tiles = (rows + MLP_TILE - 1) / MLP_TILE, cap = (M->engine == 0 ? 2 : 1) * M->max_blocks;
@@ -500,10 +515,8 @@ static mdz_status mlp_step(mdz_ctx *ctx, const uint4 *X, const float2 *Y, long l
         bc1 = 1.f - powf(b1, (float)M->adam_t);
         bc2 = 1.f - powf(b2, (float)M->adam_t);
     }
-    k_mlp_reduce<<<(MLP_NPARAM + 1 + 31) / 32, 256, 0, st>>>(nblk, M->partials, M->grad, M->params,
-                                                                     M->adam_m, M->adam_v, M->packed, lr, b1, b2,
-                                                                     1e-8f, bc1, bc2, adam, M->tc_err);
-    MDZ_LAUNCHED(ctx);
+    MDZ_PDL(ctx, k_mlp_reduce, dim3((MLP_NPARAM + 1 + 31) / 32), dim3(256), 0, st, nblk, M->partials, M->grad, M->params,
+            M->adam_m, M->adam_v, M->packed, lr, b1, b2, 1e-8f, bc1, bc2, adam, M->tc_err, loss_out);
     return MDZ_OK;
 }
 
@@ -514,24 +527,23 @@ extern "C" mdz_status mdz_mlp_train(mdz_ctx *ctx, int steps, int batch, double l
     mdz_mlp *M = ctx->mlp;
     if (M->n < batch) return mdz_fail(ctx, MDZ_ERR_STATE, "mlp_train: %lld samples < batch %d", M->n, batch);
     const long long nb = M->n / batch;
-    double loss_acc = 0.0;
-    int loss_n = 0;
+    // the losses of the last steps stay on the device until the end: a copy and
+    // a wait after each cost 8 x 7 us
+    float *losses = M->grad + MLP_NPARAM + 1;
+    const int loss_n = steps < MLP_LOSSES ? steps : MLP_LOSSES;
     for (int s = 0; s < steps; s++) {
         // cosine decay to lr / 100
         const double c = 0.5 * (1.0 + std::cos(M_PI * (double)s / (double)steps));
         const float lrs = (float)(lr * (0.01 + 0.99 * c));
-        mdz_status r = mlp_step(ctx, M->X, M->Y, (long long)(s % nb) * batch, batch, 1, lrs);
+        const int i = s - (steps - loss_n);
+        mdz_status r = mlp_step(ctx, M->X, M->Y, (long long)(s % nb) * batch, batch, 1, lrs, i >= 0 ? losses + i : nullptr);
         if (r != MDZ_OK) return r;
-        if (s >= steps - 8) {   // mean loss of the last steps
-            float h = 0.f;
-            MDZ_CUDA(ctx, cudaMemcpyAsync(&h, M->grad + MLP_NPARAM, sizeof(float), cudaMemcpyDeviceToHost,
-                                          ctx->stream));
-            MDZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            loss_acc += h / batch;
-            loss_n++;
-        }
     }
+    float h[MLP_LOSSES] = {0.f};
+    MDZ_CUDA(ctx, cudaMemcpyAsync(h, losses, sizeof(float) * loss_n, cudaMemcpyDeviceToHost, ctx->stream));
     MDZ_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    double loss_acc = 0.0;   // mean loss of the last steps
+    for (int i = 0; i < loss_n; i++) loss_acc += h[i] / batch;
     mdz_status ts = mlp_tc_status(ctx);
     if (ts != MDZ_OK) return ts;
     M->trained = true;

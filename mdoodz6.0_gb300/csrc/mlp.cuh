@@ -33,6 +33,17 @@
 #define MLP_P_W3 4736
 #define MLP_P_B3 4864
 #define MLP_NPARAM 4866
+#define MLP_LOSSES 8      // losses of the last training steps kept on the device
+// a CTA's partial gradients hold W1 and W2 by columns: the 32 rows that a warp
+// has in its lanes are consecutive
+__host__ __device__ inline int mlp_part_w1(int row, int col) { return MLP_P_W1 + col * 64 + row; }
+__host__ __device__ inline int mlp_part_w2(int row, int col) { return MLP_P_W2 + col * 64 + row; }
+// parameter at place q of a partial gradient
+__host__ __device__ inline int mlp_part_param(int q) {
+    if (q < MLP_P_B1) return MLP_P_W1 + (q & 63) * 8 + (q >> 6);
+    if (q >= MLP_P_W2 && q < MLP_P_B2) return MLP_P_W2 + ((q - MLP_P_W2) & 63) * 64 + ((q - MLP_P_W2) >> 6);
+    return q;
+}
 // packed image (BF16 element offsets), then FP32 biases b1[64] b2[64] b3[8]
 #define MLP_S1 24
 #define MLP_S2 72
@@ -53,7 +64,7 @@ struct mdz_mlp {
     float *params = nullptr, *adam_m = nullptr, *adam_v = nullptr;   // MLP_NPARAM each (FP32 master)
     unsigned char *packed = nullptr;                                  // MLP_PACK_BYTES
     float *partials = nullptr;                                        // blocks x (MLP_NPARAM + 1)
-    float *grad = nullptr;                                            // MLP_NPARAM + 1
+    float *grad = nullptr;                                            // MLP_NPARAM + 1, then MLP_LOSSES
     int max_blocks = 0;
     uint4 *X = nullptr;                  // dataset inputs, 8 BF16 per row
     float2 *Y = nullptr;                 // dataset labels
