@@ -44,7 +44,7 @@ struct mdz_reseed_ws {
     int *qcount = nullptr, *qstart = nullptr, *qpart = nullptr;   // per quarter cell
     int *flag = nullptr, *rank = nullptr, *src = nullptr, *ipart = nullptr;           // per inner quarter cell
     int *inact = nullptr, *islot = nullptr, *reuse = nullptr, *mpart = nullptr;       // per marker
-    int *status = nullptr;                               // [0] no-neighbour flag
+    int *status = nullptr;                               // [0] no-neighbour flag, [1] a marker without a position code
 };
 
 void mdz_reseed_free(mdz_ctx *ctx) {
@@ -58,11 +58,18 @@ void mdz_reseed_free(mdz_ctx *ctx) {
     ctx->reseed = nullptr;
 }
 
+// Position code of a marker for the window search: its two coordinates in
+// quarter cells, 13 fractional bits, modulo 8 (16 bits each).  The difference of
+// two codes in one window (5 x 5 quarter cells) is their distance in 16-bit
+// arithmetic.
+constexpr double RS_UNIT = 8192.0;
+
 // Quarter-grid geometry, every constant formed as the reference forms it.
 struct quarter_geom {
     int nxl, nzl, Ncx, Ncz, Nx;
     double dx, dz, idx2, idz2, xge, zge, qx0, qz0;   // extended vertex origin; quarter-index origin xc_e0 - dx/4
-    double xg0, zg0, xc0, zc0, xmin, xmax, zmin, zmax;
+    double xg0, zg0, xmin, xmax, zmin, zmax;
+    float cx, cz, width;   // window search: squares of dx, dz over the larger; box width in its units
 };
 
 static quarter_geom make_quarter_geom(const mdz_ctx *ctx) {
@@ -72,13 +79,17 @@ static quarter_geom make_quarter_geom(const mdz_ctx *ctx) {
     q.nxl = 2 * (q.Ncx + 2); q.nzl = 2 * (q.Ncz + 2);
     q.dx = d.dx; q.dz = d.dz;
     q.idx2 = 2.0 / d.dx; q.idz2 = 2.0 / d.dz;
-    q.xg0 = d.xg[0]; q.zg0 = d.zg[0]; q.xc0 = d.xc[0]; q.zc0 = d.zc[0];
+    q.xg0 = d.xg[0]; q.zg0 = d.zg[0];
     q.xge = q.xg0 - q.dx;
     q.zge = q.zg0 - q.dz;
     const double xce = 0.5 * (q.xge + (q.xge + q.dx)), zce = 0.5 * (q.zge + (q.zge + q.dz));
     q.qx0 = xce - q.dx / 4.0;
     q.qz0 = zce - q.dz / 4.0;
     q.xmin = d.xmin; q.xmax = d.xmax; q.zmin = d.zmin; q.zmax = d.zmax;
+    const double big = q.dx > q.dz ? q.dx : q.dz;
+    q.cx = (float)((q.dx / big) * (q.dx / big));
+    q.cz = (float)((q.dz / big) * (q.dz / big));
+    q.width = (float)((q.xmax - q.xmin) / (0.5 * big) * RS_UNIT);
     return q;
 }
 
@@ -87,31 +98,49 @@ __device__ __forceinline__ int nearest_of(double v) { return (int)(ceil(__dadd_r
 
 // Quarter-cell index of a marker at distance d from the first quarter line, by
 // the mantissa where the roundings cannot matter (2^-19 of a quarter cell from a
-// line), by the reference's quotient, product and sum elsewhere.
-__device__ __forceinline__ int quarter_index(double d, double h, double ih2, int n) {
-    int i;
+// line), by the reference's quotient, product and sum elsewhere; the position
+// code's 16 bits from the same mantissa.  False: outside the quarter grid, or
+// not a number (no code).
+__device__ __forceinline__ bool quarter_index(double d, double h, double ih2, int n, int &i, unsigned &code) {
+    const unsigned long long t = (unsigned long long)__double_as_longlong(__fma_rn(d, ih2, 0.5 + 6442450944.0));
     if (!line_index(d, ih2, 0.5, i)) i = nearest_of(__dmul_rn(__ddiv_rn(d, h), 2.0));
-    return i < 0 ? 0 : (i > n - 1 ? n - 1 : i);
+    code = (unsigned)(t >> 7) & 0xffffu;
+    const bool in = i >= 0 && i < n && (unsigned)(t >> 52) == 0x41Fu;
+    i = i < 0 ? 0 : (i > n - 1 ? n - 1 : i);
+    return in;
 }
 
 __global__ void k_quarter_count(int n, const double *__restrict__ x, const double *__restrict__ z,
                                 const int *__restrict__ phase, quarter_geom q, int *__restrict__ qcell,
-                                int *__restrict__ arrival, int *__restrict__ qcount) {
+                                int *__restrict__ code, int *__restrict__ arrival, int *__restrict__ qcount,
+                                int *__restrict__ status) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     if (phase[k] < 0) { qcell[k] = -1; return; }
-    const int ic = quarter_index(x[k] - q.qx0, q.dx, q.idx2, q.nxl);
-    const int jc = quarter_index(z[k] - q.qz0, q.dz, q.idz2, q.nzl);
+    int ic, jc;
+    unsigned cx, cz;
+    const bool in = quarter_index(x[k] - q.qx0, q.dx, q.idx2, q.nxl, ic, cx);
+    if (!(quarter_index(z[k] - q.qz0, q.dz, q.idz2, q.nzl, jc, cz) && in)) status[1] = 1;   // exact searches only
     const int c = ic + jc * q.nxl;
     qcell[k] = c;
+    code[k] = (int)(cx | cz << 16);
     arrival[k] = atomicAdd(&qcount[c], 1);
 }
 
-// Window of AddPartCell2's neighbour list, in the reference's visiting order.
-__constant__ signed char c_window[25][2] = {
-    {0, 0},   {-1, 0}, {1, 0},  {0, -1}, {0, 1},  {-1, -1}, {1, -1}, {-1, 1},  {1, 1},
-    {-2, 0},  {2, 0},  {0, -2}, {0, 2},  {-2, -2}, {2, -2}, {-2, 2}, {2, 2},
-    {-1, -2}, {1, -2}, {-1, 2}, {1, 2},  {-2, -1}, {-2, 1}, {2, -1}, {2, 1}};
+// Ascending marker index inside each quarter cell, and the codes in that order.
+__global__ void k_quarter_sort(int nq, const int *__restrict__ start, int *__restrict__ sorted,
+                               const int *__restrict__ code, int *__restrict__ qcode) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= nq) return;
+    const int b = start[c], e = start[c + 1];
+    for (int i = b + 1; i < e; i++) {
+        const int v = sorted[i];
+        int j = i - 1;
+        while (j >= b && sorted[j] > v) { sorted[j + 1] = sorted[j]; j--; }
+        sorted[j + 1] = v;
+    }
+    for (int i = b; i < e; i++) qcode[i] = code[sorted[i]];
+}
 
 // New-marker position of inner quarter cell (k, l): xg[0] + ic dx/2 + dx/4 with
 // ic = k - 2 (halving and quartering are exact as products with 0.5, 0.25).
@@ -131,18 +160,16 @@ __global__ void k_reseed_cells(quarter_geom q, const signed char *__restrict__ t
     const int k = 2 + t % wi, l = 2 + t / wi, qo = (k - 2) * wj + (l - 2), kd = k + l * q.nxl;
     int f = 0;
     if (qstart[kd + 1] - qstart[kd] < thr) {
-        // centroid of the quarter cell's coarse cell, for the air test
-        const double cx = __dadd_rn(__dadd_rn(q.xge, __dmul_rn(q.dx, 0.25)), __dmul_rn(__dmul_rn((double)k, q.dx), 0.5));
-        const double cz = __dadd_rn(__dadd_rn(q.zge, __dmul_rn(q.dz, 0.25)), __dmul_rn(__dmul_rn((double)l, q.dz), 0.5));
-        int ic = nearest_of(__ddiv_rn(cx - q.xc0, q.dx)), jc = nearest_of(__ddiv_rn(cz - q.zc0, q.dz));
+        // centroid nearest to the quarter cell's centre, for the air test: the centre lies a quarter of a
+        // cell from it, so nearest_of((centre - xc0) / dx) is k / 2 - 1 whatever the roundings
+        int ic = (k >> 1) - 1, jc = (l >> 1) - 1;
         ic = ic < 0 ? 0 : (ic > q.Ncx - 1 ? q.Ncx - 1 : ic);
         jc = jc < 0 ? 0 : (jc > q.Ncz - 1 ? q.Ncz - 1 : jc);
         if (tagp[ic + jc * q.Ncx] != 30) {
             int neighs = 0;
-            for (int w = 0; w < 25; w++) {
-                const int c = kd + c_window[w][0] + c_window[w][1] * q.nxl;
-                neighs += qstart[c + 1] - qstart[c];
-            }
+#pragma unroll
+            for (int w = -2; w <= 2; w++)   // the five cells of a row are one run
+                neighs += qstart[kd + w * q.nxl + 3] - qstart[kd + w * q.nxl - 2];
             if (neighs == 0) {
                 atomicOr(status, 1);
             } else {
@@ -174,51 +201,34 @@ __global__ void k_inactive_list(int n, const int *__restrict__ inact, const int 
 }
 
 // Centers2Particle, non-periodic (SOURCE/ParticleRoutines.c:259-455): bilinear
-// on the ghosted centroid lines with the reference's edge and corner folds.
-__device__ double c2p(const mdz_dgrid &g, double x, double z, const double *__restrict__ F) {
-    const int Nx = g.ncx, Nz = g.ncz;
+// on the ghosted centroid lines, a column or row outside the centroids repeating
+// the edge's (the reference's edge and corner folds); or, with vert,
+// Vertices2Particle (:461-520): bilinear on the vertices.  One body for both, so
+// that the lanes of a group take one field each in the same instructions.
+__device__ __forceinline__ double grid_to_new(const mdz_dgrid &g, double x, double z, bool vert,
+                                              const double *__restrict__ F) {
     const double dx = g.dx, dz = g.dz;
-    const int j = (int)(ceil((x - g.xvz[0]) / dx) - 1.0), i = (int)(ceil((z - g.zvx[0]) / dz) - 1.0);
-    int iSW, iSE, iNW, iNE;
-    if (j > 0 && j < Nx && i > 0 && i < Nz) {
-        iSW = (j - 1) + (i - 1) * Nx; iSE = iSW + 1; iNW = (j - 1) + i * Nx; iNE = iNW + 1;
-    } else if (j == 0 && i > 0 && i < Nz) {
-        iSW = iSE = (i - 1) * Nx; iNW = iNE = i * Nx;
-    } else if (j == Nx && i > 0 && i < Nz) {
-        iSW = iSE = (Nx - 1) + (i - 1) * Nx; iNW = iNE = (Nx - 1) + i * Nx;
-    } else if (i == 0 && j > 0 && j < Nx) {
-        iSW = iNW = j - 1; iSE = iNE = j;
-    } else if (i == Nz && j > 0 && j < Nx) {
-        iSW = iNW = (j - 1) + (Nz - 1) * Nx; iSE = iNE = j + (Nz - 1) * Nx;
-    } else if (i == 0 && j == 0) {
-        iSW = iSE = iNW = iNE = 0;
-    } else if (i == 0 && j == Nx) {
-        iSW = iSE = iNW = iNE = Nx - 1;
-    } else if (i == Nz && j == 0) {
-        iSW = iSE = iNW = iNE = (Nz - 1) * Nx;
-    } else if (i == Nz && j == Nx) {
-        iSW = iSE = iNW = iNE = (Nx - 1) + (Nz - 1) * Nx;
-    } else {
-        return 0.0;   // outside the ghosted frame: new markers lie inside the box
+    const double *X = vert ? g.xg : g.xvz, *Z = vert ? g.zg : g.zvx;
+    double dX = x - X[0], dZ = z - Z[0];
+    if (vert) { dX = fabs(dX); dZ = fabs(dZ); }
+    int j, i;
+    if (!line_index(dX, g.idx, 0.0, j)) j = (int)(ceil(dX / dx) - 1.0);
+    if (!line_index(dZ, g.idz, 0.0, i)) i = (int)(ceil(dZ / dz) - 1.0);
+    const int nx = vert ? g.Nx : g.ncx, nz = vert ? g.Nz : g.ncz;
+    int jw = j, je = j + 1, is = i, in_ = i + 1;
+    if (!vert) {
+        if (j < 0 || j > nx || i < 0 || i > nz) return 0.0;   // outside the ghosted frame: new markers lie inside the box
+        jw = j > 0 ? j - 1 : 0; je = j < nx ? j : nx - 1;
+        is = i > 0 ? i - 1 : 0; in_ = i < nz ? i : nz - 1;
     }
-    const double ax = (x - g.xvz[j]) / dx, az = (z - g.zvx[i]) / dz;
-    const signed char *t = g.BCp;
-    double val = 0.0, sw = 0.0, w;
-    if (t[iSW] != 30 && t[iSW] != 31) { w = (1.0 - ax) * (1.0 - az); val += w * F[iSW]; sw += w; }
-    if (t[iSE] != 30 && t[iSE] != 31) { w = ax * (1.0 - az); val += w * F[iSE]; sw += w; }
-    if (t[iNW] != 30 && t[iNW] != 31) { w = (1.0 - ax) * az; val += w * F[iNW]; sw += w; }
-    if (t[iNE] != 30 && t[iNE] != 31) { w = ax * az; val += w * F[iNE]; sw += w; }
-    return sw > 1e-13 ? val / sw : val;
-}
-
-// Vertices2Particle (SOURCE/ParticleRoutines.c:461-520): bilinear on the vertices.
-__device__ double v2p_vertices(const mdz_dgrid &g, double x, double z, const double *__restrict__ F) {
-    const int Nx = g.Nx;
-    const double dx = g.dx, dz = g.dz;
-    const int j = (int)(ceil(fabs(x - g.xg[0]) / dx) - 1.0), i = (int)(ceil(fabs(z - g.zg[0]) / dz) - 1.0);
-    const double ax = (x - g.xg[j]) / dx, az = (z - g.zg[i]) / dz;
-    const int iSW = j + i * Nx, iSE = iSW + 1, iNW = j + (i + 1) * Nx, iNE = iNW + 1;
-    const signed char *t = g.BCg;
+    const int iSW = jw + is * nx, iSE = je + is * nx, iNW = jw + in_ * nx, iNE = je + in_ * nx;
+    const double ax = (x - X[j]) / dx, az = (z - Z[i]) / dz;
+    const signed char *t = vert ? g.BCg : g.BCp;
+    auto rock = [](signed char v) { return v != 30 && v != 31; };
+    if (rock(t[iSW]) && rock(t[iSE]) && rock(t[iNW]) && rock(t[iNE])) {   // the weights sum to 1: no quotient
+        const double bx = 1.0 - ax, bz = 1.0 - az;
+        return bz * (bx * F[iSW] + ax * F[iSE]) + az * (bx * F[iNW] + ax * F[iNE]);
+    }
     double val = 0.0, sw = 0.0, w;
     if (t[iSW] != 30 && t[iSW] != 31) { w = (1.0 - ax) * (1.0 - az); val += w * F[iSW]; sw += w; }
     if (t[iSE] != 30 && t[iSE] != 31) { w = ax * (1.0 - az); val += w * F[iSE]; sw += w; }
@@ -231,56 +241,145 @@ struct reseed_fields {
     const double *T_n, *sxxd_n, *szzd_n, *sxz_s, *p_n;
 };
 
-// One thread per new marker r: its quarter cell, the nearest of the markers
-// in the 5x5 quarter cells around it (the reference's visiting order; a
-// candidate replaces the best only when strictly closer: the square test
-// skips the square root of every candidate that cannot be), and the copy.
+// Place of window cell (dk, dl), at [(dl + 2) 5 + dk + 2], in the order in which
+// AddPartCell2's neighbour list visits them: the cell, its four neighbours (W, E,
+// S, N) and corners (SW, SE, NW, NE), the same at two cells' distance, and the
+// remaining eight by rows (dl = -2, 2) and columns (dk = -2, 2).
+__constant__ unsigned char c_window_place[25] = {13, 17, 11, 18, 14, 21, 5, 3, 6, 23, 9, 1, 0, 2, 10, 22, 7, 4, 8, 24,
+                                                 15, 19, 12, 20, 16};
+
+// Eight lanes per new marker r: its quarter cell, the nearest of the markers in
+// the 5x5 quarter cells around it, and the copy.  The reference visits the
+// cells in that order and replaces the best by a strictly closer marker,
+// so its result is the least distance (the rounded root) and, among equals, the
+// first visited; the first of all where none is closer than the box is wide.
+// The five cells of a window row are one run of the sorted list, which the lanes
+// share.
+//
+// The lanes first look for the least distance between position codes, in FP32: a
+// code is within one unit of the position, so a distance of codes is within
+// 3 units (2 sqrt 2, in units of 2^-13 of the wider quarter cell) of the exact
+// one, and a marker that is nearer than all others by 6 is the nearest.  Else
+// (one window in 200, lattices, markers outside the quarter grid, boxes narrower
+// than the distance) the squares are formed in FP64, and where another is within
+// 8 units in the last place of the least the roots and places are compared.
+//
+// One thread per new marker followed some 100 dependent loads (list, then
+// coordinates) one after the other, with few warps on the chip: 27 000 new
+// markers 140 us, 1364 us a step at 1024 x 512.  The lanes with FP64 squares took
+// 94 and 1086 us (the FP64 pipe), with the codes 44 and 405.
+constexpr int RS_LANES = 8;
+
+// By squared distances in FP64, for the group of lanes.
+__device__ __noinline__ int exact_nearest(int nxl, double best, int kd, int lane, unsigned group,
+                                          const int *__restrict__ qstart, const int *__restrict__ qsorted,
+                                          const double *x, const double *z, double xn, double zn) {
+    typedef unsigned long long u64;
+    auto dist2 = [&](int j) {   // bits of the squared distance: they order like the value
+        const double ax = xn - x[j], az = zn - z[j];
+        return (u64)__double_as_longlong(__dadd_rn(__dmul_rn(ax, ax), __dmul_rn(az, az)));
+    };
+    u64 least = ~0ull, next = ~0ull;
+    int m = -1;
+    for (int w = 0; w < 5; w++)
+        for (int s = qstart[kd + (w - 2) * nxl - 2] + lane; s < qstart[kd + (w - 2) * nxl + 3]; s += RS_LANES) {
+            const int j = qsorted[s];
+            const u64 d2 = dist2(j);
+            if (d2 < least) { next = least; least = d2; m = j; }
+            else if (d2 < next) next = d2;
+        }
+    u64 all = least;
+    for (int o = 1; o < RS_LANES; o <<= 1) {
+        const u64 v = __shfl_xor_sync(group, all, o);
+        all = v < all ? v : all;
+    }
+    const double d = sqrt(__longlong_as_double((long long)all));
+    const u64 near = all + 8;
+    const bool closer = d < best;
+    const unsigned mine = __ballot_sync(group, least <= near), more = __ballot_sync(group, next <= near);
+    if (closer && more == 0 && __popc(mine) == 1) return __shfl_sync(group, m, __ffs(mine) - 1);
+    // the first visited of the equally close (of all, if none is closer than the box is wide)
+    u64 place = ~0ull;
+    for (int w = 0; w < 5; w++)
+        for (int c = 0; c < 5; c++) {
+            const int b = qstart[kd + (w - 2) * nxl + c - 2], e = qstart[kd + (w - 2) * nxl + c - 1];
+            for (int s = b + lane; s < e; s += RS_LANES) {
+                const int j = qsorted[s];
+                const u64 d2 = dist2(j);
+                if (closer && (d2 > near || sqrt(__longlong_as_double((long long)d2)) != d)) continue;
+                const u64 at = (u64)c_window_place[5 * w + c] << 32 | (unsigned)(s - b);
+                if (at < place) { place = at; m = j; }
+            }
+        }
+    u64 low = place;
+    for (int o = 1; o < RS_LANES; o <<= 1) {
+        const u64 v = __shfl_xor_sync(group, low, o);
+        low = v < low ? v : low;
+    }
+    return __shfl_sync(group, m, __ffs(__ballot_sync(group, place == low)) - 1);
+}
+
 __global__ void k_reseed_write(quarter_geom q, mdz_dgrid g, int n, int nnew, int nreuse, const int *__restrict__ list,
                                const int *__restrict__ qstart, const int *__restrict__ qsorted,
+                               const int *__restrict__ qcode, const int *__restrict__ inexact,
                                const int *__restrict__ reuse, double *x, double *z, int *phase, double *vx,
                                double *vz, mdz_attr_ptrs A, int direct, reseed_fields F) {
     const int wj = q.nzl - 4;
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nnew) return;
+    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = (int)(tid / RS_LANES), lane = threadIdx.x % RS_LANES;
+    if (r >= nnew) return;   // whole groups of eight
+    const unsigned group = 0xffu << (threadIdx.x & 24);
     const int qo = list[r];
     const int k = 2 + qo / wj, l = 2 + qo % wj, kd = k + l * q.nxl;
     const double xn = new_pos(q.xg0, k - 2, q.dx), zn = new_pos(q.zg0, l - 2, q.dz);
-    double best = q.xmax - q.xmin, best2 = INFINITY;
-    int m = -1;
-    for (int w = 0; w < 25; w++) {
-        const int c = kd + c_window[w][0] + c_window[w][1] * q.nxl;
-        for (int s = qstart[c], e = qstart[c + 1]; s < e; s++) {
-            const int j = qsorted[s];
-            if (m < 0) m = j;
-            const double ax = xn - x[j], az = zn - z[j];
-            const double d2 = __dadd_rn(__dmul_rn(ax, ax), __dmul_rn(az, az));
-            if (d2 < best2) {   // sqrt is monotone: d2 >= best2 cannot give d < best
-                const double d = sqrt(d2);
-                if (d < best) { best = d; best2 = d2; m = j; }
-            }
-        }
+    int st[5], en[5];
+#pragma unroll
+    for (int w = 0; w < 5; w++) {
+        st[w] = qstart[kd + (w - 2) * q.nxl - 2];
+        en[w] = qstart[kd + (w - 2) * q.nxl + 3];
     }
+    int m = -1;
+    bool sure = false;
+    if (!*inexact) {
+        const int hx = (k << 13) + 4096, hz = (l << 13) + 4096;   // the centre of quarter cell (k, l)
+        float least = INFINITY, next = INFINITY;
+        int at = 0;
+#pragma unroll
+        for (int w = 0; w < 5; w++)
+            for (int s = st[w] + lane; s < en[w]; s += RS_LANES) {
+                const int c = qcode[s];
+                const float ax = (float)(short)((c & 0xffff) - hx), az = (float)(short)((c >> 16) - hz);
+                const float d2 = q.cx * ax * ax + q.cz * az * az;
+                if (d2 < least) { next = least; least = d2; at = s; }
+                else next = fminf(next, d2);
+            }
+        float all = least;
+#pragma unroll
+        for (int o = 1; o < RS_LANES; o <<= 1) all = fminf(all, __shfl_xor_sync(group, all, o));
+        const float d = sqrtf(all), limit = (d + 6.001f) * (d + 6.001f) * 1.0001f;
+        const unsigned mine = __ballot_sync(group, least <= limit), more = __ballot_sync(group, next <= limit);
+        sure = more == 0 && __popc(mine) == 1 && (d + 3.001f) * 1.0001f < q.width;
+        m = qsorted[at];
+        m = __shfl_sync(group, m, __ffs(mine) - 1);
+    }
+    if (!sure) m = exact_nearest(q.nxl, q.xmax - q.xmin, kd, lane, group, qstart, qsorted, x, z, xn, zn);
     const int slot = r < nreuse ? reuse[r] : n + (r - nreuse);
-    x[slot] = xn;
-    z[slot] = zn;
-    phase[slot] = phase[m];
-    vx[slot] = vx[m];
-    vz[slot] = vz[m];
-    A.a[MDZ_M_STRAIN][slot] = A.a[MDZ_M_STRAIN][m];
-    A.a[MDZ_M_STRAIN_PL][slot] = A.a[MDZ_M_STRAIN_PL][m];
-    A.a[MDZ_M_CMUL][slot] = A.a[MDZ_M_CMUL][m];
-    if (direct) {
-        A.a[MDZ_M_T][slot] = A.a[MDZ_M_T][m];
-        A.a[MDZ_M_P][slot] = A.a[MDZ_M_P][m];
-        A.a[MDZ_M_SXXD][slot] = A.a[MDZ_M_SXXD][m];
-        A.a[MDZ_M_SZZD][slot] = A.a[MDZ_M_SZZD][m];
-        A.a[MDZ_M_SXZ][slot] = A.a[MDZ_M_SXZ][m];
-    } else {
-        A.a[MDZ_M_T][slot] = c2p(g, xn, zn, F.T_n);
-        A.a[MDZ_M_P][slot] = c2p(g, xn, zn, F.p_n);
-        A.a[MDZ_M_SXXD][slot] = c2p(g, xn, zn, F.sxxd_n);
-        A.a[MDZ_M_SZZD][slot] = c2p(g, xn, zn, F.szzd_n);
-        A.a[MDZ_M_SXZ][slot] = v2p_vertices(g, xn, zn, F.sxz_s);
+    // the lanes take the properties between them
+    if (lane == 5) { x[slot] = xn; z[slot] = zn; }
+    if (lane == 6) { phase[slot] = phase[m]; vx[slot] = vx[m]; vz[slot] = vz[m]; }
+    if (lane == 7) {
+        A.a[MDZ_M_STRAIN][slot] = A.a[MDZ_M_STRAIN][m];
+        A.a[MDZ_M_STRAIN_PL][slot] = A.a[MDZ_M_STRAIN_PL][m];
+        A.a[MDZ_M_CMUL][slot] = A.a[MDZ_M_CMUL][m];
+    }
+    if (lane < 5) {
+        double *a = A.a[MDZ_M_T];
+        const double *f = F.T_n;
+        if (lane == 1) { a = A.a[MDZ_M_P]; f = F.p_n; }
+        if (lane == 2) { a = A.a[MDZ_M_SXXD]; f = F.sxxd_n; }
+        if (lane == 3) { a = A.a[MDZ_M_SZZD]; f = F.szzd_n; }
+        if (lane == 4) { a = A.a[MDZ_M_SXZ]; f = F.sxz_s; }
+        a[slot] = direct ? a[m] : grid_to_new(g, xn, zn, lane == 4, f);
     }
 }
 
@@ -341,12 +440,13 @@ mdz_status mdz_dev_reseed(mdz_ctx *ctx, int min_part_cell, int direct, const dou
     if (s != MDZ_OK) return s;
     const int n = ctx->m.n, nq = W->nq, ni = W->ni;
     // quarter-cell bins, ascending marker index inside each
-    int *const arrival = W->inact;   // free until the inactive slots are listed
+    int *const arrival = W->inact, *const code = W->islot;   // free until the inactive slots are listed
+    int *const qcode = W->qcell;                             // free after the scatter
     MDZ_CUDA(ctx, cudaMemsetAsync(W->qcount, 0, sizeof(int) * (nq + 1), st));
     MDZ_CUDA(ctx, cudaMemsetAsync(W->status, 0, sizeof(int) * 4, st));
     if (n > 0) {
         k_quarter_count<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, ctx->m.x, ctx->m.z, ctx->m.phase, q, W->qcell,
-                                                               arrival, W->qcount);
+                                                               code, arrival, W->qcount, W->status);
         MDZ_LAUNCHED(ctx);
     }
     if ((s = scan_ints(ctx, nq, W->qcount, W->qstart, W->qpart, st)) != MDZ_OK) return s;
@@ -354,7 +454,7 @@ mdz_status mdz_dev_reseed(mdz_ctx *ctx, int min_part_cell, int direct, const dou
         k_bin_scatter<<<mdz_blocks(n), MDZ_THREADS, 0, st>>>(n, W->qcell, arrival, W->qstart, W->qsorted);
         MDZ_LAUNCHED(ctx);
     }
-    k_bin_sort_segments<<<mdz_blocks(nq), MDZ_THREADS, 0, st>>>(nq, W->qstart, W->qsorted);
+    k_quarter_sort<<<mdz_blocks(nq), MDZ_THREADS, 0, st>>>(nq, W->qstart, W->qsorted, code, qcode);
     MDZ_LAUNCHED(ctx);
     // deficient quarter cells and their nearest markers, then the ranks
     const int thr = (int)(std::ceil((double)min_part_cell) / 4.0);
@@ -387,8 +487,8 @@ mdz_status mdz_dev_reseed(mdz_ctx *ctx, int min_part_cell, int direct, const dou
     if (nnew > 0) {
         mdz_attr_ptrs A;
         for (int a = 0; a < MDZ_M_NATTR; a++) A.a[a] = ctx->m.attr[a];
-        k_reseed_write<<<mdz_blocks(nnew), MDZ_THREADS, 0, st>>>(q, ctx->g, n, nnew, nreuse, W->src, W->qstart,
-                                                                 W->qsorted, W->reuse, ctx->m.x, ctx->m.z,
+        k_reseed_write<<<mdz_blocks((long long)nnew * RS_LANES), MDZ_THREADS, 0, st>>>(q, ctx->g, n, nnew, nreuse, W->src, W->qstart,
+                                                                 W->qsorted, qcode, W->status + 1, W->reuse, ctx->m.x, ctx->m.z,
                                                                  ctx->m.phase, ctx->m.vx, ctx->m.vz, A, direct,
                                                                  reseed_fields{T_n, sxxd_n, szzd_n, sxz_s, p_n});
         MDZ_LAUNCHED(ctx);
