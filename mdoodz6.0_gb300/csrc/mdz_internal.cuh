@@ -170,26 +170,32 @@ void *mdz_stage(mdz_ctx *ctx, int slot, size_t bytes);
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// (cluster > 1: in thread-block clusters of that many CTAs along x)
 template <typename... KA, typename... A>
-static inline cudaError_t launch_pdl(void (*k)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... a) {
+static inline cudaError_t launch_pdl(int cluster, void (*k)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                     A... a) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, k, KA(a)...);
 }
-#define MDZ_PDL(ctx, ...)                                                             \
+#define MDZ_PDL_CLUSTER(ctx, cluster, ...)                                            \
     do {                                                                              \
         (ctx)->launches++;                                                            \
-        cudaError_t e__ = launch_pdl(__VA_ARGS__);                                    \
+        cudaError_t e__ = launch_pdl(cluster, __VA_ARGS__);                           \
         if (e__ != cudaSuccess) return mdz_cuda_check((ctx), e__, "kernel launch");   \
     } while (0)
+#define MDZ_PDL(ctx, ...) MDZ_PDL_CLUSTER(ctx, 1, __VA_ARGS__)
 
 static inline int mdz_blocks(long long n, int threads = MDZ_THREADS) {
     long long b = (n + threads - 1) / threads;

@@ -230,6 +230,7 @@ __global__ void __launch_bounds__(NT) k_st_resid_restrict(
     const int Nx = F.Nx, Nz = F.Nz, I0 = blockIdx.x * TX, J0 = blockIdx.y * TY;
     const size_t nu = (size_t)Nx * (Nz + 1), nv = (size_t)(Nx + 1) * Nz;
     mg_release<T>();
+    if (sizeof(T) == 8 && !cxu) pdl_release();   // the bottom kernel follows: 8 CTAs that load while this one runs
 #pragma unroll 1
     for (int t0 = 0; t0 < UW * UH + VW * VH; t0 += NT) {
         const int t = t0 + threadIdx.x;
@@ -452,6 +453,7 @@ __global__ void __launch_bounds__(NT) k_mg_resid_restrict(stokes_geom F, stokes_
     __shared__ visc_tile<T, TILE ? 2 * TX + 3 : 1, TILE ? 2 * TY + 3 : 1> S;   // from (2 I0 - 3, 2 J0 - 3)
     const int Nx = F.Nx, Nz = F.Nz, I0 = blockIdx.x * TX, J0 = blockIdx.y * TY;
     mg_release<T>();
+    if (sizeof(T) == 8 && !cxu) pdl_release();   // (as in k_st_resid_restrict)
     pdl_wait();
     const vel_global<T> X{xu, xv, Nx};
     if constexpr (TILE) {

@@ -833,24 +833,34 @@ __global__ void __launch_bounds__(512) k_coarse_dense_solve(int n, int nu, int n
 }
 
 // ---------------------------------------------------------------------------
-// Bottom of the V-cycle in one CTA, everything in shared memory.  As grid
-// kernels the smallest levels cost one launch per phase, several microseconds
-// for a few hundred rows.  Here the CTA copies the levels' stencils (unknown rows
-// only), inverse diagonals and the coarsest inverse into shared memory before
-// it waits for the launch that writes its right-hand side, then runs the
-// descent, the dense solve and the ascent between CTA barriers.  The first
-// bottom level is the first whose data, with all below, fit
-// (mg_bottom_bytes): 32 x 16 cells in FP32, 16 x 8 in FP64, on a 2 : 1 box.
-// An earlier form ran every level of at most 32k points in a 16-CTA cluster
-// out of L2, with a cluster barrier per phase: 89 us (FP32, from 128 x 64
-// cells) and 203 us (FP64, where 16 SMs are too few for the rows' FP64 work);
-// levels above the shared-memory limit are faster as grid kernels of two
-// phases each (mg_tiles.cuh).
+// Bottom of the V-cycle in one cluster of 8 CTAs, everything in shared memory.
+// As grid kernels the smallest levels cost one launch per phase, several
+// microseconds for a few hundred rows.  Here each CTA copies the stencils and
+// inverse diagonals of its eighth of every level's unknown rows, and its rows of
+// the coarsest inverse, into shared memory before it waits for the launch that
+// writes the right-hand side.  The vectors are held whole in every CTA: a phase
+// computes the own rows from them and stores the results into all eight
+// (st.shared::cluster), then the cluster meets.  Right-hand sides are needed on
+// the own rows only, and restriction writes the next level's first sweep.
+//
+// In FP64 a warp instruction takes its scheduler's unit 64 clocks, so a phase of
+// one warp is 36 x 64: where a CTA has few rows (MG_BOTTOM_SPLIT) four lanes
+// share one, in the four chains of the row functions (the same bits).  The
+// kernel before releases it at once, so that the stencils are loaded meanwhile
+// (6000 clocks); a phase is then 1000 to 3700 clocks and a meeting 1000.
+//
+// One CTA for all rows could take levels of up to 256 rows in FP64 (16.5 to
+// 21 us), every level above being three launches.  V-cycle, 8 CTAs after one:
+// 100 x 100 cells 85 -> 73 us, 120 x 60 73 -> 65, 256 x 128 94 -> 80, 400 x 400
+// 197 -> 184, 1024 x 512 in FP32 111 -> 109; with 16 CTAs 78, 67, 84, 190, 116,
+// with 4 79, 69, 87, 190, 109.  A cluster of 16 CTAs out of L2 (no shared
+// memory) took 89 us for 128 x 64 cells in FP32 and 203 us in FP64.
 #define MG_BOTTOM_MAX 6
-#define MG_BOTTOM_SMEM (220 * 1024)
-// (FP64: fewer threads with twice the registers, its levels have fewer rows)
+#define MG_BOTTOM_CTAS 8
+#define MG_BOTTOM_SMEM (200 * 1024)
+#define MG_BOTTOM_SPLIT 96   // FP64 rows per CTA up to which four lanes share a row
 template <typename T>
-constexpr int mg_bottom_threads() { return sizeof(T) == 8 ? 512 : 1024; }
+constexpr int mg_bottom_threads() { return sizeof(T) == 8 ? 256 : 512; }
 template <typename T>
 struct mg_bottom_args {
     int nlev, nu1, nu2, ndense;   // nlev levels, the last one the dense coarsest
@@ -863,14 +873,78 @@ struct mg_bottom_args {
     T *xu, *xv;                   // its result
 };
 
-// elements of one level: coefficients and inverse diagonals of the unknown
-// rows, then the vectors x, y (also the residual) and f in box layout
 __host__ __device__ inline int mg_bottom_rows_u(int Nx, int Nz) { return (Nx - 2) * (Nz - 1); }
 __host__ __device__ inline int mg_bottom_rows_v(int Nx, int Nz) { return (Nx - 1) * (Nz - 2); }
+__host__ __device__ inline int mg_bottom_rows(int Nx, int Nz) { return mg_bottom_rows_u(Nx, Nz) + mg_bottom_rows_v(Nx, Nz); }
 __host__ __device__ inline int mg_bottom_box(int Nx, int Nz) { return Nx * (Nz + 1) + (Nx + 1) * Nz; }
-__host__ __device__ inline long long mg_bottom_level_elems(int Nx, int Nz) {
-    return (long long)(MG_NST + 1) * (mg_bottom_rows_u(Nx, Nz) + mg_bottom_rows_v(Nx, Nz)) +
-           3LL * mg_bottom_box(Nx, Nz);
+__host__ __device__ inline int mg_bottom_share(int rows) { return (rows + MG_BOTTOM_CTAS - 1) / MG_BOTTOM_CTAS; }
+// elements of one level in a CTA: vectors x and y (also the residual) in box
+// layout, then coefficients, inverse diagonal and f of its rows
+__host__ __device__ inline int mg_bottom_level_elems(int Nx, int Nz) {
+    return 2 * mg_bottom_box(Nx, Nz) +
+           (MG_NST + 2) * (mg_bottom_share(mg_bottom_rows_u(Nx, Nz)) + mg_bottom_share(mg_bottom_rows_v(Nx, Nz)));
+}
+// A CTA's rows of a level: `Su` u rows, then v rows, S places in all.  Rows
+// meet threads by index: u rows, a gap up to a multiple of `align`, v rows, so
+// that no warp holds both kinds.
+struct mg_bottom_rank {
+    int Nx, Nz, Ru, Rv, Su, S, box, nu, rank;
+    __device__ __forceinline__ mg_bottom_rank(int Nx_, int Nz_, int rank_) : Nx(Nx_), Nz(Nz_), rank(rank_) {
+        Ru = mg_bottom_rows_u(Nx, Nz);
+        Rv = mg_bottom_rows_v(Nx, Nz);
+        Su = mg_bottom_share(Ru);
+        S = Su + mg_bottom_share(Rv);
+        box = mg_bottom_box(Nx, Nz);
+        nu = Nx * (Nz + 1);
+    }
+    __device__ __forceinline__ int count(int align) const { return (Su + align - 1) / align * align + S - Su; }
+    // row of index t: its place i among the CTA's rows, (k, j) and place in the box; false: none
+    __device__ __forceinline__ bool row(int t, int align, bool &u, int &i, int &k, int &j, int &c) const {
+        const int gap = (Su + align - 1) / align * align;
+        u = t < gap;
+        i = u ? t : Su + t - gap;
+        const int r = u ? rank * Su + t : rank * (S - Su) + t - gap, w = u ? Nx - 2 : Nx - 1;
+        k = 1 + r % w;
+        j = 1 + r / w;
+        c = u ? k + j * Nx : nu + k + j * (Nx + 1);
+        return u ? t < Su && r < Ru : t - gap < S - Su && r < Rv;
+    }
+};
+
+// Quarter s of row (k, j)'s product: coefficients s, s + 4, ... (the chains of
+// st_urow_x and st_vrow_x in FP64)
+template <typename T>
+__device__ __forceinline__ T st_row_quarter(bool u, int Nx, int Nz, const T *cf, int S, const T *x, int k, int j, int s) {
+    const T *const xv = x + Nx * (Nz + 1);
+    T a = 0;
+#pragma unroll
+    for (int t = 0; t < 8; t++) {
+        const int q = 4 * t + s;
+        if (q >= MG_NST) break;
+        const T *p;
+        if (q < 15) {
+            const int w = u ? 3 : 5, r = q / w, d = q - w * r;
+            if (u) p = x + (k - 1 + d) + min(max(j + r - 2, 0), Nz) * Nx;
+            else p = xv + (j + r - 1) * (Nx + 1) + min(max(k + d - 2, 0), Nx);
+        } else {
+            const int r = (q - 15) >> 2, d = (q - 15) & 3;
+            if (u) p = xv + (k - 1 + d) + min(max(j + r - 2, 0), Nz - 1) * (Nx + 1);
+            else p = x + (j + r - 1) * Nx + min(max(k + d - 2, 0), Nx - 1);
+        }
+        a += cf[q * S] * *p;
+    }
+    return a;
+}
+
+__device__ __forceinline__ void cluster_meet() {
+    __syncwarp();   // (.aligned: the lanes of a warp arrive together)
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
 
 template <typename T>
@@ -878,132 +952,186 @@ __global__ void __launch_bounds__(mg_bottom_threads<T>()) k_mg_bottom(const __gr
     extern __shared__ __align__(16) unsigned char bottom_sm[];
     T *const sm = reinterpret_cast<T *>(bottom_sm);
     mg_release<T>();
-    constexpr int NT = mg_bottom_threads<T>();
+    constexpr int NT = mg_bottom_threads<T>(), C = MG_BOTTOM_CTAS;
     const int tid = threadIdx.x, lc = A.nlev - 1, n = A.ndense;
+    const int rank = blockIdx.x;   // the grid is the one cluster
+    uint32_t remote[C];            // the CTAs' shared memory in the cluster's address window
+#pragma unroll
+    for (int c = 0; c < C; c++)
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                     : "=r"(remote[c])
+                     : "r"((uint32_t)__cvta_generic_to_shared(sm)), "r"(c));
+    auto put = [&](T *p, T v) {    // into this place of every CTA
+        const uint32_t o = (uint32_t)((p - sm) * sizeof(T));
+#pragma unroll
+        for (int c = 0; c < C; c++) st_cluster(remote[c] + o, v);
+    };
     // ---- static data, while the launch before is still running
     int off = 0;
     for (int l = 0; l < lc; l++) {
-        const int Nx = A.Nx[l], Nz = A.Nz[l], Ru = mg_bottom_rows_u(Nx, Nz), Rv = mg_bottom_rows_v(Nx, Nz);
-        const size_t nu = (size_t)Nx * (Nz + 1), nv = (size_t)(Nx + 1) * Nz;
-        T *cu = sm + off, *cv = cu + (MG_NST + 1) * Ru, *vec = cv + (MG_NST + 1) * Rv;
-        for (int r = tid; r < Ru + Rv; r += NT) {
-            const bool u = r < Ru;
-            const int q = u ? r : r - Ru, w = u ? Nx - 2 : Nx - 1;
-            const size_t c = u ? (size_t)(1 + q % w) + (size_t)(1 + q / w) * Nx
-                               : (size_t)(1 + q % w) + (size_t)(1 + q / w) * (Nx + 1);
+        const mg_bottom_rank L(A.Nx[l], A.Nz[l], rank);
+        const size_t nu = L.nu, nv = (size_t)(L.Nx + 1) * L.Nz;
+        T *vec = sm + off, *cf0 = vec + 2 * L.box;
+        for (int t = tid; t < L.count(32); t += NT) {
+            bool u;
+            int i, k, j, b;
+            if (!L.row(t, 32, u, i, k, j, b)) continue;
+            const size_t c = u ? (size_t)b : (size_t)b - nu;
             T cf[MG_NST];
             st_coefs<T>(u ? A.su[l] : A.sv[l], u ? nu : nv, c, cf);
-            T *d = u ? cu + q : cv + q;
-            const int R = u ? Ru : Rv;
 #pragma unroll
-            for (int e = 0; e < MG_NST; e++) d[e * R] = cf[e];
-            d[MG_NST * R] = u ? A.idu[l][c] : A.idv[l][c];
+            for (int e = 0; e < MG_NST; e++) cf0[e * L.S + i] = cf[e];
+            cf0[MG_NST * L.S + i] = u ? A.idu[l][c] : A.idv[l][c];
         }
-        for (int e = tid; e < 3 * mg_bottom_box(Nx, Nz); e += NT) vec[e] = T(0);
-        off += (int)mg_bottom_level_elems(Nx, Nz);
+        for (int e = tid; e < 2 * L.box; e += NT) vec[e] = T(0);
+        off += mg_bottom_level_elems(L.Nx, L.Nz);
     }
-    const int cbox = mg_bottom_box(A.Nx[lc], A.Nz[lc]);
-    T *const cx = sm + off, *const cf_ = cx + cbox, *const fs = cf_ + cbox, *const Ai = fs + n;
-    for (int e = tid; e < 2 * cbox; e += NT) cx[e] = T(0);
-    for (int e = tid; e < n * n; e += NT) Ai[e] = A.AinvT[e];
-    __syncthreads();   // the vectors are cleared before the right-hand side goes into one
+    const int cbox = mg_bottom_box(A.Nx[lc], A.Nz[lc]), Sn = mg_bottom_share(n), n0 = rank * Sn,
+              nown = n - n0 < Sn ? n - n0 : Sn;   // dense rows of this CTA (none: <= 0)
+    T *const cx = sm + off, *const fs = cx + cbox, *const Ai = fs + n;
+    for (int e = tid; e < cbox; e += NT) cx[e] = T(0);
+    for (int e = tid; e < n * Sn; e += NT) {
+        const int i = e % Sn;
+        if (i < nown) Ai[e] = A.AinvT[(size_t)(e / Sn) * n + n0 + i];
+    }
+    {   // the caller's vectors are 0 where there is no unknown
+        const mg_bottom_rank L(A.Nx[0], A.Nz[0], rank);
+        for (int e = rank * NT + tid; e < L.box; e += C * NT) {
+            const bool u = e < L.nu;
+            const int k = u ? e % L.Nx : (e - L.nu) % (L.Nx + 1), j = u ? e / L.Nx : (e - L.nu) / (L.Nx + 1);
+            if (u && !(k > 0 && k < L.Nx - 1 && j > 0 && j < L.Nz)) A.xu[e] = T(0);
+            if (!u && !(k > 0 && k < L.Nx && j > 0 && j < L.Nz - 1)) A.xv[e - L.nu] = T(0);
+        }
+    }
+    cluster_meet();   // every CTA has cleared its vectors before any stores into them
     pdl_wait();
-    {
-        const int nu = A.Nx[0] * (A.Nz[0] + 1), box = mg_bottom_box(A.Nx[0], A.Nz[0]);
-        T *f = sm + (MG_NST + 1) * (mg_bottom_rows_u(A.Nx[0], A.Nz[0]) + mg_bottom_rows_v(A.Nx[0], A.Nz[0])) + 2 * box;
-        for (int e = tid; e < box; e += NT) f[e] = e < nu ? A.fu[e] : A.fv[e - nu];
-    }
-    __syncthreads();
     unsigned par = 0;   // bit l: level l's x is in its second vector
-    // mode 0: x = omega D^-1 f; 1: y = x + omega D^-1 (f - A x); 2: y = f - A x
-    auto rows = [&](int base, int Nx, int Nz, bool odd, int mode) {
-        const int Ru = mg_bottom_rows_u(Nx, Nz), Rv = mg_bottom_rows_v(Nx, Nz), nu = Nx * (Nz + 1),
-                  box = mg_bottom_box(Nx, Nz);
-        const T *cu = sm + base, *cv = cu + (MG_NST + 1) * Ru;
-        T *vec = sm + base + (MG_NST + 1) * (Ru + Rv);
-        T *x = vec + (odd ? box : 0), *y = vec + (odd ? 0 : box);
-        const T *f = vec + 2 * box;
-        for (int r = tid; r < Ru + Rv; r += NT) {
-            const bool u = r < Ru;
-            const int q = u ? r : r - Ru, w = u ? Nx - 2 : Nx - 1, R = u ? Ru : Rv;
-            const int k = 1 + q % w, l = 1 + q / w, c = u ? k + l * Nx : nu + k + l * (Nx + 1);
-            const T *d = u ? cu + q : cv + q;
-            const T id = d[MG_NST * R];
-            if (mode == 0) { x[c] = A.omega * id * f[c]; continue; }
-            T cf[MG_NST];
+    // mode 1: y = x + omega D^-1 (f - A x); 2: y = f - A x; 3: as 1, into the caller's vectors
+    auto rows = [&](int base, int l, bool odd, int mode) {
+        const mg_bottom_rank L(A.Nx[l], A.Nz[l], rank);
+        T *const x = sm + base + (odd ? L.box : 0), *const y = sm + base + (odd ? 0 : L.box),
+                 *const cf0 = sm + base + 2 * L.box;
+        bool u;
+        int i, k, j, c;
+        if (sizeof(T) == 8 && L.count(8) <= MG_BOTTOM_SPLIT) {   // four lanes per row
+            const int s = tid & 3;
+            for (int t = tid >> 2; t < (L.count(8) + 7) / 8 * 8; t += NT / 4) {
+                const bool in = L.row(t, 8, u, i, k, j, c);
+                T ax = in ? st_row_quarter<T>(u, L.Nx, L.Nz, cf0 + i, L.S, x, k, j, s) : T(0);
+                ax += __shfl_xor_sync(0xffffffffu, ax, 1);
+                ax += __shfl_xor_sync(0xffffffffu, ax, 2);
+                if (!in) continue;
+                const T r = cf0[(MG_NST + 1) * L.S + i] - ax;
+                const T v = mode == 2 ? r : x[c] + A.omega * cf0[MG_NST * L.S + i] * r;
+                if (mode != 3) {   // into two CTAs each
+                    const uint32_t o = (uint32_t)((y + c - sm) * sizeof(T));
 #pragma unroll
-            for (int e = 0; e < MG_NST; e++) cf[e] = d[e * R];
-            const T ax = u ? st_urow_x<T>(Nx, Nz, cf, x, x + nu, k, l) : st_vrow_x<T>(Nx, Nz, cf, x, x + nu, k, l);
-            y[c] = mode == 1 ? x[c] + A.omega * id * (f[c] - ax) : f[c] - ax;
+                    for (int q = 0; q < C; q++)
+                        if ((q & 3) == s) st_cluster(remote[q] + o, v);
+                } else if (s == 0) {
+                    if (u) A.xu[c] = v;
+                    else A.xv[c - L.nu] = v;
+                }
+            }
+        } else {
+            for (int t = tid; t < L.count(32); t += NT) {
+                if (!L.row(t, 32, u, i, k, j, c)) continue;
+                T cf[MG_NST];
+#pragma unroll
+                for (int e = 0; e < MG_NST; e++) cf[e] = cf0[e * L.S + i];
+                const T ax = u ? st_urow_x<T>(L.Nx, L.Nz, cf, x, x + L.nu, k, j)
+                               : st_vrow_x<T>(L.Nx, L.Nz, cf, x, x + L.nu, k, j);
+                const T r = cf0[(MG_NST + 1) * L.S + i] - ax;
+                const T v = mode == 2 ? r : x[c] + A.omega * cf0[MG_NST * L.S + i] * r;
+                if (mode != 3) put(y + c, v);
+                else if (u) A.xu[c] = v;
+                else A.xv[c - L.nu] = v;
+            }
         }
-        __syncthreads();
-    };
-    auto vecs = [&](int base, int l) {   // start of level l's vectors
-        return l == lc ? cx : sm + base + (MG_NST + 1) * (mg_bottom_rows_u(A.Nx[l], A.Nz[l]) + mg_bottom_rows_v(A.Nx[l], A.Nz[l]));
+        if (mode != 3) cluster_meet();
     };
     int base = 0;
+    {   // right-hand side of the own rows and the first sweep from x = 0
+        const mg_bottom_rank L(A.Nx[0], A.Nz[0], rank);
+        T *const cf0 = sm + 2 * L.box;
+        for (int t = tid; t < L.count(32); t += NT) {
+            bool u;
+            int i, k, j, c;
+            if (!L.row(t, 32, u, i, k, j, c)) continue;
+            const T f = u ? A.fu[c] : A.fv[c - L.nu];
+            cf0[(MG_NST + 1) * L.S + i] = f;
+            put(sm + c, A.omega * cf0[MG_NST * L.S + i] * f);
+        }
+        cluster_meet();
+    }
     for (int l = 0; l < lc; l++) {
-        const int Nx = A.Nx[l], Nz = A.Nz[l], next = base + (int)mg_bottom_level_elems(Nx, Nz);
-        rows(base, Nx, Nz, false, 0);
+        const int Nx = A.Nx[l], Nz = A.Nz[l], next = base + mg_bottom_level_elems(Nx, Nz);
         bool odd = false;
-        for (int s = 1; s < A.nu1; s++) { rows(base, Nx, Nz, odd, 1); odd = !odd; }
+        for (int s = 1; s < A.nu1; s++) { rows(base, l, odd, 1); odd = !odd; }
         if (odd) par |= 1u << l;
-        rows(base, Nx, Nz, odd, 2);
+        rows(base, l, odd, 2);
         // restriction of the residual
-        const box_geom F{Nx, Nz, Nx - 1, Nz - 1}, C{A.Nx[l + 1], A.Nz[l + 1], A.Nx[l + 1] - 1, A.Nz[l + 1] - 1};
-        const int box = mg_bottom_box(Nx, Nz), nu = Nx * (Nz + 1), nuc = C.Nx * (C.Nz + 1);
-        const T *r = vecs(base, l) + (odd ? 0 : box);
-        T *f = vecs(next, l + 1) + (l + 1 == lc ? 1 : 2) * mg_bottom_box(C.Nx, C.Nz);
-        const int Ru = mg_bottom_rows_u(C.Nx, C.Nz), Rv = mg_bottom_rows_v(C.Nx, C.Nz);
-        for (int p = tid; p < Ru + Rv; p += NT) {
-            if (p < Ru) {
-                const int I = 1 + p % (C.Nx - 2), J = 1 + p / (C.Nx - 2);
-                f[I + J * C.Nx] = restricted_u<T>(F, C, r, I, J);
-            } else {
-                const int q = p - Ru, I = 1 + q % (C.Nx - 1), J = 1 + q / (C.Nx - 1);
-                f[nuc + I + J * (C.Nx + 1)] = restricted_v<T>(F, C, r + nu, I, J);
+        const box_geom F{Nx, Nz, Nx - 1, Nz - 1}, Cg{A.Nx[l + 1], A.Nz[l + 1], A.Nx[l + 1] - 1, A.Nz[l + 1] - 1};
+        const T *r = sm + base + (odd ? 0 : mg_bottom_box(Nx, Nz)), *rv = r + Nx * (Nz + 1);
+        if (l + 1 < lc) {   // and the next level's first sweep
+            const mg_bottom_rank L(Cg.Nx, Cg.Nz, rank);
+            T *const cf0 = sm + next + 2 * L.box;
+            for (int t = tid; t < L.count(32); t += NT) {
+                bool u;
+                int i, I, J, c;
+                if (!L.row(t, 32, u, i, I, J, c)) continue;
+                const T f = u ? restricted_u<T>(F, Cg, r, I, J) : restricted_v<T>(F, Cg, rv, I, J);
+                cf0[(MG_NST + 1) * L.S + i] = f;
+                put(sm + next + c, A.omega * cf0[MG_NST * L.S + i] * f);
+            }
+        } else {
+            const int nuc = Cg.Nx * (Cg.Nz + 1);
+            for (int i = tid; i < nown; i += NT) {
+                const int m = A.dmap[n0 + i], q = m - nuc;
+                put(fs + n0 + i, m < nuc ? restricted_u<T>(F, Cg, r, m % Cg.Nx, m / Cg.Nx)
+                                         : restricted_v<T>(F, Cg, rv, q % (Cg.Nx + 1), q / (Cg.Nx + 1)));
             }
         }
-        __syncthreads();
+        cluster_meet();
         base = next;
     }
-    {   // coarsest level: x = A^-1 f
-        for (int i = tid; i < n; i += NT) fs[i] = cf_[A.dmap[i]];
-        __syncthreads();
-        for (int r0 = 0; r0 < n; r0 += NT / 8) {
-            const int r = r0 + tid / 8;
-            const T s = dense_row<T>(n, Ai, fs, r, tid & 7);
-            if (r < n && (tid & 7) == 0) cx[A.dmap[r]] = s;
-        }
-        __syncthreads();
+    // coarsest level: x = A^-1 f, eight lanes per row
+    for (int r0 = 0; r0 < nown; r0 += NT / 8) {
+        const int r = r0 + tid / 8;
+        T s = 0;
+        if (r < nown)
+            for (int j = tid & 7; j < n; j += 8) s += Ai[j * Sn + r] * fs[j];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (r < nown && (tid & 7) == 0) put(cx + A.dmap[n0 + r], s);
     }
+    cluster_meet();
     for (int l = lc - 1; l >= 0; l--) {
         const int Nx = A.Nx[l], Nz = A.Nz[l], next = base;
-        base -= (int)mg_bottom_level_elems(Nx, Nz);
+        base -= mg_bottom_level_elems(Nx, Nz);
         bool odd = par >> l & 1;
-        const box_geom F{Nx, Nz, Nx - 1, Nz - 1}, C{A.Nx[l + 1], A.Nz[l + 1], A.Nx[l + 1] - 1, A.Nz[l + 1] - 1};
-        const int box = mg_bottom_box(Nx, Nz), nu = Nx * (Nz + 1), nuc = C.Nx * (C.Nz + 1);
-        T *x = vecs(base, l) + (odd ? box : 0);
-        const T *c = vecs(next, l + 1) + (par >> (l + 1) & 1 ? mg_bottom_box(C.Nx, C.Nz) : 0);
-        const int Ru = mg_bottom_rows_u(Nx, Nz), Rv = mg_bottom_rows_v(Nx, Nz);
-        for (int p = tid; p < Ru + Rv; p += NT) {
-            if (p < Ru) {
-                const int k = 1 + p % (Nx - 2), j = 1 + p / (Nx - 2);
-                x[k + j * Nx] = prolonged_u<T>(F, C, c, x, k, j);
-            } else {
-                const int q = p - Ru, i = 1 + q % (Nx - 1), j = 1 + q / (Nx - 1);
-                x[nu + i + j * (Nx + 1)] = prolonged_v<T>(F, C, c + nuc, x + nu, i, j);
-            }
+        const box_geom F{Nx, Nz, Nx - 1, Nz - 1}, Cg{A.Nx[l + 1], A.Nz[l + 1], A.Nx[l + 1] - 1, A.Nz[l + 1] - 1};
+        const mg_bottom_rank L(Nx, Nz, rank);
+        const int nuc = Cg.Nx * (Cg.Nz + 1);
+        T *x = sm + base + (odd ? L.box : 0);
+        const T *c = sm + next + (par >> (l + 1) & 1 ? mg_bottom_box(Cg.Nx, Cg.Nz) : 0);
+        const bool last = l == 0 && A.nu2 == 0;
+        for (int t = tid; t < L.count(32); t += NT) {
+            bool u;
+            int i, k, j, b;
+            if (!L.row(t, 32, u, i, k, j, b)) continue;
+            const T v = u ? prolonged_u<T>(F, Cg, c, x, k, j) : prolonged_v<T>(F, Cg, c + nuc, x + L.nu, k, j);
+            if (!last) put(x + b, v);
+            else if (u) A.xu[b] = v;
+            else A.xv[b - L.nu] = v;
         }
-        __syncthreads();
-        for (int s = 0; s < A.nu2; s++) { rows(base, Nx, Nz, odd, 1); odd = !odd; }
+        if (last) break;
+        cluster_meet();
+        for (int s = 0; s < A.nu2; s++) {
+            rows(base, l, odd, l == 0 && s == A.nu2 - 1 ? 3 : 1);
+            odd = !odd;
+        }
         par = odd ? par | 1u << l : par & ~(1u << l);
-    }
-    const int nu0 = A.Nx[0] * (A.Nz[0] + 1), box0 = mg_bottom_box(A.Nx[0], A.Nz[0]);
-    const T *x = vecs(0, 0) + (par & 1 ? box0 : 0);
-    for (int e = tid; e < box0; e += NT) {
-        if (e < nu0) A.xu[e] = x[e];
-        else A.xv[e - nu0] = x[e];
     }
 }
 
@@ -1369,27 +1497,33 @@ static mdz_status mg_setup(mdz_ctx *ctx, mg_hier<T> &H, const double *eta_n, con
 
 static inline dim3 box_grid(int Nx, int Nz) { return dim3((Nx + 1 + 31) / 32, (Nz + 1 + 7) / 8); }
 
-// Shared memory of the bottom kernel run from level l down.
+// Shared memory per CTA of the bottom kernel run from level l down.
 template <typename T>
 static size_t mg_bottom_bytes(const mg_hier<T> &H, int l) {
     long long n = 0;
     for (int q = l; q < H.nlev - 1; q++) n += mg_bottom_level_elems(H.L[q].Nx, H.L[q].Nz);
     const mg_level<T> &C = H.L[H.nlev - 1];
-    n += 2LL * mg_bottom_box(C.Nx, C.Nz) + (long long)C.ndense * (C.ndense + 1);
+    n += mg_bottom_box(C.Nx, C.Nz) + (long long)C.ndense * (1 + mg_bottom_share(C.ndense));
     return (size_t)n * sizeof(T);
 }
 
 // Whether vcycle() runs level l and all below it in the one-launch bottom
-// kernel: as soon as their data fit in one CTA's shared memory and, in FP64,
-// the level has at most 256 rows (more are too much for one SM's FP64 units:
-// 312 rows took 37 us, as grid kernels some 22).
+// kernel: as soon as their data fit the cluster's shared memory and the level
+// has at most 2048 rows in FP64 (33 x 32 cells), 4096 in FP32 (64 x 32 and a
+// little).  V-cycle of 100 x 100, 256 x 128 and 400 x 400 cells in FP64, us:
+//   limit   256     600     2048
+//           85      77      73
+//           89      84      80
+//           199     188     184
+#define MG_BOTTOM_ROWS64 2048
+#define MG_BOTTOM_ROWS32 4096
 template <typename T>
 static bool vcycle_bottom(const mg_hier<T> &H, int l) {
     const mg_level<T> &L = H.L[l];
     const bool viscous = l == 0 && !H.newton;   // level 0 of a Picard hierarchy: stencil from eta directly
     return !viscous && l < H.nlev - 1 && H.L[H.nlev - 1].ndense && H.nlev - l <= MG_BOTTOM_MAX &&
-           mg_bottom_bytes<T>(H, l) <= MG_BOTTOM_SMEM &&
-           (sizeof(T) == 4 || mg_bottom_rows_u(L.Nx, L.Nz) + mg_bottom_rows_v(L.Nx, L.Nz) <= 256);
+           mg_bottom_rows(L.Nx, L.Nz) <= (sizeof(T) == 4 ? MG_BOTTOM_ROWS32 : MG_BOTTOM_ROWS64) &&
+           mg_bottom_bytes<T>(H, l) <= MG_BOTTOM_SMEM;
 }
 
 // Whether vcycle() smooths level l with its own sweeps (not the dense
@@ -1439,7 +1573,7 @@ static mdz_status vcycle(mdz_ctx *ctx, mg_hier<T> &H, int l, int nu1, int nu2, T
             A.su[q] = B.su; A.sv[q] = B.sv; A.idu[q] = B.idu; A.idv[q] = B.idv;
         }
         A.fu = L.fu; A.fv = L.fv; A.xu = L.xu; A.xv = L.xv;
-        MDZ_PDL(ctx, k_mg_bottom<T>, 1, mg_bottom_threads<T>(), mg_bottom_bytes<T>(H, l), st, A);
+        MDZ_PDL_CLUSTER(ctx, MG_BOTTOM_CTAS, k_mg_bottom<T>, MG_BOTTOM_CTAS, mg_bottom_threads<T>(), mg_bottom_bytes<T>(H, l), st, A);
         return MDZ_OK;
     }
     const int rows_grid = mdz_blocks(L.nu() + L.nv(), ST_THREADS);
