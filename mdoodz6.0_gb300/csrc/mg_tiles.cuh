@@ -405,22 +405,22 @@ struct vel_global {
     __device__ __forceinline__ T v(int i, int j) const { return xv[i + j * (Nx + 1)]; }
 };
 
-// out = x + omega * D^-1 (f - A x)  (x == nullptr: x = 0), 32 x 8 points per block
-template <typename T>
-__global__ void __launch_bounds__(256) k_mg_smooth(stokes_geom G, stokes_coefs<T> D, const T *__restrict__ xu,
+// out = x + omega * D^-1 (f - A x)  (x == nullptr: x = 0), TW x TH points per block
+template <typename T, int TW, int TH>
+__global__ void __launch_bounds__(TW *TH) k_mg_smooth(stokes_geom G, stokes_coefs<T> D, const T *__restrict__ xu,
                                                    const T *__restrict__ xv, const T *__restrict__ fu,
                                                    const T *__restrict__ fv, const T *__restrict__ idu,
                                                    const T *__restrict__ idv, T omega, T *__restrict__ ou,
                                                    T *__restrict__ ov) {
     constexpr bool TILE = mg_stress_tile<T>();
-    __shared__ visc_tile<T, TILE ? 33 : 1, TILE ? 9 : 1> S;
+    __shared__ visc_tile<T, TILE ? TW + 1 : 1, TILE ? TH + 1 : 1> S;
     mg_release<T>();
     pdl_wait();
-    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 8, a = threadIdx.x & 31, b = threadIdx.x >> 5;
+    const int i0 = blockIdx.x * TW, j0 = blockIdx.y * TH, a = threadIdx.x % TW, b = threadIdx.x / TW;
     const int i = i0 + a, j = j0 + b, Nx = G.Nx, Nz = G.Nz;
     const vel_global<T> X{xu, xv, Nx};
     if (TILE && xu) {
-        S.fill(G, D, X, i0 - 1, j0 - 1, threadIdx.x, 256);
+        S.fill(G, D, X, i0 - 1, j0 - 1, threadIdx.x, TW * TH);
         __syncthreads();
     }
     const T ratio = gc<T>(G, GC_DZ) * gc<T>(G, GC_IDX);

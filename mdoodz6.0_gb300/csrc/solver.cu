@@ -1497,6 +1497,30 @@ static mdz_status mg_setup(mdz_ctx *ctx, mg_hier<T> &H, const double *eta_n, con
 
 static inline dim3 box_grid(int Nx, int Nz) { return dim3((Nx + 1 + 31) / 32, (Nz + 1 + 7) / 8); }
 
+// Whether the FP64 level-0 kernels of a grid take tiles of 16 x 4 points and the
+// restriction tiles of 8 x 4 coarse points: where the 32 x 8 (16 x 8) tiles leave
+// SMs idle, or little more than one to each.  A warp's FP64 instruction takes its
+// scheduler's unit 64 clocks, so eight warps on one SM in three take three times
+// as long as spread out.  V-cycle, before and after: 100 x 100 cells 72.9 and
+// 68.4 us, 120 x 60 62.6 and 58.2, 256 x 128 (153 tiles) 78.3 and 76.0; from
+// 200 tiles on (400 x 400: 181 and 181) the smaller halo of the large tiles
+// counts.  FP32 is not bound by that unit.
+#define MG_SMALL_W 16
+#define MG_SMALL_H 4
+#define MG_SMALL_TILES 200
+#define MG_RR_W 8
+#define MG_RR_H 4
+#define MG_RR_T 352
+#define MG_RR_TILES 152
+template <typename T>
+static bool mg_small_tiles(int Nx, int Nz) {
+    return sizeof(T) == 8 && ((Nx + 32) / 32) * ((Nz + 8) / 8) < MG_SMALL_TILES;
+}
+template <typename T>
+static bool mg_small_coarse(int Nxc, int Nzc) {
+    return sizeof(T) == 8 && ((Nxc + 16) / 16) * ((Nzc + 8) / 8) < MG_RR_TILES;
+}
+
 // Shared memory per CTA of the bottom kernel run from level l down.
 template <typename T>
 static size_t mg_bottom_bytes(const mg_hier<T> &H, int l) {
@@ -1577,8 +1601,14 @@ static mdz_status vcycle(mdz_ctx *ctx, mg_hier<T> &H, int l, int nu1, int nu2, T
         return MDZ_OK;
     }
     const int rows_grid = mdz_blocks(L.nu() + L.nv(), ST_THREADS);
+    const bool small = mg_small_tiles<T>(L.Nx, L.Nz);
+    auto tiles = [&](int w, int h) { return dim3((L.Nx + w) / w, (L.Nz + h) / h); };
     auto smooth = [&](const T *xu, const T *xv, T *ou, T *ov) -> mdz_status {
-        if (viscous) MDZ_PDL(ctx, k_mg_smooth<T>, gr, 256, 0, st, G, D, xu, xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
+        if (viscous && small)
+            MDZ_PDL(ctx, (k_mg_smooth<T, MG_SMALL_W, MG_SMALL_H>), tiles(MG_SMALL_W, MG_SMALL_H), MG_SMALL_W * MG_SMALL_H, 0,
+                    st, G, D, xu, xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
+        else if (viscous)
+            MDZ_PDL(ctx, (k_mg_smooth<T, 32, 8>), gr, 256, 0, st, G, D, xu, xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov);
         else MDZ_PDL(ctx, k_st_smooth<T>, rows_grid, ST_THREADS, 0, st, G, L.su, L.sv, xu, xv, L.fu, L.fv, L.idu, L.idv,
                      omega, ou, ov);
         return MDZ_OK;
@@ -1600,7 +1630,8 @@ static mdz_status vcycle(mdz_ctx *ctx, mg_hier<T> &H, int l, int nu1, int nu2, T
 #define MG_RR(kernel, TX, TY, NT, ...)                                                                                \
     MDZ_PDL(ctx, kernel<T, TX, TY, NT>, dim3((cw + TX - 1) / TX, (ch + TY - 1) / TY), NT, 0, st, G, __VA_ARGS__, L.xu, \
             L.xv, L.fu, L.fv, GC, C.fu, C.fv, C.idu, C.idv, omega, cxu, cxv)
-    if (viscous) MG_RR(k_mg_resid_restrict, 16, 8, 384, D);
+    if (viscous && mg_small_coarse<T>(C.Nx, C.Nz)) MG_RR(k_mg_resid_restrict, MG_RR_W, MG_RR_H, MG_RR_T, D);
+    else if (viscous) MG_RR(k_mg_resid_restrict, 16, 8, 384, D);
     else if (cpts > MG_TILE_LARGE) MG_RR(k_st_resid_restrict, 16, 8, 416, L.su, L.sv);
     else if (cpts > MG_TILE_SMALL) MG_RR(k_st_resid_restrict, 8, 4, 352, L.su, L.sv);
     else MG_RR(k_st_resid_restrict, 4, 2, 128, L.su, L.sv);
@@ -1613,7 +1644,11 @@ static mdz_status vcycle(mdz_ctx *ctx, mg_hier<T> &H, int l, int nu1, int nu2, T
     // prolongation and the first post-smoothing sweep in one launch; the last
     // sweep goes straight into the caller's vector
     T *ou = nu2 == 1 && out_u ? out_u : L.yu, *ov = nu2 == 1 && out_u ? out_v : L.yv;
-    if (viscous)
+    if (viscous && small)
+        MDZ_PDL(ctx, (k_mg_prolong_smooth<T, MG_SMALL_W, MG_SMALL_H>), tiles(MG_SMALL_W, MG_SMALL_H),
+                MG_SMALL_W * MG_SMALL_H, 0, st, G, D, GC, C.xu, C.xv, L.xu, L.xv, L.fu, L.fv, L.idu, L.idv, omega, ou, ov,
+                zp, H.pmean);
+    else if (viscous)
         MDZ_PDL(ctx, k_mg_prolong_smooth<T, 32, 8>, gr, 256, 0, st, G, D, GC, C.xu, C.xv, L.xu, L.xv, L.fu, L.fv, L.idu,
                 L.idv, omega, ou, ov, zp, H.pmean);
     else if ((long long)(L.Nx + 1) * (L.Nz + 1) > MG_TILE_SMALL)
@@ -1662,8 +1697,8 @@ __global__ void k_psub(int np, const signed char *__restrict__ tp, const double 
 // f = r_vel - B zp on the fine level (B: celvol-scaled pressure gradient), with xu non-null the V-cycle's first
 // sweep from x = 0, x = omega D^-1 f, and the sum, count and mean of zp over the
 // pressure equations for the zero-mean projection in the last launch.
-template <typename T>
-__global__ void __launch_bounds__(256) k_precond(stokes_geom G, const T *__restrict__ D11, const T *__restrict__ Dt,
+template <typename T, int TW, int TH>
+__global__ void __launch_bounds__(TW *TH) k_precond(stokes_geom G, const T *__restrict__ D11, const T *__restrict__ Dt,
                                                  const T *__restrict__ ru, const T *__restrict__ rv,
                                                  const T *__restrict__ rp, T *__restrict__ zp, T *__restrict__ fu,
                                                  T *__restrict__ fv, const T *__restrict__ idu,
@@ -1671,16 +1706,15 @@ __global__ void __launch_bounds__(256) k_precond(stokes_geom G, const T *__restr
                                                  T *__restrict__ xv, double *part, unsigned int *counter,
                                                  double *psum) {
     mg_release<T>();
-    __shared__ T s_z[9][33];   // zp of the centroids (i0 - 1 .. i0 + 31, j0 - 1 .. j0 + 7)
-    const int Nx = G.Nx, Nz = G.Nz, ncx = G.ncx, ncz = G.ncz, a = threadIdx.x & 31, h = threadIdx.x >> 5;
-    const int ntx = (Nx + 32) / 32, ntiles = ntx * ((Nz + 8) / 8);
+    __shared__ T s_z[TH + 1][TW + 1];   // zp of the centroids from (i0 - 1, j0 - 1)
+    const int Nx = G.Nx, Nz = G.Nz, ncx = G.ncx, ncz = G.ncz, a = threadIdx.x % TW, h = threadIdx.x / TW;
+    const int ntx = (Nx + TW) / TW, ntiles = ntx * ((Nz + TH) / TH);
     const T half_ivol = T(0.5) * gc<T>(G, GC_IXZ);
     T acc = 0;
-    int cnt = 0;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int i0 = (tile % ntx) * 32, j0 = (tile / ntx) * 8, i = i0 + a, j = j0 + h;
-        for (int t = threadIdx.x; t < 33 * 9; t += 256) {
-            const int k = i0 - 1 + t % 33, l = j0 - 1 + t / 33;
+        const int i0 = (tile % ntx) * TW, j0 = (tile / ntx) * TH, i = i0 + a, j = j0 + h;
+        for (int t = threadIdx.x; t < (TW + 1) * (TH + 1); t += TW * TH) {
+            const int k = i0 - 1 + t % (TW + 1), l = j0 - 1 + t / (TW + 1);
             T v = 0;
             if (k >= 0 && k < ncx && l >= 0 && l < ncz) {
                 const int c = k + l * ncx;
@@ -1691,7 +1725,7 @@ __global__ void __launch_bounds__(256) k_precond(stokes_geom G, const T *__restr
                 }
                 v = half_ivol * d * rp[c];
             }
-            s_z[t / 33][t % 33] = v;
+            s_z[t / (TW + 1)][t % (TW + 1)] = v;
         }
         __syncthreads();
         if (i < Nx && j <= Nz) {
@@ -1718,14 +1752,13 @@ __global__ void __launch_bounds__(256) k_precond(stokes_geom G, const T *__restr
             const T v = s_z[h + 1][a + 1];
             zp[i + j * ncx] = v;
             acc += v;
-            cnt++;
         }
         __syncthreads();
     }
-    const T v[2] = {acc, (T)cnt};   // (counts per thread are small integers: exact in T)
-    if (mdz_grid_sum<2, T>(v, part, counter, psum)) {
+    const T v[1] = {acc};
+    if (mdz_grid_sum<1, T>(v, part, counter, psum)) {
         __syncthreads();
-        if (threadIdx.x == 0) psum[2] = psum[1] > 0 ? (double)((T)psum[0] / (T)psum[1]) : 0.0;
+        if (threadIdx.x == 0) psum[2] = (double)((T)psum[0] / (T)(ncx * ncz));
     }
 }
 
@@ -1768,11 +1801,17 @@ static mdz_status precondition(mdz_ctx *ctx, mg_hier<T> &H, const T *Dt, const T
     T *const zp = z + nu + nv;
     // zero-mean pressure block: constants are the operator's null space; left
     // in, they grow in the iterates and cost the FP32 gradients their accuracy
-    int blocks = ((F.Nx + 32) / 32) * ((F.Nz + 8) / 8);
+    const bool small = mg_small_tiles<T>(F.Nx, F.Nz);
+    const int tw = small ? MG_SMALL_W : 32, th = small ? MG_SMALL_H : 8;
+    int blocks = ((F.Nx + tw) / tw) * ((F.Nz + th) / th);
     if (blocks > 152 * 8) blocks = 152 * 8;
-    k_precond<T><<<blocks, 256, 0, st>>>(G, F.D11, Dt, r, r + nu, r + nu + nv, zp, F.fu, F.fv, F.idu, F.idv,
-                                         (T)S->omega, fused ? F.xu : nullptr, fused ? F.xv : nullptr,
-                                         ctx->red_part + MDZ_RP_PRECP, ctx->red_cnt + MDZ_RC_PRECP, H.pmean);
+#define PRECOND(W, H_)                                                                                                   \
+    k_precond<T, W, H_><<<blocks, W * H_, 0, st>>>(G, F.D11, Dt, r, r + nu, r + nu + nv, zp, F.fu, F.fv, F.idu, F.idv,   \
+                                                   (T)S->omega, fused ? F.xu : nullptr, fused ? F.xv : nullptr,          \
+                                                   ctx->red_part + MDZ_RP_PRECP, ctx->red_cnt + MDZ_RC_PRECP, H.pmean)
+    if (small) PRECOND(MG_SMALL_W, MG_SMALL_H);
+    else PRECOND(32, 8);
+#undef PRECOND
     MDZ_LAUNCHED(ctx);
     mdz_status s = vcycle<T>(ctx, H, 0, S->nu1, S->nu2, (T)S->omega, st, fused, fused ? z : nullptr,
                              fused ? z + nu : nullptr, mean_fused ? zp : nullptr);

@@ -85,18 +85,19 @@ __global__ void __launch_bounds__(256) k_stokes_apply(stokes_geom G, stokes_coef
 // The FP64 Newton apply is bound by the FP64 pipe: row by row it took 200 FP64
 // instructions a point, here about 60: 401^2 77 -> 31 us, 1025 x 513 203 -> 82 us;
 // FP32 1025 x 513 25 -> 16 us.
-constexpr int SB_W = 33, SB_H = 9;   // stresses: centroids and vertices from (i0 - 1, j0 - 1)
-template <typename T, bool NEWTON, bool RES>
-__global__ void __launch_bounds__(256) k_stokes_apply_box(stokes_geom G, stokes_coefs<T> D, stokes_cvec<T> x,
+template <typename T, bool NEWTON, bool RES, int TW, int TH>
+__global__ void __launch_bounds__(TW *TH) k_stokes_apply_box(stokes_geom G, stokes_coefs<T> D, stokes_cvec<T> x,
                                                           stokes_vec<T> y, stokes_cvec<T> b) {
+    // rates: centroids from (i0 - 2, j0 - 2), vertices from (i0 - 1, j0 - 1); stresses: both from (i0 - 1, j0 - 1)
+    constexpr int RT_W = TW + 2, RT_H = TH + 2, SB_W = TW + 1, SB_H = TH + 1;
     __shared__ T s_ex[RT_H][RT_W], s_ez[RT_H][RT_W], s_g[RT_H][RT_W], s_p[NEWTON ? RT_H : 1][RT_W];
     __shared__ T s_xx[SB_H][SB_W], s_zz[SB_H][SB_W], s_xz[SB_H][SB_W];
     const int Nx = G.Nx, Nz = G.Nz, ncx = G.ncx, ncz = G.ncz, nxvz = Nx + 1;
-    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 8, tid = threadIdx.x;
+    const int i0 = blockIdx.x * TW, j0 = blockIdx.y * TH, tid = threadIdx.x;
     const T idx = gc<T>(G, GC_IDX), idz = gc<T>(G, GC_IDZ), dx = gc<T>(G, GC_DX), dz = gc<T>(G, GC_DZ);
     const T third = T(1.0 / 3.0);
     // rates at centroids from (i0 - 2, j0 - 2) and vertices from (i0 - 1, j0 - 1)
-    for (int t = tid; t < RT_W * RT_H; t += 256) {
+    for (int t = tid; t < RT_W * RT_H; t += TW * TH) {
         const int a = t % RT_W, h = t / RT_W;
         const int kc = i0 - 2 + a, lc = j0 - 2 + h, kv = kc + 1, lv = lc + 1;
         T ex = 0, ez = 0, g = 0, pc = 0;
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(256) k_stokes_apply_box(stokes_geom G, stokes_
         if (NEWTON) s_p[h][a] = pc;
     }
     __syncthreads();
-    for (int t = tid; t < SB_W * SB_H; t += 256) {
+    for (int t = tid; t < SB_W * SB_H; t += TW * TH) {
         const int a = t % SB_W, h = t / SB_W, k = i0 - 1 + a, l = j0 - 1 + h;
         T xx = 0, zz = 0, xz = 0;
         if (k >= 0 && k < ncx && l >= 0 && l < ncz) {   // centroid (k, l): vertices (k .. k+1, l .. l+1)
@@ -149,7 +150,7 @@ __global__ void __launch_bounds__(256) k_stokes_apply_box(stokes_geom G, stokes_
         s_xz[h][a] = xz;
     }
     __syncthreads();
-    const int a = (tid & 31) + 1, h = (tid >> 5) + 1, i = i0 + a - 1, j = j0 + h - 1;   // (a, h): tile position of (i, j)
+    const int a = tid % TW + 1, h = tid / TW + 1, i = i0 + a - 1, j = j0 + h - 1;   // (a, h): tile position of (i, j)
     auto gm4 = [&](int q, int e) {   // mean shear rate of the centroid at tile position (q, e), as above
         return T(0.25) * ((s_g[e][q] + s_g[e][q + 1]) + (s_g[e + 1][q] + s_g[e + 1][q + 1]));
     };
@@ -200,16 +201,26 @@ stokes_geom mdz_stokes_geom(const mdz_ctx *ctx) {
     return make_geom(g.Nx, g.Nz, g.dx, g.dz, g.BCu, g.BCv, g.BCp, g.BCg);
 }
 
+// The box kernel's tiles in FP64: 16 x 4 points where 32 x 8 would be fewer than
+// 200, one or none for most SMs (an apply of 100 x 100 cells 9.7 -> 8.3 us with
+// its launch, of 256 x 128 13.7 -> 12.2); beyond, the smaller halo counts.
+#define ST_SMALL_W 16
+#define ST_SMALL_H 4
+#define ST_SMALL_TILES 200
 // box: the context's tags are the free-slip Dirichlet box (mdz_ctx::bcs_box)
 template <typename T>
 void stokes_apply_launch(const stokes_geom &G, const stokes_coefs<T> &D, stokes_cvec<T> x, stokes_vec<T> y,
                          const stokes_cvec<T> *b, bool newton, bool box, cudaStream_t st) {
     const dim3 gr((G.Nx + 1 + 31) / 32, (G.Nz + 1 + 7) / 8);
+    const dim3 grs((G.Nx + ST_SMALL_W) / ST_SMALL_W, (G.Nz + ST_SMALL_H) / ST_SMALL_H);
+    const bool small = box && sizeof(T) == 8 && gr.x * gr.y < ST_SMALL_TILES;
     const T celvol = gc<T>(G, GC_CELVOL);
     const stokes_cvec<T> bb = b ? *b : stokes_cvec<T>{nullptr, nullptr, nullptr};
 #define APPLY(NEWTON, RES)                                                                     \
     do {                                                                                       \
-        if (box) k_stokes_apply_box<T, NEWTON, RES><<<gr, 256, 0, st>>>(G, D, x, y, bb);       \
+        if (small) k_stokes_apply_box<T, NEWTON, RES, ST_SMALL_W, ST_SMALL_H>                  \
+            <<<grs, ST_SMALL_W * ST_SMALL_H, 0, st>>>(G, D, x, y, bb);                         \
+        else if (box) k_stokes_apply_box<T, NEWTON, RES, 32, 8><<<gr, 256, 0, st>>>(G, D, x, y, bb); \
         else k_stokes_apply<T, NEWTON, RES><<<gr, dim3(32, 8), 0, st>>>(G, D, x, y, bb, celvol); \
     } while (0)
     if (b) {
