@@ -1843,42 +1843,88 @@ static mdz_status precondition(mdz_ctx *ctx, mg_hier<T> &H, const T *Dt, const T
 // The running norm also goes to the host's memory with the iteration's ticket:
 // the host decides on the next iteration while the finish is still running,
 // instead of copying sc[3] back after it.
-__device__ void gcr_scalars(int k, const double *d, double *sc, double *tri, bool second, volatile double *note,
-                            double ticket) {
+// One warp: lane q holds d[q], d[q + 32], and dd is sum d^2; wa becomes
+// sum d alpha.  (One thread took two chains of k dependent FP64
+// instructions; with the folded block sums a launch went from 8.2 .. 12.4 us to
+// 7.2 .. 8.3, for 1 .. 30 vectors of 30 000.)
+__device__ __forceinline__ double warp_sum_all(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+__device__ __forceinline__ void gcr_scalars(int k, const double *d, double dk, double dr, double dd, double *sc, double *tri,
+                                            bool second, volatile double *note, double ticket) {
     // column k of U: the pass's Gram-Schmidt coefficients (added to the first
     // pass's after a second pass) and the new direction's norm
     double *U = tri + (size_t)k * GCR_MAX_M;
-    double nrm2 = d[k], wr = d[k + 1];
-    for (int q = 0; q < k; q++) {
-        nrm2 -= d[q] * d[q];
-        wr -= d[q] * sc[8 + q];   // (w - sum beta_q W_q, r0) = (w, r0) - sum beta_q alpha_q
-        U[q] = second ? U[q] + d[q] : d[q];
+    double wa = 0.0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int q = 32 * h + (threadIdx.x & 31);
+        if (q < k) {
+            wa += d[h] * sc[8 + q];
+            U[q] = second ? U[q] + d[h] : d[h];
+        }
     }
+    wa = warp_sum_all(wa);
+    if ((threadIdx.x & 31) != 0) return;
+    const double nrm2 = dk - dd, wr = dr - wa;   // (w - sum beta_q W_q, r0) = (w, r0) - sum beta_q alpha_q
     double nrm = sqrt(nrm2 > 0 ? nrm2 : 0.0);
+    const double inrm = nrm > 0 ? 1.0 / nrm : 0.0;
     double alpha = nrm > 0 ? wr / nrm : 0.0;   // alpha_k = (W_k, r0) = (W_k, r_k): W orthonormal
     U[k] = nrm;
-    sc[0] = nrm > 0 ? 1.0 / nrm : 0.0;
+    sc[0] = inrm;
     sc[1] = alpha;
     sc[2] = nrm2;
-    sc[3] -= alpha * alpha;   // ||r_k||^2 = ||r_k-1||^2 - alpha_k^2
+    const double rr = sc[3] - alpha * alpha;   // ||r_k||^2 = ||r_k-1||^2 - alpha_k^2
+    sc[3] = rr;
     sc[8 + k] = alpha;
-    note[0] = sc[3];
+    note[0] = rr;
     __threadfence_system();
     note[1] = ticket;
 }
 
-// gamma = U^-1 alpha (back substitution, one thread): x = x0 + Z gamma with
-// the raw preconditioned vectors Z, whose orthogonalised combinations
-// Z U^-1 are the directions whose images are the orthonormal W
-__global__ void k_gcr_gamma(int k, const double *__restrict__ sc, double *__restrict__ tri) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// gamma = U^-1 alpha: x = x0 + Z gamma with the raw preconditioned vectors Z,
+// whose orthogonalised combinations Z U^-1 are the directions whose images are
+// the orthonormal W.  Back substitution by one warp, a column at a time: lane i
+// keeps rows i and i + 32, quotients by the reciprocal of the diagonal with one
+// step on the remainder (Markstein, IBM J. Res. Dev. 34, 1990).  One thread, row
+// by row, took 33 us for 30 columns, this 9.
+__global__ void __launch_bounds__(32) k_gcr_gamma(int k, const double *__restrict__ sc, double *__restrict__ tri) {
     double *g = tri + (size_t)GCR_MAX_M * GCR_MAX_M;
-    for (int i = k - 1; i >= 0; i--) {
-        double v = sc[8 + i];
-        for (int j = i + 1; j < k; j++) v -= tri[(size_t)j * GCR_MAX_M + i] * g[j];
-        const double dgl = tri[(size_t)i * GCR_MAX_M + i];
-        g[i] = dgl != 0.0 ? v / dgl : 0.0;
+    const int lane = threadIdx.x;
+    double v[2], dg[2], rd[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int i = 32 * h + lane;
+        v[h] = i < k ? sc[8 + i] : 0.0;
+        dg[h] = i < k ? tri[(size_t)i * GCR_MAX_M + i] : 0.0;
+        rd[h] = fabs(dg[h]) >= 2.2250738585072014e-308 ? 1.0 / dg[h] : 0.0;   // (no subnormal: 1 / dg overflows)
     }
+    double gv[2] = {0.0, 0.0};
+    auto column = [&](int j, double &u0, double &u1) {   // rows above the diagonal
+        const double *U = tri + (size_t)j * GCR_MAX_M;
+        u0 = lane < j ? U[lane] : 0.0;
+        u1 = 32 + lane < j ? U[32 + lane] : 0.0;
+    };
+    double u0, u1, n0 = 0.0, n1 = 0.0;   // this column and the next
+    column(k - 1, u0, u1);
+    for (int j = k - 1; j >= 0; j--) {
+        if (j > 0) column(j - 1, n0, n1);
+        const bool hi = j >= 32;
+        const double vj = hi ? v[1] : v[0], dj = hi ? dg[1] : dg[0], rj = hi ? rd[1] : rd[0];
+        double q = vj * rj;
+        q = __fma_rn(__fma_rn(-q, dj, vj), rj, q);
+        q = __shfl_sync(0xffffffffu, q, j & 31);
+        if (lane == (j & 31)) { if (hi) gv[1] = q; else gv[0] = q; }
+        v[0] -= u0 * q;
+        v[1] -= u1 * q;
+        u0 = n0;
+        u1 = n1;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+        if (32 * h + lane < k) g[32 * h + lane] = gv[h];
 }
 
 // first-pass correction w -= sum beta_q W_q, only when sc[5] asks for a
@@ -2045,6 +2091,27 @@ static mdz_status remove_pressure_mean(mdz_ctx *ctx, double *p, cudaStream_t st)
 // 4-byte loads 18.9 / 32.7 / 51.7.
 template <typename T>
 constexpr int dots_q() { return sizeof(T) == 4 ? 8 : 4; }
+// Block sums of Q FP64 values by 256 threads, valid in thread 0: 256 / Q threads
+// per value fold the partial sums in shared memory and shuffle, 64 warp
+// instructions on the FP64 pipe for Q = 4 (shuffles of every value in every warp
+// took 160, and 20 more in the first).  Sums in a fixed order.
+template <int Q>
+__device__ __forceinline__ void dots_fold(const double (&p)[Q], double (&bs)[Q], double *sh) {
+    static_assert(Q == 4, "64 threads per value");
+    const int t = threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < Q; j++) sh[j * 256 + t] = p[j];
+    __syncthreads();
+    const double *a = sh + (t >> 6) * 256 + (t & 63);
+    const double s = warp_sum_all((a[0] + a[64]) + (a[128] + a[192]));
+    if ((t & 31) == 0) sh[Q * 256 + (t >> 5)] = s;
+    __syncthreads();
+    if (t == 0)
+#pragma unroll
+        for (int j = 0; j < Q; j++) bs[j] = sh[Q * 256 + 2 * j] + sh[Q * 256 + 2 * j + 1];
+}
+template <typename T, int MDOT_Q>
+constexpr int dots_shared() { return sizeof(T) == 8 ? MDOT_Q * 256 + 8 : 32 * MDOT_Q; }
 template <typename T, int MDOT_Q>
 __device__ __forceinline__ void dots_block(int nq, size_t n, const T *const *ap, const T *__restrict__ b,
                                            double *part, double (&bs)[MDOT_Q], double *sh) {
@@ -2066,7 +2133,8 @@ __device__ __forceinline__ void dots_block(int nq, size_t n, const T *const *ap,
                 for (int e = 0; e < V::N; e++) p[j] += a[j].v[e] * bi.v[e];
             }
     }
-    mdz_block_sum<MDOT_Q, T>(p, bs, sh);
+    if constexpr (sizeof(T) == 8) dots_fold<MDOT_Q>(p, bs, sh);
+    else mdz_block_sum<MDOT_Q, T>(p, bs, sh);
     const int q0 = blockIdx.y * MDOT_Q;
     if (threadIdx.x == 0) {
 #pragma unroll
@@ -2080,7 +2148,7 @@ __global__ void __launch_bounds__(256) k_dots(int nq, size_t n, const T *const *
                                               const T *__restrict__ b, double *part, unsigned int *cnt,
                                               double *out, const double *flag) {
     if (flag && *flag == 0.0) return;
-    __shared__ double sh[32 * MDOT_Q];
+    __shared__ double sh[dots_shared<T, MDOT_Q>()];
     const int q0 = blockIdx.y * MDOT_Q;
     const T *ap[MDOT_Q];
 #pragma unroll
@@ -2107,7 +2175,7 @@ __global__ void __launch_bounds__(256) k_gcr_dots(int k, size_t n, const T *cons
                                                   double *tri, unsigned int *cnt, double *note, double ticket) {
     pdl_wait();
     if (flag && *flag == 0.0) return;
-    __shared__ double sh[32 * MDOT_Q];
+    __shared__ double sh[dots_shared<T, MDOT_Q>()];
     const int nq = k + 2, q0 = blockIdx.y * MDOT_Q;
     const T *ap[MDOT_Q];
 #pragma unroll
@@ -2121,23 +2189,25 @@ __global__ void __launch_bounds__(256) k_gcr_dots(int k, size_t n, const T *cons
     const int nrow = nq - q0 < MDOT_Q ? nq - q0 : MDOT_Q;
     mdz_sum_partials(part + (size_t)q0 * gridDim.x, gridDim.x, nrow, out + q0);
     if (!mdz_arrive_last(cnt, gridDim.y)) return;
-    if (threadIdx.x != 0) return;
-    double d[GCR_MAX_M + 2];
-    for (int q = 0; q < nq; q++) d[q] = __ldcg(out + q);
+    if (threadIdx.x >= 32) return;
+    // scalars of the iteration, one warp: lane q has d[q] and d[q + 32]
+    static_assert(GCR_MAX_M <= 64, "two coefficients per lane");
+    const int lane = threadIdx.x;
+    const double d[2] = {lane < k ? __ldcg(out + lane) : 0.0, lane + 32 < k ? __ldcg(out + lane + 32) : 0.0};
+    const double dk = __ldcg(out + k), dr = __ldcg(out + k + 1), dd = warp_sum_all(d[0] * d[0] + d[1] * d[1]);
     if (mode == 1) {
-        double nrm2 = d[k];
-        for (int q = 0; q < k; q++) nrm2 -= d[q] * d[q];
         // second pass when the first removed all but 1e-3 (FP64 basis) or 1e-1
         // (FP32 basis: its orthogonality decays faster, and alpha is taken
         // from r0 through the triangle) of w's squared norm
-        if (k > 0 && !(nrm2 > (sizeof(T) == 4 ? 1e-1 : 1e-3) * d[k])) {   // keep this pass's coefficients in U
-            for (int q = 0; q < k; q++) tri[(size_t)k * GCR_MAX_M + q] = d[q];
-            sc[5] = 1.0;
+        if (k > 0 && !(dk - dd > (sizeof(T) == 4 ? 1e-1 : 1e-3) * dk)) {   // keep this pass's coefficients in U
+            for (int h = 0; h < 2; h++)
+                if (32 * h + lane < k) tri[(size_t)k * GCR_MAX_M + 32 * h + lane] = d[h];
+            if (lane == 0) sc[5] = 1.0;
             return;
         }
-        sc[5] = 0.0;
+        if (lane == 0) sc[5] = 0.0;
     }
-    gcr_scalars(k, d, sc, tri, mode == 2, note, ticket);
+    gcr_scalars(k, d, dk, dr, dd, sc, tri, mode == 2, note, ticket);
 }
 
 // grid of a dots launch over nq vectors: block rows of Q vectors, about four
