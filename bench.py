@@ -100,8 +100,8 @@ GUESS_STEPS = [3000]
 
 # DRAM bytes (read + write) per launch of a kernel class at 1025x513, from one
 # ncu capture of the FP32 form (dram__bytes_read.sum + dram__bytes_write.sum
-# over the kernels of 8 preconditioner applications, caches left warm)
-TRAFFIC_PER_LAUNCH = {"mg_vcycle": 88.5e6}
+# over the kernels of 19 preconditioner applications, caches left warm)
+TRAFFIC_PER_LAUNCH = {"mg_vcycle": 83.1e6}
 
 
 def train_guess(ctx, cfg):

@@ -1,5 +1,5 @@
-// Marker-side kernels: cell binning (stable counting sort), batched
-// marker->grid projection as a deterministic per-node gather, marker counts,
+// Marker-side kernels: binning by cell and quadrant (counting sort), batched
+// marker->grid projection as deterministic per-node sums, marker counts,
 // grid->marker interpolation and RK4 advection.
 //
 // Reference behaviour followed (paths inside the MDOODZ 6.0 repository):

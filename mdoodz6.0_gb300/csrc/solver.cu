@@ -1,12 +1,12 @@
 // Linear solver for the decoupled Stokes correction  K dx = F  (K = Picard
 // operator or Newton Jacobian, applied matrix-free): right-preconditioned,
-// restarted GCR with classical Gram-Schmidt applied twice, FP64 dot products
-// (warp-shuffle block reductions), and an upper block-triangular
+// restarted GCR with classical Gram-Schmidt and a selective second pass, FP64
+// dot products (fixed-order block sums), and an upper block-triangular
 // preconditioner [[A, B], [0, S]]:
 //   S^-1 = eta_n / cell volume            (viscosity-scaled pressure mass)
 //   A^-1 = one geometric-multigrid V-cycle on the velocity block (Picard,
 //          or optionally the Newton Jacobian's): damped Jacobi smoothing,
-//          cell-doubling coarsening, bilinear prolongation with R = P^T,
+//          cell counts halved (odd ones rounded up), bilinear prolongation, R = P^T,
 //          Galerkin coarse operators R A P as 31-point stencils, and an
 //          explicit inverse (or a single-CTA Jacobi-PCG solve) on the
 //          coarsest level.
