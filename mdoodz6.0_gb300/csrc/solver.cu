@@ -1927,23 +1927,6 @@ __global__ void __launch_bounds__(32) k_gcr_gamma(int k, const double *__restric
         if (32 * h + lane < k) g[32 * h + lane] = gv[h];
 }
 
-// first-pass correction w -= sum beta_q W_q, only when sc[5] asks for a
-// second pass (grid-stride, so a skipped launch is short)
-template <typename P>
-__global__ void k_gcr_orth_if(size_t n, int k, const P *__restrict__ W, const double *__restrict__ beta,
-                              const double *__restrict__ sc, P *__restrict__ w) {
-    pdl_wait();
-    if (sc[5] == 0.0) return;
-    __shared__ P bsh[GCR_MAX_M];
-    for (int q = threadIdx.x; q < k; q += blockDim.x) bsh[q] = (P)beta[q];
-    __syncthreads();
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        P ws = w[i];
-        for (int q = 0; q < k; q++) ws -= bsh[q] * W[q * n + i];
-        w[i] = ws;
-    }
-}
-
 __global__ void k_set_scalar(double *dst, const double *src) {
     if (threadIdx.x == 0 && blockIdx.x == 0) *dst = *src;
 }
@@ -1983,7 +1966,8 @@ __global__ void __launch_bounds__(256) k_gcr_finish(size_t n, int k, P *__restri
     __syncthreads();
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V::N;
     if (i >= n) return;
-    V ws = *reinterpret_cast<const V *>(w + i);
+    // (a second pass left its vector in W_k)
+    V ws = *reinterpret_cast<const V *>((sc[5] != 0.0 ? W + (size_t)k * n : w) + i);
     const V zi = *reinterpret_cast<const V *>(z + i);
 #pragma unroll 4
     for (int q = 0; q < k; q++) {
@@ -2112,8 +2096,10 @@ __device__ __forceinline__ void dots_fold(const double (&p)[Q], double (&bs)[Q],
 }
 template <typename T, int MDOT_Q>
 constexpr int dots_shared() { return sizeof(T) == 8 ? MDOT_Q * 256 + 8 : 32 * MDOT_Q; }
-template <typename T, int MDOT_Q>
-__device__ __forceinline__ void dots_block(int nq, size_t n, const T *const *ap, const T *__restrict__ b,
+// (b: the vector as a function of the position; self: the place among the Q of
+// (b, b), whose ap is not read, or -1)
+template <typename T, int MDOT_Q, typename VEC>
+__device__ __forceinline__ void dots_block(int nq, size_t n, const T *const *ap, const VEC &b, int self,
                                            double *part, double (&bs)[MDOT_Q], double *sh) {
     typedef vec16<T> V;
     T p[MDOT_Q];
@@ -2121,11 +2107,13 @@ __device__ __forceinline__ void dots_block(int nq, size_t n, const T *const *ap,
     for (int j = 0; j < MDOT_Q; j++) p[j] = T(0);
     const size_t stride = (size_t)gridDim.x * blockDim.x * V::N;
     for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V::N; i < n; i += stride) {
-        const V bi = *reinterpret_cast<const V *>(b + i);
+        const V bi = b(i);
         V a[MDOT_Q];
 #pragma unroll
-        for (int j = 0; j < MDOT_Q; j++)
-            if (ap[j]) a[j] = *reinterpret_cast<const V *>(ap[j] + i);
+        for (int j = 0; j < MDOT_Q; j++) {
+            if (j == self) a[j] = bi;
+            else if (ap[j]) a[j] = *reinterpret_cast<const V *>(ap[j] + i);
+        }
 #pragma unroll
         for (int j = 0; j < MDOT_Q; j++)
             if (ap[j]) {
@@ -2154,7 +2142,7 @@ __global__ void __launch_bounds__(256) k_dots(int nq, size_t n, const T *const *
 #pragma unroll
     for (int j = 0; j < MDOT_Q; j++) ap[j] = q0 + j < nq ? a[q0 + j] : nullptr;
     double bs[MDOT_Q];
-    dots_block<T, MDOT_Q>(nq, n, ap, b, part, bs, sh);
+    dots_block<T, MDOT_Q>(nq, n, ap, [&](size_t i) { return *reinterpret_cast<const vec16<T> *>(b + i); }, -1, part, bs, sh);
     if (!mdz_arrive_last(cnt + blockIdx.y, gridDim.x)) return;
     const int nrow = nq - q0 < MDOT_Q ? nq - q0 : MDOT_Q;
     mdz_sum_partials(part + (size_t)q0 * gridDim.x, gridDim.x, nrow, out + q0);
@@ -2164,17 +2152,24 @@ __global__ void __launch_bounds__(256) k_dots(int nq, size_t n, const T *const *
 // (w, w) and (w, r) as vectors k and k + 1 (b = w), summed as k_dots does
 // (the last block of each block row adds its row's partials in block order);
 // the last row to finish (a second arrival counter) then runs the pass's
-// scalar step: mode 1 the check of the first pass (sc[5] = 1 asks for a
-// second pass, else the scalars), mode 2 the scalars of the second pass.
-// With flag (mode 2) every block returns at once when *flag is 0.
+// scalar step: the check of the first pass (sc[5] = 1 asks for a second pass,
+// else the scalars), or the scalars of the second.
 // cnt[0]: rows finished, cnt[1 + y]: blocks of row y finished.
-template <typename T, int MDOT_Q>
+// SECOND: the second pass, whose vector is w - sum beta_q W_q with the first
+// pass's sums beta; every block row forms it (all of W is read once per row, in
+// the few iterations that need it), the first writes it to W_k, where the finish
+// takes it from.  (As a launch of its own the correction cost every iteration a
+// launch that returned at once, 1.5 us.)
+template <typename T, int MDOT_Q, bool SECOND>
 __global__ void __launch_bounds__(256) k_gcr_dots(int k, size_t n, const T *const *__restrict__ a,
-                                                  const T *__restrict__ w, const T *__restrict__ r, double *part,
-                                                  double *out, const double *flag, int mode, double *sc,
-                                                  double *tri, unsigned int *cnt, double *note, double ticket) {
+                                                  const T *__restrict__ w, const T *__restrict__ r, T *W,
+                                                  const double *__restrict__ beta, double *part, double *out,
+                                                  double *sc, double *tri, unsigned int *cnt, double *note,
+                                                  double ticket) {
+    typedef vec16<T> V;
+    constexpr int mode = SECOND ? 2 : 1;
     pdl_wait();
-    if (flag && *flag == 0.0) return;
+    if (SECOND && sc[5] == 0.0) return;
     __shared__ double sh[dots_shared<T, MDOT_Q>()];
     const int nq = k + 2, q0 = blockIdx.y * MDOT_Q;
     const T *ap[MDOT_Q];
@@ -2184,7 +2179,24 @@ __global__ void __launch_bounds__(256) k_gcr_dots(int k, size_t n, const T *cons
         ap[j] = q < k ? a[q] : (q == k ? w : (q == k + 1 ? r : nullptr));
     }
     double bs[MDOT_Q];
-    dots_block<T, MDOT_Q>(nq, n, ap, w, part, bs, sh);
+    if constexpr (SECOND) {
+        __shared__ T bsh[GCR_MAX_M];
+        for (int q = threadIdx.x; q < k; q += blockDim.x) bsh[q] = (T)beta[q];
+        __syncthreads();
+        const bool write = blockIdx.y == 0;
+        dots_block<T, MDOT_Q>(nq, n, ap, [&](size_t i) {
+            V ws = *reinterpret_cast<const V *>(w + i);
+            for (int q = 0; q < k; q++) {
+                const V wq = *reinterpret_cast<const V *>(W + q * n + i);
+#pragma unroll
+                for (int e = 0; e < V::N; e++) ws.v[e] -= bsh[q] * wq.v[e];
+            }
+            if (write) *reinterpret_cast<V *>(W + (size_t)k * n + i) = ws;
+            return ws;
+        }, k - q0, part, bs, sh);
+    } else {
+        dots_block<T, MDOT_Q>(nq, n, ap, [&](size_t i) { return *reinterpret_cast<const V *>(w + i); }, -1, part, bs, sh);
+    }
     if (!mdz_arrive_last(cnt + 1 + blockIdx.y, gridDim.x)) return;
     const int nrow = nq - q0 < MDOT_Q ? nq - q0 : MDOT_Q;
     mdz_sum_partials(part + (size_t)q0 * gridDim.x, gridDim.x, nrow, out + q0);
@@ -2223,11 +2235,16 @@ static dim3 dots_grid(size_t n, int nq) {
 }
 
 template <typename T>
-static mdz_status gcr_dots_launch(mdz_ctx *ctx, gcr_space<T> &S, int k, const T *w, const T *r, double *out,
-                                  const double *flag, int mode, double *sc, double ticket, cudaStream_t st) {
-    MDZ_PDL(ctx, k_gcr_dots<T, dots_q<T>()>, dots_grid<T>(S.ld, k + 2), 256, 0, st, k, S.ld, S.dA0, w, r,
-            ctx->red_part + MDZ_RP_DOTS, out, flag, mode, sc, S.tri, ctx->red_cnt + MDZ_RC_GCR,
-            ctx->solver->sc + GCR_NOTE, ticket);
+static mdz_status gcr_dots_launch(mdz_ctx *ctx, gcr_space<T> &S, int k, const T *w, const T *r, const double *beta,
+                                  double *out, double *sc, double ticket, cudaStream_t st) {
+    if (beta)
+        MDZ_PDL(ctx, (k_gcr_dots<T, dots_q<T>(), true>), dots_grid<T>(S.ld, k + 2), 256, 0, st, k, S.ld, S.dA0, w, r, S.W,
+                beta, ctx->red_part + MDZ_RP_DOTS, out, sc, S.tri, ctx->red_cnt + MDZ_RC_GCR, ctx->solver->sc + GCR_NOTE,
+                ticket);
+    else
+        MDZ_PDL(ctx, (k_gcr_dots<T, dots_q<T>(), false>), dots_grid<T>(S.ld, k + 2), 256, 0, st, k, S.ld, S.dA0, w, r, S.W,
+                beta, ctx->red_part + MDZ_RP_DOTS, out, sc, S.tri, ctx->red_cnt + MDZ_RC_GCR, ctx->solver->sc + GCR_NOTE,
+                ticket);
     return MDZ_OK;
 }
 
@@ -2396,14 +2413,11 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
         // produced them); x, r and every sum are FP64.  First pass:
         // (w, W_q) q < k, (w, w), (w, r0); the check decides on the device
         // whether a second pass runs.
-        const int ng = nb < 152 * 8 ? nb : 152 * 8;
         double *d1 = dots1p[it & 1], *d2 = dots2p[it & 1];
         SV->ticket += 1.0;
-        if ((s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, d1, nullptr, 1, sc, SV->ticket, st)) != MDZ_OK) return s;
-        if (k > 0) {   // second pass (each launch returns at once unless sc[5] = 1)
-            MDZ_PDL(ctx, k_gcr_orth_if<P>, ng, MDZ_THREADS, 0, st, n, k, SP.W, d1, sc, SP.w);
-            if ((s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, d2, sc + 5, 2, sc, SV->ticket, st)) != MDZ_OK) return s;
-        }
+        if ((s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, nullptr, d1, sc, SV->ticket, st)) != MDZ_OK) return s;
+        // second pass (returns at once unless sc[5] = 1)
+        if (k > 0 && (s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, d1, d2, sc, SV->ticket, st)) != MDZ_OK) return s;
         MDZ_PDL(ctx, k_gcr_finish<P>, nb16, 256, 0, st, n, k, SP.W, SP.Z, d1, d2, sc, SP.z, SP.w, SP.pin,
                 dots1p[(it + 1) & 1], dots2p[(it + 1) & 1]);
         {   // algorithmic bytes (one Gram-Schmidt pass): the sums read W_q,
