@@ -167,6 +167,12 @@ void *mdz_stage(mdz_ctx *ctx, int slot, size_t bytes);
 // pdl_release() lets the next launch start now instead of when this grid's
 // blocks end; since every launch waits, calling it first is safe.  Both do
 // nothing in a kernel launched the ordinary way.
+// Parameters through which such a kernel reads what those launches write carry no
+// __restrict__: it would promise that the data are constant while the kernel
+// lives, and the compiler could read them through the non-coherent path or ahead
+// of the wait.  Data older than the chain (stencils, inverse diagonals,
+// viscosities, pointer tables) and parameters that are only written may have it
+// (tests/test_dependent_launches.py).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -83,8 +83,7 @@ __device__ __forceinline__ T prolonged_v(const GF &F, const GC &Cg, const T *cv,
 
 // fine x += P xc (a V-cycle without post-smoothing)
 template <typename T>
-__global__ void k_mg_prolong_add(stokes_geom F, stokes_geom Cg, const T *__restrict__ cu, const T *__restrict__ cv,
-                                 T *fu, T *fv) {
+__global__ void k_mg_prolong_add(stokes_geom F, stokes_geom Cg, const T *cu, const T *cv, T *fu, T *fv) {
     mg_release<T>();
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -134,9 +133,9 @@ __device__ __forceinline__ T restricted_v(const GF &F, const GC &Cg, const T *rv
 #define ST_THREADS 64
 template <typename T>
 __global__ void __launch_bounds__(ST_THREADS) k_st_smooth(
-    stokes_geom G, const T *__restrict__ su, const T *__restrict__ sv, const T *__restrict__ xu,
-    const T *__restrict__ xv, const T *__restrict__ fu, const T *__restrict__ fv, const T *__restrict__ idu,
-    const T *__restrict__ idv, T omega, T *__restrict__ ou, T *__restrict__ ov) {
+    stokes_geom G, const T *__restrict__ su, const T *__restrict__ sv, const T *xu, const T *xv, const T *fu,
+    const T *fv, const T *__restrict__ idu, const T *__restrict__ idv, T omega, T *__restrict__ ou,
+    T *__restrict__ ov) {
     mg_release<T>();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int Nx = G.Nx, Nz = G.Nz, nu = Nx * (Nz + 1), nv = (Nx + 1) * Nz;
@@ -221,10 +220,9 @@ __device__ __forceinline__ void restrict_tile(const stokes_geom &Cg,
 
 template <typename T, int TX, int TY, int NT>
 __global__ void __launch_bounds__(NT) k_st_resid_restrict(
-    stokes_geom F, const T *__restrict__ su, const T *__restrict__ sv, const T *__restrict__ xu,
-    const T *__restrict__ xv, const T *__restrict__ fu, const T *__restrict__ fv, stokes_geom Cg, T *__restrict__ cu,
-    T *__restrict__ cv, const T *__restrict__ cidu, const T *__restrict__ cidv, T omega, T *__restrict__ cxu,
-    T *__restrict__ cxv) {
+    stokes_geom F, const T *__restrict__ su, const T *__restrict__ sv, const T *xu, const T *xv, const T *fu,
+    const T *fv, stokes_geom Cg, T *__restrict__ cu, T *__restrict__ cv, const T *__restrict__ cidu,
+    const T *__restrict__ cidv, T omega, T *__restrict__ cxu, T *__restrict__ cxv) {
     constexpr int UW = 2 * TX + 1, UH = 2 * TY + 2, VW = 2 * TX + 2, VH = 2 * TY + 1;
     __shared__ T ru[UH][UW], rv[VH][VW];
     const int Nx = F.Nx, Nz = F.Nz, I0 = blockIdx.x * TX, J0 = blockIdx.y * TY;
@@ -255,10 +253,9 @@ __global__ void __launch_bounds__(NT) k_st_resid_restrict(
 // rows); each thread loads its row's coefficients before the tile is filled.
 template <typename T, int TW, int TH>
 __global__ void __launch_bounds__(2 * TW * TH) k_st_prolong_smooth(
-    stokes_geom F, stokes_geom Cg, const T *__restrict__ su, const T *__restrict__ sv, const T *__restrict__ cu,
-    const T *__restrict__ cv, const T *__restrict__ xu, const T *__restrict__ xv, const T *__restrict__ fu,
-    const T *__restrict__ fv, const T *__restrict__ idu, const T *__restrict__ idv, T omega, T *__restrict__ ou,
-    T *__restrict__ ov) {
+    stokes_geom F, stokes_geom Cg, const T *__restrict__ su, const T *__restrict__ sv, const T *cu, const T *cv,
+    const T *xu, const T *xv, const T *fu, const T *fv, const T *__restrict__ idu, const T *__restrict__ idv, T omega,
+    T *__restrict__ ou, T *__restrict__ ov) {
     constexpr int PUW = TW + 3, PUH = TH + 4, PVW = TW + 4, PVH = TH + 3, NT = 2 * TW * TH;
     __shared__ T pu[PUH][PUW], pv[PVH][PVW];   // u from (i0 - 2, j0 - 2), v from (i0 - 2, j0 - 2)
     const int Nx = F.Nx, Nz = F.Nz, i0 = blockIdx.x * TW, j0 = blockIdx.y * TH;
@@ -407,9 +404,8 @@ struct vel_global {
 
 // out = x + omega * D^-1 (f - A x)  (x == nullptr: x = 0), TW x TH points per block
 template <typename T, int TW, int TH>
-__global__ void __launch_bounds__(TW *TH) k_mg_smooth(stokes_geom G, stokes_coefs<T> D, const T *__restrict__ xu,
-                                                   const T *__restrict__ xv, const T *__restrict__ fu,
-                                                   const T *__restrict__ fv, const T *__restrict__ idu,
+__global__ void __launch_bounds__(TW *TH) k_mg_smooth(stokes_geom G, stokes_coefs<T> D, const T *xu, const T *xv,
+                                                   const T *fu, const T *fv, const T *__restrict__ idu,
                                                    const T *__restrict__ idv, T omega, T *__restrict__ ou,
                                                    T *__restrict__ ov) {
     constexpr bool TILE = mg_stress_tile<T>();
@@ -441,9 +437,8 @@ __global__ void __launch_bounds__(TW *TH) k_mg_smooth(stokes_geom G, stokes_coef
 }
 
 template <typename T, int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT) k_mg_resid_restrict(stokes_geom F, stokes_coefs<T> D, const T *__restrict__ xu,
-                                                          const T *__restrict__ xv, const T *__restrict__ fu,
-                                                          const T *__restrict__ fv, stokes_geom Cg,
+__global__ void __launch_bounds__(NT) k_mg_resid_restrict(stokes_geom F, stokes_coefs<T> D, const T *xu, const T *xv,
+                                                          const T *fu, const T *fv, stokes_geom Cg,
                                                           T *__restrict__ cu, T *__restrict__ cv,
                                                           const T *__restrict__ cidu, const T *__restrict__ cidv,
                                                           T omega, T *__restrict__ cxu, T *__restrict__ cxv) {
@@ -494,10 +489,9 @@ struct vel_tile {
 
 template <typename T, int TW, int TH>
 __global__ void __launch_bounds__(TW *TH) k_mg_prolong_smooth(
-    stokes_geom F, stokes_coefs<T> D, stokes_geom Cg, const T *__restrict__ cu, const T *__restrict__ cv,
-    const T *__restrict__ xu, const T *__restrict__ xv, const T *__restrict__ fu, const T *__restrict__ fv,
-    const T *__restrict__ idu, const T *__restrict__ idv, T omega, T *__restrict__ ou, T *__restrict__ ov,
-    T *__restrict__ zp, const double *__restrict__ pmean) {
+    stokes_geom F, stokes_coefs<T> D, stokes_geom Cg, const T *cu, const T *cv, const T *xu, const T *xv, const T *fu,
+    const T *fv, const T *__restrict__ idu, const T *__restrict__ idv, T omega, T *__restrict__ ou, T *__restrict__ ov,
+    T *zp, const double *pmean) {
     constexpr int W = TW + 2, H = TH + 2;
     constexpr bool TILE = mg_stress_tile<T>();
     __shared__ T pu[H][W], pv[H][W];

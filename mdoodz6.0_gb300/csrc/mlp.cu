@@ -252,11 +252,10 @@ __global__ void __launch_bounds__(128) k_mlp_train(const unsigned char *__restri
 // weights, which also rewrites the packed BF16 image.  Block: 32 parameters x
 // 8 slices.  Starts while the gradient pass ends (pdl_wait), as the next pass
 // does while this kernel runs.
-__global__ void __launch_bounds__(256) k_mlp_reduce(int nblk, const float *__restrict__ partials,
-                                                    float *__restrict__ grad, float *__restrict__ params,
-                                                    float *__restrict__ m, float *__restrict__ v,
+__global__ void __launch_bounds__(256) k_mlp_reduce(int nblk, const float *partials,
+                                                    float *__restrict__ grad, float *params, float *m, float *v,
                                                     unsigned char *packed, float lr, float b1, float b2, float eps,
-                                                    float bc1, float bc2, int adam, const int *__restrict__ tc_err,
+                                                    float bc1, float bc2, int adam, const int *tc_err,
                                                     float *__restrict__ loss_out) {
     __shared__ float part[8][33];
     const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, q = blockIdx.x * 32 + lane;

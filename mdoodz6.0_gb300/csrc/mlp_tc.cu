@@ -361,10 +361,8 @@ __device__ __forceinline__ void tc_handoff() {
 
 }  // namespace
 
-__global__ void __launch_bounds__(TC_THREADS, 2) k_mlp_train_tc(const unsigned char *__restrict__ packed,
-                                                                const uint4 *__restrict__ X,
-                                                                const float2 *__restrict__ Y, long long row0,
-                                                                int nrows, float scale,
+__global__ void __launch_bounds__(TC_THREADS, 2) k_mlp_train_tc(const unsigned char *packed, const uint4 *X,
+                                                                const float2 *Y, long long row0, int nrows, float scale,
                                                                 float *__restrict__ partials, int *__restrict__ err) {
     extern __shared__ __align__(1024) unsigned char sm[];
     const int tid = threadIdx.x, warp = tid >> 5;

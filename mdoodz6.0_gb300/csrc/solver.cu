@@ -225,14 +225,14 @@ __device__ __forceinline__ bool v_unknown(int i, int j, int Nx, int Nz) {
 // unknowns).  FP64 sums run in four chains: one dependent chain of 31 FP64
 // multiply-adds is longer than the loads on the small levels.
 template <typename T>
-__device__ __forceinline__ void st_coefs(const T *__restrict__ s, size_t n, size_t c, T (&cf)[MG_NST]) {
+__device__ __forceinline__ void st_coefs(const T *s, size_t n, size_t c, T (&cf)[MG_NST]) {
 #pragma unroll
     for (int q = 0; q < MG_NST; q++) cf[q] = s[(size_t)q * n + c];
 }
 
 template <typename T>
-__device__ __forceinline__ T st_urow_x(int Nx, int Nz, const T (&cf)[MG_NST], const T *__restrict__ xu,
-                                       const T *__restrict__ xv, int k, int l) {
+__device__ __forceinline__ T st_urow_x(int Nx, int Nz, const T (&cf)[MG_NST], const T *xu, const T *xv, int k,
+                                       int l) {
     constexpr int NA = sizeof(T) == 8 ? 4 : 1;
     T s[NA] = {};
 #pragma unroll
@@ -252,8 +252,8 @@ __device__ __forceinline__ T st_urow_x(int Nx, int Nz, const T (&cf)[MG_NST], co
 }
 
 template <typename T>
-__device__ __forceinline__ T st_vrow_x(int Nx, int Nz, const T (&cf)[MG_NST], const T *__restrict__ xu,
-                                       const T *__restrict__ xv, int i, int j) {
+__device__ __forceinline__ T st_vrow_x(int Nx, int Nz, const T (&cf)[MG_NST], const T *xu, const T *xv, int i,
+                                       int j) {
     constexpr int NA = sizeof(T) == 8 ? 4 : 1;
     T s[NA] = {};
     (void)Nz;
@@ -510,8 +510,8 @@ __device__ __forceinline__ void v_parents_ij(int i, int j, int ncxc, int *I, int
 #define GAL_WARPS 12
 #define GAL_THREADS (32 * GAL_WARPS)
 template <typename T, bool VISC>
-__global__ void __launch_bounds__(GAL_THREADS) k_galerkin(stokes_geom F, const T *__restrict__ suF,
-                                                          const T *__restrict__ svF, const T *__restrict__ D11,
+__global__ void __launch_bounds__(GAL_THREADS) k_galerkin(stokes_geom F, const T *suF, const T *svF,
+                                                          const T *__restrict__ D11,
                                                           const T *__restrict__ D33, stokes_geom Cg, int ublocks,
                                                           T *__restrict__ suC, T *__restrict__ svC,
                                                           T *__restrict__ idu, T *__restrict__ idv, int *bad) {
@@ -809,9 +809,8 @@ __device__ __forceinline__ T dense_row(int n, const T *AinvT, const T *fs, int r
 
 template <typename T>
 __global__ void __launch_bounds__(512) k_coarse_dense_solve(int n, int nu, int nv, const int *__restrict__ map,
-                                                            const T *__restrict__ AinvT, const T *__restrict__ fu,
-                                                            const T *__restrict__ fv, T *__restrict__ xu,
-                                                            T *__restrict__ xv) {
+                                                            const T *__restrict__ AinvT, const T *fu, const T *fv,
+                                                            T *__restrict__ xu, T *__restrict__ xv) {
     __shared__ T fs[MG_DENSE_MAX];
     mg_release<T>();
     pdl_wait();
@@ -1765,7 +1764,7 @@ __global__ void __launch_bounds__(TW *TH) k_precond(stokes_geom G, const T *__re
 // z pressure <- zero mean over the pressure equations (the mean cancels in
 // the gradient of the right-hand side, so it is removed only here)
 template <typename T>
-__global__ void k_pmean_out(int np, const double *__restrict__ psum, T *__restrict__ zp) {
+__global__ void k_pmean_out(int np, const double *psum, T *zp) {
     mg_release<T>();
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1774,9 +1773,8 @@ __global__ void k_pmean_out(int np, const double *__restrict__ psum, T *__restri
 
 // z velocity <- the V-cycle's result; z pressure <- zero mean, as k_pmean_out
 template <typename T>
-__global__ void k_copy_out(size_t nu, size_t nv, int np, const T *__restrict__ xu, const T *__restrict__ xv,
-                           const double *__restrict__ psum, T *__restrict__ zu, T *__restrict__ zv,
-                           T *__restrict__ zp) {
+__global__ void k_copy_out(size_t nu, size_t nv, int np, const T *xu, const T *xv, const double *psum,
+                           T *__restrict__ zu, T *__restrict__ zv, T *zp) {
     mg_release<T>();
     pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1948,10 +1946,8 @@ struct alignas(16) vec16 {
 // (16 bytes of each vector per thread; n is the padded length.  Memory bound:
 // 1025 x 513 in FP32, 12 vectors on average, 12.1 us, 23.6 with 4-byte loads)
 template <typename P>
-__global__ void __launch_bounds__(256) k_gcr_finish(size_t n, int k, P *__restrict__ W, P *__restrict__ Z,
-                                                    const double *__restrict__ dots1,
-                                                    const double *__restrict__ dots2, const double *__restrict__ sc,
-                                                    const P *__restrict__ z, const P *__restrict__ w,
+__global__ void __launch_bounds__(256) k_gcr_finish(size_t n, int k, P *W, P *__restrict__ Z, const double *dots1,
+                                                    const double *dots2, const double *sc, const P *z, const P *w,
                                                     P *__restrict__ pin, double *__restrict__ next1,
                                                     double *__restrict__ next2) {
     typedef vec16<P> V;
@@ -1961,7 +1957,7 @@ __global__ void __launch_bounds__(256) k_gcr_finish(size_t n, int k, P *__restri
     if (blockIdx.x == 0 && next1)
         for (int q = threadIdx.x; q < k + 3; q += blockDim.x) { next1[q] = 0.0; next2[q] = 0.0; }
     __shared__ P bsh[GCR_MAX_M];
-    const double *__restrict__ beta = sc[5] != 0.0 ? dots2 : dots1;
+    const double *beta = sc[5] != 0.0 ? dots2 : dots1;
     for (int q = threadIdx.x; q < k; q += blockDim.x) bsh[q] = (P)beta[q];
     __syncthreads();
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V::N;
@@ -2162,10 +2158,9 @@ __global__ void __launch_bounds__(256) k_dots(int nq, size_t n, const T *const *
 // launch that returned at once, 1.5 us.)
 template <typename T, int MDOT_Q, bool SECOND>
 __global__ void __launch_bounds__(256) k_gcr_dots(int k, size_t n, const T *const *__restrict__ a,
-                                                  const T *__restrict__ w, const T *__restrict__ r, T *W,
-                                                  const double *__restrict__ beta, double *part, double *out,
-                                                  double *sc, double *tri, unsigned int *cnt, double *note,
-                                                  double ticket) {
+                                                  const T *w, const T *r, T *W, const double *beta, double *part,
+                                                  double *out, double *sc, double *tri, unsigned int *cnt,
+                                                  double *note, double ticket) {
     typedef vec16<T> V;
     constexpr int mode = SECOND ? 2 : 1;
     pdl_wait();
