@@ -993,6 +993,8 @@ __global__ void __launch_bounds__(mg_bottom_threads<T>()) k_mg_bottom(const __gr
         const int i = e % Sn;
         if (i < nown) Ai[e] = A.AinvT[(size_t)(e / Sn) * n + n0 + i];
     }
+    cluster_meet();   // every CTA has cleared its vectors before any stores into them
+    pdl_wait();
     {   // the caller's vectors are 0 where there is no unknown
         const mg_bottom_rank L(A.Nx[0], A.Nz[0], rank);
         for (int e = rank * NT + tid; e < L.box; e += C * NT) {
@@ -1002,8 +1004,6 @@ __global__ void __launch_bounds__(mg_bottom_threads<T>()) k_mg_bottom(const __gr
             if (!u && !(k > 0 && k < L.Nx && j > 0 && j < L.Nz - 1)) A.xv[e - L.nu] = T(0);
         }
     }
-    cluster_meet();   // every CTA has cleared its vectors before any stores into them
-    pdl_wait();
     unsigned par = 0;   // bit l: level l's x is in its second vector
     // mode 1: y = x + omega D^-1 (f - A x); 2: y = f - A x; 3: as 1, into the caller's vectors
     auto rows = [&](int base, int l, bool odd, int mode) {

@@ -59,3 +59,16 @@ def test_no_restrict_on_what_the_chain_writes(name):
             stores = len(re.findall(r"(?<!\w)%s\[(?:[^\[\]]|\[[^\[\]]*\])*\]\s*=(?!=)" % v, body))
             uses = len(re.findall(r"(?<![\w.])%s\s*\[" % v, body))
             assert stores == uses, "%s reads %s, which is __restrict__" % (name, v)
+
+
+@pytest.mark.parametrize("name", sorted(KERNELS))
+def test_no_global_store_before_the_wait(name):
+    """Nothing may be stored into the caller's memory before the wait either:
+    earlier launches may still be at work on it.  (Shared memory and the partial
+    results in registers are the kernel's own.)"""
+    params, body = KERNELS[name]
+    before = body[:body.index("pdl_wait()")]
+    pointers = [re.search(r"(\w+)\s*$", p.strip()).group(1) for p in params.split(",") if "*" in p and not p.strip().startswith("const")]
+    for v in pointers + [r"A\.\w+"]:
+        m = re.search(r"(?<![\w.])%s\[(?:[^\[\]]|\[[^\[\]]*\])*\]\s*[-+*/]?=(?!=)" % v, before)
+        assert not m, "%s stores %s ahead of the wait" % (name, m.group(0))
