@@ -25,6 +25,7 @@
 #include <vector>
 #include "stokes.cuh"
 #include "solver.cuh"
+#include "krylov_dots.cuh"
 
 #define MG_MAX_LEVELS 16
 #define MG_DENSE_MAX 256
@@ -1845,11 +1846,6 @@ static mdz_status precondition(mdz_ctx *ctx, mg_hier<T> &H, const T *Dt, const T
 // sum d alpha.  (One thread took two chains of k dependent FP64
 // instructions; with the folded block sums a launch went from 8.2 .. 12.4 us to
 // 7.2 .. 8.3, for 1 .. 30 vectors of 30 000.)
-__device__ __forceinline__ double warp_sum_all(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 __device__ __forceinline__ void gcr_scalars(int k, const double *d, double dk, double dr, double dd, double *sc, double *tri,
                                             bool second, volatile double *note, double ticket) {
     // column k of U: the pass's Gram-Schmidt coefficients (added to the first
@@ -1937,12 +1933,7 @@ __global__ void k_set_scalar(double *dst, const double *src) {
 // iteration this reads the basis W twice (the sums and here) and nothing of
 // Z: about 2k + 7 vectors against 3k + 11 for the form that orthogonalised
 // z and updated r every iteration.
-template <typename T>
-struct alignas(16) vec16 {
-    static constexpr int N = 16 / sizeof(T);
-    T v[N];
-};
-
+//
 // (16 bytes of each vector per thread; n is the padded length.  Memory bound:
 // 1025 x 513 in FP32, 12 vectors on average, 12.1 us, 23.6 with 4-byte loads)
 template <typename P>
@@ -2055,95 +2046,6 @@ static mdz_status remove_pressure_mean(mdz_ctx *ctx, double *p, cudaStream_t st)
     return MDZ_OK;
 }
 
-// out[q] = (a_q, b) for the nq vectors of the pointer table (each of padded
-// length n, contiguous u|v|p like b).  One thread keeps Q running sums and loads
-// 16 bytes of each vector and of b at a time, so b is read once per Q vectors
-// and the loads of all of them are in flight together.  FP32 vectors (Q = 8):
-// products, sums and the warp reductions stay FP32 with only the warp sums
-// entering FP64 (FP64 instructions issue at a small fraction of the FP32 rate
-// on this part, so even a per-thread FP64 reduction tree dominated the
-// kernel).  FP64 vectors (Q = 4) are bound by their FP64 multiply-adds.  Block
-// row y handles vectors y Q .. y Q + Q - 1; its blocks write their partials to
-// part[q * gridDim.x + blockIdx.x] and the last block of the row to finish
-// adds them up in block order (reduce.cuh): deterministic.  cnt: one arrival
-// counter per block row.  A non-null flag holding 0 makes the launch a no-op.
-// 1025 x 513 in FP32, up to 8 / 16 / 24 vectors: 13.8 / 21.2 / 29.6 us, with
-// 4-byte loads 18.9 / 32.7 / 51.7.
-template <typename T>
-constexpr int dots_q() { return sizeof(T) == 4 ? 8 : 4; }
-// Block sums of Q FP64 values by 256 threads, valid in thread 0: 256 / Q threads
-// per value fold the partial sums in shared memory and shuffle, 64 warp
-// instructions on the FP64 pipe for Q = 4 (shuffles of every value in every warp
-// took 160, and 20 more in the first).  Sums in a fixed order.
-template <int Q>
-__device__ __forceinline__ void dots_fold(const double (&p)[Q], double (&bs)[Q], double *sh) {
-    static_assert(Q == 4, "64 threads per value");
-    const int t = threadIdx.x;
-#pragma unroll
-    for (int j = 0; j < Q; j++) sh[j * 256 + t] = p[j];
-    __syncthreads();
-    const double *a = sh + (t >> 6) * 256 + (t & 63);
-    const double s = warp_sum_all((a[0] + a[64]) + (a[128] + a[192]));
-    if ((t & 31) == 0) sh[Q * 256 + (t >> 5)] = s;
-    __syncthreads();
-    if (t == 0)
-#pragma unroll
-        for (int j = 0; j < Q; j++) bs[j] = sh[Q * 256 + 2 * j] + sh[Q * 256 + 2 * j + 1];
-}
-template <typename T, int MDOT_Q>
-constexpr int dots_shared() { return sizeof(T) == 8 ? MDOT_Q * 256 + 8 : 32 * MDOT_Q; }
-// (b: the vector as a function of the position; self: the place among the Q of
-// (b, b), whose ap is not read, or -1)
-template <typename T, int MDOT_Q, typename VEC>
-__device__ __forceinline__ void dots_block(int nq, size_t n, const T *const *ap, const VEC &b, int self,
-                                           double *part, double (&bs)[MDOT_Q], double *sh) {
-    typedef vec16<T> V;
-    T p[MDOT_Q];
-#pragma unroll
-    for (int j = 0; j < MDOT_Q; j++) p[j] = T(0);
-    const size_t stride = (size_t)gridDim.x * blockDim.x * V::N;
-    for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * V::N; i < n; i += stride) {
-        const V bi = b(i);
-        V a[MDOT_Q];
-#pragma unroll
-        for (int j = 0; j < MDOT_Q; j++) {
-            if (j == self) a[j] = bi;
-            else if (ap[j]) a[j] = *reinterpret_cast<const V *>(ap[j] + i);
-        }
-#pragma unroll
-        for (int j = 0; j < MDOT_Q; j++)
-            if (ap[j]) {
-#pragma unroll
-                for (int e = 0; e < V::N; e++) p[j] += a[j].v[e] * bi.v[e];
-            }
-    }
-    if constexpr (sizeof(T) == 8) dots_fold<MDOT_Q>(p, bs, sh);
-    else mdz_block_sum<MDOT_Q, T>(p, bs, sh);
-    const int q0 = blockIdx.y * MDOT_Q;
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int j = 0; j < MDOT_Q; j++)
-            if (q0 + j < nq) part[(size_t)(q0 + j) * gridDim.x + blockIdx.x] = bs[j];
-    }
-}
-
-template <typename T, int MDOT_Q>
-__global__ void __launch_bounds__(256) k_dots(int nq, size_t n, const T *const *__restrict__ a,
-                                              const T *__restrict__ b, double *part, unsigned int *cnt,
-                                              double *out, const double *flag) {
-    if (flag && *flag == 0.0) return;
-    __shared__ double sh[dots_shared<T, MDOT_Q>()];
-    const int q0 = blockIdx.y * MDOT_Q;
-    const T *ap[MDOT_Q];
-#pragma unroll
-    for (int j = 0; j < MDOT_Q; j++) ap[j] = q0 + j < nq ? a[q0 + j] : nullptr;
-    double bs[MDOT_Q];
-    dots_block<T, MDOT_Q>(nq, n, ap, [&](size_t i) { return *reinterpret_cast<const vec16<T> *>(b + i); }, -1, part, bs, sh);
-    if (!mdz_arrive_last(cnt + blockIdx.y, gridDim.x)) return;
-    const int nrow = nq - q0 < MDOT_Q ? nq - q0 : MDOT_Q;
-    mdz_sum_partials(part + (size_t)q0 * gridDim.x, gridDim.x, nrow, out + q0);
-}
-
 // One Gram-Schmidt pass's sums in one launch: (w, W_q) for q < k, then
 // (w, w) and (w, r) as vectors k and k + 1 (b = w), summed as k_dots does
 // (the last block of each block row adds its row's partials in block order);
@@ -2215,18 +2117,6 @@ __global__ void __launch_bounds__(256) k_gcr_dots(int k, size_t n, const T *cons
         if (lane == 0) sc[5] = 0.0;
     }
     gcr_scalars(k, d, dk, dr, dd, sc, tri, mode == 2, note, ticket);
-}
-
-// grid of a dots launch over nq vectors: block rows of Q vectors, about four
-// blocks per SM in all, each thread at least one 16-byte load per vector
-template <typename T>
-static dim3 dots_grid(size_t n, int nq) {
-    constexpr int Q = dots_q<T>();
-    const int rows = (nq + Q - 1) / Q;
-    int bx = mdz_blocks((long long)n, 256 * vec16<T>::N);
-    const int cap = (152 * 4 + rows - 1) / rows;
-    if (bx > cap) bx = cap;
-    return dim3(bx, rows);
 }
 
 template <typename T>
