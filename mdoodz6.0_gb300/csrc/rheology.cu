@@ -454,14 +454,19 @@ __device__ void visc_local_t(const visc_phase<Real> &m, const visc_prm<Real> &pr
     // (13 FP64 instructions, the logarithm 29) once |x| < 1/32, as in the last
     // two or three of some five iterations: 513 x 257 centroids 219 -> 207 us.  The
     // sums round at 1e-16 each, the logarithm of a viscosity at half a unit of some 50.
+    // Not beside grain-boundary sliding: the reference's f' leaves it out, so an update
+    // may overshoot to a negative viscosity, which has no logarithm but, at integer
+    // exponents, has the power.  (Without it S is convex and the iteration comes
+    // down on the root from above.)
     const Real dfl = -Real(2.0) * Eii * (iel + ifcst);
+    const bool log_it = logform && dislocation && !gbs;
     Real ln_eta = Real(0.0);
-    if (logform && dislocation && !ve_done) ln_eta = eta_ve == eta_up && start_pwl ? ln_eta_pwl : mlog(eta_ve);
+    if (log_it && !ve_done) ln_eta = eta_ve == eta_up && start_pwl ? ln_eta_pwl : mlog(eta_ve);
     for (it = 0; !ve_done && it < nitmax; it++) {
         Tii = Real(2.0) * eta_ve * Eii;
         Eii_cst = Tii * ifcst;
         if (dislocation) {
-            if (logform) Eii_pwl = mexp(lnC_pwl + n_pwl * (lnTE + ln_eta));
+            if (log_it) Eii_pwl = mexp(lnC_pwl + n_pwl * (lnTE + ln_eta));
             else Eii_pwl = C_pwl * mpow(Tii, n_pwl);
         }
         if (gbs) Eii_gbs = C_gbs * mpow(Tii, m.n_gbs);
@@ -475,7 +480,7 @@ __device__ void visc_local_t(const visc_phase<Real> &m, const visc_prm<Real> &pr
         if (peierls) S1 += Eii_exp * (ST + n_exp);
         const Real x = r / (dfl * eta_ve - S1);
         eta_ve -= x * eta_ve;
-        if (logform && dislocation) {
+        if (log_it) {
             if (mfabs(x) < Real(0.03125)) ln_eta += Real(ln1p_small(double(-x)));
             else ln_eta = mlog(eta_ve);
         }
