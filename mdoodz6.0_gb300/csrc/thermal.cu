@@ -469,12 +469,20 @@ extern "C" mdz_status mdz_EnergyDirectSolve(mdz_ctx *ctx, mdz_fields *f, const m
     const int m = ((n + G - 1) / G + 31) / 32 * 32;
     G = (n + m - 1) / m;
     const size_t cg_bytes = sizeof(double) * cg_doubles(m, ncx);
+    bool done = false;
     if (cg_bytes + 64 <= (size_t)smem) {
         MDZ_CUDA(ctx, cudaFuncSetAttribute(k_energy_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_bytes));
         cg_args A{diag, rhs, d.T, x, z, slots, sc, neg + 1, neg + 2, n, m, max_iterations, rel_tol};
         MDZ_CUDA(ctx, cudaMemsetAsync(slots, 0, 4 * CG_COPIES * sizeof(cg_slot) * G, st));
         void *args[] = {(void *)&g, (void *)&d, (void *)&B, (void *)&A};
-        MDZ_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)k_energy_cg, dim3(G), dim3(CG_THREADS), args, cg_bytes, st));
+        const cudaError_t e =
+            cudaLaunchCooperativeKernel((const void *)k_energy_cg, dim3(G), dim3(CG_THREADS), args, cg_bytes, st);
+        // a device (or a part of one) that cannot hold the whole grid refuses the launch: the steps below need no such thing
+        done = e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorLaunchOutOfResources && e != cudaErrorNotSupported;
+        if (!done) (void)cudaGetLastError();
+        else if (e != cudaSuccess) return mdz_cuda_check(ctx, e, "EnergyDirectSolve");
+    }
+    if (done) {
         MDZ_LAUNCHED(ctx);
         int out[2];
         MDZ_CUDA(ctx, cudaMemcpyAsync(&rel, sc, sizeof rel, cudaMemcpyDeviceToHost, st));
