@@ -471,7 +471,9 @@ extern "C" mdz_status mdz_EnergyDirectSolve(mdz_ctx *ctx, mdz_fields *f, const m
     const size_t cg_bytes = sizeof(double) * cg_doubles(m, ncx);
     bool done = false;
     if (cg_bytes + 64 <= (size_t)smem) {
-        MDZ_CUDA(ctx, cudaFuncSetAttribute(k_energy_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_bytes));
+        // (the kernel's limit belongs to the process: the same value from every call, whatever its grid, so that no other
+        // thread's call lowers it between here and the launch)
+        MDZ_CUDA(ctx, cudaFuncSetAttribute(k_energy_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 64));
         cg_args A{diag, rhs, d.T, x, z, slots, sc, neg + 1, neg + 2, n, m, max_iterations, rel_tol};
         MDZ_CUDA(ctx, cudaMemsetAsync(slots, 0, 4 * CG_COPIES * sizeof(cg_slot) * G, st));
         void *args[] = {(void *)&g, (void *)&d, (void *)&B, (void *)&A};

@@ -6,3 +6,17 @@
 #ifdef FAKE_REFUSED_LAUNCHES
 #define cudaLaunchCooperativeKernel(...) cudaErrorCooperativeLaunchTooLarge
 #endif
+
+#ifdef FAKE_RECORD_LIMITS
+// every limit of dynamic shared memory that a kernel of this source was given
+extern "C" {
+inline int probe_limits_n = 0, probe_limits[64];
+__attribute__((used)) inline int *probe_limits_get(int *n) { *n = probe_limits_n; return probe_limits; }
+}
+template <typename F>
+static cudaError_t probe_set_attribute(F f, cudaFuncAttribute a, int v) {
+    if (a == cudaFuncAttributeMaxDynamicSharedMemorySize && probe_limits_n < 64) probe_limits[probe_limits_n++] = v;
+    return cudaFuncSetAttribute(f, a, v);
+}
+#define cudaFuncSetAttribute(f, a, v) probe_set_attribute(f, a, v)
+#endif

@@ -2,7 +2,10 @@
 refused where the device, or the part of it that the process has, cannot hold
 them.  The library is built a second time with the runtime's calls replaced
 by such answers (native/fake_runtime.h): the calls go on by launches without that
-need and agree with the oracle."""
+need and agree with the oracle.  And a kernel's limit of shared memory, which
+belongs to the process, does not depend on the call that sets it."""
+import contextlib
+import ctypes as C
 import os
 
 import pytest
@@ -30,10 +33,9 @@ def _variant(tmp, name, sources, *flags):
     return so
 
 
-@pytest.fixture(scope="module")
-def refused(tmp_path_factory):
-    """mdz on the library whose launches are refused."""
-    so = _variant(tmp_path_factory.mktemp("refused"), "refused", ["thermal"], "-DFAKE_REFUSED_LAUNCHES")
+@contextlib.contextmanager
+def _loaded(so):
+    """mdz on the library `so`."""
     kept, mdz._lib = mdz._lib, None
     try:
         yield mdz.load_library(so)
@@ -41,6 +43,23 @@ def refused(tmp_path_factory):
         mdz._lib = kept
 
 
+@pytest.fixture(scope="module")
+def refused(tmp_path_factory):
+    return _variant(tmp_path_factory.mktemp("refused"), "refused", ["thermal"], "-DFAKE_REFUSED_LAUNCHES")
+
+
 @pytest.mark.parametrize("Nx,Nz", [(5, 4), (33, 9), (130, 259)])
 def test_energy_step_without_cooperative_launch(refused, Nx, Nz):
-    thermal.test_energy_step_sizes(Nx, Nz)
+    with _loaded(refused):
+        thermal.test_energy_step_sizes(Nx, Nz)
+
+
+def test_energy_step_sets_one_limit_for_all_grids(tmp_path):
+    """(Another thread's call may set it between this one's setting and its launch.)"""
+    with _loaded(_variant(tmp_path, "recorded", ["thermal"], "-DFAKE_RECORD_LIMITS")) as L:
+        for Nx, Nz in ((17, 18), (402, 401), (33, 9)):
+            thermal.test_energy_step_sizes(Nx, Nz)
+        n = C.c_int()
+        L.probe_limits_get.restype = C.POINTER(C.c_int)
+        limits = L.probe_limits_get(C.byref(n))[:n.value]
+    assert len(limits) == 6 and len(set(limits)) == 1, limits
