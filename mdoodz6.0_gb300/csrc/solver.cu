@@ -90,6 +90,7 @@ struct mg_hier {
     bool newton = false;          // level 0 is the probed Newton block (smoothed by its stencil)
     bool built = false;           // mg_setup has filled the levels at least once
     bool viscous = false;         // the last mg_setup left level 0 to its viscosities (no stencils stored)
+    bool bottom = false;          // the device can place k_mg_bottom's cluster
     stokes_geom setup_geom{};     // level 0 of that set-up
     double *pmean = nullptr;      // preconditioner scratch: pressure sum, count and mean
     mg_level<T> L[MG_MAX_LEVELS];
@@ -1135,6 +1136,28 @@ __global__ void __launch_bounds__(mg_bottom_threads<T>()) k_mg_bottom(const __gr
     }
 }
 
+// Whether the device, or the part of it that the process has, can place the
+// bottom's cluster at its largest; else every level runs as launches of its own.
+template <typename T>
+static bool mg_bottom_placed() {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(MG_BOTTOM_CTAS);
+    cfg.blockDim = dim3(mg_bottom_threads<T>());
+    cfg.dynamicSmemBytes = MG_BOTTOM_SMEM;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = MG_BOTTOM_CTAS;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(k_mg_bottom<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_BOTTOM_SMEM) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, k_mg_bottom<T>, &cfg) == cudaSuccess)
+        return n >= 1;
+    (void)cudaGetLastError();
+    return false;
+}
+
 // ---------------------------------------------------------------------------
 template <typename T>
 static cudaError_t alloc0(T **p, size_t n) {
@@ -1296,8 +1319,8 @@ mdz_status mdz_solver_ensure(mdz_ctx *ctx) {
     MG_SMEM_ATTR((k_galerkin<float, true>), sizeof(float) * MG_NST * GAL_THREADS);
     MG_SMEM_ATTR((k_galerkin<float, false>), sizeof(float) * MG_NST * GAL_THREADS);
 #undef MG_SMEM_ATTR
-    MDZ_CUDA(ctx, cudaFuncSetAttribute(k_mg_bottom<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_BOTTOM_SMEM));
-    MDZ_CUDA(ctx, cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_BOTTOM_SMEM));
+    S->mg64.bottom = mg_bottom_placed<double>();
+    S->mg32.bottom = mg_bottom_placed<float>();
     MDZ_CUDA(ctx, cudaFuncSetAttribute(k_coarse_dense_setup<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        MG_DENSE_SMEM));
     MDZ_CUDA(ctx, cudaFuncSetAttribute(k_coarse_dense_setup<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1545,7 +1568,7 @@ template <typename T>
 static bool vcycle_bottom(const mg_hier<T> &H, int l) {
     const mg_level<T> &L = H.L[l];
     const bool viscous = l == 0 && !H.newton;   // level 0 of a Picard hierarchy: stencil from eta directly
-    return !viscous && l < H.nlev - 1 && H.L[H.nlev - 1].ndense && H.nlev - l <= MG_BOTTOM_MAX &&
+    return H.bottom && !viscous && l < H.nlev - 1 && H.L[H.nlev - 1].ndense && H.nlev - l <= MG_BOTTOM_MAX &&
            mg_bottom_rows(L.Nx, L.Nz) <= (sizeof(T) == 4 ? MG_BOTTOM_ROWS32 : MG_BOTTOM_ROWS64) &&
            mg_bottom_bytes<T>(H, l) <= MG_BOTTOM_SMEM;
 }

@@ -5,6 +5,19 @@
 
 #ifdef FAKE_REFUSED_LAUNCHES
 #define cudaLaunchCooperativeKernel(...) cudaErrorCooperativeLaunchTooLarge
+template <typename K>
+static cudaError_t no_clusters(int *n, K, const cudaLaunchConfig_t *) {
+    *n = 0;
+    return cudaSuccess;
+}
+template <typename K, typename... A>
+static cudaError_t launch_without_clusters(const cudaLaunchConfig_t *cfg, K k, A... a) {
+    for (unsigned i = 0; i < cfg->numAttrs; i++)
+        if (cfg->attrs[i].id == cudaLaunchAttributeClusterDimension) return cudaErrorLaunchOutOfResources;
+    return cudaLaunchKernelEx(cfg, k, a...);
+}
+#define cudaOccupancyMaxActiveClusters(...) no_clusters(__VA_ARGS__)
+#define cudaLaunchKernelEx(...) launch_without_clusters(__VA_ARGS__)
 #endif
 
 #ifdef FAKE_RECORD_LIMITS

@@ -12,7 +12,9 @@ import pytest
 
 import mdz
 import mdz_build
+import test_krylov_scalars_gpu as krylov
 import test_thermal_one_launch_gpu as thermal
+import test_vcycle_gpu as vcycle
 
 pytestmark = pytest.mark.gpu
 
@@ -45,13 +47,23 @@ def _loaded(so):
 
 @pytest.fixture(scope="module")
 def refused(tmp_path_factory):
-    return _variant(tmp_path_factory.mktemp("refused"), "refused", ["thermal"], "-DFAKE_REFUSED_LAUNCHES")
+    return _variant(tmp_path_factory.mktemp("refused"), "refused", ["thermal", "solver"], "-DFAKE_REFUSED_LAUNCHES")
 
 
 @pytest.mark.parametrize("Nx,Nz", [(5, 4), (33, 9), (130, 259)])
 def test_energy_step_without_cooperative_launch(refused, Nx, Nz):
     with _loaded(refused):
         thermal.test_energy_step_sizes(Nx, Nz)
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+@pytest.mark.parametrize("Nx,Nz", [(33, 17), (67, 46), (129, 65)])
+def test_solve_without_clusters(refused, Nx, Nz, precision):
+    """The V-cycle's levels as launches of their own: one application against the
+    restatement of the cycle, and a solve whose residual the oracle confirms."""
+    with _loaded(refused):
+        vcycle.test_first_krylov_direction(Nx, Nz, precision, 2, 1)
+        krylov.test_basis_sizes(33, precision)
 
 
 def test_energy_step_sets_one_limit_for_all_grids(tmp_path):
