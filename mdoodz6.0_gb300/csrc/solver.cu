@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstring>
 #include <atomic>
+#include <thread>
 #include <vector>
 #include "stokes.cuh"
 #include "solver.cuh"
@@ -2167,10 +2168,14 @@ static mdz_status dots_launch(mdz_ctx *ctx, gcr_space<T> &S, int q0, int nq, con
 }
 
 // The running norm of the iteration with this ticket, as gcr_scalars wrote it
-// to host memory (GCR_NOTE), usually before the iteration's last launch ends.
-static mdz_status gcr_wait_note(mdz_ctx *ctx, double ticket, cudaStream_t st, double *rn2) {
+// to host memory (GCR_NOTE), usually before the iteration's last launch ends.  The
+// wait spins, as the runtime's own waits do by default; a process that asked for
+// waits that block (cudaDeviceScheduleBlockingSync) or yield gets those.
+static mdz_status gcr_wait_note(mdz_ctx *ctx, double ticket, cudaStream_t st, unsigned schedule, double *rn2) {
     volatile double *note = ctx->solver->sc + GCR_NOTE;
+    if (schedule == cudaDeviceScheduleBlockingSync) MDZ_CUDA(ctx, cudaStreamSynchronize(st));
     for (long long spin = 1; note[1] != ticket; spin++) {
+        if (schedule == cudaDeviceScheduleYield) std::this_thread::yield();
         if (spin % 4096) continue;
         const cudaError_t e = cudaStreamQuery(st);   // a failed launch never writes its ticket
         if (e == cudaErrorNotReady) continue;
@@ -2298,6 +2303,8 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
         return MDZ_OK;
     };
     const int check = SV->check > 0 ? SV->check : 1;
+    unsigned schedule = 0;
+    MDZ_CUDA(ctx, cudaGetDeviceFlags(&schedule));
     for (it = 0; it < maxit; it++) {
         if (k == S.m && (s = end_basis(true)) != MDZ_OK) return s;   // restart: fold the basis into x and r
         cudaEvent_t ev;
@@ -2338,7 +2345,7 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
         // the running norm lives on the device; the host looks every `check`
         // iterations, at each restart and at the iteration limit
         if ((it + 1) % check != 0 && k != S.m && it + 1 < maxit) continue;
-        if ((s = gcr_wait_note(ctx, SV->ticket, st, &rn2)) != MDZ_OK) return s;
+        if ((s = gcr_wait_note(ctx, SV->ticket, st, schedule & cudaDeviceScheduleMask, &rn2)) != MDZ_OK) return s;
         if (!std::isfinite(rn2)) return mdz_fail(ctx, MDZ_ERR_NAN, "GCR: NaN in the Krylov iteration");
         if (rn2 <= rtol * rtol * rn02 || (k == S.m)) {
             // fold the basis in and take the true norm of r at convergence
