@@ -28,7 +28,7 @@ __device__ __forceinline__ double warp_sum_all(double v) {
 // row y handles vectors y Q .. y Q + Q - 1; its blocks write their partials to
 // part[q * gridDim.x + blockIdx.x] and the last block of the row to finish
 // adds them up in block order (reduce.cuh): deterministic.  cnt: one arrival
-// counter per block row.  A non-null flag holding 0 makes the launch a no-op.
+// counter per block row.
 // 1025 x 513 in FP32, up to 8 / 16 / 24 vectors: 13.8 / 21.2 / 29.6 us, with
 // 4-byte loads 18.9 / 32.7 / 51.7.
 template <typename T>
@@ -100,8 +100,7 @@ __device__ __forceinline__ void dots_block(int nq, size_t n, const T *const *ap,
 template <typename T, int MDOT_Q>
 __global__ void __launch_bounds__(256) k_dots(int nq, size_t n, const T *const *__restrict__ a,
                                               const T *__restrict__ b, double *part, unsigned int *cnt,
-                                              double *out, const double *flag) {
-    if (flag && *flag == 0.0) return;
+                                              double *out) {
     __shared__ double sh[dots_shared<T, MDOT_Q>()];
     const int q0 = blockIdx.y * MDOT_Q;
     const T *ap[MDOT_Q];

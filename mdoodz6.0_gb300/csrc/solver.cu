@@ -79,7 +79,7 @@ struct gcr_space {
     T *x = nullptr, *r = nullptr, *z = nullptr, *w = nullptr, *t = nullptr;
     T *pin = nullptr;                   // the preconditioner's input (graph-captured pointer)
     double *tri = nullptr;              // Gram-Schmidt triangle U (column q at q * GCR_MAX_M), then gamma
-    const T **dA0 = nullptr, **dA1 = nullptr, **dA2 = nullptr;   // dot-product pointer tables (k_dots uses dA0)
+    const T **dA0 = nullptr;            // table of the dot products' vectors
     double *dots = nullptr;             // device scalars
     // FP32 copies of the operator (only used for T = float)
     T *Dc[12] = {nullptr};
@@ -306,9 +306,8 @@ __global__ void k_st_diag(stokes_geom G, const T *__restrict__ su, const T *__re
 
 #include "mg_tiles.cuh"
 
-// Level-0 probing: x = indicator of the unknowns of component comp with
-// (k mod 4, l mod 4) = (cx, cz); y = A x.  The level-0 operator (Picard or
-// Newton) couples a row to same-component nodes within [-1, 1]^2 and to
+// Level-0 probing of the Newton block: x = indicator of the unknowns of component
+// comp with (k mod 4, l mod 4) = (cx, cz); y = A x.  The operator couples a row to same-component nodes within [-1, 1]^2 and to
 // other-component nodes within a 4 x 4 window, so each colour class holds at
 // most one node of a row's footprint and y at the row is one coefficient.
 #define MG_PROBE 4
@@ -326,23 +325,22 @@ __global__ void k_probe_vec(stokes_geom G, int comp, int cx, int cz, T *__restri
     }
 }
 
-// velocity rows of the Picard (NEWTON = false, p0 unused) or Newton operator
-// (p0 = a zero pressure vector) applied to (xu, xv, 0)
-template <typename T, bool NEWTON>
+// velocity rows of the Newton operator applied to (xu, xv, 0); p0: a zero pressure vector
+template <typename T>
 __global__ void __launch_bounds__(256) k_mg_apply(stokes_geom G, stokes_coefs<T> D, const T *__restrict__ xu,
                                                   const T *__restrict__ xv, const T *__restrict__ p0,
                                                   T *__restrict__ yu, T *__restrict__ yv) {
     int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     const int Nx = G.Nx, Nz = G.Nz;
     const T celvol = gc<T>(G, GC_CELVOL);
-    stokes_cvec<T> x{xu, xv, NEWTON ? p0 : nullptr};
+    stokes_cvec<T> x{xu, xv, p0};
     if (i < Nx && j <= Nz) {
         int c = i + j * Nx;
-        yu[c] = G.BCu[c] == -1 ? xrow<T, NEWTON>(G, D, x, i, j) * celvol : T(0);
+        yu[c] = G.BCu[c] == -1 ? xrow<T, true>(G, D, x, i, j) * celvol : T(0);
     }
     if (i <= Nx && j < Nz) {
         int c = i + j * (Nx + 1);
-        yv[c] = G.BCv[c] == -1 ? zrow<T, NEWTON>(G, D, x, i, j) * celvol : T(0);
+        yv[c] = G.BCv[c] == -1 ? zrow<T, true>(G, D, x, i, j) * celvol : T(0);
     }
 }
 
@@ -683,8 +681,7 @@ __global__ void __launch_bounds__(1024) k_mg_coarse_cg(stokes_geom G, const T *s
 
 // Small coarsest level: the velocity block is gathered from the level's
 // stencils into a dense matrix (one CTA) and inverted by Gauss-Jordan
-// elimination with partial pivoting in FP64 (a zero pivot column sets
-// *status).  AinvT is stored column-major so that the solve's threads read it
+// elimination with partial pivoting (a zero pivot column sets *status).  AinvT is stored column-major so that the solve's threads read it
 // coalesced.  Dense numbering: u unknowns (k, l), k in 1..Nx-2, l in 1..Nz-1,
 // row by row, then v unknowns (i, j), i in 1..Nx-1, j in 1..Nz-2.
 __device__ __forceinline__ int dense_u(int Nx, int Nz, int k, int l) {
@@ -1270,20 +1267,13 @@ static mdz_status alloc_gcr(mdz_ctx *ctx, gcr_space<T> &S, int m) {
     T **v[] = {&S.x, &S.r, &S.z, &S.w, &S.t, &S.pin};
     for (T **b : v) if (e == cudaSuccess) e = alloc0(b, S.ld);
     if (e == cudaSuccess) e = cudaMalloc((void **)&S.dA0, sizeof(T *) * (GCR_MAX_M + 4));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&S.dA1, sizeof(T *) * (GCR_MAX_M + 4));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&S.dA2, sizeof(T *) * (GCR_MAX_M + 4));
-    if (e == cudaSuccess) e = alloc0(&S.dots, 8 * (GCR_MAX_M + 8));   // see the layout in gcr_solve
+    if (e == cudaSuccess) e = alloc0(&S.dots, 4 * (GCR_MAX_M + 8));   // see the layout in gcr_solve
     if (e == cudaSuccess) e = alloc0(&S.tri, (size_t)GCR_MAX_M * GCR_MAX_M + GCR_MAX_M);
     if (e != cudaSuccess) return mdz_cuda_check(ctx, e, "GCR allocation");
-    // pointer tables: rows 0..m-1 = W_i, row m = w, row m+1 = r
-    std::vector<const T *> a0(m + 2), a1(m + 2), a2(m + 2);
-    for (int i = 0; i < m + 2; i++) {
-        const T *base = i < m ? S.W + S.ld * i : (i == m ? S.w : S.r);
-        a0[i] = base; a1[i] = base + S.nu; a2[i] = base + S.nu + S.nv;
-    }
+    // pointer table: rows 0..m-1 = W_i, row m = w, row m+1 = r
+    std::vector<const T *> a0(m + 2);
+    for (int i = 0; i < m + 2; i++) a0[i] = i < m ? S.W + S.ld * i : (i == m ? S.w : S.r);
     cudaMemcpy(S.dA0, a0.data(), sizeof(T *) * (m + 2), cudaMemcpyHostToDevice);
-    cudaMemcpy(S.dA1, a1.data(), sizeof(T *) * (m + 2), cudaMemcpyHostToDevice);
-    cudaMemcpy(S.dA2, a2.data(), sizeof(T *) * (m + 2), cudaMemcpyHostToDevice);
     if (sizeof(T) == 4) {
         for (int q = 0; q < 12; q++) {
             size_t n = (q < 8) ? S.np : (size_t)g.Nx * g.Nz;
@@ -1295,7 +1285,7 @@ static mdz_status alloc_gcr(mdz_ctx *ctx, gcr_space<T> &S, int m) {
 
 template <typename T>
 static void free_gcr(gcr_space<T> &S) {
-    void *p[] = {S.Z, S.W, S.x, S.r, S.z, S.w, S.t, S.pin, S.tri, S.dA0, S.dA1, S.dA2, S.dots};
+    void *p[] = {S.Z, S.W, S.x, S.r, S.z, S.w, S.t, S.pin, S.tri, S.dA0, S.dots};
     for (void *q : p) if (q) cudaFree(q);
     for (int q = 0; q < 12; q++) if (S.Dc[q]) cudaFree(S.Dc[q]);
 }
@@ -1466,19 +1456,18 @@ static mdz_status mg_setup(mdz_ctx *ctx, mg_hier<T> &H, const double *eta_n, con
             MDZ_LAUNCHED(ctx);
         }
     } else {
-    MDZ_CUDA(ctx, cudaMemsetAsync(F.su, 0, sizeof(T) * MG_NST * F.nu(), st));
-    MDZ_CUDA(ctx, cudaMemsetAsync(F.sv, 0, sizeof(T) * MG_NST * F.nv(), st));
-    for (int comp = 0; comp < 2; comp++)
-        for (int cz = 0; cz < MG_PROBE; cz++)
-            for (int cx = 0; cx < MG_PROBE; cx++) {
-                k_probe_vec<T><<<gr0, bl, 0, st>>>(F.geom(), comp, cx, cz, F.xu, F.xv);
-                MDZ_LAUNCHED(ctx);
-                if (newton) k_mg_apply<T, true><<<gr0, bl, 0, st>>>(F.geom(), K, F.xu, F.xv, F.pz, F.ru, F.rv);
-                else k_mg_apply<T, false><<<gr0, bl, 0, st>>>(F.geom(), F.coefs(), F.xu, F.xv, nullptr, F.ru, F.rv);
-                MDZ_LAUNCHED(ctx);
-                k_probe_collect<T><<<gr0, bl, 0, st>>>(F.geom(), comp, cx, cz, F.ru, F.rv, F.su, F.sv);
-                MDZ_LAUNCHED(ctx);
-            }
+        MDZ_CUDA(ctx, cudaMemsetAsync(F.su, 0, sizeof(T) * MG_NST * F.nu(), st));
+        MDZ_CUDA(ctx, cudaMemsetAsync(F.sv, 0, sizeof(T) * MG_NST * F.nv(), st));
+        for (int comp = 0; comp < 2; comp++)
+            for (int cz = 0; cz < MG_PROBE; cz++)
+                for (int cx = 0; cx < MG_PROBE; cx++) {
+                    k_probe_vec<T><<<gr0, bl, 0, st>>>(F.geom(), comp, cx, cz, F.xu, F.xv);
+                    MDZ_LAUNCHED(ctx);
+                    k_mg_apply<T><<<gr0, bl, 0, st>>>(F.geom(), K, F.xu, F.xv, F.pz, F.ru, F.rv);
+                    MDZ_LAUNCHED(ctx);
+                    k_probe_collect<T><<<gr0, bl, 0, st>>>(F.geom(), comp, cx, cz, F.ru, F.rv, F.su, F.sv);
+                    MDZ_LAUNCHED(ctx);
+                }
     }
     {   // Jacobi diagonal of level 0: the viscosity formula (Picard) or the probed stencil (Newton)
         size_t n = F.nu() > F.nv() ? F.nu() : F.nv();
@@ -1963,14 +1952,9 @@ __global__ void k_set_scalar(double *dst, const double *src) {
 template <typename P>
 __global__ void __launch_bounds__(256) k_gcr_finish(size_t n, int k, P *W, P *__restrict__ Z, const double *dots1,
                                                     const double *dots2, const double *sc, const P *z, const P *w,
-                                                    P *__restrict__ pin, double *__restrict__ next1,
-                                                    double *__restrict__ next2) {
+                                                    P *__restrict__ pin) {
     typedef vec16<P> V;
     pdl_wait();
-    // the next iteration accumulates into the other parity's buffers, which
-    // no kernel of this iteration reads: clear them here instead of by memsets
-    if (blockIdx.x == 0 && next1)
-        for (int q = threadIdx.x; q < k + 3; q += blockDim.x) { next1[q] = 0.0; next2[q] = 0.0; }
     __shared__ P bsh[GCR_MAX_M];
     const double *beta = sc[5] != 0.0 ? dots2 : dots1;
     for (int q = threadIdx.x; q < k; q += blockDim.x) bsh[q] = (P)beta[q];
@@ -2036,10 +2020,6 @@ __global__ void k_gcr_xupdate(size_t n, int k, const P *__restrict__ Z, const do
     for (int q = 0; q < k; q++) a += ash[q] * Z[q * n + i];
     x[i] = (T)((double)x[i] + (double)a);
 }
-
-// out[0] += (w, w), out[1] += (w, r): products, sums and the block reduction
-// in the vectors' precision, block totals added in FP64 (as k_dots); a
-// non-null flag holding 0 makes the launch a no-op
 
 template <typename T>
 __global__ void k_axpby(size_t n, double a, const T *__restrict__ x, double b, T *__restrict__ y) {
@@ -2159,10 +2139,10 @@ static mdz_status gcr_dots_launch(mdz_ctx *ctx, gcr_space<T> &S, int k, const T 
 
 template <typename T>
 static mdz_status dots_launch(mdz_ctx *ctx, gcr_space<T> &S, int q0, int nq, const T *b, double *out,
-                              cudaStream_t st, const double *flag = nullptr) {
+                              cudaStream_t st) {
     if (nq <= 0) return MDZ_OK;
     k_dots<T, dots_q<T>()><<<dots_grid<T>(S.ld, nq), 256, 0, st>>>(nq, S.ld, S.dA0 + q0, b, ctx->red_part + MDZ_RP_DOTS,
-                                                                   ctx->red_cnt + MDZ_RC_DOTS, out, flag);
+                                                                   ctx->red_cnt + MDZ_RC_DOTS, out);
     MDZ_LAUNCHED(ctx);
     return MDZ_OK;
 }
@@ -2256,13 +2236,11 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
     const int nb16 = mdz_blocks((long long)n, 256 * vec16<P>::N);
     MDZ_CUDA(ctx, cudaMemsetAsync(S.x, 0, sizeof(T) * n, st));
     // ||r0||
-    // S.dots layout (doubles, B = GCR_MAX_M + 8): first-pass sums of even / odd
-    // iterations at 0 / 4B, the scalars sc at GCR_MAX_M + 4, second-pass sums
-    // at 2B / 5B, a scratch sum at 3B
+    // S.dots layout (doubles, B = GCR_MAX_M + 8): first-pass sums at 0, the
+    // scalars sc at GCR_MAX_M + 4, second-pass sums at 2B, a scratch sum at 3B
     const int B = GCR_MAX_M + 8;
-    double *sc = S.dots + (GCR_MAX_M + 4), *dots = S.dots + 3 * B;
-    double *dots1p[2] = {S.dots, S.dots + 4 * B}, *dots2p[2] = {S.dots + 2 * B, S.dots + 5 * B};
-    MDZ_CUDA(ctx, cudaMemsetAsync(S.dots, 0, sizeof(double) * 8 * B, st));
+    double *const d1 = S.dots, *const sc = d1 + (GCR_MAX_M + 4), *const d2 = d1 + 2 * B, *const dots = d1 + 3 * B;
+    MDZ_CUDA(ctx, cudaMemsetAsync(S.dots, 0, sizeof(double) * 4 * B, st));
     mdz_status s;
     cudaGraphExec_t pre = nullptr;
     long long pre_launches = 0;
@@ -2328,13 +2306,11 @@ static mdz_status gcr_solve(mdz_ctx *ctx, gcr_space<T> &S, gcr_space<P> &SP, mg_
         // produced them); x, r and every sum are FP64.  First pass:
         // (w, W_q) q < k, (w, w), (w, r0); the check decides on the device
         // whether a second pass runs.
-        double *d1 = dots1p[it & 1], *d2 = dots2p[it & 1];
         SV->ticket += 1.0;
         if ((s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, nullptr, d1, sc, SV->ticket, st)) != MDZ_OK) return s;
         // second pass (returns at once unless sc[5] = 1)
         if (k > 0 && (s = gcr_dots_launch<P>(ctx, SP, k, SP.w, SP.r, d1, d2, sc, SV->ticket, st)) != MDZ_OK) return s;
-        MDZ_PDL(ctx, k_gcr_finish<P>, nb16, 256, 0, st, n, k, SP.W, SP.Z, d1, d2, sc, SP.z, SP.w, SP.pin,
-                dots1p[(it + 1) & 1], dots2p[(it + 1) & 1]);
+        MDZ_PDL(ctx, k_gcr_finish<P>, nb16, 256, 0, st, n, k, SP.W, SP.Z, d1, d2, sc, SP.z, SP.w, SP.pin);
         {   // algorithmic bytes (one Gram-Schmidt pass): the sums read W_q,
             // w and r0 (k + 2 P vectors); the finish reads W_q, w, z and
             // writes W_k, Z_k and the next input (k + 5)

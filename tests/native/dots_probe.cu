@@ -21,7 +21,7 @@ extern "C" int probe_dots(int nq, long long n, const float *a, const float *b, d
     cudaMemset(cnt, 0, sizeof(int) * gr.y);
     double *res = part + (size_t)gr.x * gr.y * dots_q<float>();
     if (cudaGetLastError() == cudaSuccess)
-        k_dots<float, dots_q<float>()><<<gr, 256>>>(nq, (size_t)n, tab, d + (size_t)nq * n, part, cnt, res, nullptr);
+        k_dots<float, dots_q<float>()><<<gr, 256>>>(nq, (size_t)n, tab, d + (size_t)nq * n, part, cnt, res);
     cudaMemcpy(out, res, sizeof(double) * nq, cudaMemcpyDeviceToHost);
     const int e = (int)cudaDeviceSynchronize();
     cudaFree(d); cudaFree(tab); cudaFree(part); cudaFree(cnt);
