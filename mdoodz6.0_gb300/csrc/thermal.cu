@@ -454,8 +454,8 @@ extern "C" mdz_status mdz_EnergyDirectSolve(mdz_ctx *ctx, mdz_fields *f, const m
     k_energy_setup<<<mdz_blocks(n, EN_THREADS), EN_THREADS, 0, st>>>(g, d, B, dt, gz, shear_heating, adiab_heating,
                                                                       diag, rhs);
     MDZ_LAUNCHED(ctx);
-    // One launch for the solve where the rows fit the SMs' shared memory (551 000
-    // cells at 1024 in a row): 2.4 ms the call at 400 x 400 (175 iterations; 10.2 by one launch per step of the
+    // One launch for the solve where the rows fit the SMs' shared memory (cg_doubles: on 152
+    // SMs 539 904 cells at 1024 in a row, 559 000 in a square box): 2.4 ms the call at 400 x 400 (175 iterations; 10.2 by one launch per step of the
     // recurrence, three launches, two copies and a wait of the host per iteration), 1.6 at 200 x 100, 1.2 at
     // 59 x 32; beyond, the sweeps outweigh the launches
     int dev = 0, sms = 0, smem = 0, it = 0;
